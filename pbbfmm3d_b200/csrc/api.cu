@@ -91,6 +91,23 @@ static int upload(double** dst, const double* src, size_t count) {
   return PBBFMM_OK;
 }
 
+// The float64 Chebyshev matrices in fragment order (cheb_fragment_operators):
+// nlev x 316 operators (column-major rf x rs), diag(Kw) U (n3 x rf) and
+// VT diag(Kw) (rs x n3) per level.
+static int upload_cheb_f64(const std::vector<double>& Kw, const double* E, const double* U,
+                           const double* VT, int nlev, int n3, int rf, int rs, double** dE,
+                           double** dU, double** dVT) {
+  std::vector<double> e = cheb_fragment_operators(E, (int64_t)nlev * 316, rf, rs);
+  if (int rc = upload(dE, e.data(), e.size())) return rc;
+  std::vector<double> u(U, U + (size_t)nlev * n3 * rf), v(VT, VT + (size_t)nlev * rs * n3);
+  for (size_t i = 0; i < u.size(); ++i) u[i] *= Kw[i % n3];
+  for (size_t i = 0; i < v.size(); ++i) v[i] *= Kw[i / rs % n3];
+  e = cheb_fragment_operators(u.data(), nlev, n3, rf);
+  if (int rc = upload(dU, e.data(), e.size())) return rc;
+  e = cheb_fragment_operators(v.data(), nlev, rs, n3);
+  return upload(dVT, e.data(), e.size());
+}
+
 // float32 copy (rounded once from the float64 tables) for the mixed path
 static int upload_f32(float** dst, const double* src, size_t count) {
   if (*dst) cudaFree(*dst);
@@ -417,9 +434,9 @@ static int build_adjoint_ops(pbbfmm_tree* t) {
     }
   }
   int rc;
-  if ((rc = upload(&t->adj.E, E.data(), E.size()))) return rc;
-  if ((rc = upload(&t->adj.U, U.data(), U.size()))) return rc;
-  if ((rc = upload(&t->adj.VT, VT.data(), VT.size()))) return rc;
+  if ((rc = upload_cheb_f64(t->w.Kweights, E.data(), U.data(), VT.data(), nlev, n3, rs, rf,
+                            &t->adj.E, &t->adj.U, &t->adj.VT)))
+    return rc;
   if ((rc = upload_f32(&t->adj.fE, E.data(), E.size()))) return rc;
   if ((rc = upload_f32(&t->adj.fU, U.data(), U.size()))) return rc;
   if ((rc = upload_f32(&t->adj.fVT, VT.data(), VT.size()))) return rc;
@@ -455,9 +472,10 @@ static int upload_operators(pbbfmm_tree* t) {
   int rc;
   if ((rc = ensure_tc_err_flag(t))) return rc;
   if (t->p.use_chebyshev) {
-    if ((rc = upload(&t->d_E, t->ops.K.data(), t->ops.K.size()))) return rc;
-    if ((rc = upload(&t->d_U, t->ops.U.data(), t->ops.U.size()))) return rc;
-    if ((rc = upload(&t->d_VT, t->ops.VT.data(), t->ops.VT.size()))) return rc;
+    if ((rc = upload_cheb_f64(t->w.Kweights, t->ops.K.data(), t->ops.U.data(), t->ops.VT.data(),
+                              t->ops.nlev, t->n3, t->ops.rf, t->ops.rs, &t->d_E, &t->d_U,
+                              &t->d_VT)))
+      return rc;
     if ((rc = upload_f32(&t->f_E, t->ops.K.data(), t->ops.K.size()))) return rc;
     if ((rc = upload_f32(&t->f_U, t->ops.U.data(), t->ops.U.size()))) return rc;
     if ((rc = upload_f32(&t->f_VT, t->ops.VT.data(), t->ops.VT.size()))) return rc;
@@ -509,7 +527,7 @@ static void free_tree_device(pbbfmm_tree* t) {
                    &ws.tperm,     &ws.sperm, &ws.tstart,  &ws.sstart,     &ws.tpos,
                    &ws.spos,      &ws.wsorted, &ws.cub_temp, &ws.lists,    &ws.dcounts,
                    &ws.S,         &ws.F,     &ws.proxy,   &ws.pf,         &ws.io_tgt,
-                   &ws.io_src,    &ws.io_w,  &ws.io_out, &ws.halo, &ws.tc_proxy, &ws.leafpart,
+                   &ws.io_src,    &ws.io_w,  &ws.io_out, &ws.halo, &ws.tc_proxy, &ws.m2l_part, &ws.leafpart,
                    &ws.occ,       &ws.amax};
   for (DevBuf* b : all) release(*b);
   if (ws.h_in) cudaFreeHost(ws.h_in);
@@ -625,7 +643,8 @@ static int compute_chunk(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const 
   if ((rc = grow(ws.S, es * level_total(L, perS)))) return rc;
   if ((rc = grow(ws.F, es * level_total(L, perS)))) return rc;
   if (t->p.use_chebyshev) {
-    if ((rc = grow(ws.proxy, es * level_total(L, (int64_t)C * t->ops.rs)))) return rc;
+    const int rsp = precision == PBBFMM_PREC_FP64 ? cheb_rsp(t->ops.rs) : t->ops.rs;
+    if ((rc = grow(ws.proxy, es * level_total(L, (int64_t)C * rsp)))) return rc;
     if ((rc = grow(ws.pf, es * level_total(L, (int64_t)C * t->ops.rf)))) return rc;
   } else {
     if ((rc = grow(ws.proxy, 2 * es * level_total(L, (int64_t)C * t->nk)))) return rc;

@@ -45,6 +45,7 @@ struct Workspace {
   DevBuf pf;     // Cheb: sum_l 8^l * C * rf ;  Unif: accumulated spectra
   DevBuf halo;   // Unif M2L: per parent block 512 halo + 64 target cells
   DevBuf tc_proxy;  // tensor-core Cheb M2L: hi then lo proxies of one level (+ F16 exponents)
+  DevBuf m2l_part;  // float64 Cheb M2L: partial sums of levels with few tiles
   DevBuf leafpart;  // leaf phase: target leaves partitioned dense-first, then their count
   DevBuf occ;       // tensor-core uniform M2L: per-cell source / target occupancy of a level
   DevBuf amax;      // tensor-core uniform M2L: per level, largest |spectra| per (k23, column mod 8)
@@ -110,9 +111,9 @@ struct pbbfmm_tree {
   double* d_Tkz = nullptr;
   double* d_Kw = nullptr;
   double* d_Cw = nullptr;
-  double* d_E = nullptr;   // Cheb: nlev x 316 x rf x rs (col-major blocks)
-  double* d_U = nullptr;   // Cheb: nlev x n3 x rf
-  double* d_VT = nullptr;  // Cheb: nlev x rs x n3
+  double* d_E = nullptr;   // Cheb: nlev x 316 blocks in fragment order (cheb_fragment_operators)
+  double* d_U = nullptr;   // Cheb: nlev x diag(Kw) U, in the same order
+  double* d_VT = nullptr;  // Cheb: nlev x VT diag(Kw), in the same order
   double* d_op = nullptr;  // Unif: nlev x 343 x nk complex (lex-indexed, inner 27 zero)
   int* d_offs = nullptr;   // Cheb M2L: 8 types x 189 x 4 (ox, oy, oz, op index)
   double* d_twid = nullptr;  // Unif: cos/sin of 2 pi j / m, j < m
@@ -184,7 +185,7 @@ struct OpsView {
   const T* Tkz;
   const T* Kw;
   const T* Cw;
-  const T* E;
+  const T* E;   // float32 only, as U and VT (float64: cheb_fragment_operators)
   const T* U;
   const T* VT;
   const cplx_t<T>* op;
@@ -193,7 +194,7 @@ template <typename T>
 inline OpsView<T> ops_view(const pbbfmm_tree* t);
 template <>
 inline OpsView<double> ops_view<double>(const pbbfmm_tree* t) {
-  return {t->d_Tkz, t->d_Kw, t->d_Cw, t->d_E, t->d_U, t->d_VT, (const double2*)t->d_op};
+  return {t->d_Tkz, t->d_Kw, t->d_Cw, nullptr, nullptr, nullptr, (const double2*)t->d_op};
 }
 template <>
 inline OpsView<float> ops_view<float>(const pbbfmm_tree* t) {
@@ -215,6 +216,12 @@ int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d
                 const double* d_w, int C, cudaStream_t st);
 int run_upward(pbbfmm_tree* t, int C, cudaStream_t st);
 int run_m2l_cheb(pbbfmm_tree* t, int C, cudaStream_t st);
+// float64 Chebyshev far field of all levels (pre transform, M2L, post
+// transform); its proxies have rows of cheb_rsp(rs) values (zero from rs on)
+// and its matrices the fragment order
+int cheb_rsp(int rs);
+std::vector<double> cheb_fragment_operators(const double* K, int64_t nblocks, int rf, int rs);
+int run_m2l_cheb_f64(pbbfmm_tree* t, int C, cudaStream_t st);
 // tensor-core Chebyshev M2L (float path): N = rf padded to 16 must fit TMEM
 constexpr int kTcMaxN = 256;
 bool tc_eligible(const pbbfmm_tree* t);

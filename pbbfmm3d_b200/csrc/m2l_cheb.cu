@@ -1,6 +1,8 @@
-// Chebyshev far field in float64: the M2L pre-transform (proxy = VT (Kw o S)),
-// the SVD-compressed M2L over interaction lists, and the post-transform
-// (F = scale * Kw o (U Pf)).
+// Chebyshev far field of the mixed path: the M2L pre-transform (proxy =
+// VT (Kw o S)), the SVD-compressed M2L over interaction lists, and the
+// post-transform (F = scale * Kw o (U Pf)), on the tensor cores (m2l_tc.cu)
+// where they apply and with the float32 CUDA-core kernels here elsewhere.  The
+// float64 path is in m2l_cheb_f64.cu.
 //
 // Reference: UpwardPass tail (include/compute.hpp:373-396), FarFieldInteractions
 // (include/compute.hpp:402-508) and Moment2Local (include/compute.hpp:881-914).
@@ -9,8 +11,6 @@
 // (child type) share the same 189 offsets, so a tile of such targets walks
 // the 189 operators E_i once and multiplies each by the gathered proxies of
 // the tile -- one accumulated GEMM with K = 189 * r_s per tile.
-#include <type_traits>
-
 #include "fmm.cuh"
 
 namespace pbbfmm {
@@ -97,8 +97,8 @@ struct TypeTiles {
   int count[8];  // targets of each type
 };
 
-// M2L for one level on the CUDA cores (float64 path; also the float32 path
-// when r_f exceeds the tensor-core tile).  A CTA owns 128 (target, column)
+// M2L for one level on the CUDA cores (float32, when r_f exceeds the
+// tensor-core tile or the tensor cores are off).  A CTA owns 128 (target, column)
 // rows of one child type and 128 rows of r_f, and walks the offsets where
 // some row of the tile has a source.  Per offset only the rows with a source
 // take part: they are compacted (in tile-row order) into chunks of 16, so
@@ -119,8 +119,7 @@ constexpr int CG_NS = 2;           // stages: loads run one K step ahead
 constexpr int CG_SLOTS = 3;        // compacted row lists in flight (see lookup)
 constexpr int CG_APAD = CG_M + 1;  // A rows padded: conflict-free transposed stores
 
-// stages (A and B) and the running sum [CG_M][CG_N]; the float64 instance
-// takes 192 KB (two 16-deep stages next to the 128 KB running sum)
+// stages (A and B) and the running sum [CG_M][CG_N]
 template <typename T>
 __host__ __device__ constexpr size_t cg_smem_bytes() {
   return sizeof(T) * (CG_NS * CG_K * (CG_APAD + CG_N) + (size_t)CG_M * CG_N);
@@ -328,8 +327,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1)
   }
 }
 
-template <typename T>
-static int run_m2l_cheb_t(pbbfmm_tree* t, int C, cudaStream_t st) {
+static int run_m2l_cheb_f32(pbbfmm_tree* t, int C, cudaStream_t st) {
+  using T = float;
   const int L = t->p.tree_level, n3 = t->n3;
   const int rf = t->ops.rf, rs = t->ops.rs;
   Workspace& ws = t->ws;
@@ -352,14 +351,12 @@ static int run_m2l_cheb_t(pbbfmm_tree* t, int C, cudaStream_t st) {
       dim3 g((unsigned)((ns * (int64_t)C + GBN - 1) / GBN), (unsigned)((rs + GBM - 1) / GBM));
       if (int rc_ = kt_begin(t, KS_M2L_PRE, st)) return rc_;
       bool pre_tc = false;  // float path: tcgen05 (scaled F16 hi / lo) when W fits
-      if constexpr (std::is_same<T, float>::value) {
-        if (colgemm_tc_eligible(t, false)) {
-          if (int rc_ = run_colgemm_tc(t, false, lvl, lists + t->lists.src_off[l], ns * C, C,
-                                       S + level_offset(l, (int64_t)C * n3),
-                                       proxy + level_offset(l, (int64_t)C * rs), 1.f, st))
-            return rc_;
-          pre_tc = true;
-        }
+      if (colgemm_tc_eligible(t, false)) {
+        if (int rc_ = run_colgemm_tc(t, false, lvl, lists + t->lists.src_off[l], ns * C, C,
+                                     S + level_offset(l, (int64_t)C * n3),
+                                     proxy + level_offset(l, (int64_t)C * rs), 1.f, st))
+          return rc_;
+        pre_tc = true;
       }
       if (!pre_tc) {
         k_colgemm<T><<<g, kGemmThreads, 0, st>>>(rs, n3, ov.VT + (int64_t)lvl * rs * n3,
@@ -377,13 +374,11 @@ static int run_m2l_cheb_t(pbbfmm_tree* t, int C, cudaStream_t st) {
     const int nt = t->lists.ntgt[l];
     if (nt == 0) continue;
     bool on_tc = false;  // float path: the tcgen05 kernel (split F16 or TF32) when rf fits TMEM
-    if constexpr (std::is_same<T, float>::value) {
-      if (tc_eligible(t)) {
-        if (int rc_ = run_m2l_cheb_tc_level(t, C, l, lvl, proxy + level_offset(l, (int64_t)C * rs),
-                                            pf + level_offset(l, (int64_t)C * rf), st))
-          return rc_;
-        on_tc = true;
-      }
+    if (tc_eligible(t)) {
+      if (int rc_ = run_m2l_cheb_tc_level(t, C, l, lvl, proxy + level_offset(l, (int64_t)C * rs),
+                                          pf + level_offset(l, (int64_t)C * rf), st))
+        return rc_;
+      on_tc = true;
     }
     TypeTiles tt;
     const int per_tile = CG_M / C;
@@ -414,14 +409,12 @@ static int run_m2l_cheb_t(pbbfmm_tree* t, int C, cudaStream_t st) {
     dim3 g2((unsigned)((nt * (int64_t)C + GBN - 1) / GBN), (unsigned)((n3 + GBM - 1) / GBM));
     if (int rc_ = kt_begin(t, KS_M2L_POST, st)) return rc_;
     bool post_tc = false;
-    if constexpr (std::is_same<T, float>::value) {
-      if (colgemm_tc_eligible(t, true)) {
-        if (int rc_ = run_colgemm_tc(t, true, lvl, lists + t->lists.tgt_off[l], nt * C, C,
-                                     pf + level_offset(l, (int64_t)C * rf),
-                                     F + level_offset(l, (int64_t)C * n3), (float)scale, st))
-          return rc_;
-        post_tc = true;
-      }
+    if (colgemm_tc_eligible(t, true)) {
+      if (int rc_ = run_colgemm_tc(t, true, lvl, lists + t->lists.tgt_off[l], nt * C, C,
+                                   pf + level_offset(l, (int64_t)C * rf),
+                                   F + level_offset(l, (int64_t)C * n3), (float)scale, st))
+        return rc_;
+      post_tc = true;
     }
     if (!post_tc) {
       k_colgemm<T><<<g2, kGemmThreads, 0, st>>>(n3, rf, ov.U + (int64_t)lvl * n3 * rf,
@@ -437,8 +430,7 @@ static int run_m2l_cheb_t(pbbfmm_tree* t, int C, cudaStream_t st) {
 }
 
 int run_m2l_cheb(pbbfmm_tree* t, int C, cudaStream_t st) {
-  return t->cur_prec == PBBFMM_PREC_FP64 ? run_m2l_cheb_t<double>(t, C, st)
-                                         : run_m2l_cheb_t<float>(t, C, st);
+  return t->cur_prec == PBBFMM_PREC_FP64 ? run_m2l_cheb_f64(t, C, st) : run_m2l_cheb_f32(t, C, st);
 }
 
 }  // namespace pbbfmm
