@@ -483,8 +483,9 @@ static int upload_operators(pbbfmm_tree* t) {
   } else {
     std::vector<double> op;
     unif_spectra(t->n, t->ops.stencil, t->ops.nlev, &op);
-    if ((rc = upload(&t->d_op, op.data(), op.size()))) return rc;
-    if ((rc = upload_f32(&t->f_op, op.data(), op.size()))) return rc;
+    const std::vector<double> kara = unif_kara_operators(t->n, op, t->ops.nlev);
+    if ((rc = upload(&t->d_op, kara.data(), kara.size()))) return rc;
+    if ((rc = upload_f32(&t->f_op, kara.data(), kara.size()))) return rc;
     std::vector<uint16_t> tiles;
     std::vector<int> bexp;
     unif_tc_tiles(t->n, op, t->ops.nlev, &tiles, &bexp);
@@ -649,8 +650,7 @@ static int compute_chunk(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const 
   } else {
     if ((rc = grow(ws.proxy, 2 * es * level_total(L, (int64_t)C * t->nk)))) return rc;
     if ((rc = grow(ws.pf, 2 * es * level_total(L, (int64_t)C * t->nk)))) return rc;
-    // halo tables: at most 8^(L-2) parent blocks x (region + target) entries
-    if ((rc = grow(ws.halo, sizeof(int) * 576 * cells_at(L - 2)))) return rc;
+    if ((rc = grow(ws.halo, sizeof(int) * unif_halo_ints(1 << (L - 1))))) return rc;
   }
   if ((rc = run_upward(t, C, st))) return rc;
   if (t->timing) PB_CUDA(cudaEventRecord(t->ev[2], st));
@@ -752,7 +752,7 @@ static int create_tree(const pbbfmm_tree_params* params, const pbbfmm_user_kerne
   t->n = p.interpolation_order;
   t->n3 = t->n * t->n * t->n;
   t->m = 2 * t->n - 1;
-  t->nk = t->m * t->m * t->n;
+  t->nk = unif_slots(t->n);
   t->homog = is_homogeneous(t->kspec.homogen);
   t->homogen_neg = -t->kspec.homogen;  // src/H2_3D_Tree.cpp:45
   t->w = compute_weights(t->n, p.use_chebyshev);

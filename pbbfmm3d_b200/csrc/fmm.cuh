@@ -43,7 +43,7 @@ struct Workspace {
   DevBuf F;      // locals       sum_l 8^l * C * n3
   DevBuf proxy;  // Cheb: sum_l 8^l * C * rs ;  Unif: spectra sum_l 8^l * nk * C (complex)
   DevBuf pf;     // Cheb: sum_l 8^l * C * rf ;  Unif: accumulated spectra
-  DevBuf halo;   // Unif M2L: per parent block 512 halo + 64 target cells
+  DevBuf halo;   // Unif M2L: per parent block, region and target parents and their occupancy
   DevBuf tc_proxy;  // tensor-core Cheb M2L: hi then lo proxies of one level (+ F16 exponents)
   DevBuf m2l_part;  // float64 Cheb M2L: partial sums of levels with few tiles
   DevBuf leafpart;  // leaf phase: target leaves partitioned dense-first, then their count
@@ -104,7 +104,7 @@ struct pbbfmm_tree {
   bool weights_ready = false;
   bool ops_ready = false;
   int precision = PBBFMM_PREC_FP64;
-  int n = 0, n3 = 0, m = 0, nk = 0;  // order, n^3, 2n-1, complex spectrum size m*m*n
+  int n = 0, n3 = 0, m = 0, nk = 0;  // order, n^3, 2n-1, kept frequencies (unif_slots)
   bool homog = false;
   double homogen_neg = 0;
   // device operators
@@ -114,7 +114,7 @@ struct pbbfmm_tree {
   double* d_E = nullptr;   // Cheb: nlev x 316 blocks in fragment order (cheb_fragment_operators)
   double* d_U = nullptr;   // Cheb: nlev x diag(Kw) U, in the same order
   double* d_VT = nullptr;  // Cheb: nlev x VT diag(Kw), in the same order
-  double* d_op = nullptr;  // Unif: nlev x 343 x nk complex (lex-indexed, inner 27 zero)
+  double* d_op = nullptr;  // Unif: nlev x nk x 26 x 27 complex (unif_kara_operators)
   int* d_offs = nullptr;   // Cheb M2L: 8 types x 189 x 4 (ox, oy, oz, op index)
   double* d_twid = nullptr;  // Unif: cos/sin of 2 pi j / m, j < m
   double* d_kparam = nullptr;  // 4 kernel parameters
@@ -125,7 +125,7 @@ struct pbbfmm_tree {
   float* f_E = nullptr;
   float* f_U = nullptr;
   float* f_VT = nullptr;
-  float* f_op = nullptr;  // nlev x nk x 343 complex (float2)
+  float* f_op = nullptr;  // the same in float32
   // tensor-core uniform M2L: per level and frequency the operator tiles of
   // the block product (m2l_unif_tc.cu), scaled F16 hi / lo, and their
   // power-of-two exponents
@@ -246,6 +246,12 @@ int set_unif_tc_wait_limit(long long polls);
 int run_downward(pbbfmm_tree* t, int C, cudaStream_t st);
 int run_leaves(pbbfmm_tree* t, int64_t Nf, int64_t Ns, int C, double* d_out, cudaStream_t st);
 // operator spectra for the uniform path (host, float64) from the stencils
+// kept frequencies: their number, the index (k1 m + k2) n + k3 of one, the
+// operators of the CUDA-core MAC, and the size of a level's halo tables
+int unif_slots(int n);
+int unif_slot_freq(int n, int slot);
+std::vector<double> unif_kara_operators(int n, const std::vector<double>& op, int nlev);
+int64_t unif_halo_ints(int S);
 void unif_spectra(int n, const std::vector<double>& stencil, int nlev, std::vector<double>* op);
 
 // Kernel timer slots (pbbfmm_get_kernel_times).

@@ -1,4 +1,4 @@
-// Uniform-grid far field in float64: FFT of the padded moments, the
+// Uniform-grid far field: FFT of the padded moments, the
 // frequency-domain M2L, and the inverse FFT to local coefficients.
 //
 // Reference: UpwardPass padding + R2HC (include/compute.hpp:337-372),
@@ -13,11 +13,18 @@
 // which is what runs here, as a 3-D real DFT on the m^3 grid (m = 2n-1):
 // x placed at grid position b, y read at grid position (a + n) mod m, and
 // the operator spectra stored as conj(DFT3(A)).  Only the k3 < n half of each
-// spectrum is kept (Hermitian symmetry), nk = m*m*n complex values per cell
-// and column.  Same sums as the reference, different rounding.
+// spectrum is computed (Hermitian symmetry), and of its k3 = 0 plane, which is
+// Hermitian in itself, one half: nk = (m^3 + 1) / 2 complex values per cell
+// and column (365 instead of m*m*n = 405 at order 5).  Same sums as the
+// reference, different rounding.
+//
+// Frequency slots.  Jobs j number the kept (k2, k3): first k3 = 1..n-1 for
+// every k2, then k3 = 0 for k2 = 1..(m-1)/2, last (0, 0); slot j m + k1, of
+// the last job only k1 <= (m-1)/2.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <vector>
 
 #include "fmm.cuh"
 
@@ -148,7 +155,28 @@ __device__ __forceinline__ void idft_9_to_5(const cplx_t<T>* v, Out out) {
   }
 }
 
-// Spectra of a level are stored frequency-major: X[(k * ncells + cell) * C + col]
+__host__ __device__ inline constexpr int unif_jobs(int n) {
+  return (2 * n - 1) * (n - 1) + (n - 1) + 1;
+}
+__host__ __device__ inline void unif_job(int n, int j, int* k2, int* k3) {
+  const int m = 2 * n - 1, full = m * (n - 1);
+  if (j < full) {
+    *k2 = j / (n - 1);
+    *k3 = j % (n - 1) + 1;
+  } else {  // k3 = 0: k2 = 1..n-1 = (m-1)/2, then 0
+    *k2 = j < full + n - 1 ? j - full + 1 : 0;
+    *k3 = 0;
+  }
+}
+int unif_slots(int n) { return (unif_jobs(n) - 1) * (2 * n - 1) + n; }
+int unif_slot_freq(int n, int slot) {
+  const int m = 2 * n - 1;
+  int k2, k3;
+  unif_job(n, slot / m, &k2, &k3);
+  return ((slot % m) * m + k2) * n + k3;
+}
+
+// Spectra of a level are stored frequency-major: X[(slot * ncells + cell) * C + col]
 // (ncells = 8^level), so that one frequency plane of a level is contiguous.
 
 // Forward: CTAs loop over the nonempty source cells (cells[0..ncl)), columns
@@ -172,11 +200,12 @@ __global__ void k_fft_fwd(const int* __restrict__ cells, int ncl, const T* __res
   T* sin_buf = sm + 2 * m;                      // 2 x CG * n3 real moments (double-buffered)
   C2* Z = (C2*)(sin_buf + 2 * sin_stride);      // CG * n * n * n   (l1, l2, k3)
   C2* Y = Z + CG * n3;                         // CG * n * m * n   (l1, k2, k3)
-  unsigned* s_amax = reinterpret_cast<unsigned*>(Y + CG * ny);  // [m n][8]
+  constexpr int nj = unif_jobs(n);
+  unsigned* s_amax = reinterpret_cast<unsigned*>(Y + CG * ny);  // [nj][8]
   (void)twid;
   const int tid = threadIdx.x, bd = blockDim.x;
   if (amax)
-    for (int i = tid; i < m * n * 8; i += bd) s_amax[i] = 0u;
+    for (int i = tid; i < nj * 8; i += bd) s_amax[i] = 0u;
   // work units (cell, column group) of this CTA in order; each unit's moments
   // are copied (cp.async) into the other buffer while the previous unit is
   // transformed
@@ -246,25 +275,30 @@ __global__ void k_fft_fwd(const int* __restrict__ cells, int ncl, const T* __res
       }
     }
     __syncthreads();
-    // x: X[k1][k2][k3][c] = sum_l1 Y[c][l1][k2][k3] w^(k1 l1); job (k23, c), c fastest
-    for (int job = tid; job < cg * m * n; job += bd) {
-      const int cc = job % cg, k23 = job / cg;
-      const C2* y = Y + cc * ny + k23;
+    // x: X[k1][k2][k3][c] = sum_l1 Y[c][l1][k2][k3] w^(k1 l1); job (j, c), c fastest
+    for (int job = tid; job < cg * nj; job += bd) {
+      const int cc = job % cg, j = job / cg;
+      int k2, k3;
+      unif_job(n, j, &k2, &k3);
+      const C2* y = Y + cc * ny + k2 * n + k3;
       C2 v[n];
 #pragma unroll
       for (int l = 0; l < n; ++l) v[l] = y[l * m * n];
-      C2* out = X_l + ((int64_t)k23 * ncells + cell) * C + c0 + cc;
+      C2* out = X_l + ((int64_t)(j * m) * ncells + cell) * C + c0 + cc;
       if constexpr (sizeof(T) == 4) {
         if (amax) {  // |X_k1| <= sum_l |v_l| <= sum_l (|re| + |im|) for every k1
           float bnd = 0.f;
 #pragma unroll
           for (int l = 0; l < n; ++l) bnd += fabsf(v[l].x) + fabsf(v[l].y);
-          atomicMax(&s_amax[k23 * 8 + ((c0 + cc) & 7)], __float_as_uint(bnd));
+          atomicMax(&s_amax[j * 8 + ((c0 + cc) & 7)], __float_as_uint(bnd));
         }
       }
-      const int64_t kstride = (int64_t)m * n * ncells * C;
+      const int64_t kstride = ncells * C;
+      const int kend = j == nj - 1 ? n : m;  // (0, 0): the rest are conjugates
       if constexpr (m == 9) {
-        dft_5_to_9<n, T>(v, [&](int k, C2 r) { out[k * kstride] = r; });
+        dft_5_to_9<n, T>(v, [&](int k, C2 r) {
+          if (k < kend) out[k * kstride] = r;
+        });
       } else {
 #pragma unroll
         for (int k = 0; k < m; ++k) {
@@ -275,7 +309,7 @@ __global__ void k_fft_fwd(const int* __restrict__ cells, int ncl, const T* __res
             re = fma(v[l].x, c, fma(v[l].y, s, re));
             im = fma(v[l].y, c, fma(-v[l].x, s, im));
           }
-          out[k * kstride] = make_cplx<T>(re, im);
+          if (k < kend) out[k * kstride] = make_cplx<T>(re, im);
         }
       }
     }
@@ -284,7 +318,7 @@ __global__ void k_fft_fwd(const int* __restrict__ cells, int ncl, const T* __res
   cp_async_wait_all();  // the (empty) prefetch past the last unit
   if (amax) {
     __syncthreads();
-    for (int i = tid; i < m * n * 8; i += bd)
+    for (int i = tid; i < nj * 8; i += bd)
       if (s_amax[i]) atomicMax(&amax[i], s_amax[i]);
   }
 }
@@ -299,8 +333,9 @@ __global__ void k_fft_inv(const int* __restrict__ cells, const cplx_t<T>* __rest
   using W = Tw<n, T>;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
-  constexpr int m = 2 * n - 1, n2 = n * n, n3 = n2 * n, nk = m * m * n, ng = n * m * n;
-  C2* Yh = (C2*)(sm + ((2 * m + 3) & ~3));  // CG * nk   (k1, k2, k3)
+  constexpr int m = 2 * n - 1, n2 = n * n, n3 = n2 * n, ng = n * m * n;
+  constexpr int nj = unif_jobs(n), nk = (nj - 1) * m + n;
+  C2* Yh = (C2*)(sm + ((2 * m + 3) & ~3));  // CG * nk   (slots)
   C2* G = Yh + CG * nk;                     // CG * n*m*n (a1, k2, k3)
   C2* H = G + CG * ng;                      // CG * n3    (a1, a2, k3)
   (void)twid;
@@ -316,14 +351,20 @@ __global__ void k_fft_inv(const int* __restrict__ cells, const cplx_t<T>* __rest
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    // x: G[c][a1][k2][k3] = sum_k1 Yh[c][k1][k2][k3] e^{+2 pi i k1 t1 / m}; job (c, k23)
-    for (int job = tid; job < cg * m * n; job += bd) {
-      const int k23 = job % (m * n), cc = job / (m * n);
-      const C2* y = Yh + cc * nk + k23;
+    // x: G[c][a1][k2][k3] = sum_k1 Yh[c][k1][k2][k3] e^{+2 pi i k1 t1 / m}; job (c, j)
+    for (int job = tid; job < cg * nj; job += bd) {
+      const int j = job % nj, cc = job / nj;
+      int k2, k3;
+      unif_job(n, j, &k2, &k3);
+      const C2* y = Yh + cc * nk + j * m;
       C2 v[m];
 #pragma unroll
-      for (int k = 0; k < m; ++k) v[k] = y[k * m * n];
-      C2* g = G + cc * ng + k23;
+      for (int k = 0; k < m; ++k) {
+        const bool mirror = j == nj - 1 && k >= n;  // Y(-k1, 0, 0) = conj Y(k1, 0, 0)
+        v[k] = y[mirror ? m - k : k];
+        if (mirror) v[k].y = -v[k].y;
+      }
+      C2* g = G + cc * ng + k2 * n + k3;
       if constexpr (m == 9) {
         idft_9_to_5<n, T>(v, [&](int a, C2 r) { g[a * m * n] = r; });
       } else {
@@ -348,7 +389,11 @@ __global__ void k_fft_inv(const int* __restrict__ cells, const cplx_t<T>* __rest
       const C2* g = G + cc * ng + a1 * m * n + k3;
       C2 v[m];
 #pragma unroll
-      for (int k = 0; k < m; ++k) v[k] = g[k * n];
+      for (int k = 0; k < m; ++k) {
+        const bool mirror = k3 == 0 && k >= n;  // G(-k2, 0) = conj G(k2, 0)
+        v[k] = g[(mirror ? m - k : k) * n];
+        if (mirror) v[k].y = -v[k].y;
+      }
       C2* h = H + cc * n3 + a1 * n2 + k3;
       if constexpr (m == 9) {
         idft_9_to_5<n, T>(v, [&](int a, C2 r) { h[a * n] = r; });
@@ -390,225 +435,299 @@ __global__ void k_fft_inv(const int* __restrict__ cells, const cplx_t<T>* __rest
 }
 
 // ----------------------------------------------------------------- MAC
-// One CTA per (block of PBX x 2 x 2 parents = 2PBX x 4 x 4 targets,
-// frequency chunk), the frequency chunk varying slowest in the grid so that
-// resident CTAs work on the same frequency plane (one plane of level 6 is
-// 33.5 MB and stays in L2 while its halo reuse is served).  Threads =
-// (parent, kc, col); each thread accumulates the 8 children of its parent for
-// one frequency and one column, sweeping the 6x6x6 children of the parent's
-// neighbours, staged in shared memory for the whole block ((2PBX+4) x 8 x 8
-// cells).  The (child, source) interaction pattern and the operator index are
-// compile-time constants; each complex accumulator is split over four
-// independent FMA chains.
+// y_k(P)[t] = sum over parent offsets D in {-1, 0, 1}^3 and children s of
+// E_k[2 D + s - t] x_k(P + D)[s] (E = 0 for near offsets; D = 0 has near ones
+// only).  For one D this is an 8 x 8 block that is Toeplitz in each of the
+// three child coordinates, so it is taken with three products per coordinate
+// instead of four (Karatsuba):
+//   y0 = e0 x0 + e+ x1 = e0 (x0 + x1) + (e+ - e0) x1
+//   y1 = e- x0 + e0 x1 = e0 (x0 + x1) + (e- - e0) x0
+// 27 complex products per parent pair instead of 56 (64 less the near ones);
+// the 27 products of a target parent are summed over D before the (linear)
+// output step.  Counted per target parent and frequency: 26 x (108
+// multiply-adds + 38 additions) against 6048 multiply-adds.
 //
-// Per level, halo[b*stride + r] holds the source cell of region slot r of
-// parent block b (or -1: outside the domain or no sources), followed by the
-// target cell of each block slot (or -1).
+// A thread owns (target parent, slot, column) and its 27 complex sums; a CTA
+// owns a block of PX x PY x PZ target parents, KC slots and CG columns.  The
+// source parents of the block and its one-parent halo are staged in shared
+// memory as [child][parent][slot][column], so that the threads of a warp,
+// which run over column, slot and z, read consecutive words; the 26 x 27
+// coefficients of each slot lie behind them and are read by broadcast.  The
+// loop over D is not unrolled (every D has the same body).  The slot varies
+// slowest in the grid, so resident CTAs share a few frequency planes in L2.
+//
+// Bound: the FP64 pipe and the shared-memory reads beside it (float32: issue
+// slots and shared-memory reads).  Measured, M2L of one matvec at order 5
+// against the direct sum of 189 products per child and m m n frequencies:
+// 1M points, 8 columns, float64 59.7 -> 47.3 ms; 250,000 points, 1 column,
+// float64 1.66 -> 0.84 ms; 1M points, 1 column, float32 6.45 -> 3.96 ms;
+// 200,000 points, 3 columns, float32 2.79 -> 1.61 ms.  The distance of the
+// float32 pass from float64 stays where it was (2.3e-7 to 5.2e-7 over orders 3
+// to 5 and 1 to 3 columns; before, 2.9e-7 to 5.2e-7).
+//
+// Per level, halo[b * STRIDE + r] holds for the region parents of block b their
+// Morton index, then the occupancy of their 8 children (0 outside the
+// domain), then the same of the block's target parents.
+constexpr int kKaraD = 26, kKaraJ = 27;
 
-template <int PBX>
+template <int PX, int PY, int PZ>
 struct MacGeom {
-  static constexpr int RX = 2 * PBX + 4;       // region extent in x (y, z: 8)
-  static constexpr int RC = RX * 64;           // region cells
-  static constexpr int TC = 2 * PBX * 16;      // target cells of a block
-  static constexpr int STRIDE = RC + TC;       // halo table entries per block
-  static constexpr int NPAR = PBX * 4;         // parents per block
+  static constexpr int RX = PX + 2, RY = PY + 2, RZ = PZ + 2;
+  static constexpr int RP = RX * RY * RZ;  // region parents
+  static constexpr int NP = PX * PY * PZ;  // target parents
+  static constexpr int STRIDE = 2 * RP + 2 * NP;
 };
 
-template <int PBX>
-__global__ void k_halo_tables(const int* __restrict__ sstart, const int* __restrict__ tstart,
-                              int span, int lev, int* __restrict__ halo) {
-  using G = MacGeom<PBX>;
-  const int nby = 1 << (lev - 2), nbx = (1 << (lev - 1)) / PBX;  // blocks per dim
-  const int b = blockIdx.x;
-  const int bx = b / (nby * nby), by = (b / nby) % nby, bz = b % nby;
-  const int nside = 1 << lev;
-  for (int r = threadIdx.x; r < G::STRIDE; r += blockDim.x) {
-    int v = -1;
-    if (r < G::RC) {
-      const int x = 2 * PBX * bx - 2 + (r >> 6), y = 4 * by - 2 + ((r >> 3) & 7),
-                z = 4 * bz - 2 + (r & 7);
-      if (x >= 0 && y >= 0 && z >= 0 && x < nside && y < nside && z < nside) {
-        const uint32_t cm = morton_encode(x, y, z);
-        if (sstart[(int64_t)(cm + 1) * span] > sstart[(int64_t)cm * span]) v = (int)cm;
-      }
-    } else {
-      const int q = r - G::RC;
-      const uint32_t cm =
-          morton_encode(2 * PBX * bx + (q >> 4), 4 * by + ((q >> 2) & 3), 4 * bz + (q & 3));
-      if (tstart[(int64_t)(cm + 1) * span] > tstart[(int64_t)cm * span]) v = (int)cm;
-    }
-    halo[(int64_t)b * G::STRIDE + r] = v;
+__device__ __forceinline__ int parent_mask(const int* __restrict__ start, int64_t p, int span) {
+  int m = 0, lo = start[8 * p * span];
+  for (int c = 0; c < 8; ++c) {
+    const int hi = start[(8 * p + c + 1) * span];
+    m |= (hi > lo ? 1 : 0) << c;
+    lo = hi;
   }
-  (void)nbx;
+  return m;
 }
 
-// One sx slab of the MAC: the 6 x 6 (sy, sz) sources of the slab against
-// the 8 children.  F0 / F1: children with tx = 0 / 1 are far in x at this sx
-// (|sx - 2 - tx| > 1), so every interaction test is a compile-time constant.
-template <bool F0, bool F1, int RS, typename C2, typename T>
-__device__ __forceinline__ void mac_slab(const C2* __restrict__ rrow, const C2* __restrict__ orow,
-                                         int py, int pz, T* ar, T* br, T* ai, T* bi) {
-#pragma unroll
-  for (int sy = 0; sy < 6; ++sy)
-#pragma unroll
-    for (int sz = 0; sz < 6; ++sz) {
-      const int r = ((2 * py + sy) << 3) | (2 * pz + sz);
-      const C2 xv = rrow[r * RS];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const int tx = (t >> 2) & 1;
-        const int oy = sy - 2 - ((t >> 1) & 1);
-        const int oz = sz - 2 - (t & 1);
-        const bool far_yz = oy > 1 || oy < -1 || oz > 1 || oz < -1;
-        if (far_yz || (tx ? F1 : F0)) {
-          const C2 a = orow[-49 * tx + 7 * (oy + 3) + (oz + 3)];
-          ar[t] = fma(a.x, xv.x, ar[t]);
-          br[t] = fma(-a.y, xv.y, br[t]);
-          ai[t] = fma(a.x, xv.y, ai[t]);
-          bi[t] = fma(a.y, xv.x, bi[t]);
-        }
-      }
+template <int PX, int PY, int PZ>
+__global__ void k_halo_tables(const int* __restrict__ sstart, const int* __restrict__ tstart,
+                              int span, int S, int nby, int nbz, int* __restrict__ halo) {
+  using G = MacGeom<PX, PY, PZ>;
+  const int b = blockIdx.x;
+  const int x0 = PX * (b / (nby * nbz)), y0 = PY * ((b / nbz) % nby), z0 = PZ * (b % nbz);
+  int* h = halo + (int64_t)b * G::STRIDE;
+  for (int r = threadIdx.x; r < G::RP + G::NP; r += blockDim.x) {
+    const bool src = r < G::RP;
+    const int q = src ? r : r - G::RP;
+    const int x = src ? x0 - 1 + q / (G::RY * G::RZ) : x0 + q / (PY * PZ);
+    const int y = src ? y0 - 1 + (q / G::RZ) % G::RY : y0 + (q / PZ) % PY;
+    const int z = src ? z0 - 1 + q % G::RZ : z0 + q % PZ;
+    int p = 0, m = 0;
+    if (x >= 0 && y >= 0 && z >= 0 && x < S && y < S && z < S) {
+      p = (int)morton_encode(x, y, z);
+      m = parent_mask(src ? sstart : tstart, p, span);
     }
+    int* d = src ? h + q : h + 2 * G::RP + q;
+    d[0] = p;
+    d[src ? G::RP : G::NP] = m;
+  }
 }
 
-template <int PBX, int KC, int CG, typename T>
-__global__ void __launch_bounds__(4 * PBX * KC * CG)
+template <int PX, int PY, int PZ, int KC, int CG, typename T>
+struct MacSmem {
+  using G = MacGeom<PX, PY, PZ>;
+  static constexpr int Q = KC * CG;
+  // stride of a child's plane: shifted against the others, so that the copies
+  // of several children of one parent reach different banks
+  static constexpr int CS = G::RP * Q + (CG > 4 ? CG : 4);
+  static constexpr size_t bytes =
+      sizeof(cplx_t<T>) * (8 * CS + KC * kKaraD * kKaraJ) + sizeof(int) * G::STRIDE;
+};
+
+template <int PX, int PY, int PZ, int KC, int CG, typename T>
+__global__ void __launch_bounds__(PX* PY* PZ* KC* CG)
     k_m2l_unif_mac(const cplx_t<T>* __restrict__ X_l, cplx_t<T>* __restrict__ Y_l,
-                   const cplx_t<T>* __restrict__ op,  // nk x 343 for this level
-                   const int* __restrict__ halo, int64_t ncells, int C, int nk) {
-  using G = MacGeom<PBX>;
+                   const cplx_t<T>* __restrict__ op,  // [slot][26][27] of this level
+                   const int* __restrict__ halo, int64_t ncells, int C, int c0, int nk) {
+  using G = MacGeom<PX, PY, PZ>;
+  using SM = MacSmem<PX, PY, PZ, KC, CG, T>;
   using C2 = cplx_t<T>;
-  constexpr int NT = G::NPAR * KC * CG;
-  constexpr int RC = G::RC;
+  constexpr int NT = G::NP * KC * CG, Q = KC * CG, CS = SM::CS, NE = kKaraD * kKaraJ;
   extern __shared__ __align__(16) unsigned char smraw[];
-  C2* reg = reinterpret_cast<C2*>(smraw);  // RC x KC x CG
-  C2* sop = reg + RC * KC * CG;            // KC x 343
-  int* s_src = (int*)(sop + KC * 343);  // RC source cells, then TC target cells
-  int* s_tgt = s_src + RC;
+  C2* reg = reinterpret_cast<C2*>(smraw);  // [child][region parent][slot][col]
+  C2* sop = reg + 8 * CS;                  // [slot][26][27]
+  int* s_par = (int*)(sop + KC * NE);      // region parents
+  int* s_msk = s_par + G::RP;              // their children with sources
+  int* s_tgt = s_msk + G::RP;              // target parents, then their children with targets
   const int tid = threadIdx.x;
-  const int cc = tid % CG, kc = (tid / CG) % KC, p = tid / (CG * KC);
-  const int px = p >> 2, py = (p >> 1) & 1, pz = p & 1;
+  const int cc = tid % CG, kc = (tid / CG) % KC, p = tid / Q;
+  const int px = p / (PY * PZ), py = (p / PZ) % PY, pz = p % PZ;
   const int* hb = halo + (int64_t)blockIdx.x * G::STRIDE;
   int mine = 0;
   for (int r = tid; r < G::STRIDE; r += NT) {
     const int v = hb[r];
-    s_src[r] = v;
-    if (r >= RC) mine |= v >= 0;
+    s_par[r] = v;
+    if (r >= 2 * G::RP + G::NP) mine |= v;
   }
-  if (!__syncthreads_or(mine)) return;
+  if (!__syncthreads_or(mine)) return;  // no target in the block
   const int k0 = blockIdx.y * KC;
-  const int c0 = blockIdx.z * CG;
-  // stage the source halo for frequencies k0..k0+KC-1 and columns
-  // c0..c0+CG-1 with asynchronous copies (all in flight at once; empty or
-  // out-of-domain cells are zero-filled)
-  for (int i = tid; i < RC * KC * CG; i += NT) {
-    const int r = i / (KC * CG), q = i % (KC * CG), kk = q / CG, c = q % CG;
-    const int src = s_src[r];
-    const bool ok = src >= 0 && k0 + kk < nk && c0 + c < C;
-    const C2* g = ok ? &X_l[((int64_t)(k0 + kk) * ncells + src) * C + c0 + c] : X_l;
-    cp_async_cplx(&reg[i], g, ok);
+  // all copies in flight at once; empty or out-of-domain cells are zero-filled.
+  // Order (column, child, slot, parent): runs of 8 CG values are contiguous.
+  for (int i = tid; i < G::RP * 8 * Q; i += NT) {
+    const int c = i % CG, ch = (i / CG) % 8, kk = (i / (8 * CG)) % KC, r = i / (8 * Q);
+    const bool ok = ((s_msk[r] >> ch) & 1) && k0 + kk < nk;
+    const C2* g = ok ? &X_l[((int64_t)(k0 + kk) * ncells + 8 * (int64_t)s_par[r] + ch) * C + c0 + c]
+                     : X_l;
+    cp_async_cplx(&reg[ch * CS + r * Q + kk * CG + c], g, ok);
   }
-  for (int i = tid; i < KC * 343; i += NT) {
-    const int kk = i / 343, e = i % 343;
-    const bool ok = k0 + kk < nk;
-    cp_async_cplx(&sop[i], ok ? &op[(int64_t)(k0 + kk) * 343 + e] : op, ok);
+  for (int i = tid; i < KC * NE; i += NT) {
+    const bool ok = k0 + i / NE < nk;
+    cp_async_cplx(&sop[i], ok ? &op[(int64_t)k0 * NE + i] : op, ok);
   }
   cp_async_commit();
   cp_async_wait_all();
   __syncthreads();
-  T ar[8], br[8], ai[8], bi[8];  // re = ar + br, im = ai + bi
+  C2 acc[kKaraJ];
 #pragma unroll
-  for (int t = 0; t < 8; ++t) ar[t] = br[t] = ai[t] = bi[t] = T(0);
-  const C2* myop = sop + kc * 343;
-  // sx runs as a loop.  float64: the body for each sx is one of four
-  // compile-time specialisations (whether the children with tx = 0 / 1 are
-  // far in x at this sx), so no interaction test is left to run time (9 %
-  // faster than the predicated body).  float32: one predicated body; the
-  // four specialisations were 20 % slower there, the larger code costing
-  // more than the predicated-off FMAs it saves.
+  for (int j = 0; j < kKaraJ; ++j) acc[j] = make_cplx<T>(T(0), T(0));
+  const C2* e = sop + kc * NE;
+  auto add = [](C2 a, C2 b) { return make_cplx<T>(a.x + b.x, a.y + b.y); };
 #pragma unroll 1
-  for (int sx = 0; sx < 6; ++sx) {
-    const C2* rrow = reg + (((2 * px + sx) << 6) * KC + kc) * CG + cc;
-    const C2* orow = myop + 49 * (sx + 1);  // lex of ox + 3 = sx + 1 - tx
-    if constexpr (sizeof(T) == 8) {
-      if (sx == 0 || sx == 5)
-        mac_slab<true, true, KC * CG>(rrow, orow, py, pz, ar, br, ai, bi);
-      else if (sx == 1)
-        mac_slab<false, true, KC * CG>(rrow, orow, py, pz, ar, br, ai, bi);
-      else if (sx == 4)
-        mac_slab<true, false, KC * CG>(rrow, orow, py, pz, ar, br, ai, bi);
-      else
-        mac_slab<false, false, KC * CG>(rrow, orow, py, pz, ar, br, ai, bi);
-    } else {
+  for (int dx = 0; dx < 3; ++dx)
+#pragma unroll 1
+    for (int dy = 0; dy < 3; ++dy)
+#pragma unroll 1
+      for (int dz = 0; dz < 3; ++dz) {
+        if (dx == 1 && dy == 1 && dz == 1) continue;
+        const int r = ((px + dx) * G::RY + py + dy) * G::RZ + pz + dz;
+        if (s_msk[r]) {
+          const C2* xr = reg + r * Q + kc * CG + cc;
+          C2 x[8];
 #pragma unroll
-      for (int sy = 0; sy < 6; ++sy)
+          for (int ch = 0; ch < 8; ++ch) x[ch] = xr[ch * CS];
+          // j = 9 jx + 3 jy + jz, each 0: x0 + x1, 1: x1, 2: x0
 #pragma unroll
-        for (int sz = 0; sz < 6; ++sz) {
-          const int r = ((2 * py + sy) << 3) | (2 * pz + sz);
-          const C2 xv = rrow[r * KC * CG];
+          for (int jz = 0; jz < 3; ++jz) {
+            C2 u[4];  // (bx, by)
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const int tx = (t >> 2) & 1;
-            const int oy = sy - 2 - ((t >> 1) & 1);
-            const int oz = sz - 2 - (t & 1);
-            const int ox = sx - 2 - tx;
-            const bool far_yz = oy > 1 || oy < -1 || oz > 1 || oz < -1;
-            if (far_yz || ox > 1 || ox < -1) {
-              const C2 a = orow[-49 * tx + 7 * (oy + 3) + (oz + 3)];
-              ar[t] = fma(a.x, xv.x, ar[t]);
-              br[t] = fma(-a.y, xv.y, br[t]);
-              ai[t] = fma(a.x, xv.y, ai[t]);
-              bi[t] = fma(a.y, xv.x, bi[t]);
+            for (int q = 0; q < 4; ++q)
+              u[q] = jz == 0 ? add(x[2 * q], x[2 * q + 1]) : x[2 * q + (jz == 1 ? 1 : 0)];
+#pragma unroll
+            for (int jy = 0; jy < 3; ++jy) {
+              C2 v[2];  // bx
+#pragma unroll
+              for (int q = 0; q < 2; ++q)
+                v[q] = jy == 0 ? add(u[2 * q], u[2 * q + 1]) : u[2 * q + (jy == 1 ? 1 : 0)];
+#pragma unroll
+              for (int jx = 0; jx < 3; ++jx) {
+                const C2 w = jx == 0 ? add(v[0], v[1]) : v[jx == 1 ? 1 : 0];
+                const int j = 9 * jx + 3 * jy + jz;
+                const C2 a = e[j];
+                acc[j].x = fma(a.x, w.x, acc[j].x);
+                acc[j].y = fma(a.x, w.y, acc[j].y);
+                acc[j].x = fma(-a.y, w.y, acc[j].x);
+                acc[j].y = fma(a.y, w.x, acc[j].y);
+              }
             }
           }
         }
-    }
-  }
-  if (k0 + kc < nk && c0 + cc < C) {
+        e += kKaraJ;
+      }
+  if (k0 + kc >= nk) return;
+  const int tm = s_tgt[G::NP + p];
+  const int64_t tp = 8 * (int64_t)s_tgt[p];
+  C2* out = Y_l + ((int64_t)(k0 + kc) * ncells + tp) * C + c0 + cc;
+  // y0 = P + Q1, y1 = P + Q0 per coordinate
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const int q = ((2 * px + ((t >> 2) & 1)) << 4) | ((2 * py + ((t >> 1) & 1)) << 2) |
-                    (2 * pz + (t & 1));
-      const int cm = s_tgt[q];
-      if (cm >= 0)
-        Y_l[((int64_t)(k0 + kc) * ncells + cm) * C + c0 + cc] =
-            make_cplx<T>(ar[t] + br[t], ai[t] + bi[t]);
-    }
+  for (int t = 0; t < 8; ++t) {
+    const int jx = 9 * (1 + ((t >> 2) & 1)), jy = 3 * (1 + ((t >> 1) & 1)), jz = 1 + (t & 1);
+    const C2 y = add(add(add(acc[0], acc[jz]), add(acc[jy], acc[jy + jz])),
+                     add(add(acc[jx], acc[jx + jz]), add(acc[jx + jy], acc[jx + jy + jz])));
+    if ((tm >> t) & 1) out[(int64_t)t * C] = y;
   }
 }
 
-template <int PBX, int KC, int CG, typename T>
-static int launch_mac(const cplx_t<T>* X, cplx_t<T>* Y, const cplx_t<T>* op, int* halo,
-                      const int* sstart, const int* tstart, int span, int lev, int C, int nk,
-                      cudaStream_t st) {
-  using G = MacGeom<PBX>;
-  const int nby = 1 << (lev - 2), nbx = (1 << (lev - 1)) / PBX;
-  const int nblk = nbx * nby * nby;
-  k_halo_tables<PBX><<<nblk, 256, 0, st>>>(sstart, tstart, span, lev, halo);
-  PB_LAUNCH("halo_tables");
-  dim3 g((unsigned)nblk, (unsigned)((nk + KC - 1) / KC), (unsigned)((C + CG - 1) / CG));
-  const size_t smem =
-      sizeof(cplx_t<T>) * (G::RC * KC * CG + KC * 343) + sizeof(int) * G::STRIDE;
-  PB_CUDA(cudaFuncSetAttribute(k_m2l_unif_mac<PBX, KC, CG, T>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_m2l_unif_mac<PBX, KC, CG, T><<<g, G::NPAR * KC * CG, smem, st>>>(X, Y, op, halo,
-                                                                     cells_at(lev), C, nk);
-  PB_LAUNCH("m2l_unif_mac");
-  return PBBFMM_OK;
+// The coefficients [level][slot][26][27] from the spectra op[level][k][343]
+// (lex-indexed offsets, inner 27 zero): per coordinate the differences above.
+std::vector<double> unif_kara_operators(int n, const std::vector<double>& op, int nlev) {
+  const int nk = unif_slots(n), nfull = (2 * n - 1) * (2 * n - 1) * n;
+  std::vector<double> out((size_t)nlev * nk * kKaraD * kKaraJ * 2);
+  parallel_for((int64_t)nlev * nk, [&](int64_t b0, int64_t b1) {
+    for (int64_t b = b0; b < b1; ++b) {
+      const double* E = &op[(size_t)(b / nk * nfull + unif_slot_freq(n, (int)(b % nk))) * 343 * 2];
+      double* o = &out[(size_t)b * kKaraD * kKaraJ * 2];
+      for (int d = 0; d < 27; ++d) {
+        if (d == 13) continue;
+        const int c[3] = {2 * (d / 9 - 1), 2 * (d / 3 % 3 - 1), 2 * (d % 3 - 1)};
+        for (int j = 0; j < kKaraJ; ++j, o += 2) {
+          const int jd[3] = {j / 9, j / 3 % 3, j % 3};
+          o[0] = o[1] = 0.0;
+          for (int q = 0; q < 8; ++q) {  // bit i: the subtracted term of coordinate i
+            int lex = 0, sign = 1;
+            bool used = true;
+            for (int i = 0; i < 3; ++i) {
+              const int sub = (q >> i) & 1;
+              int off = c[i];
+              if (jd[i] == 0)
+                used &= !sub;
+              else if (sub)
+                sign = -sign;
+              else
+                off += jd[i] == 1 ? 1 : -1;
+              lex = 7 * lex + off + 3;
+            }
+            if (!used) continue;
+            o[0] += sign * E[2 * lex];
+            o[1] += sign * E[2 * lex + 1];
+          }
+        }
+      }
+    }
+  });
+  return out;
 }
 
-template <int PBX, typename T>
-static int launch_mac_cols(const cplx_t<T>* X, cplx_t<T>* Y, const cplx_t<T>* op, int* halo,
-                           const int* sstart, const int* tstart, int span, int lev, int C, int nk,
-                           cudaStream_t st) {
-  if (C >= 8)
-    return launch_mac<PBX, 1, 8, T>(X, Y, op, halo, sstart, tstart, span, lev, C, nk, st);
-  if (C >= 4)
-    return launch_mac<PBX, 2, 4, T>(X, Y, op, halo, sstart, tstart, span, lev, C, nk, st);
-  if (C >= 2)
-    return launch_mac<PBX, 4, 2, T>(X, Y, op, halo, sstart, tstart, span, lev, C, nk, st);
-  return launch_mac<PBX, 8, 1, T>(X, Y, op, halo, sstart, tstart, span, lev, C, nk, st);
+// ints of the halo tables of a level with S parents per side
+int64_t unif_halo_ints(int S) {
+  const int64_t b4 = (S + 3) / 4, b2 = (S + 1) / 2;
+  const int64_t a = b4 * b4 * b4 * MacGeom<4, 4, 4>::STRIDE, b = b4 * b4 * b2 * MacGeom<4, 4, 2>::STRIDE,
+                c = b4 * b2 * b2 * MacGeom<4, 2, 2>::STRIDE;
+  return std::max(a, std::max(b, c));
 }
+
+template <typename T>
+struct MacLevel {
+  const cplx_t<T>* X;
+  cplx_t<T>* Y;
+  const cplx_t<T>* op;
+  int* halo;
+  const int* sstart;
+  const int* tstart;
+  int span, lev, C, nk;
+  cudaStream_t st;
+  int last = 0;  // geometry that the halo tables hold
+
+  template <int PX, int PY, int PZ, int KC, int CG>
+  int run(int c0) {
+    using G = MacGeom<PX, PY, PZ>;
+    const int S = 1 << (lev - 1);
+    const int nbx = (S + PX - 1) / PX, nby = (S + PY - 1) / PY, nbz = (S + PZ - 1) / PZ;
+    const unsigned nblk = (unsigned)(nbx * nby * nbz);
+    if (last != G::STRIDE) {
+      k_halo_tables<PX, PY, PZ><<<nblk, 128, 0, st>>>(sstart, tstart, span, S, nby, nbz, halo);
+      PB_LAUNCH("halo_tables");
+      last = G::STRIDE;
+    }
+    auto kern = k_m2l_unif_mac<PX, PY, PZ, KC, CG, T>;
+    constexpr size_t smem = MacSmem<PX, PY, PZ, KC, CG, T>::bytes;
+    PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3(nblk, (unsigned)((nk + KC - 1) / KC)), G::NP * KC * CG, smem, st>>>(
+        X, Y, op, halo, cells_at(lev), C, c0, nk);
+    PB_LAUNCH("m2l_unif_mac");
+    return PBBFMM_OK;
+  }
+
+  // Columns in groups of 8 and one smaller group, each an instance of its own
+  // (no lanes on absent columns).  Blocks: the fewer the columns, the more
+  // parents, so that a CTA has 4 to 10 warps and two or more CTAs share an SM.
+  int columns() {
+    constexpr bool f64 = sizeof(T) == 8;
+    for (int c0 = 0; c0 < C; c0 += 8) {
+      int rc;
+      switch (std::min(8, C - c0)) {
+        case 1: rc = run<4, 4, 4, f64 ? 2 : 4, 1>(c0); break;
+        case 2: rc = run<4, 4, 4, f64 ? 1 : 2, 2>(c0); break;
+        case 3: rc = run<4, 4, 4, 1, 3>(c0); break;
+        case 4: rc = run<4, 4, f64 ? 2 : 4, 1, 4>(c0); break;
+        case 5: rc = run<4, f64 ? 2 : 4, 2, 1, 5>(c0); break;
+        case 6: rc = run<4, f64 ? 2 : 4, 2, 1, 6>(c0); break;
+        case 7: rc = run<4, f64 ? 2 : 4, 2, 1, 7>(c0); break;
+        default: rc = run<4, f64 ? 2 : 4, 2, 1, 8>(c0); break;
+      }
+      if (rc) return rc;
+    }
+    return PBBFMM_OK;
+  }
+};
 
 template <typename T>
 struct FftLaunch {
@@ -623,7 +742,7 @@ struct FftLaunch {
   unsigned* amax = nullptr;  // forward: spectra maxima of the level (tensor-core MAC)
   template <int N>
   int run() {
-    const int n3 = N * N * N, nk = (2 * N - 1) * (2 * N - 1) * N;
+    const int n3 = N * N * N, nk = t->nk;
     Workspace& ws = t->ws;
     const int* lists = ws.lists.as<int>();
     const int64_t perS = (int64_t)C * n3, perX = (int64_t)nk * C;
@@ -672,14 +791,14 @@ static int run_m2l_unif_t(pbbfmm_tree* t, int C, cudaStream_t st) {
   const int fwd_col = n3 * ts + n3 * 2 * ts + n * m * n * 2 * ts;
   const int CGf = max(1, min(C, 60000 / fwd_col));
   const size_t smem_f = (size_t)ts * (2 * m + 2 * ((CGf * n3 + 3) & ~3)) +
-                        (size_t)2 * ts * (CGf * n3 + CGf * n * m * n) + (size_t)4 * m * n * 8;
+                        (size_t)2 * ts * (CGf * n3 + CGf * n * m * n) + (size_t)4 * unif_jobs(n) * 8;
   const int inv_col = (nk + n * m * n + n3) * 2 * ts;
   const int CGi = max(1, min(C, 60000 / inv_col));
   const size_t smem_i = (size_t)ts * ((2 * m + 3) & ~3) +
                         (size_t)2 * ts * (CGi * nk + CGi * n * m * n + CGi * n3);
   FftLaunch<T> fl{t, C, CGf, CGi, smem_f, smem_i, invP, st};
   // spectra maxima per level for the tensor-core MAC's scaling (float path)
-  const size_t amax_per = (size_t)m * n * 8;
+  const size_t amax_per = (size_t)unif_jobs(n) * 8;
   bool any_tc = false;
   for (int l = 2; l <= L; ++l) any_tc |= sizeof(T) == 4 && unif_tc_eligible(t, l, C);
   if (any_tc) {
@@ -704,22 +823,21 @@ static int run_m2l_unif_t(pbbfmm_tree* t, int C, cudaStream_t st) {
   for (int l = 2; l <= L; ++l) {
     if (t->lists.ntgt[l] == 0) continue;
     const int lvl = t->homog ? 0 : l - 2;
-    const C2* op = ov.op + (int64_t)lvl * nk * 343;
+    const C2* op = ov.op + (int64_t)lvl * nk * kKaraD * kKaraJ;
     const int span = (int)cells_at(L - l);
     int rc;
     if ((rc = kt_begin(t, KS_MAC, st))) return rc;
     const C2* Xl = X + level_offset(l, perX);
     C2* Yl = Y + level_offset(l, perX);
     // float32, 16 parents per side or more, columns in groups of 8: the
-    // tensor cores (m2l_unif_tc.cu); otherwise 4x2x2 parent blocks on the
-    // CUDA cores from level 3 up (level 2 has 2 parents per side)
-    if (sizeof(T) == 4 && unif_tc_eligible(t, l, C))
+    // tensor cores (m2l_unif_tc.cu); otherwise the CUDA cores
+    if (sizeof(T) == 4 && unif_tc_eligible(t, l, C)) {
       rc = run_m2l_unif_tc_level(t, C, l, lvl, reinterpret_cast<const float2*>(Xl),
                                  reinterpret_cast<float2*>(Yl), amax_at(l), st);
-    else if (l >= 3)
-      rc = launch_mac_cols<4, T>(Xl, Yl, op, halo, sstart, tstart, span, l, C, nk, st);
-    else
-      rc = launch_mac_cols<2, T>(Xl, Yl, op, halo, sstart, tstart, span, l, C, nk, st);
+    } else {
+      MacLevel<T> ml{Xl, Yl, op, halo, sstart, tstart, span, l, C, nk, st};
+      rc = ml.columns();
+    }
     if (rc) return rc;
     if ((rc = kt_end(t, st))) return rc;
     double len = t->p.L;

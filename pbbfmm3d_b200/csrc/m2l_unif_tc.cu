@@ -135,12 +135,12 @@ struct UnifTcArgs {
   float2* Y;             // level target spectra [k][cell][C]
   const uint16_t* tiles;  // [nk][kUnifTcTileHalves] operator tiles of this level (F16)
   const int* bexp;        // [nk] exponent sB of each frequency's tiles
-  const uint32_t* amax;   // [nk23][8] largest |spectra| (float bits) per (k23, column mod 8)
+  const uint32_t* amax;   // [job][8] largest |spectra| (float bits) per (slot / m, column mod 8)
   const uint8_t* socc;   // [cell] source cell nonempty
   const uint8_t* tocc;   // [cell] target cell nonempty
   int lev;               // cells 2^lev per side, parents S = 2^(lev-1)
   int C, c0;             // columns of the arrays; first of this group of 8
-  int nk, nk23, kchunk, nchunks, nblocks;  // frequencies k = k1 nk23 + k23
+  int nk, m, kchunk, nchunks, nblocks;  // frequency slots k = job m + k1
   int* err;
 };
 
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(UT_THREADS, 1) k_m2l_unif_tc(const UnifTcArgs 
       const bool in = xs >= 0 && xs < S && ys >= 0 && ys < S && zsp != 0xffffffffu;
       if (lp.k != k_ctx) {
         k_ctx = lp.k;
-        amax_k = a.amax + 8 * (lp.k % a.nk23) + t_col;
+        amax_k = a.amax + 8 * (lp.k / a.m) + t_col;
       }
       r.amax = __ldg(amax_k);
       r.occ = 0;
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(UT_THREADS, 1) k_m2l_unif_tc(const UnifTcArgs 
         }
         tc_fence_after();
         // undo the scaling of this row's column and of the frequency's tiles
-        const float ua = exp2i(-unif_scale_exp(__ldg(a.amax + 8 * (k % a.nk23) + col)));
+        const float ua = exp2i(-unif_scale_exp(__ldg(a.amax + 8 * (k / a.m) + col)));
         const float ub = exp2i(-__ldg(a.bexp + k));
         for (int ty = 0; ty < UT_BY; ++ty) {
           const uint32_t ta = lb + (uint32_t)(fb * UT_BY * 32 + 32 * ty);
@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(UT_THREADS, 1) k_m2l_unif_tc(const UnifTcArgs 
 
 // Operator tiles of the tensor-core MAC from the spectra op[lvl][k][343]
 // (complex, lex-indexed offsets, inner 27 zero): for each level and frequency
-// nine tiles (D_x, D_z), each [kcore 2][row 96][8 halves], row = 32 dyi +
+// slot nine tiles (D_x, D_z), each [kcore 2][row 96][8 halves], row = 32 dyi +
 // 16 part + 2 t + ri_out (D_y = 1 - dyi; part 0: F16 hi, 1: lo), element
 // K = 8 kcore + e = 2 s + ri_in, value the real form of E[o] with
 // o = 2 D + bits(s) - bits(t):  (re, re) = a, (im, re) = -b, (re, im) = b,
@@ -492,13 +492,13 @@ __global__ void __launch_bounds__(UT_THREADS, 1) k_m2l_unif_tc(const UnifTcArgs 
 // frequency scaled by 2^sB (bexp), sB putting the largest in [2^14, 2^15).
 void unif_tc_tiles(int n, const std::vector<double>& op, int nlev, std::vector<uint16_t>* tiles,
                    std::vector<int>* bexp) {
-  const int m = 2 * n - 1, nk = m * m * n;
+  const int m = 2 * n - 1, nfull = m * m * n, nk = unif_slots(n);
   tiles->assign((size_t)nlev * nk * kUnifTcTileHalves, 0);
   bexp->assign((size_t)nlev * nk, 0);
   parallel_for((int64_t)nlev * nk, [&](int64_t b0, int64_t b1) {
     std::vector<float> val(UT_BFREQ / 4);  // float32 values of the hi slots, tile order
     for (int64_t b = b0; b < b1; ++b) {
-      const double* E = &op[(size_t)b * 343 * 2];
+      const double* E = &op[(size_t)(b / nk * nfull + unif_slot_freq(n, (int)(b % nk))) * 343 * 2];
       float vmax = 0.f;
       for (int tile = 0; tile < 9; ++tile) {
         const int dxi = tile / 3, dzi = tile % 3;
@@ -580,7 +580,7 @@ int run_m2l_unif_tc_level(pbbfmm_tree* t, int C, int l, int lvl, const float2* X
   a.tiles = t->f_unif_tiles + (size_t)lvl * nk * kUnifTcTileHalves;
   a.bexp = t->f_unif_bexp + (size_t)lvl * nk;
   a.amax = amax;
-  a.nk23 = (2 * t->n - 1) * t->n;
+  a.m = t->m;
   a.socc = socc;
   a.tocc = tocc;
   a.lev = l;
