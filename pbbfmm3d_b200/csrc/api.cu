@@ -533,6 +533,8 @@ static void free_tree_device(pbbfmm_tree* t) {
   for (DevBuf* b : all) release(*b);
   if (ws.h_in) cudaFreeHost(ws.h_in);
   if (ws.h_out) cudaFreeHost(ws.h_out);
+  if (ws.h_counts) cudaFreeHost(ws.h_counts);
+  ws.h_counts = ws.d_counts = nullptr;
   ws.h_in = ws.h_out = nullptr;
   ws.h_in_cap = ws.h_out_cap = 0;
   if (ws.io_stream) cudaStreamDestroy(ws.io_stream);
@@ -1273,10 +1275,10 @@ int pbbfmm_debug_copy(pbbfmm_tree* t, int what, int level, double* host, int64_t
       p = t->ws.tperm.as<int>();
       total = t->last_Nf;
     } else if (what == 4) {
-      p = t->ws.sstart.as<int>();
+      p = t->ws.sstart_p;
       total = cells_at(L) + 1;
     } else {
-      p = t->ws.sperm.as<int>();
+      p = t->ws.sperm_p;
       total = t->last_Ns;
     }
     tmp.resize(total);

@@ -8,8 +8,6 @@
 // leaves (no atomics, no symmetry assumption, sources may differ from
 // targets), and the far-field interpolation, the near-field sum and the
 // scatter to the caller's output are one kernel.
-#include <cub/cub.cuh>
-
 #include <type_traits>
 
 #include "fmm.cuh"
@@ -203,32 +201,12 @@ struct L2LLaunch {
   }
 };
 
-// counts[i] = 32-target chunks of dense leaf i (i < *nsel), 0 otherwise (i <= nl)
-__global__ void k_chunk_counts(const int* __restrict__ part, const int* __restrict__ nsel, int nl,
-                               const int* __restrict__ tstart, int* __restrict__ counts) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > nl) return;
-  int c = 0;
-  if (i < *nsel) {
-    const int leaf = part[i];
-    c = (tstart[leaf + 1] - tstart[leaf] + 31) / 32;
-  }
-  counts[i] = c;
-}
-
-struct DenseLeaf {
-  const int* tstart;
-  __host__ __device__ bool operator()(int leaf) const {
-    return tstart[leaf + 1] - tstart[leaf] >= kLaneLeafMin;
-  }
-};
-
-// The leaf kernels' arguments for this compute.  Potentials: the leaves are
-// partitioned dense-first and the dense leaves' 32-target chunks counted and
-// scanned (so that each launch's active warps are packed into the first CTAs
-// of its grid).  Gradients: all leaves, one warp each.
-static int prepare_leaf_args(pbbfmm_tree* t, int64_t Nf, int64_t Ns, int C, double* out,
-                             cudaStream_t st, pbbfmm_leaf_args* a) {
+// The leaf kernels' arguments for this compute.  Potentials: the binning's
+// leaves dense-first, with the dense leaves' first 32-target chunks (so that
+// each launch's active warps are packed into the first CTAs of its grid).
+// Gradients: all leaves, one warp each.
+static void prepare_leaf_args(pbbfmm_tree* t, int64_t Nf, int64_t Ns, int C, double* out,
+                              pbbfmm_leaf_args* a) {
   const int L = t->p.tree_level;
   const int nl = t->lists.ntgt[L];
   Workspace& ws = t->ws;
@@ -240,10 +218,10 @@ static int prepare_leaf_args(pbbfmm_tree* t, int64_t Nf, int64_t Ns, int C, doub
   a->leaves = ws.lists.as<int>() + t->lists.tgt_off[L];
   a->nleaves = nl;
   a->tstart = ws.tstart.as<int>();
-  a->sstart = ws.sstart.as<int>();
+  a->sstart = ws.sstart_p;
   a->tperm = ws.tperm.as<int>();
   a->tpos = ws.tpos.as<double>();
-  a->spos = ws.spos.as<double>();
+  a->spos = ws.spos_p;
   a->wsorted = ws.wsorted.as<double>();
   a->Nf = (int)Nf;
   a->Ns = (int)Ns;
@@ -260,38 +238,15 @@ static int prepare_leaf_args(pbbfmm_tree* t, int64_t Nf, int64_t Ns, int C, doub
     a->out = t->gl.values ? out : nullptr;
     a->contract = t->gl.contract;
     a->grad_out = t->gl.grad_out;
-    return PBBFMM_OK;
+    return;
   }
   a->out = out;
-  if (int rc_ = grow(ws.leafpart, sizeof(int) * 3 * ((size_t)nl + 1))) return rc_;
-  int* part = ws.leafpart.as<int>();
-  int* nsel = part + nl;
-  size_t tb = 0;
-  DenseLeaf pred{ws.tstart.as<int>()};
-  PB_CUDA(cub::DevicePartition::If(nullptr, tb, a->leaves, part, nsel, nl, pred, st));
-  if (int rc_ = grow(ws.cub_temp, tb)) return rc_;
-  tb = ws.cub_temp.cap;
-  PB_CUDA(cub::DevicePartition::If(ws.cub_temp.p, tb, a->leaves, part, nsel, nl, pred, st));
-  count_launches(2);
-  // 32-target chunks of the dense leaves, exclusive scan -> one warp each
-  int* chunks = part + nl + 1;  // nl + 1 counts, then nl + 1 prefixes
-  int* prefix = chunks + nl + 1;
-  k_chunk_counts<<<(unsigned)((nl + 1 + 255) / 256), 256, 0, st>>>(part, nsel, nl,
-                                                                 ws.tstart.as<int>(), chunks);
-  PB_LAUNCH("leaf_chunks");
-  size_t tb2 = 0;
-  PB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, chunks, prefix, nl + 1, st));
-  if (int rc_ = grow(ws.cub_temp, tb2)) return rc_;
-  tb2 = ws.cub_temp.cap;
-  PB_CUDA(cub::DeviceScan::ExclusiveSum(ws.cub_temp.p, tb2, chunks, prefix, nl + 1, st));
-  count_launches(2);
-  a->leaves = part;
-  a->ndense = nsel;
-  a->chunk_prefix = prefix;
+  a->leaves = ws.leafpart.as<int>();
+  a->ndense = ws.ndense;
+  a->chunk_prefix = ws.dense_prefix;
   // upper bound of the chunk count: Nf / 32 + one partial chunk per dense
   // leaf (at most Nf / kLaneLeafMin of them)
   a->max_chunks = Nf / 32 + (nl < Nf / kLaneLeafMin ? nl : Nf / kLaneLeafMin) + 1;
-  return PBBFMM_OK;
 }
 
 // Status of a leaf launcher's return value (0, a cudaError_t code, or -1 for
@@ -337,7 +292,7 @@ int run_leaves(pbbfmm_tree* t, int64_t Nf, int64_t Ns, int C, double* d_out, cud
   if (t->lists.ntgt[t->p.tree_level] == 0) return PBBFMM_OK;
   pbbfmm_leaf_args a;
   if (int rc = kt_begin(t, KS_LEAF, st)) return rc;
-  if (int rc = prepare_leaf_args(t, Nf, Ns, C, d_out, st, &a)) return rc;
+  prepare_leaf_args(t, Nf, Ns, C, d_out, &a);
   int rc;
   if (t->p.kernel == PBBFMM_KERNEL_USER) {
     if (a.gradient && !t->user.has_gradient) return leaf_status(-1);

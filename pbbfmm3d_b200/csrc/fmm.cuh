@@ -46,7 +46,13 @@ struct Workspace {
   DevBuf halo;   // Unif M2L: per parent block, region and target parents and their occupancy
   DevBuf tc_proxy;  // tensor-core Cheb M2L: hi then lo proxies of one level (+ F16 exponents)
   DevBuf m2l_part;  // float64 Cheb M2L: partial sums of levels with few tiles
-  DevBuf leafpart;  // leaf phase: target leaves partitioned dense-first, then their count
+  DevBuf leafpart;  // leaf phase: target leaves dense-first, chunk prefix of the dense ones
+  // the sources' leaf offsets, permutation and positions of the last binning
+  // (the targets' where one buffer is both), and the dense leaves' count
+  int *sperm_p = nullptr, *sstart_p = nullptr;
+  double* spos_p = nullptr;
+  int *ndense = nullptr, *dense_prefix = nullptr;
+  int *h_counts = nullptr, *d_counts = nullptr;  // mapped pinned: lengths of the lists
   DevBuf occ;       // tensor-core uniform M2L: per-cell source / target occupancy of a level
   DevBuf amax;      // tensor-core uniform M2L: per level, largest |spectra| per (k23, column mod 8)
   // staging for the host-pointer entry point

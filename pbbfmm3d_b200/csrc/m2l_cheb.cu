@@ -338,7 +338,7 @@ static int run_m2l_cheb_f32(pbbfmm_tree* t, int C, cudaStream_t st) {
   T* proxy = ws.proxy.as<T>();
   T* pf = ws.pf.as<T>();
   const OpsView<T> ov = ops_view<T>(t);
-  const int* sstart = ws.sstart.as<int>();
+  const int* sstart = ws.sstart_p;
   if (C > GBN) {
     set_error("nCols above 64 must be split by the caller");
     return PBBFMM_ERR_UNSUPPORTED;

@@ -593,7 +593,7 @@ static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
   a.rf = rf;
   a.rsp = rsp;
   fd_blocks(rf, &a.nblk, &a.ntb);
-  a.sstart = ws.sstart.as<int>();
+  a.sstart = ws.sstart_p;
   a.offs = t->d_offs;
   int nsm = 148;
   PB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, t->device));

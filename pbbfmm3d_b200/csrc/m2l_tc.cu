@@ -570,7 +570,7 @@ static int launch_tc(const pbbfmm_tree* t, unsigned tiles, int smem, int rf, int
   PB_CUDA(cudaFuncSetAttribute(k_m2l_cheb_tc<NST, F16, RSUM>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   k_m2l_cheb_tc<NST, F16, RSUM><<<tiles, TC_THREADS, smem, st>>>(
-      rf, NP, rowb, tm_h, tm_l, lvl, typed, tt, C, l, t->ws.sstart.as<int>(), span, t->d_offs,
+      rf, NP, rowb, tm_h, tm_l, lvl, typed, tt, C, l, t->ws.sstart_p, span, t->d_offs,
       ph, pl, pexp, t->tc.eexp + (int64_t)lvl * 316, pf, tc_group(NP, F16), t->d_tc_err);
   PB_LAUNCH("m2l_cheb_tc");
   return PBBFMM_OK;

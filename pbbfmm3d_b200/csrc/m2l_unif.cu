@@ -782,7 +782,7 @@ static int run_m2l_unif_t(pbbfmm_tree* t, int C, cudaStream_t st) {
   Workspace& ws = t->ws;
   C2* X = ws.proxy.as<C2>();
   C2* Y = ws.pf.as<C2>();
-  const int* sstart = ws.sstart.as<int>();
+  const int* sstart = ws.sstart_p;
   const int* tstart = ws.tstart.as<int>();
   const int64_t perX = (int64_t)nk * C;
   const double invP = 1.0 / (double)(m * m * m);

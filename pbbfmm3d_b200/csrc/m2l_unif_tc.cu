@@ -569,7 +569,7 @@ int run_m2l_unif_tc_level(pbbfmm_tree* t, int C, int l, int lvl, const float2* X
   uint8_t* tocc = socc + ncells;
   const int span = (int)cells_at(L - l);
   const unsigned g = (unsigned)((ncells + 255) / 256);
-  k_occupancy<<<g, 256, 0, st>>>(ws.sstart.as<int>(), span, ncells, socc);
+  k_occupancy<<<g, 256, 0, st>>>(ws.sstart_p, span, ncells, socc);
   PB_LAUNCH("occupancy");
   k_occupancy<<<g, 256, 0, st>>>(ws.tstart.as<int>(), span, ncells, tocc);
   PB_LAUNCH("occupancy");

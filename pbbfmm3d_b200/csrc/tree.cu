@@ -9,8 +9,6 @@
 // the device, producing the same Morton leaf index, and a stable radix sort
 // keeps the reference's within-leaf order (original index order).
 #include <cub/cub.cuh>
-#include <thrust/iterator/counting_iterator.h>
-#include <thrust/iterator/transform_iterator.h>
 
 #include "fmm.cuh"
 
@@ -59,15 +57,22 @@ __global__ void k_bbox_partial(const double* __restrict__ p, int64_t N, double* 
   }
 }
 
+// One warp: lanes over the partial boxes, then across the lanes.
 __global__ void k_bbox_final(const double* __restrict__ part, int nb, double* __restrict__ ctr) {
-  if (threadIdx.x < 3) {
-    int d = threadIdx.x;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
     double a = 1e32, b = -1e32;
-    for (int j = 0; j < nb; ++j) {
+    for (int j = lane; j < nb; j += 32) {
       a = part[j * 6 + d] < a ? part[j * 6 + d] : a;
       b = b < part[j * 6 + 3 + d] ? part[j * 6 + 3 + d] : b;
     }
-    ctr[d] = 0.5 * (a + b);  // include/compute.hpp:108-111
+    for (int o = 16; o > 0; o >>= 1) {
+      const double a2 = __shfl_xor_sync(0xffffffffu, a, o), b2 = __shfl_xor_sync(0xffffffffu, b, o);
+      a = a2 < a ? a2 : a;
+      b = b < b2 ? b2 : b;
+    }
+    if (lane == 0) ctr[d] = 0.5 * (a + b);  // include/compute.hpp:108-111
   }
 }
 
@@ -110,15 +115,20 @@ __global__ void k_leaf_start(const uint32_t* __restrict__ ks, int N, int64_t nle
   start[k] = lo;
 }
 
-__global__ void k_gather_pos(const double* __restrict__ p, const int* __restrict__ perm, int N,
-                             const double* __restrict__ ctr, double* __restrict__ soa) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Sorted positions (recentred, SoA) and, with w, the sorted weights.
+__global__ void k_gather(const double* __restrict__ p, const int* __restrict__ perm, int N,
+                         const double* __restrict__ ctr, double* __restrict__ soa,
+                         const double* __restrict__ w, int C, double* __restrict__ ws) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const int j = perm[i];
 #pragma unroll
   for (int d = 0; d < 3; ++d) soa[(int64_t)d * N + i] = p[3 * (int64_t)j + d] - ctr[d];
+  if (w)
+    for (int c = 0; c < C; ++c) ws[(int64_t)i * C + c] = w[(int64_t)c * N + j];
 }
 
+// Sorted weights, thread per (point, column): coalesced rows for several columns.
 __global__ void k_gather_w(const double* __restrict__ w, const int* __restrict__ perm, int Ns,
                            int C, double* __restrict__ ws) {
   int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -127,36 +137,145 @@ __global__ void k_gather_w(const double* __restrict__ w, const int* __restrict__
   ws[t] = w[(int64_t)c * Ns + perm[j]];
 }
 
-struct NonEmpty {
-  const int* start;
-  int span_shift;  // 3 * (L - l)
-  __host__ __device__ bool operator()(int cell) const {
-    int64_t a = (int64_t)cell << span_shift, b = (int64_t)(cell + 1) << span_shift;
-    return start[b] > start[a];
-  }
+// Lists of cells, all levels in three launches (counts per block of cells, a
+// scan of the counts, the writes): per level the nonempty source cells and
+// target cells in Morton order and the target cells ordered by (child type,
+// parent); of the leaves also the dense and the sparse target leaves, back to
+// back, with the first 32-target chunk of each dense one.  (A select per list
+// costs two launches for each of 3 (L - 1) lists: of a 20,000-point matvec on
+// 4 levels that was 0.1 of 0.64 ms, nearly all of it launches.)
+enum ListKind { LIST_SRC = 0, LIST_TGT = 1, LIST_TYPED = 2, LIST_DENSE = 3, LIST_SPARSE = 4 };
+constexpr int kListThreads = 256, kListItems = 4, kListBlock = kListThreads * kListItems;
+
+struct ListJob {
+  int kind, shift;    // shift = 3 (L - level): leaf ranges of a cell
+  int ncells, block0; // virtual cells, first block
+  int* out;           // the list
+  int* count;         // its length (device)
+  int* bounds;        // LIST_TYPED: [9] first position of each child type
+  int slot;           // index of the length in the host copy; bounds at slot + 1
+};
+struct ListArgs {
+  ListJob job[3 * (kMaxLevel - 1) + 2];
+  int njobs, nblocks;
+  const int *sstart, *tstart;
+  int *bcount, *bchunk;  // per block: cells selected, chunks of dense leaves
+  int* prefix;           // first chunk of each dense leaf, then the total
+  int* hcount;           // mapped host memory: the lengths and bounds
 };
 
-// virtual index v -> cell 8*(v % npar) + v / npar, so selection is ordered by
-// (child type, parent Morton index)
-struct TypedCell {
-  int npar;
-  __host__ __device__ int operator()(int v) const { return 8 * (v % npar) + v / npar; }
-};
+__device__ __forceinline__ int list_job(const ListArgs& a) {
+  int j = 0;
+  for (int i = 1; i < a.njobs; ++i)
+    if ((int)blockIdx.x >= a.job[i].block0) j = i;
+  return j;
+}
+// virtual cell v of a job: its Morton index and whether it is listed; for dense
+// leaves also their chunks of 32 targets
+__device__ __forceinline__ bool list_cell(const ListArgs& a, const ListJob& j, int v, int* cell,
+                                          int* chunks) {
+  if (v >= j.ncells) return false;
+  const int npar = j.ncells >> 3;
+  *cell = j.kind == LIST_TYPED ? 8 * (v % npar) + v / npar : v;
+  const int* start = j.kind == LIST_SRC ? a.sstart : a.tstart;
+  const int64_t c = *cell;
+  const int n = start[(c + 1) << j.shift] - start[c << j.shift];
+  *chunks = (n + 31) / 32;
+  if (j.kind == LIST_DENSE) return n >= kLaneLeafMin;
+  if (j.kind == LIST_SPARSE) return n > 0 && n < kLaneLeafMin;
+  return n > 0;
+}
 
-__global__ void k_type_bounds(const int* __restrict__ list, const int* __restrict__ count,
-                              int* __restrict__ bounds) {
-  int t = threadIdx.x;
-  if (t > 8) return;
-  int n = *count;
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if ((list[mid] & 7) < t)
-      lo = mid + 1;
-    else
-      hi = mid;
+// block-wide exclusive prefix of (x, y); *tx, *ty the totals
+__device__ __forceinline__ void block_scan2(int x, int y, int* ex, int* ey, int* tx, int* ty) {
+  __shared__ int sx[kListThreads / 32], sy[kListThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int ix = x, iy = y;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ax = __shfl_up_sync(0xffffffffu, ix, o), ay = __shfl_up_sync(0xffffffffu, iy, o);
+    if (lane >= o) ix += ax, iy += ay;
   }
-  bounds[t] = lo;
+  __syncthreads();  // the previous call's readers
+  if (lane == 31) sx[w] = ix, sy[w] = iy;
+  __syncthreads();
+  int bx = 0, by = 0;
+  *tx = *ty = 0;
+  for (int k = 0; k < kListThreads / 32; ++k) {
+    if (k < w) bx += sx[k], by += sy[k];
+    *tx += sx[k], *ty += sy[k];
+  }
+  *ex = bx + ix - x;
+  *ey = by + iy - y;
+}
+
+__global__ void __launch_bounds__(kListThreads) k_list_count(const __grid_constant__ ListArgs a) {
+  const ListJob& j = a.job[list_job(a)];
+  const int v0 = ((int)blockIdx.x - j.block0) * kListBlock + threadIdx.x * kListItems;
+  int n = 0, nc = 0;
+#pragma unroll
+  for (int i = 0; i < kListItems; ++i) {
+    int cell, ch;
+    if (list_cell(a, j, v0 + i, &cell, &ch)) n += 1, nc += ch;
+  }
+  int ex, ey, tx, ty;
+  block_scan2(n, nc, &ex, &ey, &tx, &ty);
+  if (threadIdx.x == 0) a.bcount[blockIdx.x] = tx, a.bchunk[blockIdx.x] = ty;
+}
+
+// one block per list: exclusive scan of its blocks' counts, in place
+__global__ void __launch_bounds__(kListThreads) k_list_scan(const __grid_constant__ ListArgs a) {
+  const ListJob& j = a.job[blockIdx.x];
+  const int b1 = blockIdx.x + 1 < a.njobs ? a.job[blockIdx.x + 1].block0 : a.nblocks;
+  int n = 0, nc = 0;
+  for (int b = j.block0; b < b1; b += kListThreads) {
+    const int k = b + threadIdx.x;
+    const int x = k < b1 ? a.bcount[k] : 0, y = k < b1 ? a.bchunk[k] : 0;
+    int ex, ey, tx, ty;
+    block_scan2(x, y, &ex, &ey, &tx, &ty);
+    if (k < b1) a.bcount[k] = n + ex, a.bchunk[k] = nc + ey;
+    n += tx;
+    nc += ty;
+  }
+  if (threadIdx.x == 0) {
+    *j.count = n;
+    if (j.kind == LIST_DENSE) a.prefix[n] = nc;
+    if (j.slot >= 0) a.hcount[j.slot] = n;
+    if (j.kind == LIST_TYPED) j.bounds[8] = a.hcount[j.slot + 9] = n;
+  }
+}
+
+__global__ void __launch_bounds__(kListThreads) k_list_write(const __grid_constant__ ListArgs a) {
+  const int ji = list_job(a);
+  const ListJob& j = a.job[ji];
+  const int v0 = ((int)blockIdx.x - j.block0) * kListBlock + threadIdx.x * kListItems;
+  int cell[kListItems], ch[kListItems], n = 0, nc = 0;
+  bool sel[kListItems];
+#pragma unroll
+  for (int i = 0; i < kListItems; ++i) {
+    sel[i] = list_cell(a, j, v0 + i, &cell[i], &ch[i]);
+    if (sel[i]) n += 1, nc += ch[i];
+  }
+  int ex, ey, tx, ty;
+  block_scan2(n, nc, &ex, &ey, &tx, &ty);
+  int at = a.bcount[blockIdx.x] + ex, cat = a.bchunk[blockIdx.x] + ey;
+  // the sparse leaves follow the dense ones (the job before)
+  const int base = j.kind == LIST_SPARSE ? *a.job[ji - 1].count : 0;
+  const int npar = j.ncells >> 3;
+#pragma unroll
+  for (int i = 0; i < kListItems; ++i) {
+    const int v = v0 + i;
+    if (j.kind == LIST_TYPED && v < j.ncells && v % npar == 0) {
+      j.bounds[v / npar] = at;
+      a.hcount[j.slot + 1 + v / npar] = at;
+    }
+    if (sel[i]) {
+      j.out[base + at] = cell[i];
+      if (j.kind == LIST_DENSE) a.prefix[at] = cat;
+      at += 1;
+      cat += ch[i];
+    }
+  }
 }
 
 int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d_src, int64_t Ns,
@@ -166,24 +285,14 @@ int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d
   const int64_t nleaf = cells_at(L);
   const int64_t Nmax = Nf > Ns ? Nf : Ns;
 
-  // CUB scratch: radix sort of Nmax keys and selection over 8^L cells
-  size_t sort_bytes = 0, sel_bytes = 0;
-  PB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const uint32_t*)nullptr,
+  // CUB scratch: radix sort of Nmax keys
+  size_t cub_need = 0;
+  PB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, cub_need, (const uint32_t*)nullptr,
                                           (uint32_t*)nullptr, (const int*)nullptr, (int*)nullptr,
                                           (int)Nmax, 0, 3 * L, st));
-  size_t sel2_bytes = 0;
-  {
-    NonEmpty pred{nullptr, 0};
-    thrust::counting_iterator<int> it(0);
-    PB_CUDA(cub::DeviceSelect::If(nullptr, sel_bytes, it, (int*)nullptr, (int*)nullptr,
-                                  (int)nleaf, pred, st));
-    auto tit = thrust::make_transform_iterator(it, TypedCell{(int)(nleaf / 8)});
-    PB_CUDA(cub::DeviceSelect::If(nullptr, sel2_bytes, tit, (int*)nullptr, (int*)nullptr,
-                                  (int)nleaf, pred, st));
-  }
-  size_t cub_need = sort_bytes > sel_bytes ? sort_bytes : sel_bytes;
-  cub_need = cub_need > sel2_bytes ? cub_need : sel2_bytes;
-
+  // one buffer given as sources and targets is binned once: the sources'
+  // arrays are the targets'
+  const bool same = d_tgt == d_src && Nf == Ns;
   int64_t list_need = 0;
   for (int l = 2; l <= L; ++l) {
     int64_t nc = cells_at(l);
@@ -196,15 +305,25 @@ int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d
   if ((rc = grow(ws.key_sorted, 4 * Nmax))) return rc;
   if ((rc = grow(ws.idx, 4 * Nmax))) return rc;
   if ((rc = grow(ws.tperm, 4 * Nf))) return rc;
-  if ((rc = grow(ws.sperm, 4 * Ns))) return rc;
+  if (!same && (rc = grow(ws.sperm, 4 * Ns))) return rc;
   if ((rc = grow(ws.tstart, 4 * (nleaf + 1)))) return rc;
-  if ((rc = grow(ws.sstart, 4 * (nleaf + 1)))) return rc;
+  if (!same && (rc = grow(ws.sstart, 4 * (nleaf + 1)))) return rc;
   if ((rc = grow(ws.tpos, 8 * 3 * Nf))) return rc;
-  if ((rc = grow(ws.spos, 8 * 3 * Ns))) return rc;
+  if (!same && (rc = grow(ws.spos, 8 * 3 * Ns))) return rc;
   if ((rc = grow(ws.wsorted, 8 * Ns * (int64_t)C))) return rc;
   if ((rc = grow(ws.cub_temp, cub_need))) return rc;
   if ((rc = grow(ws.lists, 4 * (list_need + 16)))) return rc;
   if ((rc = grow(ws.dcounts, 4 * (kMaxLevel + 1) * 12))) return rc;
+  // dense and sparse target leaves, the chunk prefix, then the block counts
+  const int64_t leaf_need = (nleaf < Nf ? nleaf : Nf) + 1;
+  int64_t list_blocks = 0;
+  for (int l = 2; l <= L; ++l)
+    list_blocks += (l == L ? 5 : 3) * ((cells_at(l) + kListBlock - 1) / kListBlock);
+  if ((rc = grow(ws.leafpart, 4 * (2 * leaf_need + 2 * list_blocks)))) return rc;
+  if (!ws.h_counts) {
+    PB_CUDA(cudaHostAlloc(&ws.h_counts, sizeof(int) * 12 * (kMaxLevel + 1), cudaHostAllocMapped));
+    PB_CUDA(cudaHostGetDevicePointer(&ws.d_counts, ws.h_counts, 0));
+  }
   double* ctr = ws.ctr.as<double>();
   uint32_t* key = ws.key.as<uint32_t>();
   uint32_t* key_sorted = ws.key_sorted.as<uint32_t>();
@@ -234,54 +353,74 @@ int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d
     PB_LAUNCH("leaf_start");
     return PBBFMM_OK;
   };
+  auto gather = [&](const double* pts, const int* perm, int64_t N, double* pos, const double* w) -> int {
+    if (N == 0) return PBBFMM_OK;
+    const bool fused = C < 4;  // few columns: the weights with the positions
+    k_gather<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(pts, perm, (int)N, ctr, pos,
+                                                         fused ? w : nullptr, C,
+                                                         ws.wsorted.as<double>());
+    PB_LAUNCH("gather");
+    if (w && !fused) {
+      k_gather_w<<<(unsigned)((N * C + 255) / 256), 256, 0, st>>>(w, perm, (int)N, C,
+                                                                 ws.wsorted.as<double>());
+      PB_LAUNCH("gather_w");
+    }
+    return PBBFMM_OK;
+  };
+  ws.sperm_p = same ? ws.tperm.as<int>() : ws.sperm.as<int>();
+  ws.sstart_p = same ? ws.tstart.as<int>() : ws.sstart.as<int>();
+  ws.spos_p = same ? ws.tpos.as<double>() : ws.spos.as<double>();
   if ((rc = bin_set(d_tgt, Nf, ws.tperm.as<int>(), ws.tstart.as<int>()))) return rc;
-  if (Nf > 0) {
-    k_gather_pos<<<(unsigned)((Nf + 255) / 256), 256, 0, st>>>(d_tgt, ws.tperm.as<int>(), (int)Nf,
-                                                               ctr, ws.tpos.as<double>());
-    PB_LAUNCH("gather_tpos");
-  }
-  if ((rc = bin_set(d_src, Ns, ws.sperm.as<int>(), ws.sstart.as<int>()))) return rc;
-  if (Ns > 0) {
-    k_gather_pos<<<(unsigned)((Ns + 255) / 256), 256, 0, st>>>(d_src, ws.sperm.as<int>(), (int)Ns,
-                                                               ctr, ws.spos.as<double>());
-    int64_t tot = Ns * (int64_t)C;
-    k_gather_w<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(d_w, ws.sperm.as<int>(), (int)Ns, C,
-                                                              ws.wsorted.as<double>());
-    PB_LAUNCH_N("gather_src", 2);
+  if ((rc = gather(d_tgt, ws.tperm.as<int>(), Nf, ws.tpos.as<double>(), same ? d_w : nullptr)))
+    return rc;
+  if (!same) {
+    if ((rc = bin_set(d_src, Ns, ws.sperm_p, ws.sstart_p))) return rc;
+    if ((rc = gather(d_src, ws.sperm_p, Ns, ws.spos_p, d_w))) return rc;
   }
 
-  // nonempty-cell lists for levels 2..L
   LevelLists& LL = t->lists;
-  int64_t off = 0;
+  ListArgs la{};
+  la.sstart = ws.sstart_p;
+  la.tstart = ws.tstart.as<int>();
+  la.hcount = ws.d_counts;
   int* cnt = ws.dcounts.as<int>();  // [l][0]=nsrc [l][1]=ntgt [l][2]=ntyp [l][3..11] type bounds
+  int* part = ws.leafpart.as<int>();
+  la.prefix = part + leaf_need;
+  la.bcount = la.prefix + leaf_need;
+  la.bchunk = la.bcount + list_blocks;
+  auto add = [&](int kind, int l, int* out, int* count, int slot) {
+    ListJob& j = la.job[la.njobs++];
+    j.kind = kind;
+    j.shift = 3 * (L - l);
+    j.ncells = (int)cells_at(l);
+    j.block0 = la.nblocks;
+    j.out = out;
+    j.count = count;
+    j.slot = slot;
+    j.bounds = kind == LIST_TYPED ? count + 1 : nullptr;
+    la.nblocks += (j.ncells + kListBlock - 1) / kListBlock;
+  };
+  int64_t off = 0;
   for (int l = 2; l <= L; ++l) {
-    const int64_t nc = cells_at(l);
-    const int shift = 3 * (L - l);
-    thrust::counting_iterator<int> it(0);
-    size_t bytes;
+    const int64_t nc = cells_at(l), ms = nc < Ns ? nc : Ns, mt = nc < Nf ? nc : Nf;
     LL.src_off[l] = off;
-    bytes = ws.cub_temp.cap;
-    PB_CUDA(cub::DeviceSelect::If(ws.cub_temp.p, bytes, it, lists + off, cnt + 12 * l + 0,
-                                  (int)nc, NonEmpty{ws.sstart.as<int>(), shift}, st));
-    off += (nc < Ns ? nc : Ns);
-    LL.tgt_off[l] = off;
-    bytes = ws.cub_temp.cap;
-    PB_CUDA(cub::DeviceSelect::If(ws.cub_temp.p, bytes, it, lists + off, cnt + 12 * l + 1,
-                                  (int)nc, NonEmpty{ws.tstart.as<int>(), shift}, st));
-    off += (nc < Nf ? nc : Nf);
-    LL.typ_off[l] = off;
-    bytes = ws.cub_temp.cap;
-    auto tit = thrust::make_transform_iterator(it, TypedCell{(int)(nc / 8)});
-    PB_CUDA(cub::DeviceSelect::If(ws.cub_temp.p, bytes, tit, lists + off, cnt + 12 * l + 2,
-                                  (int)nc, NonEmpty{ws.tstart.as<int>(), shift}, st));
-    count_launches(3 * 2);  // three DeviceSelect calls: init + scan kernels each
-    k_type_bounds<<<1, 32, 0, st>>>(lists + off, cnt + 12 * l + 2, cnt + 12 * l + 3);
-    PB_LAUNCH("type_bounds");
-    off += (nc < Nf ? nc : Nf);
+    LL.tgt_off[l] = off + ms;
+    LL.typ_off[l] = off + ms + mt;
+    for (int k = 0; k < 3; ++k)
+      add(k, l, lists + (k == 0 ? LL.src_off[l] : k == 1 ? LL.tgt_off[l] : LL.typ_off[l]),
+          cnt + 12 * l + k, 12 * l + k);
+    off += ms + 2 * mt;
   }
-  int hc[(kMaxLevel + 1) * 12];
-  PB_CUDA(cudaMemcpyAsync(hc, ws.dcounts.p, sizeof(int) * 12 * (L + 1), cudaMemcpyDeviceToHost, st));
+  add(LIST_DENSE, L, part, cnt, -1);
+  add(LIST_SPARSE, L, part, cnt + 1, -1);
+  ws.ndense = cnt;
+  ws.dense_prefix = la.prefix;
+  k_list_count<<<la.nblocks, kListThreads, 0, st>>>(la);
+  k_list_scan<<<la.njobs, kListThreads, 0, st>>>(la);
+  k_list_write<<<la.nblocks, kListThreads, 0, st>>>(la);
+  PB_LAUNCH_N("lists", 3);
   PB_CUDA(cudaStreamSynchronize(st));
+  const int* hc = ws.h_counts;
   for (int l = 2; l <= L; ++l) {
     LL.nsrc[l] = hc[12 * l + 0];
     LL.ntgt[l] = hc[12 * l + 1];

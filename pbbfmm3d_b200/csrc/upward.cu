@@ -126,7 +126,7 @@ struct P2MLaunch {
     constexpr int W = p2m_warps<N, T>();
     const OpsView<T> ov = ops_view<T>(t);
     k_p2m<N, T><<<(nl + W - 1) / W, 32 * W, 0, st>>>(
-        ws.lists.as<int>() + t->lists.src_off[L], nl, ws.sstart.as<int>(), ws.spos.as<double>(),
+        ws.lists.as<int>() + t->lists.src_off[L], nl, ws.sstart_p, ws.spos_p,
         (int)t->last_Ns, ws.wsorted.as<double>(), C, t->p.use_chebyshev, ov.Tkz, t->p.L, L,
         ws.S.as<T>() + level_offset(L, (int64_t)C * N * N * N));
     PB_LAUNCH("p2m");
@@ -342,7 +342,7 @@ struct M2MLaunch {
     const size_t smem = sizeof(T) * G::per_warp * G::warps;
     PB_CUDA(cudaFuncSetAttribute(k_m2m<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_m2m<N, T><<<(unsigned)((tasks + G::warps - 1) / G::warps), 32 * G::warps, smem, st>>>(
-        ws.lists.as<int>() + t->lists.src_off[l], np, ws.sstart.as<int>(), (int)cells_at(L - l - 1),
+        ws.lists.as<int>() + t->lists.src_off[l], np, ws.sstart_p, (int)cells_at(L - l - 1),
         ws.S.as<T>() + level_offset(l + 1, per), ws.S.as<T>() + level_offset(l, per), C,
         ops_view<T>(t).Cw);
     PB_LAUNCH("m2m");
