@@ -650,8 +650,10 @@ static int compute_chunk(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const 
     if ((rc = grow(ws.proxy, es * level_total(L, (int64_t)C * rsp)))) return rc;
     if ((rc = grow(ws.pf, es * level_total(L, (int64_t)C * t->ops.rf)))) return rc;
   } else {
-    if ((rc = grow(ws.proxy, 2 * es * level_total(L, (int64_t)C * t->nk)))) return rc;
-    if ((rc = grow(ws.pf, 2 * es * level_total(L, (int64_t)C * t->nk)))) return rc;
+    size_t xb, yb;
+    unif_spectra_bytes(t, C, precision == PBBFMM_PREC_FP64, &xb, &yb);
+    if ((rc = grow(ws.proxy, xb))) return rc;
+    if ((rc = grow(ws.pf, yb))) return rc;
     if ((rc = grow(ws.halo, sizeof(int) * unif_halo_ints(1 << (L - 1))))) return rc;
   }
   if ((rc = run_upward(t, C, st))) return rc;

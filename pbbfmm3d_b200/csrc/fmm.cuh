@@ -41,8 +41,8 @@ struct Workspace {
   // per-level coefficient arrays (levels 2..L)
   DevBuf S;      // moments      sum_l 8^l * C * n3
   DevBuf F;      // locals       sum_l 8^l * C * n3
-  DevBuf proxy;  // Cheb: sum_l 8^l * C * rs ;  Unif: spectra sum_l 8^l * nk * C (complex)
-  DevBuf pf;     // Cheb: sum_l 8^l * C * rf ;  Unif: accumulated spectra
+  DevBuf proxy;  // Cheb: sum_l 8^l * C * rs ;  Unif: spectra of one level
+  DevBuf pf;     // Cheb: sum_l 8^l * C * rf ;  Unif: accumulated spectra of one level
   DevBuf halo;   // Unif M2L: per parent block, region and target parents and their occupancy
   DevBuf tc_proxy;  // tensor-core Cheb M2L: hi then lo proxies of one level (+ F16 exponents)
   DevBuf m2l_part;  // float64 Cheb M2L: partial sums of levels with few tiles
@@ -54,7 +54,7 @@ struct Workspace {
   int *ndense = nullptr, *dense_prefix = nullptr;
   int *h_counts = nullptr, *d_counts = nullptr;  // mapped pinned: lengths of the lists
   DevBuf occ;       // tensor-core uniform M2L: per-cell source / target occupancy of a level
-  DevBuf amax;      // tensor-core uniform M2L: per level, largest |spectra| per (k23, column mod 8)
+  DevBuf amax;      // tensor-core uniform M2L: bound on a level's spectra per column of a group
   // staging for the host-pointer entry point
   DevBuf io_tgt, io_src, io_w, io_out;
   // pinned host staging of the host-buffer entry point (cudaHostAlloc)
@@ -244,8 +244,8 @@ int run_m2l_unif(pbbfmm_tree* t, int C, cudaStream_t st);
 // tensor-core uniform M2L (float path): levels with >= 16 parents per side,
 // columns in groups of 8
 bool unif_tc_eligible(const pbbfmm_tree* t, int l, int C);
-int run_m2l_unif_tc_level(pbbfmm_tree* t, int C, int l, int lvl, const float2* X, float2* Y,
-                          const uint32_t* amax, cudaStream_t st);
+// bytes of the uniform path's spectra arrays (Workspace::proxy and pf)
+void unif_spectra_bytes(const pbbfmm_tree* t, int C, bool f64, size_t* x, size_t* y);
 void unif_tc_tiles(int n, const std::vector<double>& op, int nlev, std::vector<uint16_t>* tiles,
                    std::vector<int>* bexp);
 int set_unif_tc_wait_limit(long long polls);

@@ -21,12 +21,17 @@
 // Frequency slots.  Jobs j number the kept (k2, k3): first k3 = 1..n-1 for
 // every k2, then k3 = 0 for k2 = 1..(m-1)/2, last (0, 0); slot j m + k1, of
 // the last job only k1 <= (m-1)/2.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <vector>
 
 #include "fmm.cuh"
+#include "tcgen05.cuh"
+#include "unif_tc.cuh"
 
 namespace pbbfmm {
 
@@ -179,198 +184,267 @@ int unif_slot_freq(int n, int slot) {
 // Spectra of a level are stored frequency-major: X[(slot * ncells + cell) * C + col]
 // (ncells = 8^level), so that one frequency plane of a level is contiguous.
 
-// Forward: CTAs loop over the nonempty source cells (cells[0..ncl)), columns
-// in groups of CG.  With amax (float path, levels of the tensor-core MAC), a
-// bound on |re| and |im| of the spectra per (k23, column mod 8), over the
-// level's cells and k1, as float bits: the sum of |re| + |im| of the last
-// transform's n inputs (a bound on every one of its m outputs), per CTA in
-// shared memory, then one atomicMax per slot into amax[k23][8] (zeroed by
-// the caller).
-// w = e^{-2 pi i / m}; (a + ib) w^j = (a c + b s) + i (b c - a s).
+// Both transforms run one unit = (cell, column) per lane: the U units of a CTA
+// are neighbours in memory, so that a warp's loads and stores of a frequency
+// cover consecutive words, and every thread computes whole 1-D transforms of
+// its unit.  Two stages with one array between them in shared memory
+// ([element][unit], conflict-free):
+//   forward: thread (l1): the n^2 moments of its row; for each k3 the z
+//            transform of the n lines l2 and the y transform of the results;
+//            thread (j): the x transform of (k2, k3), straight to global memory;
+//   inverse: thread (j): the x transform, straight from global memory; thread
+//            (a1): for each k3 the y transform, added into the n^2 outputs of
+//            its row by the z transform; the outputs leave through shared
+//            memory in coalesced rows.
+// Bound: HBM and the latency of the stages (shared memory admits two to three
+// CTAs per SM).  Measured, 1M points at order 5, forward + inverse, against one
+// cell per CTA with a column per lane: 1 column, float32 2.57 + 1.56 -> 0.39 +
+// 0.39 ms (its stores covered 8 bytes of each frequency plane); 8 columns,
+// float64 3.77 + 5.38 -> 2.89 + 3.61 ms.
 template <int n, typename T>
-__global__ void k_fft_fwd(const int* __restrict__ cells, int ncl, const T* __restrict__ S_l,
-                          cplx_t<T>* __restrict__ X_l, int64_t ncells, int C, int CG,
-                          const T* __restrict__ twid, unsigned* __restrict__ amax) {
-  using C2 = cplx_t<T>;
+struct FftCfg {
+  static constexpr int m = 2 * n - 1, n3 = n * n * n, nym = n * m * n;
+  static constexpr int unit = (n3 + 2 * nym) * (int)sizeof(T);  // bytes per unit (forward)
+  static constexpr int U = unit * 32 <= 110 * 1024   ? 32
+                           : unit * 16 <= 110 * 1024 ? 16
+                           : unit * 8 <= 226 * 1024  ? 8
+                                                     : 4;
+  // the rows of the k3 loop: one thread per (row, part of k3) where one per row leaves warps idle
+  static constexpr int parts = n * U < 128 ? 2 : 1;
+  static constexpr int threads = n * U * parts <= 128 ? 128 : (n * U * parts + 31) / 32 * 32;
+  static constexpr size_t smem_fwd = sizeof(T) * ((size_t)n3 * (U + 1) + 2 * (size_t)nym * U) + 16;
+  static constexpr size_t out_bytes = sizeof(T) * (size_t)U * (n3 | 1);
+  static constexpr size_t smem_inv =
+      2 * sizeof(T) * (size_t)nym * U > out_bytes ? 2 * sizeof(T) * (size_t)nym * U : out_bytes;
+  static constexpr int unroll = n <= 6 ? n : 1;  // the k3 loops: larger orders keep the code small
+};
+
+// The z and y transforms of row l1 of one unit, for k3 = K0, K0 + STEP, ...
+template <int n, typename T, int U, int K0, int STEP>
+__device__ __forceinline__ void fwd_row(const T* __restrict__ s, cplx_t<T>* __restrict__ y) {
   using W = Tw<n, T>;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  constexpr int m = 2 * n - 1, n2 = n * n, n3 = n2 * n, ny = n * m * n;
-  const int sin_stride = (CG * n3 + 3) & ~3;
-  T* sin_buf = sm + 2 * m;                      // 2 x CG * n3 real moments (double-buffered)
-  C2* Z = (C2*)(sin_buf + 2 * sin_stride);      // CG * n * n * n   (l1, l2, k3)
-  C2* Y = Z + CG * n3;                         // CG * n * m * n   (l1, k2, k3)
-  constexpr int nj = unif_jobs(n);
-  unsigned* s_amax = reinterpret_cast<unsigned*>(Y + CG * ny);  // [nj][8]
-  (void)twid;
-  const int tid = threadIdx.x, bd = blockDim.x;
-  if (amax)
-    for (int i = tid; i < nj * 8; i += bd) s_amax[i] = 0u;
-  // work units (cell, column group) of this CTA in order; each unit's moments
-  // are copied (cp.async) into the other buffer while the previous unit is
-  // transformed
-  const int ngrp = (C + CG - 1) / CG;
-  auto fetch = [&](int u, int buf) {
-    const int ci = blockIdx.x + (u / ngrp) * gridDim.x;
-    if (ci < ncl) {
-      const int c0 = (u % ngrp) * CG, cg = min(CG, C - c0);
-      const T* src = S_l + ((int64_t)cells[ci] * C + c0) * n3;
-      T* dst = sin_buf + buf * sin_stride;
-      for (int i = tid; i < cg * n3; i += bd) cp_async_elem(dst + i, src + i, true);
+  constexpr int m = 2 * n - 1;
+  using Cfg = FftCfg<n, T>;
+#pragma unroll Cfg::unroll
+  for (int k3 = K0; k3 < n; k3 += STEP) {
+    cplx_t<T> v[n];
+#pragma unroll
+    for (int l2 = 0; l2 < n; ++l2) {
+      T re = 0, im = 0;
+#pragma unroll
+      for (int l = 0; l < n; ++l) {
+        const T x = s[(l2 * n + l) * (U + 1)];
+        re = fma(x, W::c((k3 * l) % m), re);
+        im = fma(-x, W::s((k3 * l) % m), im);
+      }
+      v[l2] = make_cplx<T>(re, im);
     }
-    cp_async_commit();
-  };
-  int unit = 0;
-  fetch(0, 0);
-  for (int ci = blockIdx.x; ci < ncl; ci += gridDim.x) {
-  const int cell = cells[ci];
-  for (int c0 = 0; c0 < C; c0 += CG, ++unit) {
-    const int cg = min(CG, C - c0);
-    __syncthreads();  // the previous unit's readers of the other buffer are done
-    fetch(unit + 1, (unit + 1) & 1);
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    __syncthreads();
-    const T* sin_ = sin_buf + (unit & 1) * sin_stride;
-    // z: Z[c][l1][l2][k3] = sum_l3 S[c][l1][l2][l3] w^(k3 l3), real input
-    for (int job = tid; job < cg * n2; job += bd) {
-      const T* s = sin_ + job * n;
-      T x[n];
+    const int kend = k3 == 0 ? n : m;  // (k2 >= n, 0) are not kept
+    if constexpr (m == 9) {
+      dft_5_to_9<n, T>(v, [&](int k, cplx_t<T> r) {
+        if (k < kend) y[(k * n + k3) * U] = r;
+      });
+    } else {
 #pragma unroll
-      for (int l = 0; l < n; ++l) x[l] = s[l];
-      C2* z = Z + job * n;
-#pragma unroll
-      for (int k = 0; k < n; ++k) {
+      for (int k = 0; k < m; ++k) {
+        if (k >= kend) break;
         T re = 0, im = 0;
 #pragma unroll
         for (int l = 0; l < n; ++l) {
-          re = fma(x[l], W::c((k * l) % m), re);
-          im = fma(-x[l], W::s((k * l) % m), im);
+          const T c = W::c((k * l) % m), sn = W::s((k * l) % m);
+          re = fma(v[l].x, c, fma(v[l].y, sn, re));
+          im = fma(v[l].y, c, fma(-v[l].x, sn, im));
         }
-        z[k] = make_cplx<T>(re, im);
+        y[(k * n + k3) * U] = make_cplx<T>(re, im);
       }
     }
-    __syncthreads();
-    // y: Y[c][l1][k2][k3] = sum_l2 Z[c][l1][l2][k3] w^(k2 l2); job (c, l1, k3)
-    for (int job = tid; job < cg * n2; job += bd) {
-      const int k3 = job % n, l1 = (job / n) % n, cc = job / n2;
-      const C2* z = Z + cc * n3 + l1 * n2 + k3;
-      C2 v[n];
-#pragma unroll
-      for (int l = 0; l < n; ++l) v[l] = z[l * n];
-      C2* y = Y + cc * ny + l1 * m * n + k3;
-      if constexpr (m == 9) {
-        dft_5_to_9<n, T>(v, [&](int k, C2 r) { y[k * n] = r; });
-      } else {
-#pragma unroll
-        for (int k = 0; k < m; ++k) {
-          T re = 0, im = 0;
-#pragma unroll
-          for (int l = 0; l < n; ++l) {
-            const T c = W::c((k * l) % m), s = W::s((k * l) % m);
-            re = fma(v[l].x, c, fma(v[l].y, s, re));
-            im = fma(v[l].y, c, fma(-v[l].x, s, im));
-          }
-          y[k * n] = make_cplx<T>(re, im);
-        }
-      }
-    }
-    __syncthreads();
-    // x: X[k1][k2][k3][c] = sum_l1 Y[c][l1][k2][k3] w^(k1 l1); job (j, c), c fastest
-    for (int job = tid; job < cg * nj; job += bd) {
-      const int cc = job % cg, j = job / cg;
-      int k2, k3;
-      unif_job(n, j, &k2, &k3);
-      const C2* y = Y + cc * ny + k2 * n + k3;
-      C2 v[n];
-#pragma unroll
-      for (int l = 0; l < n; ++l) v[l] = y[l * m * n];
-      C2* out = X_l + ((int64_t)(j * m) * ncells + cell) * C + c0 + cc;
-      if constexpr (sizeof(T) == 4) {
-        if (amax) {  // |X_k1| <= sum_l |v_l| <= sum_l (|re| + |im|) for every k1
-          float bnd = 0.f;
-#pragma unroll
-          for (int l = 0; l < n; ++l) bnd += fabsf(v[l].x) + fabsf(v[l].y);
-          atomicMax(&s_amax[j * 8 + ((c0 + cc) & 7)], __float_as_uint(bnd));
-        }
-      }
-      const int64_t kstride = ncells * C;
-      const int kend = j == nj - 1 ? n : m;  // (0, 0): the rest are conjugates
-      if constexpr (m == 9) {
-        dft_5_to_9<n, T>(v, [&](int k, C2 r) {
-          if (k < kend) out[k * kstride] = r;
-        });
-      } else {
-#pragma unroll
-        for (int k = 0; k < m; ++k) {
-          T re = 0, im = 0;
-#pragma unroll
-          for (int l = 0; l < n; ++l) {
-            const T c = W::c((k * l) % m), s = W::s((k * l) % m);
-            re = fma(v[l].x, c, fma(v[l].y, s, re));
-            im = fma(v[l].y, c, fma(-v[l].x, s, im));
-          }
-          if (k < kend) out[k * kstride] = make_cplx<T>(re, im);
-        }
-      }
-    }
-  }
-  }
-  cp_async_wait_all();  // the (empty) prefetch past the last unit
-  if (amax) {
-    __syncthreads();
-    for (int i = tid; i < nj * 8; i += bd)
-      if (s_amax[i]) atomicMax(&amax[i], s_amax[i]);
   }
 }
 
-// Inverse: one CTA per nonempty target cell.  F = scale * IDFT(Y)/P at grid
-// positions (a + n) mod m; (a + ib) e^{+2 pi i j / m} = (a c - b s) + i (b c + a s).
-template <int n, typename T>
-__global__ void k_fft_inv(const int* __restrict__ cells, const cplx_t<T>* __restrict__ Y_l,
-                          T* __restrict__ F_l, int64_t ncells, int C, int CG,
-                          const T* __restrict__ twid, T invP, T scale) {
+// w = e^{-2 pi i / m}; (a + ib) w^j = (a c + b s) + i (b c - a s).
+// Units of a CTA: U consecutive (cell, column) pairs of the nonempty source
+// cells; spectra to X[(slot ncells + cell) C + column].  SPLIT (tensor-core
+// levels, one group of 8 columns from c0): units are U / 4 (parent, column)
+// rows x 4 children of one half of the children; spectra scaled by 2^s with s
+// from the column's bound, split into F16 hi and lo and stored in the layout
+// of the tensor-core MAC (UnifPlanes); zeros for empty cells.
+template <int n, typename T, bool SPLIT>
+__global__ void __launch_bounds__(FftCfg<n, T>::threads)
+    k_fft_fwd(const FftFwdArgs<T> a) {
   using C2 = cplx_t<T>;
   using W = Tw<n, T>;
+  using Cfg = FftCfg<n, T>;
+  constexpr int m = Cfg::m, n2 = n * n, n3 = Cfg::n3, U = Cfg::U, nj = unif_jobs(n);
   extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  constexpr int m = 2 * n - 1, n2 = n * n, n3 = n2 * n, ng = n * m * n;
-  constexpr int nj = unif_jobs(n), nk = (nj - 1) * m + n;
-  C2* Yh = (C2*)(sm + ((2 * m + 3) & ~3));  // CG * nk   (slots)
-  C2* G = Yh + CG * nk;                     // CG * n*m*n (a1, k2, k3)
-  C2* H = G + CG * ng;                      // CG * n3    (a1, a2, k3)
-  (void)twid;
-  const int cell = cells[blockIdx.x];
-  const int tid = threadIdx.x, bd = blockDim.x;
-  for (int c0 = 0; c0 < C; c0 += CG) {
-    const int cg = min(CG, C - c0);
-    __syncthreads();
-    for (int i = tid; i < cg * nk; i += bd) {
-      const int k = i / cg, cc = i % cg;
-      cp_async_cplx(&Yh[cc * nk + k], &Y_l[((int64_t)k * ncells + cell) * C + c0 + cc], true);
+  C2* Y = reinterpret_cast<C2*>(smraw);                        // [l1][k2][k3][U]
+  T* S = reinterpret_cast<T*>(Y + (size_t)Cfg::nym * U);       // [n^3][U + 1]
+  __shared__ int64_t s_src[U];                                 // unit: its moments, or -1
+  const int tid = threadIdx.x, u = tid % U, job0 = tid / U;
+  constexpr int JS = Cfg::threads / U;
+  int64_t dst = 0;  // this thread's unit: first output
+  bool has = false, inside = true;
+  int col = 0;  // SPLIT: its column of the group
+  if constexpr (SPLIT) {
+    // group: kplane = blockIdx.x & 1, rows (blockIdx.x >> 1) U / 4 ...
+    const int kp = blockIdx.x & 1, e = u & 3;
+    const int64_t row = (int64_t)(blockIdx.x >> 1) * (U / 4) + (u >> 2);
+    const int S_ = a.side, c = (int)(row % 8);
+    const int z = (int)(row / 8 % S_), y = (int)(row / 8 / S_ % S_), x = (int)(row / 8 / S_ / S_);
+    inside = x < S_;
+    col = c;
+    if (inside) {
+      const int64_t cell = 8 * (int64_t)morton_encode(x, y, z) + 4 * kp + e;
+      has = a.occ[cell] != 0;
+      dst = UnifPlanes::row_byte(S_, x, kp, y, z, c) + 4 * e;
+      if (job0 == 0) s_src[u] = has ? (cell * a.C + a.c0 + c) * n3 : -1;
+    } else if (job0 == 0) {
+      s_src[u] = -1;
+    }
+  } else {
+    const int64_t g = (int64_t)blockIdx.x * U + u;
+    has = g < a.nunits;
+    if (has) {
+      const int64_t cell = a.cells[g / a.C];
+      dst = cell * a.C + g % a.C;
+    }
+    if (job0 == 0) s_src[u] = has ? dst * n3 : -1;
+  }
+  const bool any = __syncthreads_or(has);
+  if (any) {
+    for (int i = tid; i < U * n3; i += Cfg::threads) {
+      const int v = i / n3, l = i % n3;
+      const int64_t o = s_src[v];
+      cp_async_elem(&S[l * (U + 1) + v], a.S + (o >= 0 ? o + l : 0), o >= 0);
     }
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    // x: G[c][a1][k2][k3] = sum_k1 Yh[c][k1][k2][k3] e^{+2 pi i k1 t1 / m}; job (c, j)
-    for (int job = tid; job < cg * nj; job += bd) {
-      const int j = job % nj, cc = job / nj;
+    for (int job = job0; job < n * Cfg::parts; job += JS) {
+      const int l1 = job % n;
+      const T* s = S + l1 * n2 * (U + 1) + u;
+      C2* y = Y + l1 * m * n * U + u;
+      if constexpr (Cfg::parts == 1)
+        fwd_row<n, T, U, 0, 1>(s, y);
+      else if (job < n)
+        fwd_row<n, T, U, 0, 2>(s, y);
+      else
+        fwd_row<n, T, U, 1, 2>(s, y);
+    }
+    __syncthreads();
+  }
+  float sc = 1.f;
+  if constexpr (SPLIT) {
+    if (!inside) return;
+    sc = exp2i(unif_scale_exp(a.amax[col]));
+  } else {
+    if (!has) return;
+  }
+  for (int j = job0; j < nj; j += JS) {
+    const int kend = j == nj - 1 ? n : m;  // (0, 0): the rest are conjugates
+    C2 v[n];
+    if (any) {
       int k2, k3;
       unif_job(n, j, &k2, &k3);
-      const C2* y = Yh + cc * nk + j * m;
+      const C2* y = Y + (k2 * n + k3) * U + u;
+#pragma unroll
+      for (int l = 0; l < n; ++l) v[l] = y[l * m * n * U];
+    } else {
+#pragma unroll
+      for (int l = 0; l < n; ++l) v[l] = make_cplx<T>(T(0), T(0));
+    }
+    auto put = [&](int k, C2 r) {
+      if (k >= kend) return;
+      if constexpr (SPLIT) {
+        const float x0 = r.x * sc, x1 = r.y * sc;
+        const __half2 h = __floats2half2_rn(x0, x1);
+        const float2 hf = __half22float2(h);
+        const __half2 l = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
+        unsigned char* p = reinterpret_cast<unsigned char*>(a.X) + (j * m + k) * a.slot_stride + dst;
+        *reinterpret_cast<__half2*>(p) = h;
+        *reinterpret_cast<__half2*>(p + a.lo_off) = l;
+      } else {
+        a.X[(j * m + k) * a.slot_stride + dst] = r;
+      }
+    };
+    if constexpr (m == 9) {
+      dft_5_to_9<n, T>(v, put);
+    } else {
+#pragma unroll
+      for (int k = 0; k < m; ++k) {
+        T re = 0, im = 0;
+#pragma unroll
+        for (int l = 0; l < n; ++l) {
+          const T c = W::c((k * l) % m), s = W::s((k * l) % m);
+          re = fma(v[l].x, c, fma(v[l].y, s, re));
+          im = fma(v[l].y, c, fma(-v[l].x, s, im));
+        }
+        put(k, make_cplx<T>(re, im));
+      }
+    }
+  }
+}
+
+// F = scale * IDFT(Y)/P at grid positions (a + n) mod m;
+// (a + ib) e^{+2 pi i j / m} = (a c - b s) + i (b c + a s).
+// Units: U consecutive (cell, column) pairs of the nonempty target cells,
+// Y[(slot ncells + cell) C + column]; SPLIT: U consecutive (parent, column)
+// rows of one child, Y as the tensor-core MAC writes it (UnifPlanes).
+template <int n, typename T, bool SPLIT>
+__global__ void __launch_bounds__(FftCfg<n, T>::threads)
+    k_fft_inv(const FftInvArgs<T> a) {
+  using C2 = cplx_t<T>;
+  using W = Tw<n, T>;
+  using Cfg = FftCfg<n, T>;
+  constexpr int m = Cfg::m, n2 = n * n, n3 = Cfg::n3, U = Cfg::U, nj = unif_jobs(n);
+  constexpr int OP = n3 | 1;  // pitch of a unit's outputs
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C2* G = reinterpret_cast<C2*>(smraw);  // [a1][k2][k3][U]
+  T* O = reinterpret_cast<T*>(smraw);    // [U][OP], after G
+  __shared__ int64_t s_dst[U];           // unit: its locals, or -1
+  const int tid = threadIdx.x, u = tid % U, job0 = tid / U;
+  constexpr int JS = Cfg::threads / U;
+  int64_t src = 0;
+  bool has;
+  if constexpr (SPLIT) {
+    const int t = blockIdx.x & 7, S_ = a.side;
+    const int64_t row = (int64_t)(blockIdx.x >> 3) * U + u;
+    const int c = (int)(row % 8);
+    const int z = (int)(row / 8 % S_), y = (int)(row / 8 / S_ % S_), x = (int)(row / 8 / S_ / S_);
+    has = x < S_;
+    int64_t cell = 0;
+    if (has) {
+      cell = 8 * (int64_t)morton_encode(x, y, z) + t;
+      has = a.occ[cell] != 0;
+      src = UnifPlanes::out_index(S_, x, t, y, z, c);
+    }
+    if (job0 == 0) s_dst[u] = has ? (cell * a.C + a.c0 + c) * n3 : -1;
+  } else {
+    const int64_t g = (int64_t)blockIdx.x * U + u;
+    has = g < a.nunits;
+    if (has) src = (int64_t)a.cells[g / a.C] * a.C + g % a.C;
+    if (job0 == 0) s_dst[u] = has ? src * n3 : -1;
+  }
+  if (!__syncthreads_or(has)) return;
+  if (has) {
+    // x: G[a1][k2][k3] = sum_k1 Y[k1][k2][k3] e^{+2 pi i k1 t1 / m}
+    for (int j = job0; j < nj; j += JS) {
+      int k2, k3;
+      unif_job(n, j, &k2, &k3);
+      const C2* y = a.Y + (int64_t)j * m * a.slot_stride + src;
       C2 v[m];
 #pragma unroll
       for (int k = 0; k < m; ++k) {
         const bool mirror = j == nj - 1 && k >= n;  // Y(-k1, 0, 0) = conj Y(k1, 0, 0)
-        v[k] = y[mirror ? m - k : k];
+        v[k] = y[(mirror ? m - k : k) * a.slot_stride];
         if (mirror) v[k].y = -v[k].y;
       }
-      C2* g = G + cc * ng + k2 * n + k3;
+      C2* g = G + (k2 * n + k3) * U + u;
       if constexpr (m == 9) {
-        idft_9_to_5<n, T>(v, [&](int a, C2 r) { g[a * m * n] = r; });
+        idft_9_to_5<n, T>(v, [&](int q, C2 r) { g[q * m * n * U] = r; });
       } else {
 #pragma unroll
-        for (int a = 0; a < n; ++a) {
-          const int t = (a + n) % m;
+        for (int q = 0; q < n; ++q) {
+          const int t = (q + n) % m;
           T re = 0, im = 0;
 #pragma unroll
           for (int k = 0; k < m; ++k) {
@@ -378,29 +452,44 @@ __global__ void k_fft_inv(const int* __restrict__ cells, const cplx_t<T>* __rest
             re = fma(v[k].x, c, fma(-v[k].y, s, re));
             im = fma(v[k].y, c, fma(v[k].x, s, im));
           }
-          g[a * m * n] = make_cplx<T>(re, im);
+          g[q * m * n * U] = make_cplx<T>(re, im);
         }
       }
     }
-    __syncthreads();
-    // y: H[c][a1][a2][k3] = sum_k2 G[c][a1][k2][k3] e^{+2 pi i k2 t2 / m}; job (c, a1, k3)
-    for (int job = tid; job < cg * n2; job += bd) {
-      const int k3 = job % n, a1 = (job / n) % n, cc = job / n2;
-      const C2* g = G + cc * ng + a1 * m * n + k3;
+  }
+  __syncthreads();
+  // y and z of row a1: H[a2][k3] = sum_k2 G[a1][k2][k3] e^{+2 pi i k2 t2 / m},
+  // out = Re H[..][0] + 2 sum_{k3>=1} Re(H[..][k3] e^{+2 pi i k3 t3 / m})
+  T acc[n][n];
+  const bool row = job0 < n && has;
+  if (row) {
+    const C2* g = G + job0 * m * n * U + u;
+#pragma unroll Cfg::unroll
+    for (int k3 = 0; k3 < n; ++k3) {
       C2 v[m];
 #pragma unroll
       for (int k = 0; k < m; ++k) {
         const bool mirror = k3 == 0 && k >= n;  // G(-k2, 0) = conj G(k2, 0)
-        v[k] = g[(mirror ? m - k : k) * n];
+        v[k] = g[((mirror ? m - k : k) * n + k3) * U];
         if (mirror) v[k].y = -v[k].y;
       }
-      C2* h = H + cc * n3 + a1 * n2 + k3;
+      auto add = [&](int q, C2 h) {
+#pragma unroll
+        for (int a3 = 0; a3 < n; ++a3) {
+          const int t = (a3 + n) % m;
+          if (k3 == 0)
+            acc[q][a3] = h.x;
+          else
+            acc[q][a3] = fma(T(2), fma(h.x, W::c((k3 * t) % m), -h.y * W::s((k3 * t) % m)),
+                             acc[q][a3]);
+        }
+      };
       if constexpr (m == 9) {
-        idft_9_to_5<n, T>(v, [&](int a, C2 r) { h[a * n] = r; });
+        idft_9_to_5<n, T>(v, add);
       } else {
 #pragma unroll
-        for (int a = 0; a < n; ++a) {
-          const int t = (a + n) % m;
+        for (int q = 0; q < n; ++q) {
+          const int t = (q + n) % m;
           T re = 0, im = 0;
 #pragma unroll
           for (int k = 0; k < m; ++k) {
@@ -408,29 +497,24 @@ __global__ void k_fft_inv(const int* __restrict__ cells, const cplx_t<T>* __rest
             re = fma(v[k].x, c, fma(-v[k].y, s, re));
             im = fma(v[k].y, c, fma(v[k].x, s, im));
           }
-          h[a * n] = make_cplx<T>(re, im);
+          add(q, make_cplx<T>(re, im));
         }
       }
     }
-    __syncthreads();
-    // z (complex to real over the Hermitian half):
-    // out = Re H[..][0] + 2 sum_{k3>=1} Re(H[..][k3] e^{+2 pi i k3 t3 / m}); job (c, a1, a2)
-    for (int job = tid; job < cg * n2; job += bd) {
-      const C2* h = H + job * n;
-      C2 v[n];
+  }
+  __syncthreads();
+  if (row) {
+    T* o = O + u * OP + job0 * n2;
 #pragma unroll
-      for (int k = 0; k < n; ++k) v[k] = h[k];
-      T* out = F_l + ((int64_t)cell * C + c0) * n3 + job * n;
+    for (int q = 0; q < n; ++q)
 #pragma unroll
-      for (int a = 0; a < n; ++a) {
-        const int t = (a + n) % m;
-        T acc = v[0].x;
-#pragma unroll
-        for (int k = 1; k < n; ++k)
-          acc = fma(T(2), fma(v[k].x, W::c((k * t) % m), -v[k].y * W::s((k * t) % m)), acc);
-        out[a] = scale * (acc * invP);
-      }
-    }
+      for (int a3 = 0; a3 < n; ++a3) o[q * n + a3] = a.scale * (acc[q][a3] * a.invP);
+  }
+  __syncthreads();
+  for (int i = tid; i < U * n3; i += Cfg::threads) {
+    const int v = i / n3, l = i % n3;
+    const int64_t o = s_dst[v];
+    if (o >= 0) a.F[o + l] = O[v * OP + l];
   }
 }
 
@@ -729,51 +813,82 @@ struct MacLevel {
   }
 };
 
-template <typename T>
-struct FftLaunch {
-  pbbfmm_tree* t;
-  int C, CGf, CGi;
-  size_t smem_f, smem_i;
-  double invP;
+template <typename T, bool SPLIT>
+struct FftFwdLaunch {
+  FftFwdArgs<T> a;
+  int64_t groups4;  // SPLIT: (parent, column) rows of the level
   cudaStream_t st;
-  int level = 2;
-  bool inverse = false;
-  double scale = 1.0;
-  unsigned* amax = nullptr;  // forward: spectra maxima of the level (tensor-core MAC)
   template <int N>
   int run() {
-    const int n3 = N * N * N, nk = t->nk;
-    Workspace& ws = t->ws;
-    const int* lists = ws.lists.as<int>();
-    const int64_t perS = (int64_t)C * n3, perX = (int64_t)nk * C;
-    const int l = level;
-    const T* twid = sizeof(T) == 8 ? (const T*)t->d_twid : (const T*)t->f_twid;
-    if (!inverse) {
-      PB_CUDA(cudaFuncSetAttribute(k_fft_fwd<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem_f));
-      // CTAs loop over the cells: as many as fit on the GPU at once
-      int per_sm = 1, dev = 0, nsm = 148;
-      PB_CUDA(cudaGetDevice(&dev));
-      PB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-      PB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft_fwd<N, T>, 128, smem_f));
-      const int ncl = t->lists.nsrc[l];
-      const int grid = std::max(1, std::min(ncl, std::max(1, per_sm) * nsm));
-      k_fft_fwd<N, T><<<grid, 128, smem_f, st>>>(
-          lists + t->lists.src_off[l], ncl, ws.S.as<T>() + level_offset(l, perS),
-          ws.proxy.as<cplx_t<T>>() + level_offset(l, perX), cells_at(l), C, CGf, twid, amax);
-      PB_LAUNCH("fft_fwd");
-    } else {
-      PB_CUDA(cudaFuncSetAttribute(k_fft_inv<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem_i));
-      k_fft_inv<N, T><<<t->lists.ntgt[l], 128, smem_i, st>>>(
-          lists + t->lists.tgt_off[l], ws.pf.as<cplx_t<T>>() + level_offset(l, perX),
-          ws.F.as<T>() + level_offset(l, perS), cells_at(l), C, CGi, twid, (T)invP, (T)scale);
-      PB_LAUNCH("fft_inv");
-    }
+    using Cfg = FftCfg<N, T>;
+    const int64_t grid = SPLIT ? 2 * ((groups4 + Cfg::U / 4 - 1) / (Cfg::U / 4))
+                               : (a.nunits + Cfg::U - 1) / Cfg::U;
+    auto kern = k_fft_fwd<N, T, SPLIT>;
+    PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)Cfg::smem_fwd));
+    kern<<<(unsigned)grid, Cfg::threads, Cfg::smem_fwd, st>>>(a);
+    PB_LAUNCH("fft_fwd");
     return PBBFMM_OK;
   }
 };
 
+template <typename T, bool SPLIT>
+struct FftInvLaunch {
+  FftInvArgs<T> a;
+  int64_t rows;  // SPLIT: (parent, column) rows of the level
+  cudaStream_t st;
+  template <int N>
+  int run() {
+    using Cfg = FftCfg<N, T>;
+    const int64_t grid = SPLIT ? 8 * ((rows + Cfg::U - 1) / Cfg::U) : (a.nunits + Cfg::U - 1) / Cfg::U;
+    auto kern = k_fft_inv<N, T, SPLIT>;
+    PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)Cfg::smem_inv));
+    kern<<<(unsigned)grid, Cfg::threads, Cfg::smem_inv, st>>>(a);
+    PB_LAUNCH("fft_inv");
+    return PBBFMM_OK;
+  }
+};
+
+// Largest sum over a cell and column of |moments|, per column of the group
+// (float bits): a bound on |re| and |im| of its spectra.  Warps over cells.
+__global__ void k_moment_bound(const int* __restrict__ cells, int ncl, const float* __restrict__ S,
+                               int C, int c0, int n3, uint32_t* __restrict__ amax) {
+  const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
+  float mx[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) mx[c] = 0.f;
+  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < ncl; i += nw) {
+    const float* s = S + ((int64_t)cells[i] * C + c0) * n3;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      float v = 0.f;
+      for (int l = lane; l < n3; l += 32) v += fabsf(s[c * n3 + l]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      mx[c] = fmaxf(mx[c], v);
+    }
+  }
+  if (lane == 0)
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (mx[c] > 0.f) atomicMax(&amax[c], __float_as_uint(mx[c]));
+}
+
+// Bytes of the spectra arrays X and Y (one level at a time uses them).
+void unif_spectra_bytes(const pbbfmm_tree* t, int C, bool f64, size_t* x, size_t* y) {
+  *x = *y = 16;
+  for (int l = 2; l <= t->p.tree_level; ++l) {
+    const bool tc = !f64 && unif_tc_eligible(t, l, C);
+    const size_t plain = (size_t)cells_at(l) * C * t->nk * (f64 ? 16 : 8);
+    const int S = 1 << (l - 1);
+    *x = std::max(*x, tc ? (size_t)t->nk * UnifPlanes::slot_bytes(S) : plain);
+    *y = std::max(*y, tc ? (size_t)t->nk * UnifPlanes::slot_outputs(S) * sizeof(float2) : plain);
+  }
+}
+
+// Level by level: forward transforms, MAC, inverse transforms (the spectra
+// arrays hold one level at a time).
 template <typename T>
 static int run_m2l_unif_t(pbbfmm_tree* t, int C, cudaStream_t st) {
   if (int rc = init_fft_twiddles()) return rc;
@@ -782,73 +897,104 @@ static int run_m2l_unif_t(pbbfmm_tree* t, int C, cudaStream_t st) {
   Workspace& ws = t->ws;
   C2* X = ws.proxy.as<C2>();
   C2* Y = ws.pf.as<C2>();
+  const int* lists = ws.lists.as<int>();
   const int* sstart = ws.sstart_p;
   const int* tstart = ws.tstart.as<int>();
-  const int64_t perX = (int64_t)nk * C;
-  const double invP = 1.0 / (double)(m * m * m);
-  const int ts = (int)sizeof(T);
-  // forward transforms of all nonempty source cells, levels 2..L
-  const int fwd_col = n3 * ts + n3 * 2 * ts + n * m * n * 2 * ts;
-  const int CGf = max(1, min(C, 60000 / fwd_col));
-  const size_t smem_f = (size_t)ts * (2 * m + 2 * ((CGf * n3 + 3) & ~3)) +
-                        (size_t)2 * ts * (CGf * n3 + CGf * n * m * n) + (size_t)4 * unif_jobs(n) * 8;
-  const int inv_col = (nk + n * m * n + n3) * 2 * ts;
-  const int CGi = max(1, min(C, 60000 / inv_col));
-  const size_t smem_i = (size_t)ts * ((2 * m + 3) & ~3) +
-                        (size_t)2 * ts * (CGi * nk + CGi * n * m * n + CGi * n3);
-  FftLaunch<T> fl{t, C, CGf, CGi, smem_f, smem_i, invP, st};
-  // spectra maxima per level for the tensor-core MAC's scaling (float path)
-  const size_t amax_per = (size_t)unif_jobs(n) * 8;
-  bool any_tc = false;
-  for (int l = 2; l <= L; ++l) any_tc |= sizeof(T) == 4 && unif_tc_eligible(t, l, C);
-  if (any_tc) {
-    if (int rc_ = grow(ws.amax, (size_t)(L + 1) * amax_per * sizeof(unsigned))) return rc_;
-    PB_CUDA(cudaMemsetAsync(ws.amax.p, 0, (size_t)(L + 1) * amax_per * sizeof(unsigned), st));
-  }
-  auto amax_at = [&](int l) -> unsigned* {
-    return sizeof(T) == 4 && unif_tc_eligible(t, l, C) ? ws.amax.as<unsigned>() + l * amax_per
-                                                       : nullptr;
-  };
-  for (int l = 2; l <= L; ++l) {
-    if (t->lists.nsrc[l] == 0) continue;
-    if (int rc_ = kt_begin(t, KS_FFT_FWD, st)) return rc_;
-    fl.level = l;
-    fl.inverse = false;
-    fl.amax = amax_at(l);
-    if (int rc_ = dispatch_order(n, fl)) return rc_;
-    if (int rc_ = kt_end(t, st)) return rc_;
-  }
   int* halo = ws.halo.as<int>();
   const OpsView<T> ov = ops_view<T>(t);
-  for (int l = 2; l <= L; ++l) {
+  int rc;
+  for (int l = L; l >= 2; --l) {
     if (t->lists.ntgt[l] == 0) continue;
     const int lvl = t->homog ? 0 : l - 2;
-    const C2* op = ov.op + (int64_t)lvl * nk * kKaraD * kKaraJ;
     const int span = (int)cells_at(L - l);
-    int rc;
-    if ((rc = kt_begin(t, KS_MAC, st))) return rc;
-    const C2* Xl = X + level_offset(l, perX);
-    C2* Yl = Y + level_offset(l, perX);
-    // float32, 16 parents per side or more, columns in groups of 8: the
-    // tensor cores (m2l_unif_tc.cu); otherwise the CUDA cores
-    if (sizeof(T) == 4 && unif_tc_eligible(t, l, C)) {
-      rc = run_m2l_unif_tc_level(t, C, l, lvl, reinterpret_cast<const float2*>(Xl),
-                                 reinterpret_cast<float2*>(Yl), amax_at(l), st);
-    } else {
-      MacLevel<T> ml{Xl, Yl, op, halo, sstart, tstart, span, l, C, nk, st};
-      rc = ml.columns();
-    }
-    if (rc) return rc;
-    if ((rc = kt_end(t, st))) return rc;
+    const T* S_l = ws.S.as<T>() + level_offset(l, (int64_t)C * n3);
+    T* F_l = ws.F.as<T>() + level_offset(l, (int64_t)C * n3);
     double len = t->p.L;
     for (int i = 0; i < l; ++i) len = 0.5 * len;
-    const double scale = pow(1.0 / len, t->homogen_neg);
-    if (int rc_ = kt_begin(t, KS_FFT_INV, st)) return rc_;
-    fl.level = l;
-    fl.inverse = true;
-    fl.scale = scale;
-    if (int rc_ = dispatch_order(n, fl)) return rc_;
-    if (int rc_ = kt_end(t, st)) return rc_;
+    const T scale = (T)pow(1.0 / len, t->homogen_neg), invP = (T)(1.0 / (double)(m * m * m));
+    // float32, 16 parents per side or more, columns in groups of 8: the
+    // tensor cores (m2l_unif_tc.cu); otherwise the CUDA cores
+    if constexpr (sizeof(T) == 4) {
+      if (unif_tc_eligible(t, l, C)) {
+        const int S = 1 << (l - 1);
+        uint8_t *socc, *tocc;
+        if ((rc = kt_begin(t, KS_MAC, st))) return rc;
+        if ((rc = run_unif_tc_occupancy(t, l, &socc, &tocc, st))) return rc;
+        if ((rc = kt_end(t, st))) return rc;
+        for (int c0 = 0; c0 < C; c0 += 8) {
+          uint32_t* amax = ws.amax.as<uint32_t>();
+          if ((rc = kt_begin(t, KS_FFT_FWD, st))) return rc;
+          PB_CUDA(cudaMemsetAsync(amax, 0, 8 * sizeof(uint32_t), st));
+          if (t->lists.nsrc[l] > 0) {
+            k_moment_bound<<<std::min((t->lists.nsrc[l] + 7) / 8, 4 * 148), 256, 0, st>>>(
+                lists + t->lists.src_off[l], t->lists.nsrc[l], S_l, C, c0, n3, amax);
+            PB_LAUNCH("moment_bound");
+          }
+          if ((rc = run_unif_tc_borders(t, S, reinterpret_cast<unsigned char*>(X), st))) return rc;
+          const int64_t rows = (int64_t)S * S * S * 8;
+          FftFwdLaunch<T, true> f{{}, rows, st};
+          f.a.S = S_l;
+          f.a.X = X;
+          f.a.slot_stride = UnifPlanes::slot_bytes(S);
+          f.a.lo_off = UnifPlanes::lo_off(S);
+          f.a.C = C;
+          f.a.c0 = c0;
+          f.a.side = S;
+          f.a.occ = socc;
+          f.a.amax = amax;
+          if ((rc = dispatch_order(n, f))) return rc;
+          if ((rc = kt_end(t, st))) return rc;
+          if ((rc = kt_begin(t, KS_MAC, st))) return rc;
+          if ((rc = run_m2l_unif_tc_level(t, l, lvl, reinterpret_cast<unsigned char*>(X),
+                                          reinterpret_cast<float2*>(Y), amax, tocc, st)))
+            return rc;
+          if ((rc = kt_end(t, st))) return rc;
+          if ((rc = kt_begin(t, KS_FFT_INV, st))) return rc;
+          FftInvLaunch<T, true> g{{}, rows, st};
+          g.a.Y = Y;
+          g.a.F = F_l;
+          g.a.slot_stride = UnifPlanes::slot_outputs(S);
+          g.a.C = C;
+          g.a.c0 = c0;
+          g.a.side = S;
+          g.a.occ = tocc;
+          g.a.scale = scale;
+          g.a.invP = invP;
+          if ((rc = dispatch_order(n, g))) return rc;
+          if ((rc = kt_end(t, st))) return rc;
+        }
+        continue;
+      }
+    }
+    if (t->lists.nsrc[l] > 0) {
+      if ((rc = kt_begin(t, KS_FFT_FWD, st))) return rc;
+      FftFwdLaunch<T, false> f{{}, 0, st};
+      f.a.S = S_l;
+      f.a.X = X;
+      f.a.slot_stride = cells_at(l) * C;
+      f.a.C = C;
+      f.a.cells = lists + t->lists.src_off[l];
+      f.a.nunits = (int64_t)t->lists.nsrc[l] * C;
+      if ((rc = dispatch_order(n, f))) return rc;
+      if ((rc = kt_end(t, st))) return rc;
+    }
+    if ((rc = kt_begin(t, KS_MAC, st))) return rc;
+    MacLevel<T> ml{X, Y, ov.op + (int64_t)lvl * nk * kKaraD * kKaraJ, halo, sstart, tstart,
+                   span, l, C, nk, st};
+    if ((rc = ml.columns())) return rc;
+    if ((rc = kt_end(t, st))) return rc;
+    if ((rc = kt_begin(t, KS_FFT_INV, st))) return rc;
+    FftInvLaunch<T, false> g{{}, 0, st};
+    g.a.Y = Y;
+    g.a.F = F_l;
+    g.a.slot_stride = cells_at(l) * C;
+    g.a.C = C;
+    g.a.cells = lists + t->lists.tgt_off[l];
+    g.a.nunits = (int64_t)t->lists.ntgt[l] * C;
+    g.a.scale = scale;
+    g.a.invP = invP;
+    if ((rc = dispatch_order(n, g))) return rc;
+    if ((rc = kt_end(t, st))) return rc;
   }
   return PBBFMM_OK;
 }
