@@ -383,7 +383,7 @@ static std::vector<int> m2l_offsets(const int* Ktable) {
 }
 
 static void free_adjoint_ops(pbbfmm_tree* t) {
-  double** d[] = {&t->adj.E, &t->adj.U, &t->adj.VT};
+  double** d[] = {&t->adj.E, &t->adj.U, &t->adj.VT, &t->adj.Ek};
   for (double** b : d) {
     if (*b) cudaFree(*b);
     *b = nullptr;
@@ -452,6 +452,7 @@ static int build_adjoint_ops(pbbfmm_tree* t) {
 // Exchange the forward and adjoint Chebyshev operator sets (an involution).
 static void swap_adjoint_ops(pbbfmm_tree* t) {
   std::swap(t->d_E, t->adj.E);
+  std::swap(t->d_Ek, t->adj.Ek);
   std::swap(t->d_U, t->adj.U);
   std::swap(t->d_VT, t->adj.VT);
   std::swap(t->f_E, t->adj.fE);
@@ -469,6 +470,8 @@ static int upload_operators(pbbfmm_tree* t) {
   }
   PB_CUDA(cudaSetDevice(t->device));
   free_adjoint_ops(t);  // rebuilt from the new operators on the next adjoint
+  if (t->d_Ek) cudaFree(t->d_Ek);  // and the combined ones on the next compute
+  t->d_Ek = nullptr;
   int rc;
   if ((rc = ensure_tc_err_flag(t))) return rc;
   if (t->p.use_chebyshev) {
@@ -502,7 +505,7 @@ static int upload_operators(pbbfmm_tree* t) {
 
 static void free_tree_device(pbbfmm_tree* t) {
   double** bufs[] = {&t->d_Tkz, &t->d_Kw, &t->d_Cw, &t->d_E,  &t->d_U,
-                     &t->d_VT,  &t->d_op, &t->d_twid, &t->d_kparam};
+                     &t->d_VT,  &t->d_op, &t->d_twid, &t->d_kparam, &t->d_Ek};
   for (double** b : bufs) {
     if (*b) cudaFree(*b);
     *b = nullptr;
@@ -528,7 +531,7 @@ static void free_tree_device(pbbfmm_tree* t) {
                    &ws.tperm,     &ws.sperm, &ws.tstart,  &ws.sstart,     &ws.tpos,
                    &ws.spos,      &ws.wsorted, &ws.cub_temp, &ws.lists,    &ws.dcounts,
                    &ws.S,         &ws.F,     &ws.proxy,   &ws.pf,         &ws.io_tgt,
-                   &ws.io_src,    &ws.io_w,  &ws.io_out, &ws.halo, &ws.tc_proxy, &ws.m2l_part, &ws.leafpart,
+                   &ws.io_src,    &ws.io_w,  &ws.io_out, &ws.halo, &ws.tc_proxy, &ws.m2l_part, &ws.kara_x, &ws.kara_y, &ws.leafpart,
                    &ws.occ,       &ws.amax};
   for (DevBuf* b : all) release(*b);
   if (ws.h_in) cudaFreeHost(ws.h_in);
@@ -789,7 +792,9 @@ static int create_tree(const pbbfmm_tree_params* params, const pbbfmm_user_kerne
       delete t;
       return rc;
     }
-    std::vector<int> offs = m2l_offsets(t->w.Ktable);
+    std::vector<int> offs = m2l_offsets(t->w.Ktable), terms;
+    cheb_kara_tables(t->w.Ktable, &offs, &terms);
+    offs.insert(offs.end(), terms.begin(), terms.end());
     cudaError_t e = cudaMalloc(&t->d_offs, offs.size() * sizeof(int));
     if (e == cudaSuccess)
       e = cudaMemcpy(t->d_offs, offs.data(), offs.size() * sizeof(int), cudaMemcpyHostToDevice);

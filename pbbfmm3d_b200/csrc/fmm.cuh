@@ -12,6 +12,11 @@
 namespace pbbfmm {
 
 constexpr int kMaxLevel = 10;
+// Toeplitz products over the child coordinates with three products per
+// coordinate instead of four: combinations of a parent's children and parent
+// offsets D != 0 (uniform M2L: m2l_unif.cu; float64 Chebyshev M2L:
+// m2l_cheb_f64.cu)
+constexpr int kKaraJ = 27, kKaraD = 26;
 
 // Grow-only device buffer.
 struct DevBuf {
@@ -45,6 +50,7 @@ struct Workspace {
   DevBuf pf;     // Cheb: sum_l 8^l * C * rf ;  Unif: accumulated spectra of one level
   DevBuf halo;   // Unif M2L: per parent block, region and target parents and their occupancy
   DevBuf tc_proxy;  // tensor-core Cheb M2L: hi then lo proxies of one level (+ F16 exponents)
+  DevBuf kara_x, kara_y;  // float64 Cheb M2L: combined proxies and sums of dense levels
   DevBuf m2l_part;  // float64 Cheb M2L: partial sums of levels with few tiles
   DevBuf leafpart;  // leaf phase: target leaves dense-first, chunk prefix of the dense ones
   // the sources' leaf offsets, permutation and positions of the last binning
@@ -121,7 +127,10 @@ struct pbbfmm_tree {
   double* d_U = nullptr;   // Cheb: nlev x diag(Kw) U, in the same order
   double* d_VT = nullptr;  // Cheb: nlev x VT diag(Kw), in the same order
   double* d_op = nullptr;  // Unif: nlev x nk x 26 x 27 complex (unif_kara_operators)
-  int* d_offs = nullptr;   // Cheb M2L: 8 types x 189 x 4 (ox, oy, oz, op index)
+  double* d_Ek = nullptr;  // Cheb: nlev x 27 x 26 combined operators, made on first use
+  // Cheb M2L: 8 types x 189 x 4 (ox, oy, oz, op index), then the same of the
+  // combinations and their operators' terms (cheb_kara_tables)
+  int* d_offs = nullptr;
   double* d_twid = nullptr;  // Unif: cos/sin of 2 pi j / m, j < m
   double* d_kparam = nullptr;  // 4 kernel parameters
   // float32 copies of the weights and operators for the mixed path
@@ -149,7 +158,7 @@ struct pbbfmm_tree {
   // VT' = U^T, so r_f' = r_s and r_s' = r_f.  Swapped with the forward set
   // (swap_adjoint_ops) for the duration of an adjoint pass.
   struct OpSet {
-    double *E = nullptr, *U = nullptr, *VT = nullptr;
+    double *E = nullptr, *U = nullptr, *VT = nullptr, *Ek = nullptr;
     float *fE = nullptr, *fU = nullptr, *fVT = nullptr;
     pbbfmm::TcOps tc;
     int rf = 0, rs = 0;
@@ -226,8 +235,11 @@ int run_m2l_cheb(pbbfmm_tree* t, int C, cudaStream_t st);
 // transform); its proxies have rows of cheb_rsp(rs) values (zero from rs on)
 // and its matrices the fragment order
 int cheb_rsp(int rs);
+void cheb_fragment_blocks(int rf, int* nblk, int* ntb);
 std::vector<double> cheb_fragment_operators(const double* K, int64_t nblocks, int rf, int rs);
 int run_m2l_cheb_f64(pbbfmm_tree* t, int C, cudaStream_t st);
+// offsets and operator terms of the combinations of its dense levels
+void cheb_kara_tables(const int* Ktable, std::vector<int>* offs, std::vector<int>* terms);
 // tensor-core Chebyshev M2L (float path): N = rf padded to 16 must fit TMEM
 constexpr int kTcMaxN = 256;
 bool tc_eligible(const pbbfmm_tree* t);

@@ -31,6 +31,14 @@
 // ms; 33,331 targets, r = 91, 3 columns 10.8 -> 1.8 ms.  The transforms of the
 // first: 0.86 + 0.90 -> 0.21 + 0.23 ms.
 //
+// Dense levels run on combinations of the children (cheb_kara.cuh): k_kara_in
+// forms the 27 combined proxies of each source parent, the same M2L kernel sums
+// the products over the 26 parent offsets with the combined operators
+// (k_kara_ops), and k_kara_out forms the 8 children's sums: 702 products per
+// parent instead of 1512.  M2L of 33,331 targets and 77,777 sources, r = 91, 3
+// columns: 1.79 -> 1.29 ms; of the 500,000 clustered points (dense at levels 3
+// to 5): 14.7 -> 12.5 ms.
+//
 // Levels with few tiles are cut along the offsets as well (`nsplit` parts, the
 // partial sums added in order by k_m2l_parts), since one tile's 189 offsets
 // are a serial chain of ~100 us; see m2l_cheb_f64_split.
@@ -38,6 +46,7 @@
 #include <cmath>
 #include <vector>
 
+#include "cheb_kara.cuh"
 #include "fmm.cuh"
 
 namespace pbbfmm {
@@ -52,8 +61,14 @@ struct FdLevel {
   const double* proxy;  // [cell * C + col][rsp]
   double* pf;           // [cell * C + col][rf]
   double* part;         // nsplit > 1: [split][row of the level][rf]
-  const int* typed;     // targets ordered by (child type, parent)
+  const int* typed;     // targets ordered by (child type, parent); combined: target parents
+  const int* src;       // combined: nonempty source parents
+  int nsrc;
   int lev, span;
+  // 0: rows are (cell, column) of the level, types are child types, 189
+  // offsets each; 27: combined, rows are (parent, combination, column), types
+  // are the combinations, 26 parent offsets each
+  int mult;
   int item0, nsplit;
   int row0, rows;       // (target, column) rows of the level, and of the levels before it
   int first[8];         // first list position of each type
@@ -67,7 +82,7 @@ struct FdArgs {
   int C, rf, rsp;       // rsp: rs padded to a multiple of 4
   int nblk, ntb;        // column blocks, column groups of 8 per block
   const int* sstart;
-  const int* offs;      // [8][189] (ox, oy, oz, operator)
+  const int* offs;      // [8][189] (ox, oy, oz, operator), then [27][26] of the combinations
 };
 
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
@@ -142,15 +157,26 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
   const int local = (int)blockIdx.x - lv.item0;
   const int split = local % lv.nsplit, rest = local / lv.nsplit;
   const int nb = rest % a.nblk, tile = rest / a.nblk;
-  int type = 0;
-  for (int i = 1; i < 8; ++i)
-    if (tile >= lv.tile0[i]) type = i;
-  const int ntb = a.ntb;                          // column groups of a block
-  const int r0 = (tile - lv.tile0[type]) * FD_R;  // first row within the type
-  const int nrow = min(FD_R, lv.count[type] * a.C - r0);
+  const int ntb = a.ntb;  // column groups of a block
+  const int4* offs = reinterpret_cast<const int4*>(a.offs);
+  int type = 0, r0, nrow, first = 0, noff = FD_OFFS, mult = 1, comb = 0;
+  if (lv.mult) {  // tile0[0] tiles per combination
+    type = comb = tile / lv.tile0[0];
+    r0 = (tile - type * lv.tile0[0]) * FD_R;  // first row within the type
+    nrow = min(FD_R, lv.count[0] * a.C - r0);
+    offs += 8 * FD_OFFS + type * kKaraD;
+    noff = kKaraD;
+    mult = kKaraJ;
+  } else {
+    for (int i = 1; i < 8; ++i)
+      if (tile >= lv.tile0[i]) type = i;
+    r0 = (tile - lv.tile0[type]) * FD_R;
+    nrow = min(FD_R, lv.count[type] * a.C - r0);
+    first = lv.first[type];
+    offs += type * FD_OFFS;
+  }
   const int nside = 1 << lv.lev, span = lv.span;
-  const int4* offs = reinterpret_cast<const int4*>(a.offs) + type * FD_OFFS;
-  const int o_lo = FD_OFFS * split / lv.nsplit, o_hi = FD_OFFS * (split + 1) / lv.nsplit;
+  const int o_lo = noff * split / lv.nsplit, o_hi = noff * (split + 1) / lv.nsplit;
 
   const int pitch = fd_pitch(ntb);
   double* Sum = reinterpret_cast<double*>(fd_raw);  // [FD_R][pitch]
@@ -162,11 +188,11 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
     int v = -1;
     if (tid < nrow) {
       int x, y, z;
-      morton_decode((uint32_t)lv.typed[lv.first[type] + (r0 + tid) / a.C], &x, &y, &z);
+      morton_decode((uint32_t)lv.typed[first + (r0 + tid) / a.C], &x, &y, &z);
       v = (x << 20) | (y << 10) | z;
     }
     s_xyz[tid] = v;
-    s_flat[tid] = lv.first[type] * a.C + r0 + tid;
+    s_flat[tid] = first * a.C + r0 + tid;
   }
   for (int i = tid; i < FD_R * pitch / 2; i += FD_THREADS)
     reinterpret_cast<double2*>(Sum)[i] = make_double2(0.0, 0.0);
@@ -229,7 +255,7 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
     const int xyz = s_xyz[tid];
     const long long cell =
         morton_encode((xyz >> 20) + d.x, ((xyz >> 10) & 1023) + d.y, (xyz & 1023) + d.z);
-    s_src[q % SL][pos] = (cell * a.C + s_flat[tid] % a.C) * a.rsp;
+    s_src[q % SL][pos] = ((cell * mult + comb) * a.C + s_flat[tid] % a.C) * a.rsp;
     s_row[q % SL][pos] = (uint8_t)tid;
   };
   // the next iteration to load: chunk lc of valid offset lq, into stage lst.  A: granules
@@ -350,14 +376,15 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
   const int col0 = 8 * nb * ntb, ncol = min(8 * ntb, a.rf - col0);
   for (int r = warp; r < nrow; r += FD_THREADS / 32) {
     const int flat = s_flat[r];
-    double* dst = lv.nsplit > 1
-                      ? lv.part + ((int64_t)split * lv.rows + flat) * a.rf
-                      : lv.pf + ((int64_t)lv.typed[flat / a.C] * a.C + flat % a.C) * a.rf;
+    double* dst =
+        lv.nsplit > 1
+            ? lv.part + ((int64_t)split * lv.rows + (int64_t)comb * lv.count[0] * a.C + flat) * a.rf
+            : lv.pf + (((int64_t)lv.typed[flat / a.C] * mult + comb) * a.C + flat % a.C) * a.rf;
     for (int n = lane; n < ncol; n += 32) dst[col0 + n] = Sum[r * pitch + n];
   }
 }
 
-// pf = the sum of the parts, in order (nsplit > 1), for every level: a warp per row.
+// pf = the sum of the parts, in order, for every level with nsplit > 1: a warp per row.
 __global__ void k_m2l_parts(const __grid_constant__ FdArgs a, int nrows) {
   const int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (r >= nrows) return;
@@ -366,7 +393,10 @@ __global__ void k_m2l_parts(const __grid_constant__ FdArgs a, int nrows) {
     if (r >= a.lv[i].row0) li = i;
   const FdLevel& lv = a.lv[li];
   const int flat = r - lv.row0;
-  double* dst = lv.pf + ((int64_t)lv.typed[flat / a.C] * a.C + flat % a.C) * a.rf;
+  const int per = lv.mult ? lv.count[0] * a.C : lv.rows;  // rows of a combination
+  const int comb = flat / per, f2 = flat % per;
+  double* dst = lv.pf + (((int64_t)lv.typed[f2 / a.C] * (lv.mult ? kKaraJ : 1) + comb) * a.C +
+                         f2 % a.C) * a.rf;
   for (int n = lane; n < a.rf; n += 32) {
     double v = 0.0;
     for (int s = 0; s < lv.nsplit; ++s) v += lv.part[((int64_t)s * lv.rows + flat) * a.rf + n];
@@ -374,10 +404,77 @@ __global__ void k_m2l_parts(const __grid_constant__ FdArgs a, int nrows) {
   }
 }
 
+// Combined proxies of the listed source parents: warp per (parent, column).
+__global__ void k_kara_in(const int* __restrict__ parents, int np, const int* __restrict__ sstart,
+                          int span, const double* __restrict__ proxy, double* __restrict__ kx,
+                          int C, int rsp) {
+  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= (int64_t)np * C) return;
+  const int64_t p = parents[w / C];
+  const int c = (int)(w % C);
+  const unsigned present = children_present(sstart, p, span);
+  for (int k = lane; k < rsp; k += 32) {
+    double v[8];
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch)
+      v[ch] = ((present >> ch) & 1) ? proxy[((8 * p + ch) * C + c) * rsp + k] : 0.0;
+    kara_combine(v, [&](int j, double x) { kx[((p * kKaraJ + j) * C + c) * rsp + k] = x; });
+  }
+}
+
+// Combined operators [level][27][26] from the level's 316, element by element;
+// terms[j * 26 + d][8]: +-(operator + 1), 0 for none.
+__global__ void k_kara_ops(const double* __restrict__ E, const int* __restrict__ terms,
+                           int64_t per_op, double* __restrict__ Ek) {
+  const int64_t op = blockIdx.y, lvl = blockIdx.z;
+  const double* e = E + lvl * 316 * per_op;
+  double* o = Ek + (lvl * kKaraJ * kKaraD + op) * per_op;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < per_op;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int s = terms[op * 8 + q];
+      if (s) v += s > 0 ? e[(s - 1) * per_op + i] : -e[(-s - 1) * per_op + i];
+    }
+    o[i] = v;
+  }
+}
+
+// Offsets of the combinations, [27][26] (dx, dy, dz, j 26 + d), behind the 189
+// per child type; and the operators' terms (k_kara_ops).
+void cheb_kara_tables(const int* Ktable, std::vector<int>* offs, std::vector<int>* terms) {
+  for (int j = 0; j < kKaraJ; ++j)
+    for (int d = 0, n = 0; d < 27; ++d) {
+      if (d == 13) continue;
+      const int D[3] = {d / 9 - 1, d / 3 % 3 - 1, d % 3 - 1}, jd[3] = {j / 9, j / 3 % 3, j % 3};
+      for (int i = 0; i < 3; ++i) offs->push_back(D[i]);
+      offs->push_back(j * kKaraD + n++);
+      for (int q = 0; q < 8; ++q) {  // bit i: the subtracted term of coordinate i
+        int lex = 0, sign = 1;
+        bool used = true;
+        for (int i = 0; i < 3; ++i) {
+          const int sub = (q >> i) & 1;
+          int off = 2 * D[i];
+          if (jd[i] == 0)
+            used &= !sub;
+          else if (sub)
+            sign = -sign;
+          else
+            off += jd[i] == 1 ? 1 : -1;
+          lex = 7 * lex + off + 3;
+        }
+        const int op = used ? Ktable[lex] : -1;  // -1: near, no operator
+        terms->push_back(op < 0 ? 0 : sign * (op + 1));
+      }
+    }
+}
+
 int cheb_rsp(int rs) { return (rs + 3) & ~3; }
 
 // column groups of 8 in blocks of at most 16, all blocks alike (the last one padded)
-static void fd_blocks(int rf, int* nblk, int* ntb) {
+void cheb_fragment_blocks(int rf, int* nblk, int* ntb) {
   const int nt = (rf + 7) / 8;
   *nblk = (nt + 15) / 16;
   *ntb = (nt + *nblk - 1) / *nblk;
@@ -388,7 +485,7 @@ static void fd_blocks(int rf, int* nblk, int* ntb) {
 // holds E[f][k]; zero padded to 4 in k and to whole blocks in f.
 std::vector<double> cheb_fragment_operators(const double* K, int64_t nops, int rf, int rs) {
   int nblk, ntb;
-  fd_blocks(rf, &nblk, &ntb);
+  cheb_fragment_blocks(rf, &nblk, &ntb);
   const int k4 = cheb_rsp(rs) / 4;
   const size_t per_blk = (size_t)k4 * ntb * 32, per_op = per_blk * nblk;
   std::vector<double> out((size_t)nops * per_op, 0.0);
@@ -529,7 +626,7 @@ static int run_colgemm_f64(pbbfmm_tree* t, bool post, int C, cudaStream_t st) {
   a.M = post ? n3 : rs;
   a.K = post ? rf : n3;
   a.ldo = post ? n3 : rsp;
-  fd_blocks(a.M, &a.nblk, &a.ntb);
+  cheb_fragment_blocks(a.M, &a.nblk, &a.ntb);
   const int64_t per_op = (int64_t)cheb_rsp(a.K) * a.nblk * a.ntb * 8;
   int64_t items = 0;
   for (int l = L; l >= 2; --l) {
@@ -585,14 +682,42 @@ static int launch_f64(const FdArgs& a, int items, cudaStream_t st) {
   return PBBFMM_OK;
 }
 
+// Combined operators of the tree's current set (made on first use, kept with it).
+static int ensure_kara_ops(pbbfmm_tree* t, int64_t per_op, cudaStream_t st) {
+  if (t->d_Ek) return PBBFMM_OK;
+  const int nlev = t->ops.nlev;
+  PB_CUDA(cudaMalloc(&t->d_Ek, sizeof(double) * nlev * kKaraJ * kKaraD * per_op));
+  k_kara_ops<<<dim3((unsigned)std::min<int64_t>((per_op + 255) / 256, 64), kKaraJ * kKaraD,
+                    (unsigned)nlev),
+               256, 0, st>>>(t->d_E, t->d_offs + 4 * (8 * FD_OFFS + kKaraJ * kKaraD), per_op,
+                             t->d_Ek);
+  PB_LAUNCH("kara_ops");
+  return PBBFMM_OK;
+}
+
 static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
   const int L = t->p.tree_level, rf = t->ops.rf, rsp = cheb_rsp(t->ops.rs);
   Workspace& ws = t->ws;
+  // levels on the combined operators, and their arrays
+  bool kara[kMaxLevel + 1] = {};
+  int64_t kx_off[kMaxLevel + 1] = {}, ky_off[kMaxLevel + 1] = {}, kxn = 0, kyn = 0;
+  for (int l = 3; l <= L; ++l) {
+    kara[l] = cheb_kara_level(t, l);
+    if (!kara[l]) continue;
+    kx_off[l] = kxn;
+    ky_off[l] = kyn;
+    kxn += cells_at(l - 1) * kKaraJ * C * rsp;
+    kyn += cells_at(l - 1) * kKaraJ * C * rf;
+  }
+  if (kxn > 0) {
+    if (int rc = grow(ws.kara_x, sizeof(double) * kxn)) return rc;
+    if (int rc = grow(ws.kara_y, sizeof(double) * kyn)) return rc;
+  }
   FdArgs a{};
   a.C = C;
   a.rf = rf;
   a.rsp = rsp;
-  fd_blocks(rf, &a.nblk, &a.ntb);
+  cheb_fragment_blocks(rf, &a.nblk, &a.ntb);
   a.sstart = ws.sstart_p;
   a.offs = t->d_offs;
   int nsm = 148;
@@ -603,6 +728,33 @@ static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
   for (int l = L; l >= 2; --l) {
     if (t->lists.ntgt[l] == 0) continue;
     FdLevel& v = a.lv[a.nlev++];
+    if (kara[l]) {
+      if (int rc = ensure_kara_ops(t, per_op, st)) return rc;
+      const int np = t->lists.ntgt[l - 1];
+      v.E = t->d_Ek + (int64_t)(t->homog ? 0 : l - 2) * kKaraJ * kKaraD * per_op;
+      v.proxy = ws.kara_x.as<double>() + kx_off[l];
+      v.pf = ws.kara_y.as<double>() + ky_off[l];
+      v.typed = ws.lists.as<int>() + t->lists.tgt_off[l - 1];
+      v.src = ws.lists.as<int>() + t->lists.src_off[l - 1];
+      v.nsrc = t->lists.nsrc[l - 1];
+      v.lev = l - 1;
+      v.span = (int)cells_at(L - l + 1);
+      v.mult = kKaraJ;
+      v.count[0] = np;
+      v.tile0[0] = (int)(((int64_t)np * C + FD_R - 1) / FD_R);
+      v.tile0[8] = kKaraJ * v.tile0[0];
+      v.rows = kKaraJ * np * C;
+      items += (int64_t)v.tile0[8] * a.nblk;
+      const int64_t warps = (int64_t)v.nsrc * C;
+      if (warps > 0) {
+        k_kara_in<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
+            v.src, v.nsrc, ws.sstart_p, (int)cells_at(L - l),
+            ws.proxy.as<double>() + level_offset(l, (int64_t)C * rsp),
+            ws.kara_x.as<double>() + kx_off[l], C, rsp);
+        PB_LAUNCH("kara_in");
+      }
+      continue;
+    }
     v.E = t->d_E + (int64_t)(t->homog ? 0 : l - 2) * 316 * per_op;
     v.proxy = ws.proxy.as<double>() + level_offset(l, (int64_t)C * rsp);
     v.pf = ws.pf.as<double>() + level_offset(l, (int64_t)C * rf);
@@ -626,19 +778,22 @@ static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
   for (int i = 0; i < a.nlev; ++i) {
     FdLevel& v = a.lv[i];
     v.item0 = (int)items;
-    v.nsplit = nsplit;
+    // (of the combinations' 26 offsets at least 6 to a part)
+    v.nsplit = v.mult ? std::min(nsplit, kKaraD / 6) : nsplit;
     v.row0 = (int)rows;
+    items += (int64_t)v.tile0[8] * a.nblk * v.nsplit;
+    if (v.nsplit == 1) continue;
     rows += v.rows;
-    items += (int64_t)v.tile0[8] * a.nblk * nsplit;
-    part += (int64_t)nsplit * v.rows * rf;
+    part += (int64_t)v.nsplit * v.rows * rf;
   }
   if (items == 0) return PBBFMM_OK;
-  if (nsplit > 1) {
+  if (rows > 0) {
     if (int rc = grow(ws.m2l_part, sizeof(double) * part)) return rc;
     double* p = ws.m2l_part.as<double>();
     for (int i = 0; i < a.nlev; ++i) {
+      if (a.lv[i].nsplit == 1) continue;
       a.lv[i].part = p;
-      p += (int64_t)nsplit * a.lv[i].rows * rf;
+      p += (int64_t)a.lv[i].nsplit * a.lv[i].rows * rf;
     }
   }
   // slices of TN column groups so that all 8 warps have work; the deepest
@@ -663,9 +818,18 @@ static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
   else
     rc = launch_f64<16, 3, 1, 1>(a, n, st);
   if (rc) return rc;
-  if (nsplit > 1) {
+  if (rows > 0) {
     k_m2l_parts<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a, (int)rows);
     PB_LAUNCH("m2l_parts");
+  }
+  for (int l = 3; l <= L; ++l) {
+    const int64_t warps = (int64_t)t->lists.ntgt[l - 1] * C;
+    if (!kara[l] || warps == 0) continue;
+    k_kara_out<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
+        ws.lists.as<int>() + t->lists.tgt_off[l - 1], t->lists.ntgt[l - 1],
+        ws.kara_y.as<double>() + ky_off[l],
+        ws.pf.as<double>() + level_offset(l, (int64_t)C * rf), C, rf);
+    PB_LAUNCH("kara_out");
   }
   return PBBFMM_OK;
 }

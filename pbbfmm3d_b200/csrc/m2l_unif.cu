@@ -552,8 +552,6 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
 // Per level, halo[b * STRIDE + r] holds for the region parents of block b their
 // Morton index, then the occupancy of their 8 children (0 outside the
 // domain), then the same of the block's target parents.
-constexpr int kKaraD = 26, kKaraJ = 27;
-
 template <int PX, int PY, int PZ>
 struct MacGeom {
   static constexpr int RX = PX + 2, RY = PY + 2, RZ = PZ + 2;
