@@ -132,7 +132,7 @@ static float tf32_round(float x) {
 }
 
 static void free_tc_ops(TcOps* o) {
-  void* b[] = {o->eth, o->etl, o->eh16, o->el16, o->eexp, o->vth, o->vtl, o->uh, o->ul};
+  void* b[] = {o->eth, o->etl, o->eh16, o->el16, o->eexp, o->kh16, o->kl16, o->kexp, o->vth, o->vtl, o->uh, o->ul};
   for (void* p : b)
     if (p) cudaFree(p);
   *o = TcOps{};

@@ -49,8 +49,8 @@ struct Workspace {
   DevBuf proxy;  // Cheb: sum_l 8^l * C * rs ;  Unif: spectra of one level
   DevBuf pf;     // Cheb: sum_l 8^l * C * rf ;  Unif: accumulated spectra of one level
   DevBuf halo;   // Unif M2L: per parent block, region and target parents and their occupancy
-  DevBuf tc_proxy;  // tensor-core Cheb M2L: hi then lo proxies of one level (+ F16 exponents)
-  DevBuf kara_x, kara_y;  // float64 Cheb M2L: combined proxies and sums of dense levels
+  DevBuf tc_proxy;  // tensor-core Cheb M2L: per level hi then lo proxies (+ F16 exponents)
+  DevBuf kara_x, kara_y;  // Cheb M2L: combined proxies (float64) and sums of dense levels
   DevBuf m2l_part;  // float64 Cheb M2L: partial sums of levels with few tiles
   DevBuf leafpart;  // leaf phase: target leaves dense-first, chunk prefix of the dense ones
   // the sources' leaf offsets, permutation and positions of the last binning
@@ -93,6 +93,10 @@ struct TcOps {
   uint16_t* eh16 = nullptr;
   uint16_t* el16 = nullptr;
   int* eexp = nullptr;
+  // F16, made on first use: the combined operators of the dense levels, [level]
+  // [27][26] (cheb_kara.cuh), and their exponents
+  uint16_t *kh16 = nullptr, *kl16 = nullptr;
+  int* kexp = nullptr;
   int np = 0, kp = 0, kp16 = 0;
   // M2L pre / post transforms on the tensor cores: W = VT (rs x n^3) and
   // U (n^3 x r_f) as [level][mp][kp] F16 hi / lo rows (row m holds W[m][k]
@@ -250,8 +254,7 @@ bool tc_eligible(const pbbfmm_tree* t);
 bool colgemm_tc_eligible(const pbbfmm_tree* t, bool post);
 int run_colgemm_tc(pbbfmm_tree* t, bool post, int lvl, const int* cells, int ncols, int C,
                    const float* X, float* Out, float alpha, cudaStream_t st);
-int run_m2l_cheb_tc_level(pbbfmm_tree* t, int C, int l, int lvl, const float* proxy, float* pf,
-                          cudaStream_t st);
+int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st);
 int run_m2l_unif(pbbfmm_tree* t, int C, cudaStream_t st);
 // tensor-core uniform M2L (float path): levels with >= 16 parents per side,
 // columns in groups of 8

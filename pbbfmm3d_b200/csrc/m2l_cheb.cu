@@ -369,17 +369,14 @@ static int run_m2l_cheb_f32(pbbfmm_tree* t, int C, cudaStream_t st) {
       if (int rc_ = kt_end(t, st)) return rc_;
     }
   }
+  // the tcgen05 kernel (split F16 or TF32) when rf fits TMEM
+  const bool on_tc = tc_eligible(t);
+  if (on_tc)
+    if (int rc_ = run_m2l_cheb_tc(t, C, st)) return rc_;
   for (int l = 2; l <= L; ++l) {
     const int lvl = t->homog ? 0 : l - 2;
     const int nt = t->lists.ntgt[l];
     if (nt == 0) continue;
-    bool on_tc = false;  // float path: the tcgen05 kernel (split F16 or TF32) when rf fits TMEM
-    if (tc_eligible(t)) {
-      if (int rc_ = run_m2l_cheb_tc_level(t, C, l, lvl, proxy + level_offset(l, (int64_t)C * rs),
-                                          pf + level_offset(l, (int64_t)C * rf), st))
-        return rc_;
-      on_tc = true;
-    }
     TypeTiles tt;
     const int per_tile = CG_M / C;
     int tiles = 0;

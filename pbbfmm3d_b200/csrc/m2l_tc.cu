@@ -37,6 +37,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "cheb_kara.cuh"
 #include "fmm.cuh"
 #include "tcgen05.cuh"
 
@@ -55,10 +56,28 @@ constexpr int TC_TMEM_COLS = 512;  // columns allocated (accumulators and runnin
 // keep the full bound.
 __device__ long long g_pipe_wait_iters = kWaitIters;
 
-struct TcTiles {
-  int start[9];  // first tile of each child type; start[8] = total tiles
-  int first[8];  // first list position of each type
-  int count[8];  // targets of each type
+// One level of the launch: its tiles of each child type, or (mult = 27, dense
+// levels, cheb_kara.cuh) of each combination of the children, whose rows are
+// (parent, combination, column) and whose offsets are 26 parent offsets.
+struct TcLevel {
+  const int* typed;                // targets by child type; combined: target parents
+  const unsigned char *ph, *pl;    // proxy hi / lo, rows of rowb bytes
+  const int* pexp;                 // F16: scale exponent of each row
+  float* pf;                       // output rows of rf floats
+  int lev, span, item0;            // item0: first tile of the level
+  int mult;                        // 1, or 27 (start[1] tiles per combination)
+  int op0;                         // first operator of the level
+  int start[9];                    // first tile of each type; start[8] = total tiles
+  int first[8];                    // first list position of each type
+  int count[8];                    // targets of each type
+};
+struct TcArgs {
+  TcLevel lv[kMaxLevel - 1];
+  int nlev, C, rf, NP, rowb, group;
+  const int* sstart;
+  const int* offs;                 // [8][189], then [27][26] (ox, oy, oz, operator)
+  const int *eexp, *kexp;          // F16: scale exponents of the operators / combined ones
+  int* err;
 };
 
 // Stage layout: A_hi 16 KB | A_lo 16 KB | B_hi NP*128 | B_lo NP*128, each
@@ -79,14 +98,18 @@ __host__ __device__ constexpr bool tc_sum_in_tmem(int NP) { return NP <= 160; }
 // registers (the CTA is alone on its SM, so they cost no occupancy).
 constexpr int TC_REG_SUM = 128;
 
-// One CTA per tile of 128 (target, col) rows of one child type; NST stages.
-//   tm_eh, tm_el : [nlev][316][NP] rows of hi / lo of E_o^T (row f holds
-//                  E_o[f][s] over s), zero padded to rowb bytes
-//   Ph, Pl : proxy hi / lo, row (cell * C + col) of rowb bytes, zero padded
-//   pexp   : F16 only: the scale exponent of each proxy row (read for
-//            nonempty source cells only, like Ph / Pl)
-//   eexp   : F16 only: the scale exponent of each operator of this level
-//   pf     : output rows (cell * C + col) of rf floats
+// One CTA per tile of 128 (target, col) rows of one child type (or
+// combination); NST stages; the tiles of all levels in one launch (a level
+// alone leaves a last wave that is nearly empty, the shallow ones a single one).
+// One launch and the combinations, against a launch per level on direct lists:
+// M2L of 4M clustered points, order 6: 18.1 -> 15.3 ms; of 250,000 points, r =
+// 125, 4 columns, forward and adjoint: 7.7 -> 4.4 ms (and 0.35 ms more for the
+// split, which forms the combinations).
+//   tm_eh, tm_el : [operator][NP] rows of hi / lo of E_o^T (row f holds
+//                  E_o[f][s] over s), zero padded to rowb bytes;
+//   tm_kh, tm_kl : the same of the combined operators
+//   proxies, exponents and outputs: TcLevel (pexp and the proxy rows are read
+//   for nonempty source cells only)
 // Warp roles:
 //   warps 0-3  producers: each warp gathers its 32 rows of A with cp.async and
 //              signals the stage's full barrier when its copies land
@@ -109,14 +132,26 @@ constexpr int TC_REG_SUM = 128;
 //   s_acce[b]  : accumulator b drained (128 drainer arrivals)
 template <int NST, bool F16, bool RSUM>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-    k_m2l_cheb_tc(int rf, int NP, int rowb, const __grid_constant__ CUtensorMap tm_eh,
-                  const __grid_constant__ CUtensorMap tm_el, int lvl,
-                  const int* __restrict__ typed, TcTiles tt, int C,
-                  int lev, const int* __restrict__ sstart, int span, const int* __restrict__ offs,
-                  const unsigned char* __restrict__ Ph, const unsigned char* __restrict__ Pl,
-                  const int* __restrict__ pexp, const int* __restrict__ eexp,
-                  float* __restrict__ pf, int group, int* __restrict__ err) {
+    k_m2l_cheb_tc(const __grid_constant__ CUtensorMap tm_eh,
+                  const __grid_constant__ CUtensorMap tm_el,
+                  const __grid_constant__ CUtensorMap tm_kh,
+                  const __grid_constant__ CUtensorMap tm_kl, const __grid_constant__ TcArgs a) {
   extern __shared__ unsigned char smraw[];
+  int li = 0;
+  for (int i = 1; i < a.nlev; ++i)
+    if ((int)blockIdx.x >= a.lv[i].item0) li = i;
+  const TcLevel& lv = a.lv[li];
+  const int rf = a.rf, NP = a.NP, rowb = a.rowb, C = a.C, lev = lv.lev, span = lv.span;
+  const int group = a.group, mult = lv.mult;
+  const bool kara = mult > 1;
+  const int* __restrict__ sstart = a.sstart;
+  const int* __restrict__ typed = lv.typed;
+  const unsigned char* __restrict__ Ph = lv.ph;
+  const unsigned char* __restrict__ Pl = lv.pl;
+  const int* __restrict__ pexp = lv.pexp;
+  float* __restrict__ pf = lv.pf;
+  int* __restrict__ err = a.err;
+  const int tile = (int)blockIdx.x - lv.item0;
   const int bbytes = NP * 128;
   const int stage_bytes = tc_stage_bytes(NP);
   unsigned char* base = smraw + ((1024 - (smem_u32(smraw) & 1023)) & 1023);
@@ -136,21 +171,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long piters = g_pipe_wait_iters;  // poll limit of the pipeline waits
 
-  // child type of this tile (unrolled so the parameter arrays stay in registers)
-  int type = 0, tstart = 0, tlist = 0, tcount = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    if ((int)blockIdx.x >= tt.start[i]) {
-      type = i;
-      tstart = tt.start[i];
-      tlist = tt.first[i];
-      tcount = tt.count[i];
-    }
+  // child type (or combination) of this tile
+  int type = 0, tstart = 0, tlist = 0, tcount = 0, noff = 189, comb = 0;
+  const int* my_offs = a.offs;
+  if (kara) {
+    type = comb = tile / lv.start[1];
+    tstart = type * lv.start[1];
+    tcount = lv.count[0];
+    noff = kKaraD;
+    my_offs += 4 * (8 * 189 + type * kKaraD);
+  } else {
+    for (int i = 1; i < 8; ++i)
+      if (tile >= lv.start[i]) type = i;
+    tstart = lv.start[type];
+    tlist = lv.first[type];
+    tcount = lv.count[type];
+    my_offs += type * 189 * 4;
+  }
   const int per_tile = TC_M / C;
-  const int tfirst = (blockIdx.x - tstart) * per_tile;
+  const int tfirst = (tile - tstart) * per_tile;
   const int ntile = min(per_tile, tcount - tfirst);
   const int nside = 1 << lev;
-  const int* my_offs = offs + type * 189 * 4;
 
   if (tid < TC_M) {
     const int cell = (tid < per_tile * C && tid / C < ntile) ? typed[tlist + tfirst + tid / C] : -1;
@@ -185,8 +226,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   // which (target, offset) pairs of the tile have a source cell: all threads,
   // one pair per item, independent loads
 #pragma unroll 4
-  for (int i = tid; i < ntile * 189; i += TC_THREADS) {
-    const int tg = i / 189, o = i - tg * 189;
+  for (int i = tid; i < ntile * noff; i += TC_THREADS) {
+    const int tg = i / noff, o = i - tg * noff;
     const int xyz = s_xyz[tg * C];
     const int bx = (xyz >> 20) + my_offs[4 * o], by = ((xyz >> 10) & 1023) + my_offs[4 * o + 1],
               bz = (xyz & 1023) + my_offs[4 * o + 2];
@@ -200,7 +241,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   if (tid == 0) {
     int nv = 0;
-    for (int o = 0; o < 189; ++o)
+    for (int o = 0; o < noff; ++o)
       if ((s_valid[o >> 5] >> (o & 31)) & 1) {
         s_oidx[nv] = (uint8_t)o;
         s_off[nv++] = make_int4(my_offs[4 * o], my_offs[4 * o + 1], my_offs[4 * o + 2],
@@ -210,7 +251,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   }
   __syncthreads();
   if constexpr (F16)
-    for (int q = tid; q < s_nvalid; q += TC_THREADS) s_oexp[q] = eexp[s_off[q].w];
+    for (int q = tid; q < s_nvalid; q += TC_THREADS)
+      s_oexp[q] = (kara ? a.kexp : a.eexp)[lv.op0 + s_off[q].w];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -252,7 +294,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         cur_row = -1;
         if (ocell >= 0 && ((s_tmask[otg][o >> 5] >> (o & 31)) & 1)) {
           const int4 d = s_off[q];
-          cur_row = ((long long)morton_encode(ox + d.x, oy + d.y, oz + d.z) * C + ocol) * rowb;
+          cur_row = (((long long)morton_encode(ox + d.x, oy + d.y, oz + d.z) * mult + comb) * C +
+                     ocol) * rowb;
         }
         cur_q = q;
       }
@@ -268,11 +311,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       if (tid == 0) {
         // the operator tile (NP rows x 128 bytes, hi and lo) by TMA; x in
         // elements: 64 per 128 bytes for F16, 32 for TF32
-        const int y = (lvl * 316 + s_off[q].w) * NP;
+        const int y = (lv.op0 + s_off[q].w) * NP;
         const int x = kc * (F16 ? 64 : 32);
         mbar_arrive_expect_tx(&s_tfull[s], 2u * NP * 128u);
-        tma_load_2d(st + 32768, &tm_eh, x, y, &s_tfull[s]);
-        tma_load_2d(st + 32768 + bbytes, &tm_el, x, y, &s_tfull[s]);
+        tma_load_2d(st + 32768, kara ? &tm_kh : &tm_eh, x, y, &s_tfull[s]);
+        tma_load_2d(st + 32768 + bbytes, kara ? &tm_kl : &tm_el, x, y, &s_tfull[s]);
         tma_last[s] = j;
       }
       cp_async_arrive(&s_full[s]);
@@ -340,7 +383,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     // ---------------------------------------------------------------- drainers
     const int row = 32 * (warp & 3) + lane;  // TMEM lane quadrant of this warp
     const int cell = s_cell[row];
-    float* dst = cell >= 0 ? pf + ((int64_t)cell * C + row % C) * rf : nullptr;
+    float* dst = cell >= 0 ? pf + (((int64_t)cell * mult + comb) * C + row % C) * rf : nullptr;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     const int astride = tc_acc_stride(NP);
     const bool tsum = tc_sum_in_tmem(NP);
@@ -361,7 +404,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     auto src_row = [&](int q, bool ok) -> int64_t {
       if (!ok) return 0;
       const int4 o = s_off[q];
-      return (int64_t)morton_encode(rx + o.x, ry + o.y, rz + o.z) * C + rcol;
+      return ((int64_t)morton_encode(rx + o.x, ry + o.y, rz + o.z) * mult + comb) * C + rcol;
     };
     bool v1 = has_src(0), v2 = has_src(1);
     int x1 = F16 ? pexp[src_row(0, v1)] : 0, x2 = F16 && nvalid > 1 ? pexp[src_row(1, v2)] : 0;
@@ -503,6 +546,93 @@ __global__ void k_split_proxy_f16(const int* __restrict__ cells, int64_t nrows, 
   if (lane == 0) pexp[row] = e;
 }
 
+// The 27 combined proxies of each listed source parent (cheb_kara.cuh), split
+// as above into rows (parent 27 + j) C + column: warp per (parent, column), a
+// first pass over K for the rows' magnitudes, a second for the split.
+__global__ void k_split_kara_f16(const int* __restrict__ parents, int np,
+                                 const int* __restrict__ sstart, int span, int C, int rs, int KP,
+                                 const float* __restrict__ proxy, __half* __restrict__ ph,
+                                 __half* __restrict__ pl, int* __restrict__ pexp) {
+  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= (int64_t)np * C) return;  // uniform over the warp
+  const int64_t p = parents[w / C];
+  const int c = (int)(w % C);
+  const unsigned present = children_present(sstart, p, span);
+  auto load = [&](int k, float* v) {
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch)
+      v[ch] = ((present >> ch) & 1) && k < rs ? proxy[((8 * p + ch) * C + c) * rs + k] : 0.f;
+  };
+  float m[kKaraJ];
+#pragma unroll
+  for (int j = 0; j < kKaraJ; ++j) m[j] = 0.f;
+  for (int k = lane; k < rs; k += 32) {
+    float v[8];
+    load(k, v);
+    kara_combine(v, [&](int j, float x) { m[j] = fmaxf(m[j], fabsf(x)); });
+  }
+  int e[kKaraJ];
+#pragma unroll
+  for (int j = 0; j < kKaraJ; ++j) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m[j] = fmaxf(m[j], __shfl_xor_sync(0xffffffffu, m[j], o));
+    e[j] = m[j] > 0.f ? 15 - exponent_of(m[j]) : 0;
+    if (lane == 0) pexp[(p * kKaraJ + j) * C + c] = e[j];
+  }
+  for (int k = lane; k < KP; k += 32) {
+    float v[8];
+    load(k, v);
+    kara_combine(v, [&](int j, float x0) {
+      const float x = scale2(x0, e[j]);
+      const __half h = __float2half_rn(x);
+      const int64_t at = ((p * kKaraJ + j) * C + c) * KP + k;
+      ph[at] = h;
+      pl[at] = __float2half_rn(x - __half2float(h));
+    });
+  }
+}
+
+// Combined operators as the M2L's F16 operands, from the float64 operators in
+// fragment order (cheb_fragment_operators: element (f, k) of an operator at
+// frag(f, k)): a block per (combination, parent offset) and level.
+__global__ void k_kara_ops_f16(const double* __restrict__ E, const int* __restrict__ terms, int rf,
+                               int rs, int ntb, int64_t per_blk, int64_t per_op, int NP, int KP,
+                               __half* __restrict__ eh, __half* __restrict__ el,
+                               int* __restrict__ kexp) {
+  const int op = blockIdx.x, lvl = blockIdx.y;
+  const double* e = E + (int64_t)lvl * 316 * per_op;
+  const int64_t o = (int64_t)lvl * gridDim.x + op;
+  auto value = [&](int f, int k) {
+    const int64_t i = (f / 8 / ntb) * per_blk + ((int64_t)(k / 4) * ntb + f / 8 % ntb) * 32 +
+                      (f % 8) * 4 + k % 4;
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int s = terms[op * 8 + q];
+      if (s) v += s > 0 ? e[(s - 1) * per_op + i] : -e[(-s - 1) * per_op + i];
+    }
+    return (float)v;
+  };
+  __shared__ float sm[32];
+  float m = 0.f;
+  for (int i = threadIdx.x; i < rf * rs; i += blockDim.x) m = fmaxf(m, fabsf(value(i / rs, i % rs)));
+#pragma unroll
+  for (int q = 16; q; q >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, q));
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  for (int q = 0; q < (int)blockDim.x / 32; ++q) m = fmaxf(m, sm[q]);
+  const int ex = m > 0.f ? 15 - exponent_of(m) : 0;
+  if (threadIdx.x == 0) kexp[o] = ex;
+  for (int i = threadIdx.x; i < NP * KP; i += blockDim.x) {
+    const int f = i / KP, k = i % KP;
+    const float x = f < rf && k < rs ? scale2(value(f, k), ex) : 0.f;
+    const __half h = __float2half_rn(x);
+    eh[o * NP * KP + i] = h;
+    el[o * NP * KP + i] = __float2half_rn(x - __half2float(h));
+  }
+}
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (the
 // library links no driver library).
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -563,23 +693,38 @@ bool tc_eligible(const pbbfmm_tree* t) {
 }
 
 template <int NST, bool F16, bool RSUM>
-static int launch_tc(const pbbfmm_tree* t, unsigned tiles, int smem, int rf, int NP, int rowb,
-                     const CUtensorMap& tm_h, const CUtensorMap& tm_l, int lvl, const int* typed,
-                     const TcTiles& tt, int C, int l, int span, const unsigned char* ph,
-                     const unsigned char* pl, const int* pexp, float* pf, cudaStream_t st) {
+static int launch_tc(const TcArgs& a, unsigned tiles, int smem, const CUtensorMap* tm,
+                     cudaStream_t st) {
   PB_CUDA(cudaFuncSetAttribute(k_m2l_cheb_tc<NST, F16, RSUM>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  k_m2l_cheb_tc<NST, F16, RSUM><<<tiles, TC_THREADS, smem, st>>>(
-      rf, NP, rowb, tm_h, tm_l, lvl, typed, tt, C, l, t->ws.sstart_p, span, t->d_offs,
-      ph, pl, pexp, t->tc.eexp + (int64_t)lvl * 316, pf, tc_group(NP, F16), t->d_tc_err);
+  k_m2l_cheb_tc<NST, F16, RSUM><<<tiles, TC_THREADS, smem, st>>>(tm[0], tm[1], tm[2], tm[3], a);
   PB_LAUNCH("m2l_cheb_tc");
   return PBBFMM_OK;
 }
 
-// Level l of the tensor-core M2L: split the proxies, then the MMA kernel.
-// proxy / pf are the level's float arrays (rows cell * C + col).
-int run_m2l_cheb_tc_level(pbbfmm_tree* t, int C, int l, int lvl, const float* proxy, float* pf,
-                          cudaStream_t st) {
+// The combined operators of the tree's current set (made on first use).
+static int ensure_kara_tc_ops(pbbfmm_tree* t, cudaStream_t st) {
+  TcOps& o = t->tc;
+  if (o.kh16) return PBBFMM_OK;
+  constexpr int nops = kKaraJ * kKaraD;
+  const int nlev = t->ops.nlev, rf = t->ops.rf, rs = t->ops.rs;
+  const size_t n = (size_t)nlev * nops * o.np * o.kp16;
+  PB_CUDA(cudaMalloc(&o.kexp, sizeof(int) * nlev * nops));
+  PB_CUDA(cudaMalloc(&o.kl16, 2 * n));
+  PB_CUDA(cudaMalloc(&o.kh16, 2 * n));
+  int nblk, ntb;
+  cheb_fragment_blocks(rf, &nblk, &ntb);
+  const int64_t per_blk = (int64_t)(cheb_rsp(rs) / 4) * ntb * 32;
+  k_kara_ops_f16<<<dim3(nops, (unsigned)nlev), 256, 0, st>>>(
+      t->d_E, t->d_offs + 4 * (8 * 189 + nops), rf, rs, ntb, per_blk, per_blk * nblk, o.np, o.kp16,
+      reinterpret_cast<__half*>(o.kh16), reinterpret_cast<__half*>(o.kl16), o.kexp);
+  PB_LAUNCH("kara_ops_f16");
+  return PBBFMM_OK;
+}
+
+// The tensor-core M2L of all levels: split the proxies, then one MMA launch
+// (deepest level first, so that the shallow ones fill the last wave).
+int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
   const int L = t->p.tree_level, rf = t->ops.rf, rs = t->ops.rs;
   const bool f16 = t->tc_fmt == PBBFMM_TC_F16;
   const int NP = t->tc.np, KP = f16 ? t->tc.kp16 : t->tc.kp, esize = f16 ? 2 : 4;
@@ -590,64 +735,134 @@ int run_m2l_cheb_tc_level(pbbfmm_tree* t, int C, int l, int lvl, const float* pr
     set_error("tensor-core M2L takes at most 128 columns per block");
     return PBBFMM_ERR_UNSUPPORTED;
   }
-  // hi rows | lo rows | (F16) row exponents, every cell of the level
-  const int64_t rows = cells_at(l) * C, pbytes = rows * rowb;
-  if (int rc = grow(ws.tc_proxy, 2 * pbytes + (f16 ? rows * (int64_t)sizeof(int) : 0))) return rc;
-  unsigned char* ph = ws.tc_proxy.as<unsigned char>();
-  unsigned char* pl = ph + pbytes;
-  int* pexp = f16 ? reinterpret_cast<int*>(pl + pbytes) : nullptr;
-  const int ns = t->lists.nsrc[l];
-  if (ns > 0) {
-    const int64_t nrows = (int64_t)ns * C;
-    if (int rc = kt_begin(t, KS_M2L_SPLIT, st)) return rc;
-    if (f16)
-      k_split_proxy_f16<<<(unsigned)((nrows * 32 + 255) / 256), 256, 0, st>>>(
-          lists + t->lists.src_off[l], nrows, C, rs, KP, proxy, reinterpret_cast<__half*>(ph),
-          reinterpret_cast<__half*>(pl), pexp);
-    else
-      k_split_proxy<<<(unsigned)((nrows * KP + 255) / 256), 256, 0, st>>>(
-          lists + t->lists.src_off[l], nrows, C, rs, KP, proxy, reinterpret_cast<float*>(ph),
-          reinterpret_cast<float*>(pl));
-    PB_LAUNCH("m2l_split");
-    if (int rc = kt_end(t, st)) return rc;
+  // per level: hi rows | lo rows | (F16) row exponents, then the combined sums
+  bool kara[kMaxLevel + 1] = {}, any_kara = false;
+  int64_t off[kMaxLevel + 1] = {}, total = 0, koff[kMaxLevel + 1] = {}, ktotal = 0;
+  auto rows_at = [&](int l) { return kara[l] ? cells_at(l - 1) * kKaraJ * C : cells_at(l) * C; };
+  for (int l = 2; l <= L; ++l) {
+    kara[l] = f16 && cheb_kara_level(t, l);
+    any_kara |= kara[l];
+    off[l] = total;
+    total += (rows_at(l) * (2 * rowb + (f16 ? 4 : 0)) + 255) / 256 * 256;
+    koff[l] = ktotal;
+    if (kara[l]) ktotal += rows_at(l) * rf;
   }
-  TcTiles tt;
+  int rc;
+  if ((rc = grow(ws.tc_proxy, total))) return rc;
+  if (any_kara && (rc = grow(ws.kara_y, sizeof(float) * ktotal))) return rc;
+  if (any_kara && (rc = ensure_kara_tc_ops(t, st))) return rc;
+  TcArgs a{};
+  a.C = C;
+  a.rf = rf;
+  a.NP = NP;
+  a.rowb = rowb;
+  a.group = tc_group(NP, f16);
+  a.sstart = ws.sstart_p;
+  a.offs = t->d_offs;
+  a.eexp = t->tc.eexp;
+  a.kexp = t->tc.kexp;
+  a.err = t->d_tc_err;
   const int per_tile = TC_M / C;
-  int tiles = 0;
-  for (int ty = 0; ty < 8; ++ty) {
-    tt.start[ty] = tiles;
-    tt.first[ty] = t->lists.ntyp[l][ty];
-    tt.count[ty] = t->lists.ntyp[l][ty + 1] - t->lists.ntyp[l][ty];
-    tiles += (tt.count[ty] + per_tile - 1) / per_tile;
+  int64_t tiles = 0;
+  if ((rc = kt_begin(t, KS_M2L_SPLIT, st))) return rc;
+  for (int l = L; l >= 2; --l) {
+    if (t->lists.ntgt[l] == 0) continue;
+    const int lvl = t->homog ? 0 : l - 2;
+    const int64_t pbytes = rows_at(l) * rowb;
+    unsigned char* ph = ws.tc_proxy.as<unsigned char>() + off[l];
+    unsigned char* pl = ph + pbytes;
+    int* pexp = f16 ? reinterpret_cast<int*>(pl + pbytes) : nullptr;
+    const float* proxy = ws.proxy.as<float>() + level_offset(l, (int64_t)C * rs);
+    const int ns = t->lists.nsrc[kara[l] ? l - 1 : l];
+    const int* src = lists + t->lists.src_off[kara[l] ? l - 1 : l];
+    const int64_t nrows = (int64_t)ns * C;
+    if (ns > 0) {
+      if (kara[l])
+        k_split_kara_f16<<<(unsigned)((nrows * 32 + 255) / 256), 256, 0, st>>>(
+            src, ns, ws.sstart_p, (int)cells_at(L - l), C, rs, KP, proxy,
+            reinterpret_cast<__half*>(ph), reinterpret_cast<__half*>(pl), pexp);
+      else if (f16)
+        k_split_proxy_f16<<<(unsigned)((nrows * 32 + 255) / 256), 256, 0, st>>>(
+            src, nrows, C, rs, KP, proxy, reinterpret_cast<__half*>(ph),
+            reinterpret_cast<__half*>(pl), pexp);
+      else
+        k_split_proxy<<<(unsigned)((nrows * KP + 255) / 256), 256, 0, st>>>(
+            src, nrows, C, rs, KP, proxy, reinterpret_cast<float*>(ph),
+            reinterpret_cast<float*>(pl));
+      PB_LAUNCH("m2l_split");
+    }
+    TcLevel& v = a.lv[a.nlev++];
+    v.ph = ph;
+    v.pl = pl;
+    v.pexp = pexp;
+    v.item0 = (int)tiles;
+    v.mult = 1;
+    v.lev = l;
+    v.span = (int)cells_at(L - l);
+    v.op0 = lvl * 316;
+    v.typed = lists + t->lists.typ_off[l];
+    v.pf = ws.pf.as<float>() + level_offset(l, (int64_t)C * rf);
+    if (kara[l]) {
+      v.mult = kKaraJ;
+      v.lev = l - 1;
+      v.span = (int)cells_at(L - l + 1);
+      v.op0 = lvl * kKaraJ * kKaraD;
+      v.typed = lists + t->lists.tgt_off[l - 1];
+      v.pf = ws.kara_y.as<float>() + koff[l];
+      v.count[0] = t->lists.ntgt[l - 1];
+      v.start[1] = (v.count[0] + per_tile - 1) / per_tile;
+      v.start[8] = kKaraJ * v.start[1];
+    } else {
+      int n = 0;
+      for (int ty = 0; ty < 8; ++ty) {
+        v.start[ty] = n;
+        v.first[ty] = t->lists.ntyp[l][ty];
+        v.count[ty] = t->lists.ntyp[l][ty + 1] - t->lists.ntyp[l][ty];
+        n += (v.count[ty] + per_tile - 1) / per_tile;
+      }
+      v.start[8] = n;
+    }
+    tiles += v.start[8];
   }
-  tt.start[8] = tiles;
+  if ((rc = kt_end(t, st))) return rc;
   if (tiles == 0) return PBBFMM_OK;
   // three stages when they fit in shared memory next to the static arrays
   const int nst = tc_smem_bytes(NP, 3) + 8192 <= 232448 ? 3 : 2;
   const int smem = tc_smem_bytes(NP, nst);
-  CUtensorMap tm_h, tm_l;
+  CUtensorMap tm[4];
   const int64_t nrows = (int64_t)t->ops.nlev * 316 * NP;
   const void* eh = f16 ? (const void*)t->tc.eh16 : (const void*)t->tc.eth;
   const void* el = f16 ? (const void*)t->tc.el16 : (const void*)t->tc.etl;
-  if (int rc = operator_tensor_map(&tm_h, eh, f16, NP, KP, nrows)) return rc;
-  if (int rc = operator_tensor_map(&tm_l, el, f16, NP, KP, nrows)) return rc;
-  if (int rc = kt_begin(t, KS_M2L, st)) return rc;
-  const int* typed = lists + t->lists.typ_off[l];
-  const int span = (int)cells_at(L - l);
+  if ((rc = operator_tensor_map(&tm[0], eh, f16, NP, KP, nrows))) return rc;
+  if ((rc = operator_tensor_map(&tm[1], el, f16, NP, KP, nrows))) return rc;
+  tm[2] = tm[0];
+  tm[3] = tm[1];
+  if (any_kara) {
+    const int64_t krows = (int64_t)t->ops.nlev * kKaraJ * kKaraD * NP;
+    if ((rc = operator_tensor_map(&tm[2], t->tc.kh16, true, NP, KP, krows))) return rc;
+    if ((rc = operator_tensor_map(&tm[3], t->tc.kl16, true, NP, KP, krows))) return rc;
+  }
+  if ((rc = kt_begin(t, KS_M2L, st))) return rc;
   // register running sum up to TC_REG_SUM columns (three stages always fit there)
   const bool rsum = NP <= TC_REG_SUM && nst == 3;
-#define PB_TC_LAUNCH(NSTV, F, R)                                                              \
-  launch_tc<NSTV, F, R>(t, tiles, smem, rf, NP, rowb, tm_h, tm_l, lvl, typed, tt, C, l, span, \
-                        ph, pl, pexp, pf, st)
-  int rc;
+  const unsigned nt = (unsigned)tiles;
   if (f16)
-    rc = rsum ? PB_TC_LAUNCH(3, true, true)
-              : (nst == 3 ? PB_TC_LAUNCH(3, true, false) : PB_TC_LAUNCH(2, true, false));
+    rc = rsum ? launch_tc<3, true, true>(a, nt, smem, tm, st)
+              : (nst == 3 ? launch_tc<3, true, false>(a, nt, smem, tm, st)
+                          : launch_tc<2, true, false>(a, nt, smem, tm, st));
   else
-    rc = rsum ? PB_TC_LAUNCH(3, false, true)
-              : (nst == 3 ? PB_TC_LAUNCH(3, false, false) : PB_TC_LAUNCH(2, false, false));
-#undef PB_TC_LAUNCH
+    rc = rsum ? launch_tc<3, false, true>(a, nt, smem, tm, st)
+              : (nst == 3 ? launch_tc<3, false, false>(a, nt, smem, tm, st)
+                          : launch_tc<2, false, false>(a, nt, smem, tm, st));
   if (rc) return rc;
+  for (int l = 3; l <= L; ++l) {
+    const int64_t warps = (int64_t)t->lists.ntgt[l - 1] * C;
+    if (!kara[l] || warps == 0) continue;
+    k_kara_out<float><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
+        lists + t->lists.tgt_off[l - 1], t->lists.ntgt[l - 1], ws.kara_y.as<float>() + koff[l],
+        ws.pf.as<float>() + level_offset(l, (int64_t)C * rf), C, rf);
+    PB_LAUNCH("kara_out");
+  }
   return kt_end(t, st);
 }
 
