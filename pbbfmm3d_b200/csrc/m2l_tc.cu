@@ -113,8 +113,8 @@ constexpr int TC_REG_SUM = 128;
 // Warp roles:
 //   warps 0-3  producers: each warp gathers its 32 rows of A with cp.async and
 //              signals the stage's full barrier when its copies land
-//              (cp.async.mbarrier.arrive); thread 0 also loads B (the
-//              operator tile, hi and lo) with two TMA copies;
+//              (cp.async.mbarrier.arrive); one thread of warp 0 also loads B
+//              (the operator tile, hi and lo) with two TMA copies;
 //   warp 4     allocates TMEM; one thread waits for full stages, issues the
 //              MMAs and commits them to the stage's empty barrier;
 //   warps 5-8  drain accumulators into the running sum (TMEM lane quadrant
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const uint32_t soff0 = sw128_off(r0, ch);  // row r0 + 16 i lies 2048 i bytes further
     int cur_q = -1;
     long long cur_row = -1;  // this lane's own row: source row offset or -1
-    int tma_last[NST];       // thread 0: last iteration whose TMA went into each stage
+    int tma_last[NST];       // the TMA thread: last iteration whose TMA went into each stage
 #pragma unroll
     for (int i = 0; i < NST; ++i) tma_last[i] = -1;
     for (int j = 0; j < niter; ++j) {
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         cp_async16(st + soff0 + 2048 * i, Ph + off, ok ? 16 : 0);
         cp_async16(st + 16384 + soff0 + 2048 * i, Pl + off, ok ? 16 : 0);
       }
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         // the operator tile (NP rows x 128 bytes, hi and lo) by TMA; x in
         // elements: 64 per 128 bytes for F16, 32 for TF32
         const int y = (lv.op0 + s_off[q].w) * NP;
@@ -323,13 +323,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     cp_async_wait_all();
     // no TMA may still be writing when the CTA ends: wait (bounded) for the
     // last load issued into each stage
-    if (tid == 0)
+    __syncwarp();
+    if (warp == 0 && elect_one())
       for (int s2 = 0; s2 < NST; ++s2)
         if (tma_last[s2] >= 0 && !mbar_wait(&s_tfull[s2], (tma_last[s2] / NST) & 1, nullptr))
           *s_abort = 1;
   } else if (warp == TC_MMA_WARP) {
     // ---------------------------------------------------------------- MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = F16 ? f16_idesc(TC_M, NP) : tf32_idesc(TC_M, NP);
       const int astride = tc_acc_stride(NP);
       int last = -1;  // last iteration whose MMAs were committed

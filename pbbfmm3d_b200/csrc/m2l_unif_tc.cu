@@ -39,7 +39,7 @@
 // The forward transform (k_fft_fwd, SPLIT) writes the spectra already scaled,
 // split and padded in the stage's layout (UnifPlanes), so that a stage is 12
 // contiguous bulk copies and no thread touches an operand.  M2L of 1M points
-// with 8 columns at order 5: 7.6 ms; with float32 spectra loaded and split by 9
+// with 8 columns at order 5: 6.1 ms; with float32 spectra loaded and split by 9
 // producer warps 19.2 ms: each value was split about four times, and the loads
 // and conversions kept the MMA thread waiting for 55 % of its time.
 //
@@ -250,53 +250,45 @@ __global__ void __launch_bounds__(UT_THREADS, 1) k_m2l_unif_tc(const UnifTcArgs 
 
   if (warp == 0) {
     // ------------------------------------------------------------ copies
-    // Lane 0 waits and arms the barrier, lanes 0-11 each issue one of a
-    // stage's copies (part, line).
-    int li = 0, f = 0, slot = -1;
-    bool ok = true;
-    const int64_t pitch = (int64_t)(S + 2) * 8 * 16, part = UnifPlanes::part_bytes(S);
-    const int cp = lane / 3, cy = lane % 3;  // this lane's copy
-    for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-      const Item t = item_of(w);
-      if (!has_targets(t)) continue;
-      const uint32_t pm = planes(t);
-      if (t.slot != slot) {
-        slot = t.slot;
-        const int fb = f & 1;
-        if (lane == 0) {
+    if (elect_one()) {
+      int li = 0, f = 0, slot = -1;
+      bool ok = true;
+      const int64_t pitch = (int64_t)(S + 2) * 8 * 16, part = UnifPlanes::part_bytes(S);
+      for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+        const Item t = item_of(w);
+        if (!has_targets(t)) continue;
+        const uint32_t pm = planes(t);
+        if (t.slot != slot) {
+          slot = t.slot;
+          const int fb = f & 1;
           ok = f < 2 || mbar_wait_sleep(&s_bempty[fb], ((f - 2) >> 1) & 1, s_abort, piters);
-          if (ok) {
-            mbar_arrive_expect_tx(&s_bfull[fb], UT_BFREQ);
-            bulk_load(bbuf + fb * UT_BFREQ, a.tiles + (int64_t)slot * kUnifTcTileHalves, UT_BFREQ,
-                      &s_bfull[fb]);
-          }
+          if (!ok) break;
+          mbar_arrive_expect_tx(&s_bfull[fb], UT_BFREQ);
+          bulk_load(bbuf + fb * UT_BFREQ, a.tiles + (int64_t)slot * kUnifTcTileHalves, UT_BFREQ,
+                    &s_bfull[fb]);
+          ++f;
         }
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-        if (!ok) break;
-        ++f;
-      }
-      const unsigned char* src0 = a.X + (int64_t)slot * UnifPlanes::slot_bytes(S) +
-                                  (int64_t)cp * part + (t.y + cy) * pitch +
-                                  (int64_t)t.zb * UT_LINE * 8 * 16;
-      for (int i = 0; i < UT_SRC; ++i) {
-        if (!((pm >> i) & 1)) continue;
-        const int s = li % UT_NST;
-        if (lane == 0) {
+        const unsigned char* src0 = a.X + (int64_t)slot * UnifPlanes::slot_bytes(S) +
+                                    t.y * pitch + (int64_t)t.zb * UT_LINE * 8 * 16;
+        for (int i = 0; i < UT_SRC; ++i) {
+          if (!((pm >> i) & 1)) continue;
+          const int s = li % UT_NST;
           ok = li < UT_NST || mbar_wait_sleep(&s_empty[s], (li / UT_NST - 1) & 1, s_abort, piters);
-          if (ok) mbar_arrive_expect_tx(&s_full[s], UT_ASTAGE);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&s_full[s], UT_ASTAGE);
+          const unsigned char* src = src0 + (int64_t)(t.x0 - 1 + i) * 4 * part;
+#pragma unroll
+          for (int cp = 0; cp < 4; ++cp)  // part
+#pragma unroll
+            for (int cy = 0; cy < 3; ++cy)  // line
+              bulk_load(astage + s * UT_ASTAGE + cp * UT_PART + cy * UT_LINEB,
+                        src + cp * part + cy * pitch, UT_LINEB, &s_full[s]);
+          ++li;
         }
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-        if (!ok) break;
-        if (lane < 12)
-          bulk_load(astage + s * UT_ASTAGE + cp * UT_PART + cy * UT_LINEB,
-                    src0 + (int64_t)(t.x0 - 1 + i) * 4 * part, UT_LINEB, &s_full[s]);
-        ++li;
       }
-    }
-    if (!ok) *s_abort = 1;
-    // no copy may still be writing when the CTA ends: wait (bounded) for the
-    // last load into each stage and buffer
-    if (lane == 0) {
+      if (!ok) *s_abort = 1;
+      // no copy may still be writing when the CTA ends: wait (bounded) for the
+      // last load into each stage and buffer
       for (int i = 0; i < UT_NST; ++i) {
         const int uses = li / UT_NST + (i < li % UT_NST ? 1 : 0);
         if (uses > 0 && !mbar_wait(&s_full[i], (uses - 1) & 1, nullptr)) *s_abort = 1;
@@ -309,7 +301,7 @@ __global__ void __launch_bounds__(UT_THREADS, 1) k_m2l_unif_tc(const UnifTcArgs 
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       int li = 0, f = 0, it = 0, slot = -1;
       bool ok = true, bused = false;
       for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
