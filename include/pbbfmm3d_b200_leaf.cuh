@@ -100,6 +100,33 @@ __device__ __forceinline__ T basis_one(int n, int cheb, T x, const T* Tkz, int m
   return num / den;
 }
 
+// The nodes and denominators of the uniform basis for a runtime order, held in
+// shared memory: basis_tab gives basis_one's values bit for bit without its
+// divisions (one instead of 2 n - 1 per value).
+template <typename T>
+struct BasisTab {
+  T node[kMaxOrder], den[kMaxOrder];
+  // by the first n threads of a block (a barrier before its use)
+  __device__ __forceinline__ void fill(int n) {
+    const int m = threadIdx.x;
+    if (m >= n) return;
+    node[m] = T(1) - T(2) * T(m) / T(n - 1);
+    T d = 1;
+    for (int j = 0; j < n; j++)
+      if (m != j) d *= T(-2) * (T(m) - T(j)) / T(n - 1);
+    den[m] = d;
+  }
+};
+template <typename T>
+__device__ __forceinline__ T basis_tab(int n, int cheb, T x, const T* Tkz, const BasisTab<T>& tab,
+                                       int m) {
+  if (cheb) return basis_one<T>(n, 1, x, Tkz, m);
+  T num = 1;
+  for (int j = 0; j < n; j++)
+    if (m != j) num *= x - tab.node[j];
+  return num / tab.den[m];
+}
+
 // dS_m/dx on [-1, 1].  Chebyshev: S_m(x) = (2/n) (1/2 + sum_{k>=1} T_k(x_m)
 // T_k(x)), so S_m'(x) = (2/n) sum_{k>=1} T_k(x_m) k U_{k-1}(x) with U the
 // Chebyshev polynomials of the second kind.  Uniform: the derivative of the
@@ -282,6 +309,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kLeafBlocks<T, KC>)
   constexpr bool kMixed = sizeof(T) == 4;
   using V4 = vec4_t<T>;
   __shared__ T sTkz[kMaxOrder * kMaxOrder];
+  __shared__ BasisTab<T> s_tab;
   __shared__ double kp[4];
   __shared__ int s_nb[kLeafWarps][27][2];  // neighbour source ranges
   __shared__ int s_pre[kLeafWarps][28];    // exclusive prefix of their lengths
@@ -292,6 +320,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kLeafBlocks<T, KC>)
   // basis values of each lane's target, [warp][dim][m < n][lane] (dynamic, sized by n)
   extern __shared__ __align__(16) unsigned char leaf_dyn[];
   T* s_bw = reinterpret_cast<T*>(leaf_dyn) + (threadIdx.x >> 5) * 3 * n * 32;
+  s_tab.fill(n);
   for (int i = threadIdx.x; i < n * n; i += blockDim.x) sTkz[i] = Tkz_g[i];
   if (threadIdx.x < 4) kp[threadIdx.x] = kparam_g[threadIdx.x];
   __syncthreads();
@@ -356,9 +385,9 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kLeafBlocks<T, KC>)
       {
         T* b = s_bw + lane;  // b[(d n + m) 32]: conflict-free, no local memory
         for (int m = 0; m < n; ++m) {
-          b[m * 32] = basis_one<T>(n, cheb, (T)(ihalfL * (x - c[0])), sTkz, m);
-          b[(n + m) * 32] = basis_one<T>(n, cheb, (T)(ihalfL * (y - c[1])), sTkz, m);
-          b[(2 * n + m) * 32] = basis_one<T>(n, cheb, (T)(ihalfL * (z - c[2])), sTkz, m);
+          b[m * 32] = basis_tab<T>(n, cheb, (T)(ihalfL * (x - c[0])), sTkz, s_tab, m);
+          b[(n + m) * 32] = basis_tab<T>(n, cheb, (T)(ihalfL * (y - c[1])), sTkz, s_tab, m);
+          b[(2 * n + m) * 32] = basis_tab<T>(n, cheb, (T)(ihalfL * (z - c[2])), sTkz, s_tab, m);
         }
         const T* Fl = F_L + ((int64_t)leaf * C + c0) * n3;
         T* sF = s_F[wl];
@@ -508,12 +537,139 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kLeafBlocks<T, KC>)
   }
 }
 
+// Sparse leaves, one column: one warp per leaf, its lanes as T' targets x 32 / T'
+// source slots (T' = the power of two that holds the leaf's targets).  The
+// neighbours' sources are staged 32 at a time; each lane sums its target's
+// pairs with every (32 / T')-th source of the tile, and its far field over
+// every (32 / T')-th row of coefficients; one reduction over the slots ends the
+// leaf.  A lane holds one target and one sum, so the kernel is a small loop:
+// with every target's sum in each lane and the targets unrolled, instruction
+// fetch was the top stall (4.7 of 12 cycles per instruction).  Measured against
+// that, leaf phase with exp(-r / l): 1M uniform points (3.8 per leaf), mixed
+// 2.13 -> 1.01 ms; 250,000 points (7.6 per leaf), float64 0.98 -> 0.59 ms.
+template <typename T>
+constexpr int kSingleBlocks = sizeof(T) == 4 ? 8 : 5;
+
+template <class KF, typename T>
+__global__ void __launch_bounds__(32 * kLeafWarps, kSingleBlocks<T>)
+    k_leaf_single(const int* __restrict__ leaves, int nleaves, const int* __restrict__ part_count,
+                  const int* __restrict__ tstart, const int* __restrict__ sstart,
+                  const int* __restrict__ tperm, const double* __restrict__ tpos,
+                  const double* __restrict__ spos, const double* __restrict__ wsorted, int Nf,
+                  int Ns, const T* __restrict__ F_L, int n, int cheb, const T* __restrict__ Tkz_g,
+                  double box, int L, const double* __restrict__ kparam_g,
+                  double* __restrict__ out) {
+  constexpr bool kMixed = sizeof(T) == 4;
+  constexpr int kMaxT = kLaneLeafMin - 1;  // targets of a sparse leaf
+  using V4 = vec4_t<T>;
+  __shared__ T sTkz[kMaxOrder * kMaxOrder];
+  __shared__ BasisTab<T> s_tab;
+  __shared__ double kp[4];
+  __shared__ int s_nb[kLeafWarps][27];   // first source of each neighbour
+  __shared__ int s_pre[kLeafWarps][28];  // exclusive prefix of their lengths
+  __shared__ T s_b[kLeafWarps][kMaxT][3 * kMaxOrder];  // the targets' basis values
+  // source tile: position (hi) and weight, position (lo)
+  __shared__ V4 s_sh[kLeafWarps][32], s_sl[kLeafWarps][kMixed ? 32 : 1];
+  s_tab.fill(n);
+  for (int i = threadIdx.x; i < n * n; i += blockDim.x) sTkz[i] = Tkz_g[i];
+  if (threadIdx.x < 4) kp[threadIdx.x] = kparam_g[threadIdx.x];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int wid = blockIdx.x * kLeafWarps + wl;
+  const int nd = *part_count;  // dense leaves come first in the list
+  if (wid >= nleaves - nd) return;
+  const int leaf = leaves[nd + wid];
+  int ax, ay, az;
+  morton_decode((uint32_t)leaf, &ax, &ay, &az);
+  const int nside = 1 << L;
+  int nb_cnt = 0;
+  if (lane < 27) {
+    const int q = lane;
+    const int bx = ax + q / 9 - 1, by = ay + (q / 3) % 3 - 1, bz = az + q % 3 - 1;
+    int a = 0, e = 0;
+    if (bx >= 0 && by >= 0 && bz >= 0 && bx < nside && by < nside && bz < nside) {
+      const uint32_t bm = morton_encode(bx, by, bz);
+      a = sstart[bm];
+      e = sstart[bm + 1];
+    }
+    s_nb[wl][q] = a;
+    nb_cnt = e - a;
+  }
+  const int ta = tstart[leaf], nt = tstart[leaf + 1] - ta;
+  if (nt >= kLaneLeafMin || nt <= 0) return;  // (dense leaves run elsewhere)
+  double c[3];
+  cell_center_d((uint32_t)leaf, L, box, c);
+  double len = box;
+  for (int i = 0; i < L; ++i) len = 0.5 * len;
+  const double ihalfL = 2. / len;
+  const int lt = nt > 1 ? 32 - __clz(nt - 1) : 0;  // T' = 2^lt
+  const int t = lane & ((1 << lt) - 1), slot = lane >> lt, nslot = 32 >> lt;
+  const bool mine = t < nt;
+  const int ti = ta + (mine ? t : 0);
+  const double x = tpos[ti], y = tpos[(int64_t)Nf + ti], z = tpos[2 * (int64_t)Nf + ti];
+  RelPos<T> tp;
+  tp.set(x - c[0], y - c[1], z - c[2]);
+  for (int idx = lane; idx < nt * 3 * n; idx += 32) {
+    const int u = idx / (3 * n), d = (idx / n) % 3, m = idx % n;
+    const double xd = tpos[(int64_t)d * Nf + ta + u];
+    s_b[wl][u][d * n + m] = basis_tab<T>(n, cheb, (T)(ihalfL * (xd - c[d])), sTkz, s_tab, m);
+  }
+  __syncwarp();
+  neighbour_prefix(nb_cnt, lane, s_pre[wl]);
+  __syncwarp();
+  const int nsrc_total = s_pre[wl][27];
+  LeafAcc<T> acc;
+  // far field: rows (l1, l2) of the leaf's coefficients
+  if (mine) {
+    const T* Fl = F_L + (int64_t)leaf * n * n * n;
+    const T* b = s_b[wl][t];
+    for (int r = slot; r < n * n; r += nslot) {
+      const T b12 = b[r / n] * b[n + r % n];
+      for (int l3 = 0; l3 < n; ++l3) acc.add(Fl[r * n + l3] * (b12 * b[2 * n + l3]));
+    }
+  }
+  // near field: the neighbours' sources in tiles of 32
+  int q = 0;
+  for (int v0 = 0; v0 < nsrc_total; v0 += 32) {
+    const int v = v0 + lane, m = min(32, nsrc_total - v0);
+    __syncwarp();
+    if (v < nsrc_total) {
+      while (v >= s_pre[wl][q + 1]) ++q;
+      const int j = s_nb[wl][q] + (v - s_pre[wl][q]);
+      RelPos<T> sp;
+      sp.set(spos[j] - c[0], spos[(int64_t)Ns + j] - c[1], spos[2 * (int64_t)Ns + j] - c[2]);
+      V4 h;
+      h.x = sp.h[0], h.y = sp.h[1], h.z = sp.h[2], h.w = (T)wsorted[j];
+      s_sh[wl][lane] = h;
+      if constexpr (kMixed) {
+        V4 lo;
+        lo.x = sp.l[0], lo.y = sp.l[1], lo.z = sp.l[2], lo.w = 0;
+        s_sl[wl][lane] = lo;
+      }
+    }
+    __syncwarp();
+    if (mine) {
+      T part = 0;
+#pragma unroll 2
+      for (int jj = slot; jj < m; jj += nslot) {
+        const V4 sh = s_sh[wl][jj];
+        T d[3];
+        tp.diff(sh, s_sl[wl][kMixed ? jj : 0], d);
+        T kv = KF::template eval<T>(d[0], d[1], d[2], kp);
+        if (isinf(kv)) kv = 0;  // coincident points (include/compute.hpp:767)
+        part = fma(kv, sh.w, part);
+      }
+      acc.add(part);
+    }
+  }
+  double v = mine ? acc.value() : 0.0;
+  for (int o = 16; o >= (1 << lt); o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (mine && slot == 0) out[tperm[ti]] += v;
+}
+
 // Sparse leaves (fewer than kLaneLeafMin targets): one warp per leaf, all its
-// targets at once, their positions and basis values computed once.  With few
-// (target, column) pairs (up to TA targets) the lanes run over the sources
-// of the 27 neighbour leaves and over the local coefficients, every lane
-// holds every pair's partial sum, and one warp reduction per pair ends the
-// leaf.  Otherwise the warp stages the sources 32 at a time in shared memory
+// targets at once, several columns (k_leaf_single: one column).  The warp
+// stages the sources of the 27 neighbour leaves 32 at a time in shared memory
 // (positions relative to the leaf centre and the weights of KC columns),
 // evaluates the kernel once per (target, source) pair with the lanes over
 // sources, and lane (t, c) -- target group member t, column c -- accumulates
@@ -532,14 +688,11 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kSparseBlocks<T>)
                   const double* __restrict__ kparam_g, double* __restrict__ out) {
   constexpr bool kMixed = sizeof(T) == 4;
   constexpr int kMaxT = kLaneLeafMin - 1;             // targets of a sparse leaf
-  constexpr int G = KC == 1 ? kMaxT : 32 / KC;        // targets per lane group
-  // up to TA targets: every (target, column) sum in each lane instead (one
-  // column only: with several, the per-lane sums and reductions cost more
-  // than the idle lanes of a short group)
-  constexpr int TA = KC == 1 ? kMaxT : 0;
+  constexpr int G = 32 / KC;                          // targets per lane group
   static_assert(G * KC <= 32, "a lane group fits the warp");
   using V4 = vec4_t<T>;
   __shared__ T sTkz[kMaxOrder * kMaxOrder];
+  __shared__ BasisTab<T> s_tab;
   __shared__ double kp[4];
   __shared__ int s_nb[kLeafWarps][27][2];
   __shared__ int s_pre[kLeafWarps][28];
@@ -551,6 +704,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kSparseBlocks<T>)
   // (rows padded to 33: lanes of different targets read different banks)
   __shared__ T s_k[kLeafWarps][kMaxT][33];
   __shared__ T s_F[kLeafWarps][KC * 33];  // staged local coefficients [column][coefficient]
+  s_tab.fill(n);
   for (int i = threadIdx.x; i < n * n; i += blockDim.x) sTkz[i] = Tkz_g[i];
   if (threadIdx.x < 4) kp[threadIdx.x] = kparam_g[threadIdx.x];
   __syncthreads();
@@ -601,7 +755,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kSparseBlocks<T>)
     const int t = idx / (3 * n), d = (idx / n) % 3, m = idx % n;
     const int i = ta + t;
     const double xd = tpos[(int64_t)d * Nf + i];
-    s_b[wl][t][d * n + m] = basis_one<T>(n, cheb, (T)(ihalfL * (xd - c[d])), sTkz, m);
+    s_b[wl][t][d * n + m] = basis_tab<T>(n, cheb, (T)(ihalfL * (xd - c[d])), sTkz, s_tab, m);
   }
   __syncwarp();
   neighbour_prefix(nb_cnt, lane, s_pre[wl]);
@@ -610,85 +764,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kSparseBlocks<T>)
   const int tl = lane / KC, cl = lane % KC;  // this lane's target-group member and column
   for (int c0 = 0; c0 < C; c0 += KC) {
     const int kce = min(KC, C - c0);  // columns of this pass
-    if constexpr (TA > 0) {
-    if (nt <= TA) {
-      // Few (target, column) pairs: lanes over sources (and over the
-      // coefficients), every pair's sum in each lane, one warp reduction
-      // per pair at the end.
-      LeafAcc<T> acc[TA][KC];
-      // the coefficients four per lane at a time, their loads issued together
-      for (int l0 = lane; l0 < n3; l0 += 128) {
-        T fv[4][KC];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int l = l0 + 32 * r;
-#pragma unroll
-          for (int cc = 0; cc < KC; ++cc)
-            fv[r][cc] = (l < n3 && cc < kce) ? F_L[((int64_t)leaf * C + c0 + cc) * n3 + l] : T(0);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int l = l0 + 32 * r;
-          if (l >= n3) break;
-          const int l1 = l / (n * n), l2 = (l / n) % n, l3 = l % n;
-#pragma unroll
-          for (int t = 0; t < TA; ++t)
-            if (t < nt) {
-              const T* b = s_b[wl][t];
-              const T v = b[l1] * b[n + l2] * b[2 * n + l3];
-#pragma unroll
-              for (int cc = 0; cc < KC; ++cc)
-                if (cc < kce) acc[t][cc].add(fv[r][cc] * v);
-            }
-        }
-      }
-      int q = 0;
-      for (int v = lane; v < nsrc_total; v += 32) {
-        while (v >= s_pre[wl][q + 1]) ++q;
-        const int j = s_nb[wl][q][0] + (v - s_pre[wl][q]);
-        RelPos<T> sp;
-        sp.set(spos[j] - c[0], spos[(int64_t)Ns + j] - c[1], spos[2 * (int64_t)Ns + j] - c[2]);
-        V4 sh, sl;
-        sh.x = sp.h[0], sh.y = sp.h[1], sh.z = sp.h[2], sh.w = 0;
-        sl.x = 0, sl.y = 0, sl.z = 0, sl.w = 0;
-        if constexpr (kMixed) sl.x = sp.l[0], sl.y = sp.l[1], sl.z = sp.l[2];
-        T w[KC];
-        const double* wj = wsorted + (int64_t)j * C + c0;
-#pragma unroll
-        for (int cc = 0; cc < KC; ++cc) w[cc] = cc < kce ? (T)wj[cc] : T(0);
-#pragma unroll
-        for (int t = 0; t < TA; ++t)
-          if (t < nt) {
-            RelPos<T> tp;
-            const V4 th = s_th[wl][t];
-            tp.h[0] = th.x, tp.h[1] = th.y, tp.h[2] = th.z;
-            if constexpr (kMixed) {
-              const V4 tlo = s_tl[wl][t];
-              tp.l[0] = tlo.x, tp.l[1] = tlo.y, tp.l[2] = tlo.z;
-            }
-            T d[3];
-            tp.diff(sh, sl, d);
-            T kv = KF::template eval<T>(d[0], d[1], d[2], kp);
-            if (isinf(kv)) kv = 0;  // coincident points (include/compute.hpp:767)
-#pragma unroll
-            for (int cc = 0; cc < KC; ++cc)
-              if (cc < kce) acc[t][cc].add(kv * w[cc]);
-          }
-      }
-#pragma unroll
-      for (int t = 0; t < TA; ++t)
-#pragma unroll
-        for (int cc = 0; cc < KC; ++cc) {
-          if (t >= nt || cc >= kce) continue;  // uniform over the warp
-          double v = acc[t][cc].value();
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) out[(int64_t)(c0 + cc) * Nf + tperm[ta + t]] += v;
-        }
-      continue;
-    }
-    }
-    // Many pairs: the targets in groups of G; for each group, lane (t, c)
+    // The targets in groups of G; for each group, lane (t, c)
     // owns group member t and column c, the sources are staged 32 at a time
     // and the kernel is evaluated once per (target, source) pair.  Groups run
     // one after the other (a loop, not unrolled: one accumulator, little
@@ -952,9 +1028,14 @@ inline int launch_leaf_kernels_t(const pbbfmm_leaf_args& a, cudaStream_t st) {
       kern<<<(unsigned)((a.max_chunks + kLeafWarps - 1) / kLeafWarps), 32 * kLeafWarps, dyn, st>>>(
           a.leaves, a.nleaves, a.ndense, a.chunk_prefix, a.tstart, a.sstart, a.tperm, a.tpos,
           a.spos, a.wsorted, a.Nf, a.Ns, a.C, F, a.n, a.cheb, Tkz, a.box, a.L, a.kparam, a.out);
+    } else if (a.C == 1) {
+      k_leaf_single<KF, T><<<(unsigned)((a.nleaves + kLeafWarps - 1) / kLeafWarps), 32 * kLeafWarps,
+                             0, st>>>(
+          a.leaves, a.nleaves, a.ndense, a.tstart, a.sstart, a.tperm, a.tpos, a.spos, a.wsorted,
+          a.Nf, a.Ns, F, a.n, a.cheb, Tkz, a.box, a.L, a.kparam, a.out);
     } else {
-      auto kern = a.C == 1 ? k_leaf_sparse<KF, T, 1> : k_leaf_sparse<KF, T, kLeafCols>;
-      kern<<<(unsigned)((a.nleaves + kLeafWarps - 1) / kLeafWarps), 32 * kLeafWarps, 0, st>>>(
+      k_leaf_sparse<KF, T, kLeafCols><<<(unsigned)((a.nleaves + kLeafWarps - 1) / kLeafWarps),
+                                        32 * kLeafWarps, 0, st>>>(
           a.leaves, a.nleaves, a.ndense, a.tstart, a.sstart, a.tperm, a.tpos, a.spos, a.wsorted,
           a.Nf, a.Ns, a.C, F, a.n, a.cheb, Tkz, a.box, a.L, a.kparam, a.out);
     }
