@@ -309,6 +309,37 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
+// Rows of n3 consecutive values of U units, a warp per unit and its lanes over
+// the row (one address per row), to and from shared memory as
+// [element][PITCH]: off(v) gives unit v's row, or -1 for none (zeros in, no
+// write out).  The copies in are asynchronous (cp_async_commit is the caller's).
+template <int U, int n3, int NT, int PITCH, class Off, typename T>
+__device__ __forceinline__ void units_in(T* d, const T* __restrict__ src, Off off) {
+  const int lane = threadIdx.x & 31;
+  for (int v = threadIdx.x >> 5; v < U; v += NT / 32) {
+    const int64_t o = off(v);
+    const T* s = src + (o >= 0 ? o : 0);
+#pragma unroll
+    for (int r = 0; r < (n3 + 31) / 32; ++r) {
+      const int e = lane + 32 * r;
+      if (e < n3) cp_async_elem(d + e * PITCH + v, s + e, o >= 0);
+    }
+  }
+}
+template <int U, int n3, int NT, int PITCH, class Off, typename T>
+__device__ __forceinline__ void units_out(const T* s, T* __restrict__ dst, Off off) {
+  const int lane = threadIdx.x & 31;
+  for (int v = threadIdx.x >> 5; v < U; v += NT / 32) {
+    const int64_t o = off(v);
+    if (o < 0) continue;
+#pragma unroll
+    for (int r = 0; r < (n3 + 31) / 32; ++r) {
+      const int e = lane + 32 * r;
+      if (e < n3) dst[o + e] = s[e * PITCH + v];
+    }
+  }
+}
+
 // Run `f.template run<N>()` for the runtime interpolation order N (2..10).
 template <typename F>
 inline int dispatch_order(int n, F&& f) {

@@ -11,10 +11,12 @@
 #include <type_traits>
 
 #include "fmm.cuh"
+#include "interp.cuh"
 
 namespace pbbfmm {
 
-// L2L, one warp per nonempty target parent and column: the parent's local
+// L2L of the higher orders (k_l2l_units: the others), one warp per nonempty
+// target parent and column: the parent's local
 // coefficients are staged once and pushed through the x, y and z passes for
 // each nonempty child, which is updated in place (F_child += ...).
 template <int N>
@@ -54,128 +56,170 @@ __global__ void __launch_bounds__(32 * L2LCfg<N>::warps)
   for (int ch = 0; ch < 8; ++ch)
     present |= (__shfl_sync(0xffffffffu, bound, ch + 1) != __shfl_sync(0xffffffffu, bound, ch))
                    ? 1u << ch : 0u;
-  constexpr int PER = (n3 + 31) / 32;
-  constexpr bool kRows = N <= (sizeof(T) == 4 ? 6 : 5);  // passes as row tasks
-  constexpr bool kBatch = sizeof(T) == 4 && N <= 5;
-  constexpr int TPL = (n2 + 31) / 32;                    // row tasks per lane
-  if constexpr (kRows) {
-    // Each pass as row tasks: a lane loads the N inputs of one 1-D transform
-    // once and forms its N outputs (operator rows read by broadcast).  The
-    // z pass of task r updates the child's coefficients r n .. r n + n-1,
-    // read up front for all children (kBatch) so those loads are in flight
-    // together.
-    T cur[kBatch ? 8 : 1][kBatch ? TPL : 1][kBatch ? N : 1];
-    if constexpr (kBatch) {
+  __syncwarp();
+  for (int ch = 0; ch < 8; ++ch) {
+    const int cell = par * 8 + ch;
+    if (!((present >> ch) & 1)) continue;  // child without targets
+    const T* wx = sCw + (((ch >> 2) & 1) ? n2 : 0);
+    const T* wy = sCw + (((ch >> 1) & 1) ? n2 : 0);
+    const T* wz = sCw + ((ch & 1) ? n2 : 0);
+    // x: Fx[l1 n2 + l2 n + l3] = sum_k F[k n2 + l2 n + l3] wx[l1 + k n]
+    for (int i = lane; i < n3; i += 32) {
+      const int l1 = i / n2, rem = i % n2;
+      T v = 0;
 #pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        const T* d = Fch + ((int64_t)(par * 8 + ch) * C + col) * n3;
-#pragma unroll
-        for (int t = 0; t < TPL; ++t) {
-          const int r = lane + 32 * t;
-#pragma unroll
-          for (int l3 = 0; l3 < N; ++l3)
-            cur[ch][t][l3] = ((present >> ch) & 1) && r < n2 ? d[r * N + l3] : T(0);
-        }
-      }
+      for (int k = 0; k < N; ++k) v += sp[k * n2 + rem] * wx[l1 + k * N];
+      b0[i] = v;
     }
     __syncwarp();
+    // y: Fy[l1 n2 + l2 n + l3] = sum_k Fx[l1 n2 + k n + l3] wy[l2 + k n]
+    for (int i = lane; i < n3; i += 32) {
+      const int l1 = i / n2, l2 = (i / N) % N, l3 = i % N;
+      T v = 0;
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      const int cell = par * 8 + ch;
-      if (!((present >> ch) & 1)) continue;  // child without targets
-      const T* wx = sCw + (((ch >> 2) & 1) ? n2 : 0);
-      const T* wy = sCw + (((ch >> 1) & 1) ? n2 : 0);
-      const T* wz = sCw + ((ch & 1) ? n2 : 0);
-      // x: Fx[l1 n2 + rem] = sum_k F[k n2 + rem] wx[l1 + k n]   (task rem)
-      for (int q = lane; q < n2; q += 32) {
-        T x[N];
+      for (int k = 0; k < N; ++k) v += b0[l1 * n2 + k * N + l3] * wy[l2 + k * N];
+      b1[i] = v;
+    }
+    __syncwarp();
+    // z: Fchild[l1 n + l3] += sum_k Fy[l1 n + k] wz[l3 + k n]   (l1 over n^2)
+    T* dst = Fch + ((int64_t)cell * C + col) * n3;
+    for (int i = lane; i < n3; i += 32) {
+      const int l1 = i / N, l3 = i % N;
+      T v = 0;
 #pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = sp[k * n2 + q];
+      for (int k = 0; k < N; ++k) v += b1[l1 * N + k] * wz[l3 + k * N];
+      dst[i] += v;
+    }
+    __syncwarp();
+  }
+}
+
+// L2L for orders with InterpCfg::use (interp.cuh): the x pass once per x half,
+// the y pass once per (x, y) quarter, the z pass per child.
+template <int N, typename T>
+__global__ void __launch_bounds__(InterpCfg<N, T>::threads)
+    k_l2l_units(const int* __restrict__ parents, int64_t nunits, const int* __restrict__ tstart,
+                int span_child, const T* __restrict__ Fpar, T* __restrict__ Fch, int C,
+                const __grid_constant__ InterpOps<N, T> op) {
+  using G = InterpCfg<N, T>;
+  constexpr int n2 = G::n2, n3 = G::n3, U = G::U, NT = G::threads;
+  // units per warp and values per lane of the children's updates
+  constexpr int VPW = (U + NT / 32 - 1) / (NT / 32), RPU = (n3 + 31) / 32;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T* sp = reinterpret_cast<T*>(smraw);  // [n^3][U + 1] parent, then the children's updates
+  T* mid = sp + n3 * (U + 1);           // 2 x [n^3][U] after x
+  __shared__ int64_t s_row[U];    // unit: its parent's locals, or -1
+  __shared__ int64_t s_child[U];  // its first child's locals
+  __shared__ unsigned s_present[U];
+  const int tid = threadIdx.x, u = tid % U, l1 = tid / U, warp = tid >> 5, lane = tid & 31;
+  if (tid < U) {
+    const int64_t g = (int64_t)blockIdx.x * U + tid;
+    int64_t row = -1, child = 0;
+    unsigned present = 0;
+    if (g < nunits) {
+      const int64_t p = parents[g / C];
+      row = (p * C + g % C) * n3;
+      child = (8 * p * C + g % C) * n3;
+      int lo = tstart[8 * p * span_child];
+      for (int ch = 0; ch < 8; ++ch) {
+        const int hi = tstart[(8 * p + ch + 1) * span_child];
+        present |= hi != lo ? 1u << ch : 0u;
+        lo = hi;
+      }
+    }
+    s_row[tid] = row;
+    s_child[tid] = child;
+    s_present[tid] = present;
+  }
+  __syncthreads();
+  units_in<U, n3, NT, U + 1>(sp, Fpar, [&](int v) { return s_row[v]; });
+  cp_async_commit();
+  cp_async_wait_all();
+  __syncthreads();
+  if (l1 < N) {
 #pragma unroll
-        for (int l1 = 0; l1 < N; ++l1) {
+    for (int i = 0; i < N; ++i) {
+      const int rem = l1 + N * i;
+      T x[N];
+#pragma unroll
+      for (int k = 0; k < N; ++k) x[k] = sp[(k * n2 + rem) * (U + 1) + u];
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int o = 0; o < N; ++o) {
           T v = 0;
 #pragma unroll
-          for (int k = 0; k < N; ++k) v = fma(x[k], wx[l1 + k * N], v);
-          b0[l1 * n2 + q] = v;
+          for (int k = 0; k < N; ++k) v = fma(x[k], op.w[b][o + k * N], v);
+          mid[(b * n3 + o * n2 + rem) * U + u] = v;
         }
-      }
-      __syncwarp();
-      // y: Fy[l1 n2 + l2 n + l3] = sum_k Fx[l1 n2 + k n + l3] wy[l2 + k n]   (task (l1, l3))
-      for (int q = lane; q < n2; q += 32) {
-        const int l1 = q / N, l3 = q % N;
-        T x[N];
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int bx = 0; bx < 2; ++bx)
 #pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = b0[l1 * n2 + k * N + l3];
+    for (int by = 0; by < 2; ++by) {
+      T y[N][N];
+      if (l1 < N) {
+        const T* m = mid + (bx * n3 + l1 * n2) * U + u;
 #pragma unroll
-        for (int l2 = 0; l2 < N; ++l2) {
-          T v = 0;
-#pragma unroll
-          for (int k = 0; k < N; ++k) v = fma(x[k], wy[l2 + k * N], v);
-          b1[l1 * n2 + l2 * N + l3] = v;
-        }
-      }
-      __syncwarp();
-      // z: Fchild[r n + l3] += sum_k Fy[r n + k] wz[l3 + k n]   (task row r over n^2)
-      T* dst = Fch + ((int64_t)cell * C + col) * n3;
-#pragma unroll
-      for (int t = 0; t < TPL; ++t) {
-        const int r = lane + 32 * t;
-        if (r < n2) {
+        for (int l3 = 0; l3 < N; ++l3) {
           T x[N];
 #pragma unroll
-          for (int k = 0; k < N; ++k) x[k] = b1[r * N + k];
+          for (int k = 0; k < N; ++k) x[k] = m[(k * N + l3) * U];
 #pragma unroll
-          for (int l3 = 0; l3 < N; ++l3) {
+          for (int l2 = 0; l2 < N; ++l2) {
             T v = 0;
 #pragma unroll
-            for (int k = 0; k < N; ++k) v = fma(x[k], wz[l3 + k * N], v);
-            if constexpr (kBatch) dst[r * N + l3] = cur[ch][t][l3] + v;
-            else dst[r * N + l3] += v;
+            for (int k = 0; k < N; ++k) v = fma(x[k], op.w[by][l2 + k * N], v);
+            y[l2][l3] = v;
           }
         }
       }
-      __syncwarp();
+#pragma unroll
+      for (int bz = 0; bz < 2; ++bz) {
+        const int ch = 4 * bx + 2 * by + bz;
+        // the child's coefficients, loaded while its update is computed (a warp
+        // per unit, lanes over its row, as units_out)
+        T cur[VPW][RPU];
+#pragma unroll
+        for (int i = 0; i < VPW; ++i) {
+          const int v = warp + i * (NT / 32);
+          const bool ok = v < U && ((s_present[v] >> ch) & 1);
+          const T* f = Fch + (ok ? s_child[v] + (int64_t)ch * C * n3 : 0);
+#pragma unroll
+          for (int r = 0; r < RPU; ++r) cur[i][r] = ok && lane + 32 * r < n3 ? f[lane + 32 * r] : T(0);
+        }
+        if (l1 < N) {
+          T* d = sp + l1 * n2 * (U + 1) + u;
+#pragma unroll
+          for (int l2 = 0; l2 < N; ++l2)
+#pragma unroll
+            for (int l3 = 0; l3 < N; ++l3) {
+              T v = 0;
+#pragma unroll
+              for (int k = 0; k < N; ++k) v = fma(y[l2][k], op.w[bz][l3 + k * N], v);
+              d[(l2 * N + l3) * (U + 1)] = v;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < VPW; ++i) {
+          const int v = warp + i * (NT / 32);
+          if (v < U && ((s_present[v] >> ch) & 1)) {
+            T* f = Fch + s_child[v] + (int64_t)ch * C * n3;
+#pragma unroll
+            for (int r = 0; r < RPU; ++r) {
+              const int e = lane + 32 * r;
+              if (e < n3) f[e] = cur[i][r] + sp[e * (U + 1) + v];
+            }
+          }
+        }
+        __syncthreads();
+      }
     }
-  } else {
-    __syncwarp();
-    for (int ch = 0; ch < 8; ++ch) {
-      const int cell = par * 8 + ch;
-      if (!((present >> ch) & 1)) continue;  // child without targets
-      const T* wx = sCw + (((ch >> 2) & 1) ? n2 : 0);
-      const T* wy = sCw + (((ch >> 1) & 1) ? n2 : 0);
-      const T* wz = sCw + ((ch & 1) ? n2 : 0);
-      // x: Fx[l1 n2 + l2 n + l3] = sum_k F[k n2 + l2 n + l3] wx[l1 + k n]
-      for (int i = lane; i < n3; i += 32) {
-        const int l1 = i / n2, rem = i % n2;
-        T v = 0;
-#pragma unroll
-        for (int k = 0; k < N; ++k) v += sp[k * n2 + rem] * wx[l1 + k * N];
-        b0[i] = v;
-      }
-      __syncwarp();
-      // y: Fy[l1 n2 + l2 n + l3] = sum_k Fx[l1 n2 + k n + l3] wy[l2 + k n]
-      for (int i = lane; i < n3; i += 32) {
-        const int l1 = i / n2, l2 = (i / N) % N, l3 = i % N;
-        T v = 0;
-#pragma unroll
-        for (int k = 0; k < N; ++k) v += b0[l1 * n2 + k * N + l3] * wy[l2 + k * N];
-        b1[i] = v;
-      }
-      __syncwarp();
-      // z: Fchild[l1 n + l3] += sum_k Fy[l1 n + k] wz[l3 + k n]   (l1 over n^2)
-      T* dst = Fch + ((int64_t)cell * C + col) * n3;
-      for (int i = lane; i < n3; i += 32) {
-        const int l1 = i / N, l3 = i % N;
-        T v = 0;
-#pragma unroll
-        for (int k = 0; k < N; ++k) v += b1[l1 * N + k] * wz[l3 + k * N];
-        dst[i] += v;
-      }
-      __syncwarp();
-    }
-  }
-  (void)PER;
 }
+
 
 template <typename T>
 struct L2LLaunch {
@@ -184,11 +228,23 @@ struct L2LLaunch {
   cudaStream_t st;
   template <int N>
   int run() {
-    using G = L2LCfg<N>;
     const int L = t->p.tree_level;
     Workspace& ws = t->ws;
-    const int64_t per = (int64_t)C * G::n3;
+    const int64_t per = (int64_t)C * N * N * N;
     const int np = t->lists.ntgt[l - 1];
+    if constexpr (InterpCfg<N, T>::use) {
+      using I = InterpCfg<N, T>;
+      const int64_t units = (int64_t)np * C;
+      PB_CUDA(cudaFuncSetAttribute(k_l2l_units<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)I::smem));
+      k_l2l_units<N, T><<<(unsigned)((units + I::U - 1) / I::U), I::threads, I::smem, st>>>(
+          ws.lists.as<int>() + t->lists.tgt_off[l - 1], units, ws.tstart.as<int>(),
+          (int)cells_at(L - l), ws.F.as<T>() + level_offset(l - 1, per),
+          ws.F.as<T>() + level_offset(l, per), C, interp_ops<N, T>(t));
+      PB_LAUNCH("l2l");
+      return PBBFMM_OK;
+    } else {
+    using G = L2LCfg<N>;
     const int64_t tasks = (int64_t)np * C;
     const size_t smem = sizeof(T) * G::per_warp * G::warps;
     PB_CUDA(cudaFuncSetAttribute(k_l2l<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -198,6 +254,7 @@ struct L2LLaunch {
         ws.F.as<T>() + level_offset(l, per), C, ops_view<T>(t).Cw);
     PB_LAUNCH("l2l");
     return PBBFMM_OK;
+    }
   }
 };
 

@@ -198,9 +198,9 @@ int unif_slot_freq(int n, int slot) {
 //            memory in coalesced rows.
 // Bound: HBM and the latency of the stages (shared memory admits two to three
 // CTAs per SM).  Measured, 1M points at order 5, forward + inverse, against one
-// cell per CTA with a column per lane: 1 column, float32 2.57 + 1.56 -> 0.39 +
-// 0.39 ms (its stores covered 8 bytes of each frequency plane); 8 columns,
-// float64 3.77 + 5.38 -> 2.89 + 3.61 ms.
+// cell per CTA with a column per lane: 1 column, float32 2.57 + 1.56 -> 0.38 +
+// 0.34 ms (its stores covered 8 bytes of each frequency plane); 8 columns,
+// float64 3.77 + 5.38 -> 2.75 + 3.30 ms, float32 with the split 2.57 + 2.19 ms.
 template <int n, typename T>
 struct FftCfg {
   static constexpr int m = 2 * n - 1, n3 = n * n * n, nym = n * m * n;
@@ -311,11 +311,7 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   }
   const bool any = __syncthreads_or(has);
   if (any) {
-    for (int i = tid; i < U * n3; i += Cfg::threads) {
-      const int v = i / n3, l = i % n3;
-      const int64_t o = s_src[v];
-      cp_async_elem(&S[l * (U + 1) + v], a.S + (o >= 0 ? o + l : 0), o >= 0);
-    }
+    units_in<U, n3, Cfg::threads, U + 1>(S, a.S, [&](int v) { return s_src[v]; });
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
@@ -511,10 +507,15 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
       for (int a3 = 0; a3 < n; ++a3) o[q * n + a3] = a.scale * (acc[q][a3] * a.invP);
   }
   __syncthreads();
-  for (int i = tid; i < U * n3; i += Cfg::threads) {
-    const int v = i / n3, l = i % n3;
+  // (a warp per unit, lanes over its row)
+  for (int v = tid >> 5; v < U; v += Cfg::threads / 32) {
     const int64_t o = s_dst[v];
-    if (o >= 0) a.F[o + l] = O[v * OP + l];
+    if (o < 0) continue;
+#pragma unroll
+    for (int r = 0; r < (n3 + 31) / 32; ++r) {
+      const int l = (tid & 31) + 32 * r;
+      if (l < n3) a.F[o + l] = O[v * OP + l];
+    }
   }
 }
 

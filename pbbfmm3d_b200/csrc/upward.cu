@@ -9,6 +9,7 @@
 // Layout: moments of level l live at S + level_offset(l, C*n3), cell-major,
 // S[(cell*C + col)*n3 + (l1*n + l2)*n + l3] as in the reference's sourceval.
 #include "fmm.cuh"
+#include "interp.cuh"
 
 namespace pbbfmm {
 
@@ -134,7 +135,8 @@ struct P2MLaunch {
   }
 };
 
-// M2M, one warp per nonempty parent and column: the column's moments of all
+// M2M of the higher orders (k_m2m_units: the others), one warp per nonempty
+// parent and column: the column's moments of all
 // nonempty children are staged in the warp's shared slice (cp.async), then
 // each child goes through the z, y and x passes and is added to the parent
 // (children in order 0..7, as the reference accumulates them).
@@ -165,8 +167,7 @@ __global__ void __launch_bounds__(32 * M2MCfg<N, T>::warps)
   T* b0 = sch + 8 * n3;
   T* b1 = b0 + n3;
   // which children hold sources: lanes 0..8 read the 9 leaf-range bounds at
-  // once; then (float32, orders up to 6) every child's moments are loaded
-  // with all loads in flight (an empty child's moments are never read)
+  // once
   int bound = 0;
   if (lane <= 8) bound = sstart[(int64_t)(par * 8 + lane) * span_child];
   unsigned present = 0;
@@ -175,107 +176,12 @@ __global__ void __launch_bounds__(32 * M2MCfg<N, T>::warps)
     present |= (__shfl_sync(0xffffffffu, bound, ch + 1) != __shfl_sync(0xffffffffu, bound, ch))
                    ? 1u << ch : 0u;
   constexpr int PER = (n3 + 31) / 32;
-  if constexpr (N > 6 || sizeof(T) == 8) {
-    for (int ch = 0; ch < 8; ++ch) {
-      if (!((present >> ch) & 1)) continue;
-      const T* src = Schild + ((int64_t)(par * 8 + ch) * C + col) * n3;
-      for (int i = lane; i < n3; i += 32) sch[ch * n3 + i] = src[i];
-    }
-  } else {
-    T v[8][PER];
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      const T* src = Schild + ((int64_t)(par * 8 + ch) * C + col) * n3;
-#pragma unroll
-      for (int r = 0; r < PER; ++r) {
-        const int i = lane + 32 * r;
-        v[ch][r] = ((present >> ch) & 1) && i < n3 ? src[i] : T(0);
-      }
-    }
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch)
-#pragma unroll
-      for (int r = 0; r < PER; ++r) {
-        const int i = lane + 32 * r;
-        if (i < n3) sch[ch * n3 + i] = v[ch][r];
-      }
-  }
-  __syncwarp();
-  // Orders up to 6 (float32) or 5 (float64): each pass as row tasks, a lane
-  // loading the N inputs of one 1-D transform once and forming its N outputs
-  // (the operator rows read by broadcast).  Higher orders (registers):
-  // element tasks, one output per lane and pass.
-  if constexpr (N <= (sizeof(T) == 4 ? 6 : 5)) {
-  constexpr int TPL = (n2 + 31) / 32;  // x-pass tasks per lane
-  T acc[TPL][N];
-#pragma unroll
-  for (int t = 0; t < TPL; ++t)
-#pragma unroll
-    for (int l = 0; l < N; ++l) acc[t][l] = 0;
   for (int ch = 0; ch < 8; ++ch) {
     if (!((present >> ch) & 1)) continue;
-    const T* wx = sCw + (((ch >> 2) & 1) ? n2 : 0);
-    const T* wy = sCw + (((ch >> 1) & 1) ? n2 : 0);
-    const T* wz = sCw + ((ch & 1) ? n2 : 0);
-    const T* sc = sch + ch * n3;
-    // z: Sz[r n + l3] = sum_k S[r n + k] wz[l3 n + k]   (row r over n^2)
-    for (int r = lane; r < n2; r += 32) {
-      T x[N];
-#pragma unroll
-      for (int k = 0; k < N; ++k) x[k] = sc[r * N + k];
-#pragma unroll
-      for (int l3 = 0; l3 < N; ++l3) {
-        T v = 0;
-#pragma unroll
-        for (int k = 0; k < N; ++k) v = fma(x[k], wz[l3 * N + k], v);
-        b0[r * N + l3] = v;
-      }
-    }
-    __syncwarp();
-    // y: Sy[l1 n2 + l2 n + l3] = sum_k Sz[l1 n2 + k n + l3] wy[l2 n + k]   (task (l1, l3))
-    for (int q = lane; q < n2; q += 32) {
-      const int l1 = q / N, l3 = q % N;
-      T x[N];
-#pragma unroll
-      for (int k = 0; k < N; ++k) x[k] = b0[l1 * n2 + k * N + l3];
-#pragma unroll
-      for (int l2 = 0; l2 < N; ++l2) {
-        T v = 0;
-#pragma unroll
-        for (int k = 0; k < N; ++k) v = fma(x[k], wy[l2 * N + k], v);
-        b1[l1 * n2 + l2 * N + l3] = v;
-      }
-    }
-    __syncwarp();
-    // x: SS[l1 n2 + rem] += sum_k Sy[k n2 + rem] wx[l1 n + k]   (task rem)
-#pragma unroll
-    for (int t = 0; t < TPL; ++t) {
-      const int rem = lane + 32 * t;
-      if (rem < n2) {
-        T x[N];
-#pragma unroll
-        for (int k = 0; k < N; ++k) x[k] = b1[k * n2 + rem];
-#pragma unroll
-        for (int l1 = 0; l1 < N; ++l1) {
-          T v = acc[t][l1];
-#pragma unroll
-          for (int k = 0; k < N; ++k) v = fma(x[k], wx[l1 * N + k], v);
-          acc[t][l1] = v;
-        }
-      }
-    }
-    __syncwarp();
+    const T* src = Schild + ((int64_t)(par * 8 + ch) * C + col) * n3;
+    for (int i = lane; i < n3; i += 32) sch[ch * n3 + i] = src[i];
   }
-  T* dst = Spar + ((int64_t)par * C + col) * n3;
-#pragma unroll
-  for (int t = 0; t < TPL; ++t) {
-    const int rem = lane + 32 * t;
-    if (rem < n2)
-#pragma unroll
-      for (int l1 = 0; l1 < N; ++l1) dst[l1 * n2 + rem] = acc[t][l1];
-  }
-  } else {
-  constexpr int PER = (n3 + 31) / 32;
+  __syncwarp();
   T acc[PER];
 #pragma unroll
   for (int r = 0; r < PER; ++r) acc[r] = 0;
@@ -323,7 +229,126 @@ __global__ void __launch_bounds__(32 * M2MCfg<N, T>::warps)
     const int i = lane + 32 * r;
     if (i < n3) dst[i] = acc[r];
   }
+}
+
+// M2M for orders with InterpCfg::use (interp.cuh): children in pairs along z,
+// then y, then x; one child's moments are copied while the previous one is
+// transformed.
+template <int N, typename T>
+__global__ void __launch_bounds__(InterpCfg<N, T>::threads)
+    k_m2m_units(const int* __restrict__ parents, int64_t nunits, const int* __restrict__ sstart,
+                int span_child, const T* __restrict__ Schild, T* __restrict__ Spar, int C,
+                const __grid_constant__ InterpOps<N, T> op) {
+  using G = InterpCfg<N, T>;
+  constexpr int n2 = G::n2, n3 = G::n3, U = G::U, NT = G::threads;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T* sch = reinterpret_cast<T*>(smraw);  // 2 x [n^3][U + 1] children
+  T* mid = sch + 2 * n3 * (U + 1);       // [n^3][U] after z and y
+  __shared__ int64_t s_row[U];           // unit: its parent's moments, or -1
+  __shared__ int64_t s_child[U];         // its first child's moments
+  __shared__ unsigned s_present[U];
+  const int tid = threadIdx.x, u = tid % U, l1 = tid / U;
+  if (tid < U) {
+    const int64_t g = (int64_t)blockIdx.x * U + tid;
+    int64_t row = -1, child = 0;
+    unsigned present = 0;
+    if (g < nunits) {
+      const int64_t p = parents[g / C];
+      row = (p * C + g % C) * n3;
+      child = (8 * p * C + g % C) * n3;
+      int lo = sstart[8 * p * span_child];
+      for (int ch = 0; ch < 8; ++ch) {
+        const int hi = sstart[(8 * p + ch + 1) * span_child];
+        present |= hi != lo ? 1u << ch : 0u;
+        lo = hi;
+      }
+    }
+    s_row[tid] = row;
+    s_child[tid] = child;
+    s_present[tid] = present;
   }
+  __syncthreads();
+  auto fetch = [&](int ch) {  // zeros for absent children
+    units_in<U, n3, NT, U + 1>(sch + (ch & 1) * n3 * (U + 1), Schild, [&](int v) -> int64_t {
+      return (s_present[v] >> ch) & 1 ? s_child[v] + (int64_t)ch * C * n3 : -1;
+    });
+    cp_async_commit();
+  };
+  fetch(0);
+  T acc[N][N];  // x pass: pairs l1 + N i, outputs
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int o = 0; o < N; ++o) acc[i][o] = 0;
+#pragma unroll
+  for (int bx = 0; bx < 2; ++bx) {
+    T a[N][N];
+#pragma unroll
+    for (int by = 0; by < 2; ++by) {
+      T tz[N][N];
+#pragma unroll
+      for (int bz = 0; bz < 2; ++bz) {
+        const int ch = 4 * bx + 2 * by + bz;
+        cp_async_wait_all();
+        __syncthreads();  // child ch is here; the other buffer's readers are done
+        if (ch < 7) fetch(ch + 1);
+        if (l1 < N) {
+          const T* s = sch + (ch & 1) * n3 * (U + 1) + l1 * n2 * (U + 1) + u;
+#pragma unroll
+          for (int l2 = 0; l2 < N; ++l2) {
+            T x[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) x[k] = s[(l2 * N + k) * (U + 1)];
+#pragma unroll
+            for (int l3 = 0; l3 < N; ++l3) {
+              T v = bz == 0 ? T(0) : tz[l2][l3];
+#pragma unroll
+              for (int k = 0; k < N; ++k) v = fma(x[k], op.w[bz][l3 * N + k], v);
+              tz[l2][l3] = v;
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int l3 = 0; l3 < N; ++l3)
+#pragma unroll
+        for (int l2 = 0; l2 < N; ++l2) {
+          T v = by == 0 ? T(0) : a[l2][l3];
+#pragma unroll
+          for (int k = 0; k < N; ++k) v = fma(tz[k][l3], op.w[by][l2 * N + k], v);
+          a[l2][l3] = v;
+        }
+    }
+    if (l1 < N) {
+      T* d = mid + l1 * n2 * U + u;
+#pragma unroll
+      for (int e = 0; e < n2; ++e) d[e * U] = a[e / N][e % N];
+    }
+    __syncthreads();
+    if (l1 < N) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const T* d = mid + (l1 + N * i) * U + u;
+        T x[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) x[k] = d[k * n2 * U];
+#pragma unroll
+        for (int o = 0; o < N; ++o)
+#pragma unroll
+          for (int k = 0; k < N; ++k) acc[i][o] = fma(x[k], op.w[bx][o * N + k], acc[i][o]);
+      }
+    }
+    // (the next write of mid lies behind the barriers of the next children)
+  }
+  __syncthreads();
+  if (l1 < N) {  // through shared memory: coalesced rows
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int o = 0; o < N; ++o) sch[(o * n2 + l1 + N * i) * (U + 1) + u] = acc[i][o];
+  }
+  __syncthreads();
+  units_out<U, n3, NT, U + 1>(sch, Spar, [&](int v) { return s_row[v]; });
 }
 
 template <typename T>
@@ -333,11 +358,23 @@ struct M2MLaunch {
   cudaStream_t st;
   template <int N>
   int run() {
-    using G = M2MCfg<N, T>;
     const int L = t->p.tree_level;
     Workspace& ws = t->ws;
-    const int64_t per = (int64_t)C * G::n3;
+    const int64_t per = (int64_t)C * N * N * N;
     const int np = t->lists.nsrc[l];
+    if constexpr (InterpCfg<N, T>::use) {
+      using I = InterpCfg<N, T>;
+      const int64_t units = (int64_t)np * C;
+      PB_CUDA(cudaFuncSetAttribute(k_m2m_units<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)I::smem));
+      k_m2m_units<N, T><<<(unsigned)((units + I::U - 1) / I::U), I::threads, I::smem, st>>>(
+          ws.lists.as<int>() + t->lists.src_off[l], units, ws.sstart_p, (int)cells_at(L - l - 1),
+          ws.S.as<T>() + level_offset(l + 1, per), ws.S.as<T>() + level_offset(l, per), C,
+          interp_ops<N, T>(t));
+      PB_LAUNCH("m2m");
+      return PBBFMM_OK;
+    } else {
+    using G = M2MCfg<N, T>;
     const int64_t tasks = (int64_t)np * C;
     const size_t smem = sizeof(T) * G::per_warp * G::warps;
     PB_CUDA(cudaFuncSetAttribute(k_m2m<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -347,6 +384,7 @@ struct M2MLaunch {
         ops_view<T>(t).Cw);
     PB_LAUNCH("m2m");
     return PBBFMM_OK;
+    }
   }
 };
 
