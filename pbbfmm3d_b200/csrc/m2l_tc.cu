@@ -873,13 +873,20 @@ int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
 // for the columns n < ncols, row_n = cells[n / C] * C + n % C (reference:
 // UpwardPass tail, include/compute.hpp:373-396, and the Moment2Local
 // post-transform, include/compute.hpp:881-914).  One CTA of 128 threads per
-// 128 columns; thread t owns column n = 128 blockIdx.x + t:
-//   A = its row of X (times bscale), scaled by its own power of two and split
+// 128 columns n = 128 blockIdx.x + t:
+//   A = row t of X (times bscale), scaled by its own power of two and split
 //       into F16 hi / lo, written to shared memory (SW128 K-major) one K chunk
-//       of 64 at a time;
+//       of 64 at a time by warp t / 32, lanes over K, 8 rows in flight;
 //   B = W (mp rows, pre-split with one exponent per level), by TMA;
 //   D[n][m] (128 lanes x mp columns, TMEM) accumulates three products per
 //       K step; thread t drains lane t, unscales and writes row_n of Out.
+// Bound: latency of the row loads (few CTAs per SM, one stage).  A row per
+// thread, read with a stride of K floats between lanes, moved a 32-byte sector
+// for every 16 bytes used and wrote the outputs one scattered float per lane;
+// with lanes over K and outputs through shared memory, order 5 with 4 columns
+// (K = 125, not a multiple of 4; 250,000 points, forward and adjoint) pre + post
+// 1.33 -> 0.89 ms, order 6 with 1 column (4M points) 2.51 -> 2.12 ms, all of it
+// in the post-transform.
 // Chunks run one after another (one stage); two CTAs share an SM (one when
 // mp > 256: then each product is two MMAs of N = mp / 2 and the CTA holds all
 // 512 TMEM columns).  When
@@ -911,29 +918,32 @@ __global__ void __launch_bounds__(CG_TC_THREADS, 1)
   const int n = blockIdx.x * CG_TC_THREADS + tid;
   const bool valid = n < ncols;
   const int64_t row = valid ? (int64_t)cells[n / C] * C + n % C : 0;
-  const float* xr = X + row * K;
-  // 16-byte loads when rows (K floats, from 16-byte aligned level bases) are
-  // 16-byte aligned
-  const bool vec4 = (K & 3) == 0;
-  // this column's exponent: max |bscale x| 2^e in [2^14, 2^15)
-  float mx = 0.f;
-  if (valid) {
-    if (vec4) {
-      const float4* x4 = reinterpret_cast<const float4*>(xr);
-#pragma unroll 4
-      for (int k4 = 0; k4 < K / 4; ++k4) {
-        float4 v = x4[k4];
-        if (BSCALE) {
-          const float4 b = reinterpret_cast<const float4*>(bscale)[k4];
-          v.x *= b.x, v.y *= b.y, v.z *= b.z, v.w *= b.w;
-        }
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-      }
-    } else {
-      for (int k = 0; k < K; ++k) mx = fmaxf(mx, fabsf(BSCALE ? xr[k] * bscale[k] : xr[k]));
+  __shared__ int64_t s_row[CG_TC_THREADS];  // row_n, or -1 past the end
+  __shared__ int s_exp[CG_TC_THREADS];      // its exponent: max |bscale x| 2^e in [2^14, 2^15)
+  const int lane = tid & 31;
+  s_row[tid] = valid ? row : -1;
+  __syncwarp();
+  for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += 8) {
+    float mx[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx[i] = 0.f;
+    for (int k = lane; k < K; k += 32) {
+      const float b = BSCALE ? bscale[k] : 1.f;
+      float x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = s_row[r0 + i] >= 0 ? X[s_row[r0 + i] * K + k] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx[i] = fmaxf(mx[i], fabsf(BSCALE ? x[i] * b : x[i]));
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+      for (int o = 16; o; o >>= 1) mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], o));
+      if (lane == 0) s_exp[r0 + i] = mx[i] > 0.f ? 15 - exponent_of(mx[i]) : 0;
     }
   }
-  const int e = mx > 0.f ? 15 - exponent_of(mx) : 0;
+  __syncwarp();
+  const int e = s_exp[tid];
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                      smem_u32(&s_tmem)),
@@ -960,45 +970,35 @@ __global__ void __launch_bounds__(CG_TC_THREADS, 1)
   for (int i = 0; i < 128; ++i) racc[i] = 0.f;
   int last_tma = -1;  // thread 0: the last chunk whose TMA was issued
   for (int c = 0; c < nchunks; ++c) {
-    // A chunk: this column's 64 values (zero past K), scaled and split
+    // A chunk: 64 values of each row (zero past K), scaled and split; lane k / 2
+    // of a row's warp takes values k and k + 1
+    for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += 8) {
+      const int k = c * 64 + 2 * lane;
+      const bool k0 = k < K, k1 = k + 1 < K;
+      float x[8][2];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      uint32_t h[4], l[4];
-      float v8[8];
-      const int kb = c * 64 + j * 8;
-      if (vec4) {  // two 16-byte loads; a block of 4 lies wholly below or above K
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int k = kb + 4 * q;
-          float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (valid && k < K) {
-            x = *reinterpret_cast<const float4*>(xr + k);
-            if (BSCALE) {
-              const float4 b = *reinterpret_cast<const float4*>(bscale + k);
-              x.x *= b.x, x.y *= b.y, x.z *= b.z, x.w *= b.w;
-            }
-          }
-          v8[4 * q] = scale2(x.x, e), v8[4 * q + 1] = scale2(x.y, e);
-          v8[4 * q + 2] = scale2(x.z, e), v8[4 * q + 3] = scale2(x.w, e);
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int k = kb + u;
-          v8[u] = (valid && k < K) ? scale2(BSCALE ? xr[k] * bscale[k] : xr[k], e) : 0.f;
-        }
+      for (int i = 0; i < 8; ++i) {
+        const int64_t r = s_row[r0 + i];
+        x[i][0] = r >= 0 && k0 ? X[r * K + k] : 0.f;
+        x[i][1] = r >= 0 && k1 ? X[r * K + k + 1] : 0.f;
       }
+      const float b0 = BSCALE && k0 ? bscale[k] : 1.f, b1 = BSCALE && k1 ? bscale[k + 1] : 1.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float v[2] = {v8[2 * i], v8[2 * i + 1]};
-        const __half2 vh = __floats2half2_rn(v[0], v[1]);
+      for (int i = 0; i < 8; ++i) {
+        const int er = s_exp[r0 + i];  // uniform over the warp
+        float v0 = BSCALE ? x[i][0] * b0 : x[i][0], v1 = BSCALE ? x[i][1] * b1 : x[i][1];
+        if (er >= -126 && er <= 127) {
+          const float f = exp2i(er);
+          v0 *= f, v1 *= f;
+        } else {
+          v0 = scale2(v0, er), v1 = scale2(v1, er);
+        }
+        const __half2 vh = __floats2half2_rn(v0, v1);
         const float2 vf = __half22float2(vh);
-        const __half2 vl = __floats2half2_rn(v[0] - vf.x, v[1] - vf.y);
-        h[i] = *reinterpret_cast<const uint32_t*>(&vh);
-        l[i] = *reinterpret_cast<const uint32_t*>(&vl);
+        const uint32_t off = sw128_off(r0 + i, lane >> 2) + (lane & 3) * 4;
+        *reinterpret_cast<__half2*>(a_hi + off) = vh;
+        *reinterpret_cast<__half2*>(a_lo + off) = __floats2half2_rn(v0 - vf.x, v1 - vf.y);
       }
-      *reinterpret_cast<uint4*>(a_hi + sw128_off(tid, j)) = make_uint4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<uint4*>(a_lo + sw128_off(tid, j)) = make_uint4(l[0], l[1], l[2], l[3]);
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // to the tensor pipe
     if (tid == 0) {
@@ -1061,30 +1061,37 @@ __global__ void __launch_bounds__(CG_TC_THREADS, 1)
     if (tid == 0 && err) atomicExch(err, 1);
   } else {
     // every lane of the warp takes part in the (warp-collective) TMEM loads;
-    // only valid columns store
+    // only valid rows are written
     tc_fence_after();
     // the unscaling 2^-(e + wexp) as two exact power-of-two factors applied
     // one after the other (never multiplied together, which could leave the
     // float range although the result lies inside it), then alpha
     const int kt = -(e + wexp), k1 = min(max(kt, -126), 127), k2 = min(max(kt - k1, -149), 127);
     const float sc = exp2i(k1), sc2 = exp2i(k2);
-    float* o = valid ? Out + row * M : nullptr;
-    if (rdrain) {
-      if (o) {
+    float* so = reinterpret_cast<float*>(base);  // [128 rows][129] (the tiles are done with)
+    for (int m0 = 0; m0 < mp; m0 += 128) {  // uniform
+      __syncthreads();
+      if (rdrain) {
 #pragma unroll
         for (int m = 0; m < 128; ++m)
-          if (m < M) o[m] = racc[m] * sc * sc2 * alpha * (OSCALE ? oscale[m] : 1.f);
-      }
-    } else {
-      for (int m0 = 0; m0 < mp; m0 += 16) {
-        uint32_t r[16];
-        tc_ld16_wait(lane_base + (uint32_t)m0, r);
-        if (o) {
+          if (m < mp) so[tid * 129 + m] = racc[m] * sc * sc2 * alpha;
+      } else {
+        for (int q = 0; q < min(128, mp - m0); q += 16) {
+          uint32_t r[16];
+          tc_ld16_wait(lane_base + (uint32_t)(m0 + q), r);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int m = m0 + i;
-            if (m < M) o[m] = __uint_as_float(r[i]) * sc * sc2 * alpha * (OSCALE ? oscale[m] : 1.f);
-          }
+          for (int i = 0; i < 16; ++i)
+            so[tid * 129 + q + i] = __uint_as_float(r[i]) * sc * sc2 * alpha;
+        }
+      }
+      __syncthreads();
+      for (int r = warp; r < CG_TC_THREADS; r += CG_TC_THREADS / 32) {
+        if (s_row[r] < 0) continue;
+        float* o = Out + s_row[r] * M + m0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int m = lane + 32 * q;
+          if (m0 + m < M) o[m] = OSCALE ? so[r * 129 + m] * oscale[m0 + m] : so[r * 129 + m];
         }
       }
     }
