@@ -173,6 +173,11 @@ __host__ __device__ inline void unif_job(int n, int j, int* k2, int* k3) {
     *k3 = 0;
   }
 }
+// job of (k2, k3); k3 = 0: k2 < n
+__host__ __device__ inline constexpr int unif_job_of(int n, int k2, int k3) {
+  const int full = (2 * n - 1) * (n - 1);
+  return k3 > 0 ? k2 * (n - 1) + k3 - 1 : k2 > 0 ? full + k2 - 1 : full + n - 1;
+}
 int unif_slots(int n) { return (unif_jobs(n) - 1) * (2 * n - 1) + n; }
 int unif_slot_freq(int n, int slot) {
   const int m = 2 * n - 1;
@@ -196,14 +201,17 @@ int unif_slot_freq(int n, int slot) {
 //            (a1): for each k3 the y transform, added into the n^2 outputs of
 //            its row by the z transform; the outputs leave through shared
 //            memory in coalesced rows.
-// Bound: HBM and the latency of the stages (shared memory admits two to three
-// CTAs per SM).  Measured, 1M points at order 5, forward + inverse, against one
+// Spectra between the stages: the jobs (k2, k3) that are kept, n nj elements per
+// unit.  Bound: HBM and the latency of the stages (shared memory admits two to
+// four CTAs per SM).  Measured, 1M points at order 5, forward + inverse, against one
 // cell per CTA with a column per lane: 1 column, float32 2.57 + 1.56 -> 0.38 +
 // 0.34 ms (its stores covered 8 bytes of each frequency plane); 8 columns,
-// float64 3.77 + 5.38 -> 2.75 + 3.30 ms, float32 with the split 2.57 + 2.19 ms.
+// float64 3.77 + 5.38 -> 2.75 + 3.30 ms, float32 with the split 3.32 + 3.10 -> 2.57 +
+// 2.19 ms, and with four CTAs per SM instead of three (the conjugate elements not
+// stored, the forward's moments under its spectra) 2.27 + 1.99 ms.
 template <int n, typename T>
 struct FftCfg {
-  static constexpr int m = 2 * n - 1, n3 = n * n * n, nym = n * m * n;
+  static constexpr int m = 2 * n - 1, n3 = n * n * n, nj = unif_jobs(n), nym = n * nj;
   static constexpr int unit = (n3 + 2 * nym) * (int)sizeof(T);  // bytes per unit (forward)
   static constexpr int U = unit * 32 <= 110 * 1024   ? 32
                            : unit * 16 <= 110 * 1024 ? 16
@@ -212,15 +220,26 @@ struct FftCfg {
   // the rows of the k3 loop: one thread per (row, part of k3) where one per row leaves warps idle
   static constexpr int parts = n * U < 128 ? 2 : 1;
   static constexpr int threads = n * U * parts <= 128 ? 128 : (n * U * parts + 31) / 32 * 32;
-  static constexpr size_t smem_fwd = sizeof(T) * ((size_t)n3 * (U + 1) + 2 * (size_t)nym * U) + 16;
+  // forward: the moments take the place of the spectra until every thread has
+  // its row in registers
+  static constexpr bool alias = parts == 1 && sizeof(T) == 4 && n <= 5;
+  static constexpr size_t smem_y = 2 * sizeof(T) * (size_t)nym * U;
+  static constexpr size_t smem_s = sizeof(T) * (size_t)n3 * (U + 1);
+  static constexpr size_t smem_fwd = alias ? (smem_y > smem_s ? smem_y : smem_s) : smem_y + smem_s + 16;
   static constexpr size_t out_bytes = sizeof(T) * (size_t)U * (n3 | 1);
-  static constexpr size_t smem_inv =
-      2 * sizeof(T) * (size_t)nym * U > out_bytes ? 2 * sizeof(T) * (size_t)nym * U : out_bytes;
+  // inverse: plain levels ask for n m n elements per unit and so keep three CTAs
+  // per SM at order 5, float32 (with four: 1M points, 1 column 0.334 -> 0.356 ms;
+  // 200,000 points, 3 columns 0.146 -> 0.166 ms); the split ones gain from four
+  // (2.20 -> 1.99 ms)
+  static constexpr size_t smem_inv(bool split) {
+    const size_t b = split ? smem_y : 2 * sizeof(T) * (size_t)(n * m * n) * U;
+    return b > out_bytes ? b : out_bytes;
+  }
   static constexpr int unroll = n <= 6 ? n : 1;  // the k3 loops: larger orders keep the code small
 };
 
 // The z and y transforms of row l1 of one unit, for k3 = K0, K0 + STEP, ...
-template <int n, typename T, int U, int K0, int STEP>
+template <int n, typename T, int U, int K0, int STEP, int PITCH>
 __device__ __forceinline__ void fwd_row(const T* __restrict__ s, cplx_t<T>* __restrict__ y) {
   using W = Tw<n, T>;
   constexpr int m = 2 * n - 1;
@@ -233,7 +252,7 @@ __device__ __forceinline__ void fwd_row(const T* __restrict__ s, cplx_t<T>* __re
       T re = 0, im = 0;
 #pragma unroll
       for (int l = 0; l < n; ++l) {
-        const T x = s[(l2 * n + l) * (U + 1)];
+        const T x = s[(l2 * n + l) * PITCH];
         re = fma(x, W::c((k3 * l) % m), re);
         im = fma(-x, W::s((k3 * l) % m), im);
       }
@@ -242,7 +261,7 @@ __device__ __forceinline__ void fwd_row(const T* __restrict__ s, cplx_t<T>* __re
     const int kend = k3 == 0 ? n : m;  // (k2 >= n, 0) are not kept
     if constexpr (m == 9) {
       dft_5_to_9<n, T>(v, [&](int k, cplx_t<T> r) {
-        if (k < kend) y[(k * n + k3) * U] = r;
+        if (k < kend) y[unif_job_of(n, k, k3) * U] = r;
       });
     } else {
 #pragma unroll
@@ -255,7 +274,7 @@ __device__ __forceinline__ void fwd_row(const T* __restrict__ s, cplx_t<T>* __re
           re = fma(v[l].x, c, fma(v[l].y, sn, re));
           im = fma(v[l].y, c, fma(-v[l].x, sn, im));
         }
-        y[(k * n + k3) * U] = make_cplx<T>(re, im);
+        y[unif_job_of(n, k, k3) * U] = make_cplx<T>(re, im);
       }
     }
   }
@@ -276,8 +295,8 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   using Cfg = FftCfg<n, T>;
   constexpr int m = Cfg::m, n2 = n * n, n3 = Cfg::n3, U = Cfg::U, nj = unif_jobs(n);
   extern __shared__ __align__(16) unsigned char smraw[];
-  C2* Y = reinterpret_cast<C2*>(smraw);                        // [l1][k2][k3][U]
-  T* S = reinterpret_cast<T*>(Y + (size_t)Cfg::nym * U);       // [n^3][U + 1]
+  C2* Y = reinterpret_cast<C2*>(smraw);                        // [l1][job][U]
+  T* S = reinterpret_cast<T*>(Cfg::alias ? Y : Y + (size_t)Cfg::nym * U);  // [n^3][U + 1]
   __shared__ int64_t s_src[U];                                 // unit: its moments, or -1
   const int tid = threadIdx.x, u = tid % U, job0 = tid / U;
   constexpr int JS = Cfg::threads / U;
@@ -315,16 +334,27 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    for (int job = job0; job < n * Cfg::parts; job += JS) {
-      const int l1 = job % n;
-      const T* s = S + l1 * n2 * (U + 1) + u;
-      C2* y = Y + l1 * m * n * U + u;
-      if constexpr (Cfg::parts == 1)
-        fwd_row<n, T, U, 0, 1>(s, y);
-      else if (job < n)
-        fwd_row<n, T, U, 0, 2>(s, y);
-      else
-        fwd_row<n, T, U, 1, 2>(s, y);
+    if constexpr (Cfg::alias) {
+      T row[n2];
+      if (job0 < n) {
+        const T* s = S + job0 * n2 * (U + 1) + u;
+#pragma unroll
+        for (int l = 0; l < n2; ++l) row[l] = s[l * (U + 1)];
+      }
+      __syncthreads();
+      if (job0 < n) fwd_row<n, T, U, 0, 1, 1>(row, Y + job0 * nj * U + u);
+    } else {
+      for (int job = job0; job < n * Cfg::parts; job += JS) {
+        const int l1 = job % n;
+        const T* s = S + l1 * n2 * (U + 1) + u;
+        C2* y = Y + l1 * nj * U + u;
+        if constexpr (Cfg::parts == 1)
+          fwd_row<n, T, U, 0, 1, U + 1>(s, y);
+        else if (job < n)
+          fwd_row<n, T, U, 0, 2, U + 1>(s, y);
+        else
+          fwd_row<n, T, U, 1, 2, U + 1>(s, y);
+      }
     }
     __syncthreads();
   }
@@ -339,11 +369,9 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
     const int kend = j == nj - 1 ? n : m;  // (0, 0): the rest are conjugates
     C2 v[n];
     if (any) {
-      int k2, k3;
-      unif_job(n, j, &k2, &k3);
-      const C2* y = Y + (k2 * n + k3) * U + u;
+      const C2* y = Y + j * U + u;
 #pragma unroll
-      for (int l = 0; l < n; ++l) v[l] = y[l * m * n * U];
+      for (int l = 0; l < n; ++l) v[l] = y[l * nj * U];
     } else {
 #pragma unroll
       for (int l = 0; l < n; ++l) v[l] = make_cplx<T>(T(0), T(0));
@@ -394,7 +422,7 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   constexpr int m = Cfg::m, n2 = n * n, n3 = Cfg::n3, U = Cfg::U, nj = unif_jobs(n);
   constexpr int OP = n3 | 1;  // pitch of a unit's outputs
   extern __shared__ __align__(16) unsigned char smraw[];
-  C2* G = reinterpret_cast<C2*>(smraw);  // [a1][k2][k3][U]
+  C2* G = reinterpret_cast<C2*>(smraw);  // [a1][job][U]
   T* O = reinterpret_cast<T*>(smraw);    // [U][OP], after G
   __shared__ int64_t s_dst[U];           // unit: its locals, or -1
   const int tid = threadIdx.x, u = tid % U, job0 = tid / U;
@@ -424,8 +452,6 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   if (has) {
     // x: G[a1][k2][k3] = sum_k1 Y[k1][k2][k3] e^{+2 pi i k1 t1 / m}
     for (int j = job0; j < nj; j += JS) {
-      int k2, k3;
-      unif_job(n, j, &k2, &k3);
       const C2* y = a.Y + (int64_t)j * m * a.slot_stride + src;
       C2 v[m];
 #pragma unroll
@@ -434,9 +460,9 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
         v[k] = y[(mirror ? m - k : k) * a.slot_stride];
         if (mirror) v[k].y = -v[k].y;
       }
-      C2* g = G + (k2 * n + k3) * U + u;
+      C2* g = G + j * U + u;
       if constexpr (m == 9) {
-        idft_9_to_5<n, T>(v, [&](int q, C2 r) { g[q * m * n * U] = r; });
+        idft_9_to_5<n, T>(v, [&](int q, C2 r) { g[q * nj * U] = r; });
       } else {
 #pragma unroll
         for (int q = 0; q < n; ++q) {
@@ -448,7 +474,7 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
             re = fma(v[k].x, c, fma(-v[k].y, s, re));
             im = fma(v[k].y, c, fma(v[k].x, s, im));
           }
-          g[q * m * n * U] = make_cplx<T>(re, im);
+          g[q * nj * U] = make_cplx<T>(re, im);
         }
       }
     }
@@ -459,14 +485,14 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   T acc[n][n];
   const bool row = job0 < n && has;
   if (row) {
-    const C2* g = G + job0 * m * n * U + u;
+    const C2* g = G + job0 * nj * U + u;
 #pragma unroll Cfg::unroll
     for (int k3 = 0; k3 < n; ++k3) {
       C2 v[m];
 #pragma unroll
       for (int k = 0; k < m; ++k) {
         const bool mirror = k3 == 0 && k >= n;  // G(-k2, 0) = conj G(k2, 0)
-        v[k] = g[((mirror ? m - k : k) * n + k3) * U];
+        v[k] = g[unif_job_of(n, mirror ? m - k : k, k3) * U];
         if (mirror) v[k].y = -v[k].y;
       }
       auto add = [&](int q, C2 h) {
@@ -842,8 +868,8 @@ struct FftInvLaunch {
     const int64_t grid = SPLIT ? 8 * ((rows + Cfg::U - 1) / Cfg::U) : (a.nunits + Cfg::U - 1) / Cfg::U;
     auto kern = k_fft_inv<N, T, SPLIT>;
     PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Cfg::smem_inv));
-    kern<<<(unsigned)grid, Cfg::threads, Cfg::smem_inv, st>>>(a);
+                                 (int)Cfg::smem_inv(SPLIT)));
+    kern<<<(unsigned)grid, Cfg::threads, Cfg::smem_inv(SPLIT), st>>>(a);
     PB_LAUNCH("fft_inv");
     return PBBFMM_OK;
   }
