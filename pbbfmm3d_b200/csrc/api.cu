@@ -566,7 +566,7 @@ static int take_tc_timeout(pbbfmm_tree* t) {
 }
 
 // ---- host staging of the host-buffer entry point
-constexpr size_t kStageChunk = 16u << 20;
+constexpr size_t kStagePiece = 1u << 20;
 
 static int grow_pinned(void** p, size_t* cap, size_t bytes) {
   if (bytes == 0) bytes = 16;
@@ -581,47 +581,35 @@ static int grow_pinned(void** p, size_t* cap, size_t bytes) {
 
 static int host_threads(size_t bytes) {
   const unsigned hw = std::thread::hardware_concurrency();
-  const size_t by_size = bytes / (1u << 20) + 1;  // about 1 MB per thread at least
+  // 3 MB per thread at least: starting one costs 50 to 100 us here (14 MB in and
+  // out, whole call: 1 MB per thread 4.8, 3 MB 3.9, 8 MB 3.9 ms)
+  const size_t by_size = bytes / (3u << 20) + 1;
   size_t n = hw ? (hw < 16 ? hw : 16) : 4;
   return (int)(n < by_size ? n : by_size);
 }
 
-// memcpy split over host threads (pageable source into pinned staging)
-static void host_copy_mt(void* dst, const void* src, size_t bytes) {
-  const int nt = host_threads(bytes);
-  if (nt <= 1) {
-    memcpy(dst, src, bytes);
-    return;
-  }
-  std::vector<std::thread> th;
-  const size_t per = (bytes + nt - 1) / nt;
-  for (int i = 0; i < nt; ++i) {
-    const size_t a = i * per, b = a + per < bytes ? a + per : bytes;
-    if (a >= b) break;
-    th.emplace_back([=] {
-      memcpy(static_cast<unsigned char*>(dst) + a, static_cast<const unsigned char*>(src) + a, b - a);
-    });
-  }
-  for (auto& x : th) x.join();
-}
-
-// dst[i] += src[i], split over host threads
-static void host_add_mt(double* dst, const double* src, size_t n) {
-  const int nt = host_threads(n * sizeof(double));
-  auto add = [](double* d, const double* s, size_t a, size_t b) {
-    for (size_t i = a; i < b; ++i) d[i] += s[i];
+// work(i) for i < n on the calling thread and up to nt - 1 others, each taking
+// the next index; own(take) runs on the calling thread, which helps through
+// take() (false when no index is left).  No thread outlives the call; one that
+// cannot be started is done without.
+template <typename W, typename O>
+static void host_pieces(size_t n, int nt, W work, O own) {
+  std::atomic<size_t> next{0};
+  auto take = [&]() -> bool {
+    const size_t i = next.fetch_add(1, std::memory_order_relaxed);
+    if (i < n) work(i);
+    return i < n;
   };
-  if (nt <= 1) {
-    add(dst, src, 0, n);
-    return;
-  }
   std::vector<std::thread> th;
-  const size_t per = (n + nt - 1) / nt;
-  for (int i = 0; i < nt; ++i) {
-    const size_t a = i * per, b = a + per < n ? a + per : n;
-    if (a >= b) break;
-    th.emplace_back(add, dst, src, a, b);
+  try {
+    for (int k = 1; k < nt; ++k)
+      th.emplace_back([&] {
+        while (take()) {
+        }
+      });
+  } catch (...) {
   }
+  own(take);
   for (auto& x : th) x.join();
 }
 
@@ -1170,9 +1158,18 @@ int pbbfmm_compute(pbbfmm_tree* t, const double* target, int64_t Nf, const doubl
   if ((rc = grow_pinned(&ws.h_out, &ws.h_out_cap, bo))) return rc;
   double* dt = ws.io_tgt.as<double>();
   double* ds = same ? dt : ws.io_src.as<double>();
-  // inputs: multithreaded copy into pinned staging, chunk by chunk, each
-  // chunk's DMA overlapping the next chunk's host copy
+  // inputs: into pinned staging by pieces, over host threads started once; a
+  // piece's transfer is queued as soon as it and those before it are there, and
+  // overlaps the copies of the next.  (Threads started for each array, whole
+  // arrays up to 16 MB at a time: 200,003 points, 3 columns, 5.3 -> 3.9 ms per
+  // call, 2.5 ms of it on the device.)
   unsigned char* hin = static_cast<unsigned char*>(ws.h_in);
+  struct Piece {
+    const unsigned char* src;
+    unsigned char *host, *dev;
+    size_t bytes;
+  };
+  std::vector<Piece> pieces;
   struct Seg {
     const void* src;
     void* dev;
@@ -1180,13 +1177,30 @@ int pbbfmm_compute(pbbfmm_tree* t, const double* target, int64_t Nf, const doubl
   } segs[3] = {{target, dt, bt}, {source, ds, bs}, {weight, ws.io_w.p, bw}};
   size_t off = 0;
   for (const Seg& g : segs)
-    for (size_t c = 0; c < g.bytes; c += kStageChunk) {
-      const size_t n = g.bytes - c < kStageChunk ? g.bytes - c : kStageChunk;
-      host_copy_mt(hin + off, static_cast<const unsigned char*>(g.src) + c, n);
-      PB_CUDA(cudaMemcpyAsync(static_cast<unsigned char*>(g.dev) + c, hin + off, n,
-                              cudaMemcpyHostToDevice, st));
+    for (size_t c = 0; c < g.bytes; c += kStagePiece) {
+      const size_t n = std::min(g.bytes - c, kStagePiece);
+      pieces.push_back({static_cast<const unsigned char*>(g.src) + c, hin + off,
+                        static_cast<unsigned char*>(g.dev) + c, n});
       off += n;
     }
+  std::vector<std::atomic<int>> there(pieces.size());
+  cudaError_t ce = cudaSuccess;
+  host_pieces(
+      pieces.size(), host_threads(off),
+      [&](size_t i) {
+        memcpy(pieces[i].host, pieces[i].src, pieces[i].bytes);
+        there[i].store(1, std::memory_order_release);
+      },
+      [&](auto& take) {
+        for (size_t i = 0; i < pieces.size(); ++i) {
+          while (!there[i].load(std::memory_order_acquire))
+            if (!take()) std::this_thread::yield();
+          if (ce == cudaSuccess)
+            ce = cudaMemcpyAsync(pieces[i].dev, pieces[i].host, pieces[i].bytes,
+                                 cudaMemcpyHostToDevice, st);
+        }
+      });
+  PB_CUDA(ce);
   // the result comes back into a zeroed buffer and is added to the caller's
   // output on the host (accumulate semantics without uploading the output)
   PB_CUDA(cudaMemsetAsync(ws.io_out.p, 0, bo, st));
@@ -1194,32 +1208,46 @@ int pbbfmm_compute(pbbfmm_tree* t, const double* target, int64_t Nf, const doubl
                              ws.io_out.as<double>(), t->precision, st);
   if (rc) return rc;
   double* hout = static_cast<double*>(ws.h_out);
-  const size_t chunk_d = kStageChunk / sizeof(double);
+  const size_t piece_d = kStagePiece / sizeof(double);
   const size_t total_d = (size_t)Nf * nCols;
-  std::vector<cudaEvent_t> evs;
-  for (size_t c = 0; c < total_d; c += chunk_d) {
-    const size_t n = total_d - c < chunk_d ? total_d - c : chunk_d;
+  struct Events : std::vector<cudaEvent_t> {
+    ~Events() {
+      for (cudaEvent_t e : *this) cudaEventDestroy(e);
+    }
+  } evs;
+  for (size_t c = 0; c < total_d; c += piece_d) {
+    const size_t n = std::min(total_d - c, piece_d);
     PB_CUDA(cudaMemcpyAsync(hout + c, ws.io_out.as<double>() + c, n * sizeof(double),
                             cudaMemcpyDeviceToHost, st));
     cudaEvent_t e;
     PB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    PB_CUDA(cudaEventRecord(e, st));
     evs.push_back(e);
+    PB_CUDA(cudaEventRecord(e, st));
   }
-  int status = PBBFMM_OK;
-  size_t k = 0;
-  for (size_t c = 0; c < total_d; c += chunk_d, ++k) {
-    const size_t n = total_d - c < chunk_d ? total_d - c : chunk_d;
-    cudaError_t e = cudaEventSynchronize(evs[k]);
-    if (e != cudaSuccess && status == PBBFMM_OK) status = cuda_status(e, "result copy");
-    // The compute's kernels finished before the first result chunk landed,
-    // so a timed-out tensor-core wait has set its flag by now: nothing is
-    // added to the caller's output from an invalid compute.
-    if (k == 0 && status == PBBFMM_OK) status = take_tc_timeout(t);
-    if (status == PBBFMM_OK) host_add_mt(output + c, hout + c, n);
-  }
-  for (cudaEvent_t e : evs) cudaEventDestroy(e);
-  return status;
+  PB_CUDA(cudaEventSynchronize(evs[0]));
+  // The compute's kernels finished before the first piece of the result
+  // landed, so a timed-out tensor-core wait has set its flag by now: nothing is
+  // added to the caller's output from an invalid compute.
+  if ((rc = take_tc_timeout(t))) return rc;
+  std::atomic<int> bad{(int)cudaSuccess};
+  host_pieces(
+      evs.size(), host_threads(bo),
+      [&](size_t k) {
+        cudaError_t e = cudaSetDevice(t->device);
+        if (e == cudaSuccess) e = cudaEventSynchronize(evs[k]);
+        if (e != cudaSuccess) {
+          bad = (int)e;
+          return;
+        }
+        const size_t a = k * piece_d, b = std::min(a + piece_d, total_d);
+        for (size_t i = a; i < b; ++i) output[i] += hout[i];
+      },
+      [](auto& take) {
+        while (take()) {
+        }
+      });
+  PB_CUDA((cudaError_t)bad.load());
+  return PBBFMM_OK;
 }
 
 int pbbfmm_set_tensor_cores(pbbfmm_tree* t, int mode) {
