@@ -456,24 +456,24 @@ def per_step(kt, steps):
 
 # DRAM bytes per (cell, frequency, column) of the frequency-domain M2L, from
 # the ncu capture in profiles/k_m2l_unif_tc_expcov0.3_unif5_N262144_C8_L5.md
-# (the level-5 launch of k_m2l_unif_tc: 1021.17 MB read + 815.66 MB written
-# for 32,768 cells x 405 frequencies x 8 columns)
-MAC_DRAM_BYTES_PER_UNIT = (1021.168e6 + 815.659e6) / (32768 * 405 * 8)
-# tensor-core MAC tiling (csrc/m2l_unif_tc.cu): 8 target lines of 16 parents
-# per CTA, 3 x 10 source lines per frequency, 6 MMAs (M = 128, K = 16) per
-# source line with N = 32 x (target lines it serves)
-UT_BY, UT_LINE = 8, 16
+# (the level-5 launch of k_m2l_unif_tc: 979.03 MB read + 725.68 MB written
+# for 32,768 cells x 365 frequencies x 8 columns)
+MAC_DRAM_BYTES_PER_UNIT = (979.034e6 + 725.678e6) / (32768 * 365 * 8)
+# tensor-core MAC tiling (csrc/m2l_unif_tc.cu): items of 8 x 1 x 16 target
+# parents at one frequency, 10 source planes per item, 18 MMAs (M = 128,
+# K = 16) per plane with N = 32 x (target planes it serves)
+UT_BX, UT_LINE = 8, 16
 
 
 def unif_tc_issued_flops(L, nk):
     """Tensor-pipe flops the MMAs of k_m2l_unif_tc issue per step (empty
-    source lines skipped at run time are counted: an upper bound)."""
-    nl = [min(UT_BY - 1, sy + 1) - max(0, sy - 1) + 1 for sy in range(-1, UT_BY + 1)]
-    per_cta_freq = 3 * sum(6 * 128 * 32 * k * 16 * 2 for k in nl)
+    source planes skipped at run time are counted: an upper bound)."""
+    served = [min(UT_BX - 1, sx + 1) - max(0, sx - 1) + 1 for sx in range(-1, UT_BX + 1)]
+    per_item = sum(18 * 128 * 32 * k * 16 * 2 for k in served)
     total = 0
     for l in range(5, L + 1):
         S = 1 << (l - 1)
-        total += S * (S // UT_BY) * (S // UT_LINE) * nk * per_cta_freq
+        total += (S // UT_BX) * S * (S // UT_LINE) * nk * per_item
     return float(total)
 
 
@@ -487,7 +487,7 @@ def unif_roofline(fmm, tree, wl, results, steps, local_rank):
     pairs = interaction_pairs(tstart, wl["L"])
     n, C = wl["n"], wl["C"]
     m = 2 * n - 1
-    nk = m * m * n
+    nk = (m ** 3 + 1) // 2  # the other frequencies are conjugates
     flops = sum(pairs.values()) * nk * C * 8.0
     nonempty = {l: int((np.diff(tstart).reshape(-1, 8 ** (wl["L"] - l)).sum(1) > 0).sum())
                 for l in range(2, wl["L"] + 1)}
@@ -513,7 +513,9 @@ def unif_roofline(fmm, tree, wl, results, steps, local_rank):
         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the level-5 "
                           "launch of bench.py --workload profile, scaled per (cell, frequency, "
                           "column); bytes per step",
-        "fp64_path": {"kernel": "k_m2l_unif_mac<double> (CUDA cores)",
+        "fp64_path": {"kernel": "k_m2l_unif_mac<double> (CUDA cores; 27 of the 56 "
+                                "products of a full parent pair, so frac counts work "
+                                "that it does not do)",
                       "achieved": flops / (mac64_ms * 1e-3) / 1e12, "peak": fp64_peak,
                       "frac": flops / (mac64_ms * 1e-3) / 1e12 / fp64_peak, "unit": "TFLOP/s"},
         "algorithmic": "%.4g useful flops per step = %d M2L pairs x %d freqs x %d cols x 8; "
@@ -543,6 +545,14 @@ def cheb_roofline(fmm, tree, wl, results, steps, local_rank):
     ms = kt["m2l"][0] / steps
     ms64 = results["fp64"]["ktimes"]["m2l"][0] / steps
     achieved = flops / (ms * 1e-3) / 1e12
+    # levels with nearly full parents take 702 combined products per parent
+    # instead of 1512 (csrc/cheb_kara.cuh)
+    done = 0.0
+    for l in pairs:
+        cnt = np.diff(tstart).reshape(-1, 8 ** (wl["L"] - l)).sum(1) > 0
+        a = cnt.sum() / max(1, int(cnt.reshape(-1, 8).any(1).sum()))
+        done += pairs[l] * (702 / 1512 if a * a > 36 else 1.0)
+    issued = 3.0 * done * rf * rs * C * 2.0
     fp64_peak = fmm.measure_fma_peak(local_rank, fmm.PREC_FP64)
     on_tc = fmt is not None
     kernels = {"f16": "k_m2l_cheb_tc (tcgen05 kind::f16, power-of-two scaled F16 hi/lo split, "
@@ -556,11 +566,11 @@ def cheb_roofline(fmm, tree, wl, results, steps, local_rank):
                         "TFLOP/s)" if fmt != "tf32" else
                         "dense TF32 = half the %s bf16 tensor figure of MEASURED_PEAKS.json "
                         "(%.0f TFLOP/s)") % (peak_kind, peaks["bf16_tflops"]),
-        "tensor_pipe_issued_frac": 3.0 * achieved / tc_peak,
+        "tensor_pipe_issued_frac": issued / (ms * 1e-3) / 1e12 / tc_peak,
         "algorithmic": "%.4g useful flops per step = %d M2L pairs x rf %d x rs %d x %d cols x 2"
                        % (flops, sum(pairs.values()), rf, rs, C),
         "launches_per_step": kt["m2l"][1] / steps,
-        "fp64_path": {"kernel": "k_m2l_cheb<double> (CUDA cores, rows compacted per offset)",
+        "fp64_path": {"kernel": "k_m2l_cheb_f64 (mma.sync f64, rows compacted per offset)",
                       "achieved": flops / (ms64 * 1e-3) / 1e12, "peak": fp64_peak,
                       "frac": flops / (ms64 * 1e-3) / 1e12 / fp64_peak, "unit": "TFLOP/s"},
     }
