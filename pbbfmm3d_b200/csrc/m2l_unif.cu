@@ -876,28 +876,39 @@ struct FftInvLaunch {
 };
 
 // Largest sum over a cell and column of |moments|, per column of the group
-// (float bits): a bound on |re| and |im| of its spectra.  Warps over cells.
+// (float bits): a bound on |re| and |im| of its spectra.  Warps over cells, lanes
+// over the moments, the 8 columns' loads in flight together; the 8 sums meet in
+// 9 shuffles, lane l ending with column l / 4.  Bound: HBM (one read of the
+// moments).  Against a column at a time with 5 shuffles each, 1M points, 8 columns:
+// forward phase 2.27 -> 2.18 ms.
 __global__ void k_moment_bound(const int* __restrict__ cells, int ncl, const float* __restrict__ S,
                                int C, int c0, int n3, uint32_t* __restrict__ amax) {
   const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
-  float mx[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) mx[c] = 0.f;
+  float mx = 0.f;
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < ncl; i += nw) {
     const float* s = S + ((int64_t)cells[i] * C + c0) * n3;
+    float v[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      float v = 0.f;
-      for (int l = lane; l < n3; l += 32) v += fabsf(s[c * n3 + l]);
+    for (int c = 0; c < 8; ++c) v[c] = 0.f;
+#pragma unroll 4
+    for (int l = lane; l < n3; l += 32) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      mx[c] = fmaxf(mx[c], v);
+      for (int c = 0; c < 8; ++c) v[c] += fabsf(s[c * n3 + l]);
     }
-  }
-  if (lane == 0)
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-      if (mx[c] > 0.f) atomicMax(&amax[c], __float_as_uint(mx[c]));
+    for (int h = 4; h > 0; h >>= 1) {  // the lanes of the upper half keep the upper columns
+      const bool up = (lane & (4 * h)) != 0;
+#pragma unroll
+      for (int c = 0; c < h; ++c) {
+        const float keep = up ? v[c + h] : v[c];
+        v[c] = keep + __shfl_xor_sync(0xffffffffu, up ? v[c] : v[c + h], 4 * h);
+      }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    mx = fmaxf(mx, v[0]);
+  }
+  if ((lane & 3) == 0 && mx > 0.f) atomicMax(&amax[lane >> 2], __float_as_uint(mx));
 }
 
 // Bytes of the spectra arrays X and Y (one level at a time uses them).
