@@ -542,10 +542,12 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kLeafBlocks<T, KC>)
 // neighbours' sources are staged 32 at a time; each lane sums its target's
 // pairs with every (32 / T')-th source of the tile, and its far field over
 // every (32 / T')-th row of coefficients; one reduction over the slots ends the
-// leaf.  A lane holds one target and one sum, so the kernel is a small loop:
-// with every target's sum in each lane and the targets unrolled, instruction
-// fetch was the top stall (4.7 of 12 cycles per instruction).  Measured against
-// that, leaf phase with exp(-r / l): 1M uniform points (3.8 per leaf), mixed
+// leaf.  Every pair goes into the lane's compensated sum by itself (plain float32
+// sums over a tile lose up to 2e-4 where large weights cancel, and were no
+// faster: 1.01 ms for the first of the figures below either way).  A lane holds
+// one target and one sum, so the kernel is a small loop: with every target's sum
+// in each lane and the targets unrolled, instruction fetch was the top stall (4.7
+// of 12 cycles per instruction).  Measured against that, leaf phase with exp(-r / l): 1M uniform points (3.8 per leaf), mixed
 // 2.13 -> 1.01 ms; 250,000 points (7.6 per leaf), float64 0.98 -> 0.59 ms.
 template <typename T>
 constexpr int kSingleBlocks = sizeof(T) == 4 ? 8 : 5;
@@ -649,7 +651,6 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kSingleBlocks<T>)
     }
     __syncwarp();
     if (mine) {
-      T part = 0;
 #pragma unroll 2
       for (int jj = slot; jj < m; jj += nslot) {
         const V4 sh = s_sh[wl][jj];
@@ -657,9 +658,8 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kSingleBlocks<T>)
         tp.diff(sh, s_sl[wl][kMixed ? jj : 0], d);
         T kv = KF::template eval<T>(d[0], d[1], d[2], kp);
         if (isinf(kv)) kv = 0;  // coincident points (include/compute.hpp:767)
-        part = fma(kv, sh.w, part);
+        acc.add(kv * sh.w);
       }
-      acc.add(part);
     }
   }
   double v = mine ? acc.value() : 0.0;
