@@ -882,9 +882,11 @@ __global__ void __launch_bounds__(32 * kLeafWarps, kSparseBlocks<T>)
 // holds the 4 x kGradCols sums of one target, the sources are staged once per
 // tile for all targets.  (One target at a time over all lanes gathered every
 // source again for each target and reduced 16 sums over 32 lanes: leaf phases of
-// forward and backward, 250,000 + 250,000 points, 4 columns, mixed 2.07 -> 1.36
+// forward and backward, 250,000 + 250,000 points, 4 columns, mixed 2.07 -> 1.39
 // ms; 30,000 + 20,011 points, 2 columns, float64, two gradients 0.38 -> 0.23 ms,
-// both with the forward phase in passes of 4 columns.)
+// both with the forward phase in passes of 4 columns.  The first is 1.36 ms with
+// plain float32 sums over a tile instead of every pair in the compensated sums,
+// which loses up to 2e-4 where large weights cancel.)
 constexpr int kGradCols = 4;  // columns per pass (4 accumulators each)
 constexpr int kGradT = 16;    // targets of a pass
 
@@ -997,29 +999,21 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
         }
         __syncwarp();
         if (mine) {
-          T pv[kGradCols], pg[kGradCols][3];  // the tile's sums
-#pragma unroll
-          for (int cc = 0; cc < kGradCols; ++cc) pv[cc] = pg[cc][0] = pg[cc][1] = pg[cc][2] = 0;
           for (int jj = slot; jj < m; jj += nslot) {
             T gk[3];
             T kv = KF::template grad<T>((T)(s_pos[wl][0][jj] - x), (T)(s_pos[wl][1][jj] - y),
                                         (T)(s_pos[wl][2][jj] - z), kp, gk);
             if (isinf(kv)) kv = 0;  // coincident points (include/compute.hpp:767)
 #pragma unroll
-            for (int cc = 0; cc < kGradCols; ++cc) {
-              const T w = s_w[wl][jj][cc];
-              pv[cc] = fma(kv, w, pv[cc]);
-              // d K(x, y_j) / d x = -dK/dd with d = y_j - x
-              pg[cc][0] = fma(-gk[0], w, pg[cc][0]);
-              pg[cc][1] = fma(-gk[1], w, pg[cc][1]);
-              pg[cc][2] = fma(-gk[2], w, pg[cc][2]);
-            }
-          }
-#pragma unroll
-          for (int cc = 0; cc < kGradCols; ++cc) {
-            v[cc].add(pv[cc]);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) g[cc][d].add(pg[cc][d]);
+            for (int cc = 0; cc < kGradCols; ++cc)
+              if (cc < cg) {
+                const T w = s_w[wl][jj][cc];
+                v[cc].add(kv * w);
+                // d K(x, y_j) / d x = -dK/dd with d = y_j - x
+                g[cc][0].add(-gk[0] * w);
+                g[cc][1].add(-gk[1] * w);
+                g[cc][2].add(-gk[2] * w);
+              }
           }
         }
       }

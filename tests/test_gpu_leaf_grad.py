@@ -9,7 +9,7 @@ import pytest
 
 import pbbfmm3d_b200 as fmm
 from helpers import make_tree
-from test_gpu_leaf_sizes import _per_leaf
+from test_gpu_leaf_sizes import _per_leaf, cancelling_sources, eight_leaves
 
 pytestmark = pytest.mark.gpu
 
@@ -43,4 +43,40 @@ def test_leaf_gradients(size, cols):
         # the kernel (1e-4) and, differentiated, ten times that
         assert (a - r).norm() < 2e-3 * n
         assert (a - b).norm() < 4e-5 * n
+    t.close()
+
+
+@pytest.mark.parametrize("cols", [1, 4])
+@pytest.mark.parametrize("size", [8, 11, 16])
+def test_gradient_sums_are_compensated_pair_by_pair(size, cols):
+    import torch
+
+    rng = np.random.default_rng(size)
+    src, w, bound = cancelling_sources()
+    tgt = eight_leaves(rng, size)
+    t = make_tree("Laplacian", 0.0, 1.0, 2, 3, 1e-6, 1)
+    t.buildFMMTree()
+    dev = lambda a: torch.tensor(a, device="cuda")
+    d = tgt - src[0]
+    r = np.linalg.norm(d, axis=1)
+    for prec, tol in ((fmm.PREC_FP64, 1e-11), (fmm.PREC_MIXED, bound + 1e-6)):
+        # forward: the targets' gradients sum over the sources
+        gt = torch.zeros(len(tgt), 3, dtype=torch.float64, device="cuda")
+        fmm.compute_adjoint_device(t, dev(tgt), dev(src), dev(np.tile(w, (cols, 1))),
+                                   dev(np.ones((cols, len(tgt)))), cols, grad_target=gt,
+                                   precision=prec)
+        ref = -cols * w.sum() * d / r[:, None] ** 3
+        err = np.linalg.norm(gt.cpu().numpy() - ref, axis=1) / np.linalg.norm(ref, axis=1)
+        assert err.max() < tol, prec
+        # transposed: the same points as targets (the corners keep the box), the
+        # weights' gradients sum over them
+        many = np.vstack([src, [[-0.22] * 3, [0.22] * 3]])
+        g = np.tile(np.append(w, [0.0, 0.0]), (cols, 1))
+        gw = torch.zeros(cols, len(tgt), dtype=torch.float64, device="cuda")
+        gs = torch.zeros(len(tgt), 3, dtype=torch.float64, device="cuda")
+        fmm.compute_adjoint_device(t, dev(many), dev(tgt), dev(np.ones((cols, len(tgt)))), dev(g),
+                                   cols, grad_weight=gw, grad_source=gs, precision=prec)
+        assert np.abs(gw.cpu().numpy() / (w.sum() / r) - 1).max() < tol, prec
+        err = np.linalg.norm(gs.cpu().numpy() - ref, axis=1) / np.linalg.norm(ref, axis=1)
+        assert err.max() < tol, prec
     t.close()
