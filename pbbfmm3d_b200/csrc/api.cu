@@ -58,20 +58,25 @@ int cuda_status(cudaError_t e, const char* what) {
   return PBBFMM_ERR_CUDA;
 }
 
+// cudaMalloc; on failure *p is null and the runtime's last error is cleared, so
+// that a later launch check does not report it again.
+int dev_alloc(void** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return PBBFMM_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  set_error("device allocation of " + std::to_string(bytes) + " bytes failed: " +
+            cudaGetErrorString(e));
+  return PBBFMM_ERR_ALLOC;
+}
+
 int grow(DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
   if (b.p && b.cap >= bytes) return PBBFMM_OK;
   if (b.p) cudaFree(b.p);
   b.p = nullptr;
   b.cap = 0;
-  cudaError_t e = cudaMalloc(&b.p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    b.p = nullptr;
-    set_error("device allocation of " + std::to_string(bytes) + " bytes failed: " +
-              cudaGetErrorString(e));
-    return PBBFMM_ERR_ALLOC;
-  }
+  if (int rc = dev_alloc(&b.p, bytes)) return rc;
   b.cap = bytes;
   return PBBFMM_OK;
 }
@@ -132,7 +137,7 @@ static float tf32_round(float x) {
 }
 
 static void free_tc_ops(TcOps* o) {
-  void* b[] = {o->eth, o->etl, o->eh16, o->el16, o->eexp, o->kh16, o->kl16, o->kexp, o->vth, o->vtl, o->uh, o->ul};
+  void* b[] = {o->eth, o->etl, o->eh16, o->el16, o->eexp, o->kh16, o->vth, o->vtl, o->uh, o->ul};
   for (void* p : b)
     if (p) cudaFree(p);
   *o = TcOps{};

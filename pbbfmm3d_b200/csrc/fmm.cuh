@@ -28,6 +28,7 @@ struct DevBuf {
   }
 };
 int grow(DevBuf& b, size_t bytes);  // PBBFMM_OK or PBBFMM_ERR_ALLOC
+int dev_alloc(void** p, size_t bytes);
 void release(DevBuf& b);
 
 // Device arrays of one compute, grown on demand and kept by the tree.
@@ -94,7 +95,7 @@ struct TcOps {
   uint16_t* el16 = nullptr;
   int* eexp = nullptr;
   // F16, made on first use: the combined operators of the dense levels, [level]
-  // [27][26] (cheb_kara.cuh), and their exponents
+  // [27][26] (cheb_kara.cuh), and their exponents, in one allocation at kh16
   uint16_t *kh16 = nullptr, *kl16 = nullptr;
   int* kexp = nullptr;
   int np = 0, kp = 0, kp16 = 0;

@@ -686,12 +686,19 @@ static int launch_f64(const FdArgs& a, int items, cudaStream_t st) {
 static int ensure_kara_ops(pbbfmm_tree* t, int64_t per_op, cudaStream_t st) {
   if (t->d_Ek) return PBBFMM_OK;
   const int nlev = t->ops.nlev;
-  PB_CUDA(cudaMalloc(&t->d_Ek, sizeof(double) * nlev * kKaraJ * kKaraD * per_op));
+  if (int rc = dev_alloc((void**)&t->d_Ek, sizeof(double) * nlev * kKaraJ * kKaraD * per_op))
+    return rc;
   k_kara_ops<<<dim3((unsigned)std::min<int64_t>((per_op + 255) / 256, 64), kKaraJ * kKaraD,
                     (unsigned)nlev),
                256, 0, st>>>(t->d_E, t->d_offs + 4 * (8 * FD_OFFS + kKaraJ * kKaraD), per_op,
                              t->d_Ek);
-  PB_LAUNCH("kara_ops");
+  count_launches(1);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {  // (a kernel's first launch may need memory of its own)
+    cudaFree(t->d_Ek);
+    t->d_Ek = nullptr;
+    return cuda_status(e, "kara_ops");
+  }
   return PBBFMM_OK;
 }
 

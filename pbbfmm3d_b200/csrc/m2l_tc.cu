@@ -703,23 +703,31 @@ static int launch_tc(const TcArgs& a, unsigned tiles, int smem, const CUtensorMa
   return PBBFMM_OK;
 }
 
-// The combined operators of the tree's current set (made on first use).
+// The combined operators of the tree's current set (made on first use): one
+// allocation, hi parts, lo parts, exponents, so that they are there as a whole or
+// not at all.
 static int ensure_kara_tc_ops(pbbfmm_tree* t, cudaStream_t st) {
   TcOps& o = t->tc;
   if (o.kh16) return PBBFMM_OK;
   constexpr int nops = kKaraJ * kKaraD;
   const int nlev = t->ops.nlev, rf = t->ops.rf, rs = t->ops.rs;
   const size_t n = (size_t)nlev * nops * o.np * o.kp16;
-  PB_CUDA(cudaMalloc(&o.kexp, sizeof(int) * nlev * nops));
-  PB_CUDA(cudaMalloc(&o.kl16, 2 * n));
-  PB_CUDA(cudaMalloc(&o.kh16, 2 * n));
+  if (int rc = dev_alloc((void**)&o.kh16, 4 * n + sizeof(int) * nlev * nops)) return rc;
+  o.kl16 = o.kh16 + n;
+  o.kexp = reinterpret_cast<int*>(o.kl16 + n);
   int nblk, ntb;
   cheb_fragment_blocks(rf, &nblk, &ntb);
   const int64_t per_blk = (int64_t)(cheb_rsp(rs) / 4) * ntb * 32;
   k_kara_ops_f16<<<dim3(nops, (unsigned)nlev), 256, 0, st>>>(
       t->d_E, t->d_offs + 4 * (8 * 189 + nops), rf, rs, ntb, per_blk, per_blk * nblk, o.np, o.kp16,
       reinterpret_cast<__half*>(o.kh16), reinterpret_cast<__half*>(o.kl16), o.kexp);
-  PB_LAUNCH("kara_ops_f16");
+  count_launches(1);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {  // (a kernel's first launch may need memory of its own)
+    cudaFree(o.kh16);
+    o.kh16 = nullptr;
+    return cuda_status(e, "kara_ops_f16");
+  }
   return PBBFMM_OK;
 }
 
