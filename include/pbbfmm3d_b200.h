@@ -228,6 +228,12 @@ int pbbfmm_tensor_core_m2l(const pbbfmm_tree *tree);
  * next compute runs normally once the limit is restored. */
 int pbbfmm_debug_set_pipeline_wait_limit(int device, long long polls);
 
+/* Test access to the arrays of the dense Chebyshev levels' combinations (no
+ * reference counterpart).  bound >= 0: the bytes that they may take at a time
+ * (8 GiB by default; 0: none, every level on its direct list); results differ by
+ * rounding only.  *held (may be NULL): the bytes they take now. */
+int pbbfmm_debug_combined_bytes(pbbfmm_tree *tree, int64_t bound, int64_t *held);
+
 /* Per-phase device times (ms) of the last compute, when timing is enabled
  * with pbbfmm_set_timing(tree, 1).  names: comma-separated phase names. */
 int pbbfmm_set_timing(pbbfmm_tree *tree, int enable);

@@ -74,6 +74,7 @@ EXPORTS = {
                                   ctypes.c_int),
     "pbbfmm_measure_fma_peak": ([ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double)], ctypes.c_int),
     "pbbfmm_debug_set_pipeline_wait_limit": ([ctypes.c_int, ctypes.c_longlong], ctypes.c_int),
+    "pbbfmm_debug_combined_bytes": ([_vp, _i64, ctypes.POINTER(_i64)], ctypes.c_int),
 }
 
 

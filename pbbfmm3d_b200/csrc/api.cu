@@ -621,9 +621,36 @@ static void host_pieces(size_t n, int nt, W work, O own) {
 static const char* kPhaseNames = "binning,upward,far_field,downward,near_field";
 constexpr int kNumPhases = 5;
 
-static int compute_chunk(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d_src,
-                         int64_t Ns, const double* d_w, int C, double* d_out, int precision,
-                         cudaStream_t st) {
+// Frees what the combinations of dense Chebyshev levels hold, which a call can do
+// without (the direct lists need none of it); false when there was nothing.
+static bool release_combined(pbbfmm_tree* t) {
+  bool any = false;
+  for (DevBuf* b : {&t->ws.kara_x, &t->ws.kara_y}) {
+    any |= b->p != nullptr;
+    release(*b);
+  }
+  for (double** e : {&t->d_Ek, &t->adj.Ek}) {
+    any |= *e != nullptr;
+    if (*e) cudaFree(*e);
+    *e = nullptr;
+  }
+  for (TcOps* o : {&t->tc, &t->adj.tc}) {
+    any |= o->kh16 != nullptr;
+    if (o->kh16) cudaFree(o->kh16);
+    o->kh16 = nullptr;
+  }
+  return any;
+}
+
+// grow() for a buffer that the call cannot do without
+static int grow_needed(pbbfmm_tree* t, DevBuf& b, size_t bytes) {
+  const int rc = grow(b, bytes);
+  return rc == PBBFMM_ERR_ALLOC && release_combined(t) ? grow(b, bytes) : rc;
+}
+
+// All phases ahead of the leaves: the first writes to the output are theirs.
+static int compute_far(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d_src,
+                       int64_t Ns, const double* d_w, int C, int precision, cudaStream_t st) {
   const int L = t->p.tree_level, n3 = t->n3;
   Workspace& ws = t->ws;
   int rc;
@@ -662,6 +689,26 @@ static int compute_chunk(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const 
   if (t->timing) PB_CUDA(cudaEventRecord(t->ev[3], st));
   if ((rc = run_downward(t, C, st))) return rc;
   if (t->timing) PB_CUDA(cudaEventRecord(t->ev[4], st));
+  return PBBFMM_OK;
+}
+
+static int compute_chunk(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d_src,
+                         int64_t Ns, const double* d_w, int C, double* d_out, int precision,
+                         cudaStream_t st) {
+  const size_t kused = t->kused;
+  int rc = compute_far(t, d_tgt, Nf, d_src, Ns, d_w, C, precision, st);
+  if (rc == PBBFMM_ERR_ALLOC && release_combined(t)) {
+    // once more in the memory of the direct lists
+    const int64_t bytes = t->kara_bytes;
+    t->kused = kused;
+    t->kara_bytes = 0;
+    rc = compute_far(t, d_tgt, Nf, d_src, Ns, d_w, C, precision, st);
+    t->kara_bytes = bytes;
+  }
+  if (rc) {
+    t->kused = kused;  // (no half pairs of timing events)
+    return rc;
+  }
   if ((rc = run_leaves(t, Nf, Ns, C, d_out, st))) return rc;
   if (t->timing) PB_CUDA(cudaEventRecord(t->ev[5], st));
   t->have_last = true;
@@ -1155,10 +1202,10 @@ int pbbfmm_compute(pbbfmm_tree* t, const double* target, int64_t Nf, const doubl
   const bool same = (source == target && Ns == Nf);
   const size_t bt = sizeof(double) * 3 * Nf, bs = same ? 0 : sizeof(double) * 3 * Ns;
   const size_t bw = sizeof(double) * (size_t)Ns * nCols, bo = sizeof(double) * (size_t)Nf * nCols;
-  if ((rc = grow(ws.io_tgt, bt))) return rc;
-  if (!same && (rc = grow(ws.io_src, bs ? bs : 16))) return rc;
-  if ((rc = grow(ws.io_w, bw ? bw : 16))) return rc;
-  if ((rc = grow(ws.io_out, bo))) return rc;
+  if ((rc = grow_needed(t, ws.io_tgt, bt))) return rc;
+  if (!same && (rc = grow_needed(t, ws.io_src, bs ? bs : 16))) return rc;
+  if ((rc = grow_needed(t, ws.io_w, bw ? bw : 16))) return rc;
+  if ((rc = grow_needed(t, ws.io_out, bo))) return rc;
   if ((rc = grow_pinned(&ws.h_in, &ws.h_in_cap, bt + bs + bw))) return rc;
   if ((rc = grow_pinned(&ws.h_out, &ws.h_out_cap, bo))) return rc;
   double* dt = ws.io_tgt.as<double>();
@@ -1334,6 +1381,16 @@ int pbbfmm_debug_copy(pbbfmm_tree* t, int what, int level, double* host, int64_t
   if (written) *written = total;
   int64_t nc = count < total ? count : total;
   if (host && nc > 0) PB_CUDA(cudaMemcpy(host, src, sizeof(double) * nc, cudaMemcpyDeviceToHost));
+  return PBBFMM_OK;
+}
+
+int pbbfmm_debug_combined_bytes(pbbfmm_tree* t, int64_t bound, int64_t* held) {
+  if (!t) {
+    set_error("null tree");
+    return PBBFMM_ERR_ARG;
+  }
+  if (bound >= 0) t->kara_bytes = bound;
+  if (held) *held = (int64_t)(t->ws.kara_x.cap + t->ws.kara_y.cap);
   return PBBFMM_OK;
 }
 

@@ -17,6 +17,13 @@ constexpr int kMaxLevel = 10;
 // offsets D != 0 (uniform M2L: m2l_unif.cu; float64 Chebyshev M2L:
 // m2l_cheb_f64.cu)
 constexpr int kKaraJ = 27, kKaraD = 26;
+// Bytes that the Chebyshev combinations of a call may hold at a time: room for
+// one column of the largest levels that are in use (level 7, r = 125: 4.8 GB), a
+// few per cent of the card, and so much work per launch (100 us at least) that
+// more groups cost nothing.
+constexpr int64_t kKaraBytes = (int64_t)8 << 30;
+// The next smaller amount to ask for.
+constexpr int64_t kara_less(int64_t bytes) { return bytes > ((int64_t)256 << 20) ? bytes / 4 : 0; }
 
 // Grow-only device buffer.
 struct DevBuf {
@@ -179,6 +186,7 @@ struct pbbfmm_tree {
     bool values = true;                // also add the potentials to the compute's output
   } gl;
   int cur_prec = PBBFMM_PREC_FP64;  // precision of the compute in flight
+  int64_t kara_bytes = pbbfmm::kKaraBytes;
   pbbfmm::Workspace ws;
   pbbfmm::LevelLists lists;
   // last compute (debug access)

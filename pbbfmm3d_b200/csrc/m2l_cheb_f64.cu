@@ -62,13 +62,12 @@ struct FdLevel {
   double* pf;           // [cell * C + col][rf]
   double* part;         // nsplit > 1: [split][row of the level][rf]
   const int* typed;     // targets ordered by (child type, parent); combined: target parents
-  const int* src;       // combined: nonempty source parents
-  int nsrc;
   int lev, span;
   // 0: rows are (cell, column) of the level, types are child types, 189
-  // offsets each; 27: combined, rows are (parent, combination, column), types
-  // are the combinations, 26 parent offsets each
-  int mult;
+  // offsets each; otherwise combined, rows are (parent, combination, column) of
+  // the `mult` combinations from j0 on, types are these, 26 parent offsets each
+  int mult, j0;
+  int C;                // columns of the rows
   int item0, nsplit;
   int row0, rows;       // (target, column) rows of the level, and of the levels before it
   int first[8];         // first list position of each type
@@ -77,9 +76,9 @@ struct FdLevel {
 };
 
 struct FdArgs {
-  FdLevel lv[kMaxLevel - 1];
+  FdLevel lv[kChebParts];
   int nlev;
-  int C, rf, rsp;       // rsp: rs padded to a multiple of 4
+  int rf, rsp;          // rsp: rs padded to a multiple of 4
   int nblk, ntb;        // column blocks, column groups of 8 per block
   const int* sstart;
   const int* offs;      // [8][189] (ox, oy, oz, operator), then [27][26] of the combinations
@@ -158,20 +157,21 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
   const int split = local % lv.nsplit, rest = local / lv.nsplit;
   const int nb = rest % a.nblk, tile = rest / a.nblk;
   const int ntb = a.ntb;  // column groups of a block
+  const int C = lv.C;
   const int4* offs = reinterpret_cast<const int4*>(a.offs);
   int type = 0, r0, nrow, first = 0, noff = FD_OFFS, mult = 1, comb = 0;
   if (lv.mult) {  // tile0[0] tiles per combination
     type = comb = tile / lv.tile0[0];
     r0 = (tile - type * lv.tile0[0]) * FD_R;  // first row within the type
-    nrow = min(FD_R, lv.count[0] * a.C - r0);
-    offs += 8 * FD_OFFS + type * kKaraD;
+    nrow = min(FD_R, lv.count[0] * C - r0);
+    offs += 8 * FD_OFFS + (lv.j0 + type) * kKaraD;
     noff = kKaraD;
-    mult = kKaraJ;
+    mult = lv.mult;
   } else {
     for (int i = 1; i < 8; ++i)
       if (tile >= lv.tile0[i]) type = i;
     r0 = (tile - lv.tile0[type]) * FD_R;
-    nrow = min(FD_R, lv.count[type] * a.C - r0);
+    nrow = min(FD_R, lv.count[type] * C - r0);
     first = lv.first[type];
     offs += type * FD_OFFS;
   }
@@ -188,11 +188,11 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
     int v = -1;
     if (tid < nrow) {
       int x, y, z;
-      morton_decode((uint32_t)lv.typed[first + (r0 + tid) / a.C], &x, &y, &z);
+      morton_decode((uint32_t)lv.typed[first + (r0 + tid) / C], &x, &y, &z);
       v = (x << 20) | (y << 10) | z;
     }
     s_xyz[tid] = v;
-    s_flat[tid] = first * a.C + r0 + tid;
+    s_flat[tid] = first * C + r0 + tid;
   }
   for (int i = tid; i < FD_R * pitch / 2; i += FD_THREADS)
     reinterpret_cast<double2*>(Sum)[i] = make_double2(0.0, 0.0);
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
     const int xyz = s_xyz[tid];
     const long long cell =
         morton_encode((xyz >> 20) + d.x, ((xyz >> 10) & 1023) + d.y, (xyz & 1023) + d.z);
-    s_src[q % SL][pos] = ((cell * mult + comb) * a.C + s_flat[tid] % a.C) * a.rsp;
+    s_src[q % SL][pos] = ((cell * mult + comb) * C + s_flat[tid] % C) * a.rsp;
     s_row[q % SL][pos] = (uint8_t)tid;
   };
   // the next iteration to load: chunk lc of valid offset lq, into stage lst.  A: granules
@@ -378,8 +378,8 @@ __global__ void __launch_bounds__(FD_THREADS, 2) k_m2l_cheb_f64(const __grid_con
     const int flat = s_flat[r];
     double* dst =
         lv.nsplit > 1
-            ? lv.part + ((int64_t)split * lv.rows + (int64_t)comb * lv.count[0] * a.C + flat) * a.rf
-            : lv.pf + (((int64_t)lv.typed[flat / a.C] * mult + comb) * a.C + flat % a.C) * a.rf;
+            ? lv.part + ((int64_t)split * lv.rows + (int64_t)comb * lv.count[0] * C + flat) * a.rf
+            : lv.pf + (((int64_t)lv.typed[flat / C] * mult + comb) * C + flat % C) * a.rf;
     for (int n = lane; n < ncol; n += 32) dst[col0 + n] = Sum[r * pitch + n];
   }
 }
@@ -393,10 +393,10 @@ __global__ void k_m2l_parts(const __grid_constant__ FdArgs a, int nrows) {
     if (r >= a.lv[i].row0) li = i;
   const FdLevel& lv = a.lv[li];
   const int flat = r - lv.row0;
-  const int per = lv.mult ? lv.count[0] * a.C : lv.rows;  // rows of a combination
+  const int per = lv.mult ? lv.count[0] * lv.C : lv.rows;  // rows of a combination
   const int comb = flat / per, f2 = flat % per;
-  double* dst = lv.pf + (((int64_t)lv.typed[f2 / a.C] * (lv.mult ? kKaraJ : 1) + comb) * a.C +
-                         f2 % a.C) * a.rf;
+  double* dst = lv.pf + (((int64_t)lv.typed[f2 / lv.C] * (lv.mult ? lv.mult : 1) + comb) * lv.C +
+                         f2 % lv.C) * a.rf;
   for (int n = lane; n < a.rf; n += 32) {
     double v = 0.0;
     for (int s = 0; s < lv.nsplit; ++s) v += lv.part[((int64_t)s * lv.rows + flat) * a.rf + n];
@@ -404,22 +404,25 @@ __global__ void k_m2l_parts(const __grid_constant__ FdArgs a, int nrows) {
   }
 }
 
-// Combined proxies of the listed source parents: warp per (parent, column).
+// Combined proxies j0 <= j < j0 + nj of columns [c0, c0 + nc) of the listed source
+// parents: warp per (parent, column).
 __global__ void k_kara_in(const int* __restrict__ parents, int np, const int* __restrict__ sstart,
                           int span, const double* __restrict__ proxy, double* __restrict__ kx,
-                          int C, int rsp) {
+                          int C, int c0, int nc, int j0, int nj, int rsp) {
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (w >= (int64_t)np * C) return;
-  const int64_t p = parents[w / C];
-  const int c = (int)(w % C);
+  if (w >= (int64_t)np * nc) return;
+  const int64_t p = parents[w / nc];
+  const int c = (int)(w % nc);
   const unsigned present = children_present(sstart, p, span);
   for (int k = lane; k < rsp; k += 32) {
     double v[8];
 #pragma unroll
     for (int ch = 0; ch < 8; ++ch)
-      v[ch] = ((present >> ch) & 1) ? proxy[((8 * p + ch) * C + c) * rsp + k] : 0.0;
-    kara_combine(v, [&](int j, double x) { kx[((p * kKaraJ + j) * C + c) * rsp + k] = x; });
+      v[ch] = ((present >> ch) & 1) ? proxy[((8 * p + ch) * C + c0 + c) * rsp + k] : 0.0;
+    kara_combine(v, [&](int j, double x) {
+      if ((unsigned)(j - j0) < (unsigned)nj) kx[((p * nj + j - j0) * nc + c) * rsp + k] = x;
+    });
   }
 }
 
@@ -702,62 +705,57 @@ static int ensure_kara_ops(pbbfmm_tree* t, int64_t per_op, cudaStream_t st) {
   return PBBFMM_OK;
 }
 
-static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
+// The parts of the far field and their arrays.  What the combinations need is not
+// needed by the direct lists: where it cannot be allocated, less is asked for, in
+// the end nothing.
+static int plan_m2l_f64(pbbfmm_tree* t, int C, int64_t per_op, ChebPlan* plan, cudaStream_t st) {
   const int L = t->p.tree_level, rf = t->ops.rf, rsp = cheb_rsp(t->ops.rs);
+  bool dense[kMaxLevel + 1] = {}, used[kMaxLevel + 1] = {};
+  for (int l = 2; l <= L; ++l) {
+    used[l] = t->lists.ntgt[l] > 0;
+    dense[l] = cheb_kara_level(t, l);
+  }
+  for (int64_t bound = t->kara_bytes;; bound = kara_less(bound)) {
+    *plan = cheb_plan(dense, used, L, C, 8 * rsp, 8 * rf, 0, bound);
+    if (plan->y_bytes == 0) return PBBFMM_OK;
+    int rc = ensure_kara_ops(t, per_op, st);
+    if (!rc) rc = grow(t->ws.kara_x, plan->x_bytes);
+    if (!rc) rc = grow(t->ws.kara_y, plan->y_bytes);
+    if (rc != PBBFMM_ERR_ALLOC) return rc;
+  }
+}
+
+static int launch_m2l_f64(pbbfmm_tree* t, int C, const std::vector<ChebPart>& parts, FdArgs a,
+                          int64_t per_op, int nsm, cudaStream_t st) {
+  const int L = t->p.tree_level, rf = t->ops.rf, rsp = a.rsp;
   Workspace& ws = t->ws;
-  // levels on the combined operators, and their arrays
-  bool kara[kMaxLevel + 1] = {};
-  int64_t kx_off[kMaxLevel + 1] = {}, ky_off[kMaxLevel + 1] = {}, kxn = 0, kyn = 0;
-  for (int l = 3; l <= L; ++l) {
-    kara[l] = cheb_kara_level(t, l);
-    if (!kara[l]) continue;
-    kx_off[l] = kxn;
-    ky_off[l] = kyn;
-    kxn += cells_at(l - 1) * kKaraJ * C * rsp;
-    kyn += cells_at(l - 1) * kKaraJ * C * rf;
-  }
-  if (kxn > 0) {
-    if (int rc = grow(ws.kara_x, sizeof(double) * kxn)) return rc;
-    if (int rc = grow(ws.kara_y, sizeof(double) * kyn)) return rc;
-  }
-  FdArgs a{};
-  a.C = C;
-  a.rf = rf;
-  a.rsp = rsp;
-  cheb_fragment_blocks(rf, &a.nblk, &a.ntb);
-  a.sstart = ws.sstart_p;
-  a.offs = t->d_offs;
-  int nsm = 148;
-  PB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, t->device));
-  // deepest level first: the shallow levels' few items fill the last wave
-  const int64_t per_op = (int64_t)rsp * a.nblk * a.ntb * 8;
   int64_t items = 0;
-  for (int l = L; l >= 2; --l) {
-    if (t->lists.ntgt[l] == 0) continue;
+  for (const ChebPart& q : parts) {
+    const int l = q.level;
     FdLevel& v = a.lv[a.nlev++];
-    if (kara[l]) {
-      if (int rc = ensure_kara_ops(t, per_op, st)) return rc;
+    v.C = q.nc;
+    if (q.nj) {
       const int np = t->lists.ntgt[l - 1];
       v.E = t->d_Ek + (int64_t)(t->homog ? 0 : l - 2) * kKaraJ * kKaraD * per_op;
-      v.proxy = ws.kara_x.as<double>() + kx_off[l];
-      v.pf = ws.kara_y.as<double>() + ky_off[l];
+      v.proxy = ws.kara_x.as<double>() + q.x / 8;
+      v.pf = ws.kara_y.as<double>() + q.y / 8;
       v.typed = ws.lists.as<int>() + t->lists.tgt_off[l - 1];
-      v.src = ws.lists.as<int>() + t->lists.src_off[l - 1];
-      v.nsrc = t->lists.nsrc[l - 1];
       v.lev = l - 1;
       v.span = (int)cells_at(L - l + 1);
-      v.mult = kKaraJ;
+      v.mult = q.nj;
+      v.j0 = q.j0;
       v.count[0] = np;
-      v.tile0[0] = (int)(((int64_t)np * C + FD_R - 1) / FD_R);
-      v.tile0[8] = kKaraJ * v.tile0[0];
-      v.rows = kKaraJ * np * C;
+      v.tile0[0] = (int)(((int64_t)np * q.nc + FD_R - 1) / FD_R);
+      v.tile0[8] = q.nj * v.tile0[0];
+      v.rows = q.nj * np * q.nc;
       items += (int64_t)v.tile0[8] * a.nblk;
-      const int64_t warps = (int64_t)v.nsrc * C;
+      const int ns = t->lists.nsrc[l - 1];
+      const int64_t warps = (int64_t)ns * q.nc;
       if (warps > 0) {
         k_kara_in<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
-            v.src, v.nsrc, ws.sstart_p, (int)cells_at(L - l),
+            ws.lists.as<int>() + t->lists.src_off[l - 1], ns, ws.sstart_p, (int)cells_at(L - l),
             ws.proxy.as<double>() + level_offset(l, (int64_t)C * rsp),
-            ws.kara_x.as<double>() + kx_off[l], C, rsp);
+            ws.kara_x.as<double>() + q.x / 8, C, q.c0, q.nc, q.j0, q.nj, rsp);
         PB_LAUNCH("kara_in");
       }
       continue;
@@ -779,23 +777,27 @@ static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
     v.rows = t->lists.ntyp[l][8] * C;
     items += (int64_t)tiles * a.nblk;
   }
-  const int nsplit = m2l_cheb_f64_split(items, nsm);
-  int64_t part = 0, rows = 0;
-  items = 0;
-  for (int i = 0; i < a.nlev; ++i) {
-    FdLevel& v = a.lv[i];
-    v.item0 = (int)items;
-    // (of the combinations' 26 offsets at least 6 to a part)
-    v.nsplit = v.mult ? std::min(nsplit, kKaraD / 6) : nsplit;
-    v.row0 = (int)rows;
-    items += (int64_t)v.tile0[8] * a.nblk * v.nsplit;
-    if (v.nsplit == 1) continue;
-    rows += v.rows;
-    part += (int64_t)v.nsplit * v.rows * rf;
-  }
   if (items == 0) return PBBFMM_OK;
+  int64_t part = 0, rows = 0;
+  // (without the parts where there is no room for them)
+  for (int nsplit = m2l_cheb_f64_split(items, nsm);; nsplit = 1) {
+    items = part = rows = 0;
+    for (int i = 0; i < a.nlev; ++i) {
+      FdLevel& v = a.lv[i];
+      v.item0 = (int)items;
+      // (of the combinations' 26 offsets at least 6 to a part)
+      v.nsplit = v.mult ? std::min(nsplit, kKaraD / 6) : nsplit;
+      v.row0 = (int)rows;
+      items += (int64_t)v.tile0[8] * a.nblk * v.nsplit;
+      if (v.nsplit == 1) continue;
+      rows += v.rows;
+      part += (int64_t)v.nsplit * v.rows * rf;
+    }
+    const int rc = rows > 0 ? grow(ws.m2l_part, sizeof(double) * part) : PBBFMM_OK;
+    if (!rc) break;
+    if (rc != PBBFMM_ERR_ALLOC) return rc;
+  }
   if (rows > 0) {
-    if (int rc = grow(ws.m2l_part, sizeof(double) * part)) return rc;
     double* p = ws.m2l_part.as<double>();
     for (int i = 0; i < a.nlev; ++i) {
       if (a.lv[i].nsplit == 1) continue;
@@ -829,15 +831,29 @@ static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
     k_m2l_parts<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a, (int)rows);
     PB_LAUNCH("m2l_parts");
   }
-  for (int l = 3; l <= L; ++l) {
-    const int64_t warps = (int64_t)t->lists.ntgt[l - 1] * C;
-    if (!kara[l] || warps == 0) continue;
-    k_kara_out<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
-        ws.lists.as<int>() + t->lists.tgt_off[l - 1], t->lists.ntgt[l - 1],
-        ws.kara_y.as<double>() + ky_off[l],
-        ws.pf.as<double>() + level_offset(l, (int64_t)C * rf), C, rf);
-    PB_LAUNCH("kara_out");
-  }
+  for (const ChebPart& q : parts)
+    if (q.nj && t->lists.ntgt[q.level - 1] > 0)
+      if ((rc = launch_kara_out(t, q, ws.kara_y.as<double>() + q.y / 8,
+                                ws.pf.as<double>() + level_offset(q.level, (int64_t)C * rf), C, rf,
+                                st)))
+        return rc;
+  return PBBFMM_OK;
+}
+
+static int run_m2l_f64(pbbfmm_tree* t, int C, cudaStream_t st) {
+  FdArgs a{};
+  a.rf = t->ops.rf;
+  a.rsp = cheb_rsp(t->ops.rs);
+  cheb_fragment_blocks(a.rf, &a.nblk, &a.ntb);
+  a.sstart = t->ws.sstart_p;
+  a.offs = t->d_offs;
+  int nsm = 148;
+  PB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, t->device));
+  const int64_t per_op = (int64_t)a.rsp * a.nblk * a.ntb * 8;
+  ChebPlan plan;
+  if (int rc = plan_m2l_f64(t, C, per_op, &plan, st)) return rc;
+  for (const std::vector<ChebPart>& parts : plan.launches)
+    if (int rc = launch_m2l_f64(t, C, parts, a, per_op, nsm, st)) return rc;
   return PBBFMM_OK;
 }
 

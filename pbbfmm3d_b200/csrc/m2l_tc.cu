@@ -869,7 +869,7 @@ int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
     if (!kara[l] || warps == 0) continue;
     k_kara_out<float><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
         lists + t->lists.tgt_off[l - 1], t->lists.ntgt[l - 1], ws.kara_y.as<float>() + koff[l],
-        ws.pf.as<float>() + level_offset(l, (int64_t)C * rf), C, rf);
+        ws.pf.as<float>() + level_offset(l, (int64_t)C * rf), C, 0, C, rf);
     PB_LAUNCH("kara_out");
   }
   return kt_end(t, st);

@@ -78,3 +78,92 @@ def test_combined_operators_that_do_not_fit():
     torch.cuda.empty_cache()
     assert rel(run(t, p, w, fmm.PREC_MIXED), ref) < 2e-6
     t.close()
+
+
+def combined_bytes(t, bound=-1):
+    """Sets the bound on the arrays of the combinations; the bytes they take."""
+    import ctypes
+
+    held = ctypes.c_int64()
+    _lib.check(_lib.lib().pbbfmm_debug_combined_bytes(t._h, bound, ctypes.byref(held)))
+    return held.value
+
+
+def coefficient_bytes(t, level, order, cols, width):
+    """Moments, locals, proxies and sums of levels 2 to `level`."""
+    o = t.get_operators()
+    return sum(8 ** l for l in range(2, level + 1)) * cols * width * (
+        2 * order ** 3 + o["rf"] + o["rs"])
+
+
+def test_dense_levels_run_without_room_for_combinations():
+    """Room for the level arrays but not for the combinations of dense levels:
+    the direct lists run.  Room that the combinations of an earlier call hold is
+    given back to a call that needs it."""
+    level, order, cols, n = 5, 4, 8, 100000
+    t = make_tree("Laplacian", 0.0, 1.0, level, order, 1e-5, 1)
+    t.buildFMMTree()
+    p, w = points(n, 1), weights(cols, n, 2)
+    ref = run(t, p, w, fmm.PREC_FP64)
+    held = combined_bytes(t)
+    needed = coefficient_bytes(t, level, order, cols, 8)
+    assert held > 1.3 * needed
+    t.close()
+    import torch
+
+    t = make_tree("Laplacian", 0.0, 1.0, level, order, 1e-5, 1)
+    t.buildFMMTree()
+    full = fill_but(needed + 200 * MB)
+    assert rel(run(t, p, w, fmm.PREC_FP64), ref) < 1e-13
+    assert combined_bytes(t) < 200 * MB
+    del full
+    torch.cuda.empty_cache()
+    run(t, p, w, fmm.PREC_FP64)
+    assert combined_bytes(t) == held
+    # 16 columns: twice the level arrays, in less than what the combinations hold
+    w2 = weights(2 * cols, n, 3)
+    full = fill_but(needed // 2)
+    two = run(t, p, w2, fmm.PREC_FP64)
+    assert combined_bytes(t) < held
+    del full
+    torch.cuda.empty_cache()
+    assert rel(run(t, p, w2, fmm.PREC_FP64), two) < 1e-13
+    t.close()
+
+
+# Laplacian, order 4 (r = 48), level 4: the combinations of a level's column take
+# 512, 64 and 8 parents x 27 x 96 values
+COLUMN = 512 * 27 * 96
+
+
+@pytest.mark.parametrize("cols", [1, 5])
+@pytest.mark.parametrize("share", [1.02, 2.02, 0.35, 0.7, 0.13, 0.0],
+                         ids=["column", "columns", "third", "two_thirds", "shallow", "none"])
+def test_groups_of_combinations(share, cols):
+    """Groups of columns, groups of 9 combinations of one column, the direct list
+    below that, level by level: equal but for rounding."""
+    t = make_tree("Laplacian", 0.0, 1.0, 4, 4, 1e-5, 1)
+    t.buildFMMTree()
+    p, w = points(20000, 5), weights(cols, 20000, 6)
+    ref = run(t, p, w, fmm.PREC_FP64)
+    all_held = combined_bytes(t)
+    t.close()
+    t = make_tree("Laplacian", 0.0, 1.0, 4, 4, 1e-5, 1)
+    t.buildFMMTree()
+    bound = int(share * COLUMN * 8)
+    combined_bytes(t, bound)
+    assert rel(run(t, p, w, fmm.PREC_FP64), ref) < 1e-13
+    held = combined_bytes(t)
+    assert held <= bound < all_held or bound >= all_held
+    assert (held > 0) == (share > 0)
+    g = weights(cols, 20000, 7)
+    import torch
+
+    got = []
+    for b in (bound, 1 << 40):
+        combined_bytes(t, b)
+        o = torch.zeros(cols, 20000, dtype=torch.float64, device="cuda")
+        fmm.compute_adjoint_device(t, p, p, w, g, cols, grad_weight=o)
+        got.append(o.cpu().numpy())
+    assert rel(got[0], got[1]) < 1e-13
+    t.close()
