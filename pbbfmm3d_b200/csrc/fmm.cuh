@@ -57,8 +57,10 @@ struct Workspace {
   DevBuf proxy;  // Cheb: sum_l 8^l * C * rs ;  Unif: spectra of one level
   DevBuf pf;     // Cheb: sum_l 8^l * C * rf ;  Unif: accumulated spectra of one level
   DevBuf halo;   // Unif M2L: per parent block, region and target parents and their occupancy
-  DevBuf tc_proxy;  // tensor-core Cheb M2L: per level hi then lo proxies (+ F16 exponents)
-  DevBuf kara_x, kara_y;  // Cheb M2L: combined proxies (float64) and sums of dense levels
+  DevBuf tc_proxy;  // tensor-core Cheb M2L: direct levels' hi then lo proxies (+ F16 exponents)
+  // Cheb M2L: combined proxies (tensor cores: as tc_proxy) and sums of dense
+  // levels, bounded (cheb_plan)
+  DevBuf kara_x, kara_y;
   DevBuf m2l_part;  // float64 Cheb M2L: partial sums of levels with few tiles
   DevBuf leafpart;  // leaf phase: target leaves dense-first, chunk prefix of the dense ones
   // the sources' leaf offsets, permutation and positions of the last binning

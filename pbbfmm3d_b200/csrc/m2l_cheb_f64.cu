@@ -405,10 +405,14 @@ __global__ void k_m2l_parts(const __grid_constant__ FdArgs a, int nrows) {
 }
 
 // Combined proxies j0 <= j < j0 + nj of columns [c0, c0 + nc) of the listed source
-// parents: warp per (parent, column).
+// parents: warp per (parent, column).  NJ = nj (27: j0 is 0), fixed so
+// that the stores need no test of j.
+template <int NJ>
 __global__ void k_kara_in(const int* __restrict__ parents, int np, const int* __restrict__ sstart,
                           int span, const double* __restrict__ proxy, double* __restrict__ kx,
-                          int C, int c0, int nc, int j0, int nj, int rsp) {
+                          int C, int c0, int nc, int j0_, int rsp) {
+  constexpr int nj = NJ;
+  const int j0 = NJ == kKaraJ ? 0 : j0_;
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= (int64_t)np * nc) return;
@@ -752,10 +756,11 @@ static int launch_m2l_f64(pbbfmm_tree* t, int C, const std::vector<ChebPart>& pa
       const int ns = t->lists.nsrc[l - 1];
       const int64_t warps = (int64_t)ns * q.nc;
       if (warps > 0) {
-        k_kara_in<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
-            ws.lists.as<int>() + t->lists.src_off[l - 1], ns, ws.sstart_p, (int)cells_at(L - l),
-            ws.proxy.as<double>() + level_offset(l, (int64_t)C * rsp),
-            ws.kara_x.as<double>() + q.x / 8, C, q.c0, q.nc, q.j0, q.nj, rsp);
+        (q.nj == kKaraJ ? k_kara_in<kKaraJ> : k_kara_in<kKaraJ / 3>)
+            <<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
+                ws.lists.as<int>() + t->lists.src_off[l - 1], ns, ws.sstart_p, (int)cells_at(L - l),
+                ws.proxy.as<double>() + level_offset(l, (int64_t)C * rsp),
+                ws.kara_x.as<double>() + q.x / 8, C, q.c0, q.nc, q.j0, rsp);
         PB_LAUNCH("kara_in");
       }
       continue;

@@ -56,24 +56,25 @@ constexpr int TC_TMEM_COLS = 512;  // columns allocated (accumulators and runnin
 // keep the full bound.
 __device__ long long g_pipe_wait_iters = kWaitIters;
 
-// One level of the launch: its tiles of each child type, or (mult = 27, dense
-// levels, cheb_kara.cuh) of each combination of the children, whose rows are
-// (parent, combination, column) and whose offsets are 26 parent offsets.
+// One part of the launch (ChebPart): a level's tiles of each child type, or (mult
+// > 0, dense levels, cheb_kara.cuh) of each combination of the children, whose rows
+// are (parent, combination, column) and whose offsets are 26 parent offsets.
 struct TcLevel {
   const int* typed;                // targets by child type; combined: target parents
   const unsigned char *ph, *pl;    // proxy hi / lo, rows of rowb bytes
   const int* pexp;                 // F16: scale exponent of each row
   float* pf;                       // output rows of rf floats
   int lev, span, item0;            // item0: first tile of the level
-  int mult;                        // 1, or 27 (start[1] tiles per combination)
+  int mult;                        // 0: direct; combined: combinations from j0 on (start[1] tiles each)
+  int j0, C;                       // C: columns of the rows
   int op0;                         // first operator of the level
   int start[9];                    // first tile of each type; start[8] = total tiles
   int first[8];                    // first list position of each type
   int count[8];                    // targets of each type
 };
 struct TcArgs {
-  TcLevel lv[kMaxLevel - 1];
-  int nlev, C, rf, NP, rowb, group;
+  TcLevel lv[kChebParts];
+  int nlev, rf, NP, rowb, group;
   const int* sstart;
   const int* offs;                 // [8][189], then [27][26] (ox, oy, oz, operator)
   const int *eexp, *kexp;          // F16: scale exponents of the operators / combined ones
@@ -141,9 +142,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   for (int i = 1; i < a.nlev; ++i)
     if ((int)blockIdx.x >= a.lv[i].item0) li = i;
   const TcLevel& lv = a.lv[li];
-  const int rf = a.rf, NP = a.NP, rowb = a.rowb, C = a.C, lev = lv.lev, span = lv.span;
-  const int group = a.group, mult = lv.mult;
-  const bool kara = mult > 1;
+  const int rf = a.rf, NP = a.NP, rowb = a.rowb, C = lv.C, lev = lv.lev, span = lv.span;
+  const int group = a.group, mult = max(lv.mult, 1);
+  const bool kara = lv.mult > 0;
   const int* __restrict__ sstart = a.sstart;
   const int* __restrict__ typed = lv.typed;
   const unsigned char* __restrict__ Ph = lv.ph;
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     tstart = type * lv.start[1];
     tcount = lv.count[0];
     noff = kKaraD;
-    my_offs += 4 * (8 * 189 + type * kKaraD);
+    my_offs += 4 * (8 * 189 + (lv.j0 + type) * kKaraD);
   } else {
     for (int i = 1; i < 8; ++i)
       if (tile >= lv.start[i]) type = i;
@@ -547,24 +548,30 @@ __global__ void k_split_proxy_f16(const int* __restrict__ cells, int64_t nrows, 
   if (lane == 0) pexp[row] = e;
 }
 
-// The 27 combined proxies of each listed source parent (cheb_kara.cuh), split
-// as above into rows (parent 27 + j) C + column: warp per (parent, column), a
-// first pass over K for the rows' magnitudes, a second for the split.
+// Combined proxies j0 <= j < j0 + nj of columns [c0, c0 + nc) of each listed source
+// parent (cheb_kara.cuh), split as above into rows (parent nj + j - j0) nc + column:
+// warp per (parent, column), a first pass over K for the rows' magnitudes, a second
+// for the split.  NJ = nj (27: j0 is 0), fixed so that the stores need no test of j.
+template <int NJ>
 __global__ void k_split_kara_f16(const int* __restrict__ parents, int np,
-                                 const int* __restrict__ sstart, int span, int C, int rs, int KP,
-                                 const float* __restrict__ proxy, __half* __restrict__ ph,
-                                 __half* __restrict__ pl, int* __restrict__ pexp) {
+                                 const int* __restrict__ sstart, int span, int C, int c0, int nc,
+                                 int j0_, int rs, int KP, const float* __restrict__ proxy,
+                                 __half* __restrict__ ph, __half* __restrict__ pl,
+                                 int* __restrict__ pexp) {
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (w >= (int64_t)np * C) return;  // uniform over the warp
-  const int64_t p = parents[w / C];
-  const int c = (int)(w % C);
+  if (w >= (int64_t)np * nc) return;  // uniform over the warp
+  constexpr int nj = NJ;
+  const int j0 = NJ == kKaraJ ? 0 : j0_;
+  const int64_t p = parents[w / nc];
+  const int c = (int)(w % nc);
   const unsigned present = children_present(sstart, p, span);
   auto load = [&](int k, float* v) {
 #pragma unroll
     for (int ch = 0; ch < 8; ++ch)
-      v[ch] = ((present >> ch) & 1) && k < rs ? proxy[((8 * p + ch) * C + c) * rs + k] : 0.f;
+      v[ch] = ((present >> ch) & 1) && k < rs ? proxy[((8 * p + ch) * C + c0 + c) * rs + k] : 0.f;
   };
+  auto in = [&](int j) { return (unsigned)(j - j0) < (unsigned)nj; };
   float m[kKaraJ];
 #pragma unroll
   for (int j = 0; j < kKaraJ; ++j) m[j] = 0.f;
@@ -579,15 +586,16 @@ __global__ void k_split_kara_f16(const int* __restrict__ parents, int np,
 #pragma unroll
     for (int o = 16; o; o >>= 1) m[j] = fmaxf(m[j], __shfl_xor_sync(0xffffffffu, m[j], o));
     e[j] = m[j] > 0.f ? 15 - exponent_of(m[j]) : 0;
-    if (lane == 0) pexp[(p * kKaraJ + j) * C + c] = e[j];
+    if (lane == 0 && in(j)) pexp[(p * nj + j - j0) * nc + c] = e[j];
   }
   for (int k = lane; k < KP; k += 32) {
     float v[8];
     load(k, v);
     kara_combine(v, [&](int j, float x0) {
+      if (!in(j)) return;
       const float x = scale2(x0, e[j]);
       const __half h = __float2half_rn(x);
-      const int64_t at = ((p * kKaraJ + j) * C + c) * KP + k;
+      const int64_t at = ((p * nj + j - j0) * nc + c) * KP + k;
       ph[at] = h;
       pl[at] = __float2half_rn(x - __half2float(h));
     });
@@ -731,65 +739,54 @@ static int ensure_kara_tc_ops(pbbfmm_tree* t, cudaStream_t st) {
   return PBBFMM_OK;
 }
 
-// The tensor-core M2L of all levels: split the proxies, then one MMA launch
-// (deepest level first, so that the shallow ones fill the last wave).
-int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
-  const int L = t->p.tree_level, rf = t->ops.rf, rs = t->ops.rs;
-  const bool f16 = t->tc_fmt == PBBFMM_TC_F16;
-  const int NP = t->tc.np, KP = f16 ? t->tc.kp16 : t->tc.kp, esize = f16 ? 2 : 4;
-  const int rowb = KP * esize;  // a multiple of 128
+// The parts of the far field and their arrays (see plan_m2l_f64).  Direct levels
+// hold their split proxies together up to the same bound, or one level at a time
+// where that is larger.
+static int plan_m2l_tc(pbbfmm_tree* t, int C, bool f16, int rowb, ChebPlan* plan, cudaStream_t st) {
+  const int L = t->p.tree_level, rf = t->ops.rf, row = 2 * rowb + (f16 ? 4 : 0);
+  bool dense[kMaxLevel + 1] = {}, used[kMaxLevel + 1] = {};
+  for (int l = 2; l <= L; ++l) {
+    used[l] = t->lists.ntgt[l] > 0;
+    dense[l] = f16 && cheb_kara_level(t, l);
+  }
+  for (int64_t bound = t->kara_bytes;; bound = kara_less(bound)) {
+    *plan = cheb_plan(dense, used, L, C, row, 4 * rf, row, bound);
+    int rc = PBBFMM_OK;
+    if (plan->y_bytes > 0) {
+      rc = ensure_kara_tc_ops(t, st);
+      if (!rc) rc = grow(t->ws.kara_x, plan->x_bytes);
+      if (!rc) rc = grow(t->ws.kara_y, plan->y_bytes);
+    }
+    if (!rc) rc = grow(t->ws.tc_proxy, plan->direct_bytes);
+    if (rc != PBBFMM_ERR_ALLOC || bound == 0) return rc;
+  }
+}
+
+static int launch_m2l_tc(pbbfmm_tree* t, int C, const std::vector<ChebPart>& parts, TcArgs a,
+                         bool f16, int KP, const CUtensorMap* tm, cudaStream_t st) {
+  const int L = t->p.tree_level, rf = a.rf, rs = t->ops.rs, NP = a.NP, rowb = a.rowb;
   Workspace& ws = t->ws;
   const int* lists = ws.lists.as<int>();
-  if (C > TC_M) {
-    set_error("tensor-core M2L takes at most 128 columns per block");
-    return PBBFMM_ERR_UNSUPPORTED;
-  }
-  // per level: hi rows | lo rows | (F16) row exponents, then the combined sums
-  bool kara[kMaxLevel + 1] = {}, any_kara = false;
-  int64_t off[kMaxLevel + 1] = {}, total = 0, koff[kMaxLevel + 1] = {}, ktotal = 0;
-  auto rows_at = [&](int l) { return kara[l] ? cells_at(l - 1) * kKaraJ * C : cells_at(l) * C; };
-  for (int l = 2; l <= L; ++l) {
-    kara[l] = f16 && cheb_kara_level(t, l);
-    any_kara |= kara[l];
-    off[l] = total;
-    total += (rows_at(l) * (2 * rowb + (f16 ? 4 : 0)) + 255) / 256 * 256;
-    koff[l] = ktotal;
-    if (kara[l]) ktotal += rows_at(l) * rf;
-  }
   int rc;
-  if ((rc = grow(ws.tc_proxy, total))) return rc;
-  if (any_kara && (rc = grow(ws.kara_y, sizeof(float) * ktotal))) return rc;
-  if (any_kara && (rc = ensure_kara_tc_ops(t, st))) return rc;
-  TcArgs a{};
-  a.C = C;
-  a.rf = rf;
-  a.NP = NP;
-  a.rowb = rowb;
-  a.group = tc_group(NP, f16);
-  a.sstart = ws.sstart_p;
-  a.offs = t->d_offs;
-  a.eexp = t->tc.eexp;
-  a.kexp = t->tc.kexp;
-  a.err = t->d_tc_err;
-  const int per_tile = TC_M / C;
   int64_t tiles = 0;
   if ((rc = kt_begin(t, KS_M2L_SPLIT, st))) return rc;
-  for (int l = L; l >= 2; --l) {
-    if (t->lists.ntgt[l] == 0) continue;
-    const int lvl = t->homog ? 0 : l - 2;
-    const int64_t pbytes = rows_at(l) * rowb;
-    unsigned char* ph = ws.tc_proxy.as<unsigned char>() + off[l];
-    unsigned char* pl = ph + pbytes;
-    int* pexp = f16 ? reinterpret_cast<int*>(pl + pbytes) : nullptr;
+  for (const ChebPart& q : parts) {
+    const int l = q.level, lvl = t->homog ? 0 : l - 2, per_tile = TC_M / q.nc;
+    const bool kara = q.nj > 0;
+    const int64_t rows = kara ? cells_at(l - 1) * q.nj * q.nc : cells_at(l) * q.nc;
+    unsigned char* ph = (kara ? ws.kara_x : ws.tc_proxy).as<unsigned char>() + q.x;
+    unsigned char* pl = ph + rows * rowb;
+    int* pexp = f16 ? reinterpret_cast<int*>(pl + rows * rowb) : nullptr;
     const float* proxy = ws.proxy.as<float>() + level_offset(l, (int64_t)C * rs);
-    const int ns = t->lists.nsrc[kara[l] ? l - 1 : l];
-    const int* src = lists + t->lists.src_off[kara[l] ? l - 1 : l];
-    const int64_t nrows = (int64_t)ns * C;
+    const int ns = t->lists.nsrc[kara ? l - 1 : l];
+    const int* src = lists + t->lists.src_off[kara ? l - 1 : l];
+    const int64_t nrows = (int64_t)ns * q.nc;
     if (ns > 0) {
-      if (kara[l])
-        k_split_kara_f16<<<(unsigned)((nrows * 32 + 255) / 256), 256, 0, st>>>(
-            src, ns, ws.sstart_p, (int)cells_at(L - l), C, rs, KP, proxy,
-            reinterpret_cast<__half*>(ph), reinterpret_cast<__half*>(pl), pexp);
+      if (kara)
+        (q.nj == kKaraJ ? k_split_kara_f16<kKaraJ> : k_split_kara_f16<kKaraJ / 3>)
+            <<<(unsigned)((nrows * 32 + 255) / 256), 256, 0, st>>>(
+                src, ns, ws.sstart_p, (int)cells_at(L - l), C, q.c0, q.nc, q.j0, rs, KP, proxy,
+                reinterpret_cast<__half*>(ph), reinterpret_cast<__half*>(pl), pexp);
       else if (f16)
         k_split_proxy_f16<<<(unsigned)((nrows * 32 + 255) / 256), 256, 0, st>>>(
             src, nrows, C, rs, KP, proxy, reinterpret_cast<__half*>(ph),
@@ -805,22 +802,23 @@ int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
     v.pl = pl;
     v.pexp = pexp;
     v.item0 = (int)tiles;
-    v.mult = 1;
+    v.C = q.nc;
     v.lev = l;
     v.span = (int)cells_at(L - l);
     v.op0 = lvl * 316;
     v.typed = lists + t->lists.typ_off[l];
     v.pf = ws.pf.as<float>() + level_offset(l, (int64_t)C * rf);
-    if (kara[l]) {
-      v.mult = kKaraJ;
+    if (kara) {
+      v.mult = q.nj;
+      v.j0 = q.j0;
       v.lev = l - 1;
       v.span = (int)cells_at(L - l + 1);
       v.op0 = lvl * kKaraJ * kKaraD;
       v.typed = lists + t->lists.tgt_off[l - 1];
-      v.pf = ws.kara_y.as<float>() + koff[l];
+      v.pf = ws.kara_y.as<float>() + q.y / 4;
       v.count[0] = t->lists.ntgt[l - 1];
       v.start[1] = (v.count[0] + per_tile - 1) / per_tile;
-      v.start[8] = kKaraJ * v.start[1];
+      v.start[8] = q.nj * v.start[1];
     } else {
       int n = 0;
       for (int ty = 0; ty < 8; ++ty) {
@@ -838,19 +836,6 @@ int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
   // three stages when they fit in shared memory next to the static arrays
   const int nst = tc_smem_bytes(NP, 3) + 8192 <= 232448 ? 3 : 2;
   const int smem = tc_smem_bytes(NP, nst);
-  CUtensorMap tm[4];
-  const int64_t nrows = (int64_t)t->ops.nlev * 316 * NP;
-  const void* eh = f16 ? (const void*)t->tc.eh16 : (const void*)t->tc.eth;
-  const void* el = f16 ? (const void*)t->tc.el16 : (const void*)t->tc.etl;
-  if ((rc = operator_tensor_map(&tm[0], eh, f16, NP, KP, nrows))) return rc;
-  if ((rc = operator_tensor_map(&tm[1], el, f16, NP, KP, nrows))) return rc;
-  tm[2] = tm[0];
-  tm[3] = tm[1];
-  if (any_kara) {
-    const int64_t krows = (int64_t)t->ops.nlev * kKaraJ * kKaraD * NP;
-    if ((rc = operator_tensor_map(&tm[2], t->tc.kh16, true, NP, KP, krows))) return rc;
-    if ((rc = operator_tensor_map(&tm[3], t->tc.kl16, true, NP, KP, krows))) return rc;
-  }
   if ((rc = kt_begin(t, KS_M2L, st))) return rc;
   // register running sum up to TC_REG_SUM columns (three stages always fit there)
   const bool rsum = NP <= TC_REG_SUM && nst == 3;
@@ -864,15 +849,53 @@ int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
               : (nst == 3 ? launch_tc<3, false, false>(a, nt, smem, tm, st)
                           : launch_tc<2, false, false>(a, nt, smem, tm, st));
   if (rc) return rc;
-  for (int l = 3; l <= L; ++l) {
-    const int64_t warps = (int64_t)t->lists.ntgt[l - 1] * C;
-    if (!kara[l] || warps == 0) continue;
-    k_kara_out<float><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
-        lists + t->lists.tgt_off[l - 1], t->lists.ntgt[l - 1], ws.kara_y.as<float>() + koff[l],
-        ws.pf.as<float>() + level_offset(l, (int64_t)C * rf), C, 0, C, rf);
-    PB_LAUNCH("kara_out");
-  }
+  for (const ChebPart& q : parts)
+    if (q.nj && t->lists.ntgt[q.level - 1] > 0)
+      if ((rc = launch_kara_out(t, q, ws.kara_y.as<float>() + q.y / 4,
+                                ws.pf.as<float>() + level_offset(q.level, (int64_t)C * rf), C, rf,
+                                st)))
+        return rc;
   return kt_end(t, st);
+}
+
+// The tensor-core M2L: per launch of the plan (one, where the arrays of all levels
+// fit its bound) split the proxies, then the MMA kernel.
+int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
+  const bool f16 = t->tc_fmt == PBBFMM_TC_F16;
+  const int NP = t->tc.np, KP = f16 ? t->tc.kp16 : t->tc.kp, esize = f16 ? 2 : 4;
+  if (C > TC_M) {
+    set_error("tensor-core M2L takes at most 128 columns per block");
+    return PBBFMM_ERR_UNSUPPORTED;
+  }
+  TcArgs a{};
+  a.rf = t->ops.rf;
+  a.NP = NP;
+  a.rowb = KP * esize;
+  a.group = tc_group(NP, f16);
+  int rc;
+  ChebPlan plan;
+  if ((rc = plan_m2l_tc(t, C, f16, a.rowb, &plan, st))) return rc;
+  a.sstart = t->ws.sstart_p;
+  a.offs = t->d_offs;
+  a.eexp = t->tc.eexp;
+  a.kexp = t->tc.kexp;
+  a.err = t->d_tc_err;
+  CUtensorMap tm[4];
+  const int64_t nrows = (int64_t)t->ops.nlev * 316 * NP;
+  const void* eh = f16 ? (const void*)t->tc.eh16 : (const void*)t->tc.eth;
+  const void* el = f16 ? (const void*)t->tc.el16 : (const void*)t->tc.etl;
+  if ((rc = operator_tensor_map(&tm[0], eh, f16, NP, KP, nrows))) return rc;
+  if ((rc = operator_tensor_map(&tm[1], el, f16, NP, KP, nrows))) return rc;
+  tm[2] = tm[0];
+  tm[3] = tm[1];
+  if (plan.y_bytes > 0) {
+    const int64_t krows = (int64_t)t->ops.nlev * kKaraJ * kKaraD * NP;
+    if ((rc = operator_tensor_map(&tm[2], t->tc.kh16, true, NP, KP, krows))) return rc;
+    if ((rc = operator_tensor_map(&tm[3], t->tc.kl16, true, NP, KP, krows))) return rc;
+  }
+  for (const std::vector<ChebPart>& parts : plan.launches)
+    if ((rc = launch_m2l_tc(t, C, parts, a, f16, KP, tm, st))) return rc;
+  return PBBFMM_OK;
 }
 
 // ------------------------------------------------------------------------

@@ -96,17 +96,19 @@ def coefficient_bytes(t, level, order, cols, width):
         2 * order ** 3 + o["rf"] + o["rs"])
 
 
-def test_dense_levels_run_without_room_for_combinations():
+@pytest.mark.parametrize("precision", [fmm.PREC_FP64, fmm.PREC_MIXED], ids=["f64", "mixed"])
+def test_dense_levels_run_without_room_for_combinations(precision):
     """Room for the level arrays but not for the combinations of dense levels:
     the direct lists run.  Room that the combinations of an earlier call hold is
     given back to a call that needs it."""
     level, order, cols, n = 5, 4, 8, 100000
+    tol = 1e-13 if precision == fmm.PREC_FP64 else 2e-6
     t = make_tree("Laplacian", 0.0, 1.0, level, order, 1e-5, 1)
     t.buildFMMTree()
     p, w = points(n, 1), weights(cols, n, 2)
-    ref = run(t, p, w, fmm.PREC_FP64)
+    ref = run(t, p, w, precision)
     held = combined_bytes(t)
-    needed = coefficient_bytes(t, level, order, cols, 8)
+    needed = coefficient_bytes(t, level, order, cols, 8 if precision == fmm.PREC_FP64 else 4)
     assert held > 1.3 * needed
     t.close()
     import torch
@@ -114,45 +116,50 @@ def test_dense_levels_run_without_room_for_combinations():
     t = make_tree("Laplacian", 0.0, 1.0, level, order, 1e-5, 1)
     t.buildFMMTree()
     full = fill_but(needed + 200 * MB)
-    assert rel(run(t, p, w, fmm.PREC_FP64), ref) < 1e-13
+    assert rel(run(t, p, w, precision), ref) < tol
     assert combined_bytes(t) < 200 * MB
     del full
     torch.cuda.empty_cache()
-    run(t, p, w, fmm.PREC_FP64)
+    run(t, p, w, precision)
     assert combined_bytes(t) == held
     # 16 columns: twice the level arrays, in less than what the combinations hold
     w2 = weights(2 * cols, n, 3)
     full = fill_but(needed // 2)
-    two = run(t, p, w2, fmm.PREC_FP64)
+    two = run(t, p, w2, precision)
     assert combined_bytes(t) < held
     del full
     torch.cuda.empty_cache()
-    assert rel(run(t, p, w2, fmm.PREC_FP64), two) < 1e-13
+    assert rel(run(t, p, w2, precision), two) < tol
     t.close()
 
 
-# Laplacian, order 4 (r = 48), level 4: the combinations of a level's column take
-# 512, 64 and 8 parents x 27 x 96 values
-COLUMN = 512 * 27 * 96
+# Laplacian, order 4 (r = 48), level 4: bytes of the combinations of one column of
+# the deepest level, 512 parents x 27 proxies (mixed: hi and lo parts of 64 values
+# and an exponent) and sums
+COLUMN = {fmm.PREC_FP64: 512 * 27 * 96 * 8, fmm.PREC_MIXED: 512 * 27 * (2 * 64 * 2 + 4 + 48 * 4)}
 
 
+@pytest.mark.parametrize("precision", [fmm.PREC_FP64, fmm.PREC_MIXED], ids=["f64", "mixed"])
 @pytest.mark.parametrize("cols", [1, 5])
 @pytest.mark.parametrize("share", [1.02, 2.02, 0.35, 0.7, 0.13, 0.0],
                          ids=["column", "columns", "third", "two_thirds", "shallow", "none"])
-def test_groups_of_combinations(share, cols):
+def test_groups_of_combinations(share, cols, precision):
     """Groups of columns, groups of 9 combinations of one column, the direct list
-    below that, level by level: equal but for rounding."""
+    below that, level by level: equal but for rounding (float32: the direct list's
+    against the combinations', each within 1e-6 of float64)."""
+    column = COLUMN[precision]
+    tol = 1e-13 if precision == fmm.PREC_FP64 else 2e-6
     t = make_tree("Laplacian", 0.0, 1.0, 4, 4, 1e-5, 1)
     t.buildFMMTree()
     p, w = points(20000, 5), weights(cols, 20000, 6)
-    ref = run(t, p, w, fmm.PREC_FP64)
+    ref = run(t, p, w, precision)
     all_held = combined_bytes(t)
     t.close()
     t = make_tree("Laplacian", 0.0, 1.0, 4, 4, 1e-5, 1)
     t.buildFMMTree()
-    bound = int(share * COLUMN * 8)
+    bound = int(share * column)
     combined_bytes(t, bound)
-    assert rel(run(t, p, w, fmm.PREC_FP64), ref) < 1e-13
+    assert rel(run(t, p, w, precision), ref) < tol
     held = combined_bytes(t)
     assert held <= bound < all_held or bound >= all_held
     assert (held > 0) == (share > 0)
@@ -163,7 +170,7 @@ def test_groups_of_combinations(share, cols):
     for b in (bound, 1 << 40):
         combined_bytes(t, b)
         o = torch.zeros(cols, 20000, dtype=torch.float64, device="cuda")
-        fmm.compute_adjoint_device(t, p, p, w, g, cols, grad_weight=o)
+        fmm.compute_adjoint_device(t, p, p, w, g, cols, grad_weight=o, precision=precision)
         got.append(o.cpu().numpy())
-    assert rel(got[0], got[1]) < 1e-13
+    assert rel(got[0], got[1]) < tol
     t.close()
