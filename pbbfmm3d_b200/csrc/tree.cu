@@ -147,19 +147,27 @@ __global__ void k_gather_w(const double* __restrict__ w, const int* __restrict__
 enum ListKind { LIST_SRC = 0, LIST_TGT = 1, LIST_TYPED = 2, LIST_DENSE = 3, LIST_SPARSE = 4 };
 constexpr int kListThreads = 256, kListItems = 4, kListBlock = kListThreads * kListItems;
 
+constexpr int kScanItems = 16;  // counts of a thread of k_list_scan
+// Blocks of a list at most: a deep level's blocks take several pieces of kListBlock
+// cells each, and there are still enough to fill the chip (20,000 points at level 9,
+// binning: a piece per block 5.9, so 4.8 ms; at level 8 0.79 and 0.68 ms).
+constexpr int kListBlocksMax = 2048;
+
 struct ListJob {
-  int kind, shift;    // shift = 3 (L - level): leaf ranges of a cell
-  int ncells, block0; // virtual cells, first block
-  int* out;           // the list
-  int* count;         // its length (device)
-  int* bounds;        // LIST_TYPED: [9] first position of each child type
-  int slot;           // index of the length in the host copy; bounds at slot + 1
+  int kind, shift;     // shift = 3 (L - level): leaf ranges of a cell
+  int ncells, block0;  // cells (LIST_TYPED: parents), first block
+  int pieces;          // of kListBlock cells per block
+  int count0, ncounts; // its counts: one per block (LIST_TYPED: per child type and block)
+  int* out;            // the list
+  int* count;          // its length (device)
+  int slot;            // index of the length in the host copy; LIST_TYPED: the first
+                       // position of each child type, then the length, from slot + 1 on
 };
 struct ListArgs {
   ListJob job[3 * (kMaxLevel - 1) + 2];
-  int njobs, nblocks;
+  int njobs, nblocks, ncounts;
   const int *sstart, *tstart;
-  int *bcount, *bchunk;  // per block: cells selected, chunks of dense leaves
+  int *bcount, *bchunk;  // the jobs' counts: cells selected, chunks of dense leaves
   int* prefix;           // first chunk of each dense leaf, then the total
   int* hcount;           // mapped host memory: the lengths and bounds
 };
@@ -170,20 +178,34 @@ __device__ __forceinline__ int list_job(const ListArgs& a) {
     if ((int)blockIdx.x >= a.job[i].block0) j = i;
   return j;
 }
-// virtual cell v of a job: its Morton index and whether it is listed; for dense
-// leaves also their chunks of 32 targets
-__device__ __forceinline__ bool list_cell(const ListArgs& a, const ListJob& j, int v, int* cell,
+// whether cell c of a job is listed; for dense leaves also their chunks of 32
+// targets
+__device__ __forceinline__ bool list_cell(const ListArgs& a, const ListJob& j, int64_t c,
                                           int* chunks) {
-  if (v >= j.ncells) return false;
-  const int npar = j.ncells >> 3;
-  *cell = j.kind == LIST_TYPED ? 8 * (v % npar) + v / npar : v;
+  if (c >= j.ncells) return false;
   const int* start = j.kind == LIST_SRC ? a.sstart : a.tstart;
-  const int64_t c = *cell;
   const int n = start[(c + 1) << j.shift] - start[c << j.shift];
   *chunks = (n + 31) / 32;
   if (j.kind == LIST_DENSE) return n >= kLaneLeafMin;
   if (j.kind == LIST_SPARSE) return n > 0 && n < kLaneLeafMin;
   return n > 0;
+}
+
+// LIST_TYPED: bit t: child t of parent p has targets.  A thread reads its parent's
+// nine bounds, neighbours in memory, and serves all eight types (a cell at a time in
+// the order of the list, types outermost, every sector of bounds is read eight
+// times: 20,000 points at level 9, binning 8.3 ms, so 5.9).
+__device__ __forceinline__ unsigned list_children(const ListArgs& a, const ListJob& j, int64_t p) {
+  if (p >= j.ncells) return 0;
+  unsigned m = 0;
+  int lo = a.tstart[(8 * p) << j.shift];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int hi = a.tstart[(8 * p + t + 1) << j.shift];
+    m |= hi > lo ? 1u << t : 0u;
+    lo = hi;
+  }
+  return m;
 }
 
 // block-wide exclusive prefix of (x, y); *tx, *ty the totals
@@ -211,70 +233,139 @@ __device__ __forceinline__ void block_scan2(int x, int y, int* ex, int* ey, int*
 
 __global__ void __launch_bounds__(kListThreads) k_list_count(const __grid_constant__ ListArgs a) {
   const ListJob& j = a.job[list_job(a)];
-  const int v0 = ((int)blockIdx.x - j.block0) * kListBlock + threadIdx.x * kListItems;
-  int n = 0, nc = 0;
+  const int b = (int)blockIdx.x - j.block0, tid = threadIdx.x;
+  if (j.kind == LIST_TYPED) {
+    __shared__ int s_n[8];
+    if (tid < 8) s_n[tid] = 0;
+    __syncthreads();
+    int n[8] = {};
+    for (int i = 0; i < kListItems * j.pieces; ++i) {
+      const unsigned m =
+          list_children(a, j, (int64_t)b * j.pieces * kListBlock + i * kListThreads + tid);
 #pragma unroll
-  for (int i = 0; i < kListItems; ++i) {
-    int cell, ch;
-    if (list_cell(a, j, v0 + i, &cell, &ch)) n += 1, nc += ch;
+      for (int t = 0; t < 8; ++t) n[t] += __popc(__ballot_sync(0xffffffffu, (m >> t) & 1u));
+    }
+    if ((tid & 31) == 0)
+#pragma unroll
+      for (int t = 0; t < 8; ++t) atomicAdd(&s_n[t], n[t]);
+    __syncthreads();
+    if (tid < 8) a.bcount[j.count0 + tid * (j.ncounts / 8) + b] = s_n[tid];
+    return;
+  }
+  int n = 0, nc = 0;
+  for (int k = 0; k < j.pieces; ++k) {
+    const int64_t c0 = ((int64_t)b * j.pieces + k) * kListBlock + tid * kListItems;
+#pragma unroll
+    for (int i = 0; i < kListItems; ++i) {
+      int ch;
+      if (list_cell(a, j, c0 + i, &ch)) n += 1, nc += ch;
+    }
   }
   int ex, ey, tx, ty;
   block_scan2(n, nc, &ex, &ey, &tx, &ty);
-  if (threadIdx.x == 0) a.bcount[blockIdx.x] = tx, a.bchunk[blockIdx.x] = ty;
+  if (tid == 0) a.bcount[j.count0 + b] = tx, a.bchunk[j.count0 + b] = ty;
 }
 
-// one block per list: exclusive scan of its blocks' counts, in place
+// one block per list: exclusive scan of its counts, in place, kScanItems of them per
+// thread and step
 __global__ void __launch_bounds__(kListThreads) k_list_scan(const __grid_constant__ ListArgs a) {
   const ListJob& j = a.job[blockIdx.x];
-  const int b1 = blockIdx.x + 1 < a.njobs ? a.job[blockIdx.x + 1].block0 : a.nblocks;
+  const bool dense = j.kind == LIST_DENSE;
   int n = 0, nc = 0;
-  for (int b = j.block0; b < b1; b += kListThreads) {
-    const int k = b + threadIdx.x;
-    const int x = k < b1 ? a.bcount[k] : 0, y = k < b1 ? a.bchunk[k] : 0;
+  for (int k0 = 0; k0 < j.ncounts; k0 += kListThreads * kScanItems) {
+    const int first = k0 + threadIdx.x * kScanItems;
+    int x[kScanItems], y[kScanItems], sx = 0, sy = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      const bool ok = first + i < j.ncounts;
+      x[i] = ok ? a.bcount[j.count0 + first + i] : 0;
+      y[i] = ok && dense ? a.bchunk[j.count0 + first + i] : 0;
+      sx += x[i], sy += y[i];
+    }
     int ex, ey, tx, ty;
-    block_scan2(x, y, &ex, &ey, &tx, &ty);
-    if (k < b1) a.bcount[k] = n + ex, a.bchunk[k] = nc + ey;
+    block_scan2(sx, sy, &ex, &ey, &tx, &ty);
+    ex += n, ey += nc;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      if (first + i < j.ncounts) {
+        a.bcount[j.count0 + first + i] = ex;
+        if (dense) a.bchunk[j.count0 + first + i] = ey;
+      }
+      ex += x[i], ey += y[i];
+    }
     n += tx;
     nc += ty;
   }
   if (threadIdx.x == 0) {
     *j.count = n;
-    if (j.kind == LIST_DENSE) a.prefix[n] = nc;
+    if (dense) a.prefix[n] = nc;
     if (j.slot >= 0) a.hcount[j.slot] = n;
-    if (j.kind == LIST_TYPED) j.bounds[8] = a.hcount[j.slot + 9] = n;
+    if (j.kind == LIST_TYPED) a.hcount[j.slot + 9] = n;
   }
 }
 
 __global__ void __launch_bounds__(kListThreads) k_list_write(const __grid_constant__ ListArgs a) {
   const int ji = list_job(a);
   const ListJob& j = a.job[ji];
-  const int v0 = ((int)blockIdx.x - j.block0) * kListBlock + threadIdx.x * kListItems;
-  int cell[kListItems], ch[kListItems], n = 0, nc = 0;
-  bool sel[kListItems];
+  const int b = (int)blockIdx.x - j.block0, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (j.kind == LIST_TYPED) {
+    __shared__ int s_w[2][8][kListThreads / 32];  // listed children of a type in a warp
+    const int nb = j.ncounts / 8;
+    const unsigned below = (1u << lane) - 1u;
+    int at[8];
 #pragma unroll
-  for (int i = 0; i < kListItems; ++i) {
-    sel[i] = list_cell(a, j, v0 + i, &cell[i], &ch[i]);
-    if (sel[i]) n += 1, nc += ch[i];
+    for (int t = 0; t < 8; ++t) at[t] = a.bcount[j.count0 + t * nb + b];
+    if (b == 0 && tid < 8) a.hcount[j.slot + 1 + tid] = a.bcount[j.count0 + tid * nb];
+    for (int i = 0; i < kListItems * j.pieces; ++i) {
+      const int64_t p = (int64_t)b * j.pieces * kListBlock + i * kListThreads + tid;
+      const unsigned m = list_children(a, j, p);
+      unsigned v[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        v[t] = __ballot_sync(0xffffffffu, (m >> t) & 1u);
+        if (lane == 0) s_w[i & 1][t][warp] = __popc(v[t]);
+      }
+      __syncthreads();  // (two buffers: a warp is at most one step ahead)
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        int mine = at[t] + __popc(v[t] & below), all = 0;
+        for (int w = 0; w < kListThreads / 32; ++w) {
+          const int x = s_w[i & 1][t][w];
+          if (w < warp) mine += x;
+          all += x;
+        }
+        if ((m >> t) & 1u) j.out[mine] = (int)(8 * p + t);
+        at[t] += all;
+      }
+    }
+    return;
   }
-  int ex, ey, tx, ty;
-  block_scan2(n, nc, &ex, &ey, &tx, &ty);
-  int at = a.bcount[blockIdx.x] + ex, cat = a.bchunk[blockIdx.x] + ey;
   // the sparse leaves follow the dense ones (the job before)
   const int base = j.kind == LIST_SPARSE ? *a.job[ji - 1].count : 0;
-  const int npar = j.ncells >> 3;
+  int at0 = a.bcount[j.count0 + b], cat0 = j.kind == LIST_DENSE ? a.bchunk[j.count0 + b] : 0;
+  for (int k = 0; k < j.pieces; ++k) {
+    const int64_t c0 = ((int64_t)b * j.pieces + k) * kListBlock + tid * kListItems;
+    int ch[kListItems], n = 0, nc = 0;
+    bool sel[kListItems];
 #pragma unroll
-  for (int i = 0; i < kListItems; ++i) {
-    const int v = v0 + i;
-    if (j.kind == LIST_TYPED && v < j.ncells && v % npar == 0) {
-      j.bounds[v / npar] = at;
-      a.hcount[j.slot + 1 + v / npar] = at;
+    for (int i = 0; i < kListItems; ++i) {
+      sel[i] = list_cell(a, j, c0 + i, &ch[i]);
+      if (sel[i]) n += 1, nc += ch[i];
     }
-    if (sel[i]) {
-      j.out[base + at] = cell[i];
-      if (j.kind == LIST_DENSE) a.prefix[at] = cat;
-      at += 1;
-      cat += ch[i];
+    int ex, ey, tx, ty;
+    block_scan2(n, nc, &ex, &ey, &tx, &ty);
+    int at = at0 + ex, cat = cat0 + ey;
+#pragma unroll
+    for (int i = 0; i < kListItems; ++i) {
+      if (sel[i]) {
+        j.out[base + at] = (int)(c0 + i);
+        if (j.kind == LIST_DENSE) a.prefix[at] = cat;
+        at += 1;
+        cat += ch[i];
+      }
     }
+    at0 += tx;
+    cat0 += ty;
   }
 }
 
@@ -313,13 +404,20 @@ int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d
   if ((rc = grow(ws.wsorted, 8 * Ns * (int64_t)C))) return rc;
   if ((rc = grow(ws.cub_temp, cub_need))) return rc;
   if ((rc = grow(ws.lists, 4 * (list_need + 16)))) return rc;
-  if ((rc = grow(ws.dcounts, 4 * (kMaxLevel + 1) * 12))) return rc;
+  if ((rc = grow(ws.dcounts, 4 * (kMaxLevel + 1) * 3))) return rc;
   // dense and sparse target leaves, the chunk prefix, then the block counts
   const int64_t leaf_need = (nleaf < Nf ? nleaf : Nf) + 1;
-  int64_t list_blocks = 0;
+  auto list_pieces = [](int64_t cells) {
+    return (cells + (int64_t)kListBlock * kListBlocksMax - 1) / ((int64_t)kListBlock * kListBlocksMax);
+  };
+  auto list_blocks = [&](int64_t cells) {
+    const int64_t per = kListBlock * list_pieces(cells);
+    return (cells + per - 1) / per;
+  };
+  int64_t list_counts = 0;
   for (int l = 2; l <= L; ++l)
-    list_blocks += (l == L ? 5 : 3) * ((cells_at(l) + kListBlock - 1) / kListBlock);
-  if ((rc = grow(ws.leafpart, 4 * (2 * leaf_need + 2 * list_blocks)))) return rc;
+    list_counts += (l == L ? 4 : 2) * list_blocks(cells_at(l)) + 8 * list_blocks(cells_at(l - 1));
+  if ((rc = grow(ws.leafpart, 4 * (2 * leaf_need + 2 * list_counts)))) return rc;
   if (!ws.h_counts) {
     PB_CUDA(cudaHostAlloc(&ws.h_counts, sizeof(int) * 12 * (kMaxLevel + 1), cudaHostAllocMapped));
     PB_CUDA(cudaHostGetDevicePointer(&ws.d_counts, ws.h_counts, 0));
@@ -383,22 +481,25 @@ int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d
   la.sstart = ws.sstart_p;
   la.tstart = ws.tstart.as<int>();
   la.hcount = ws.d_counts;
-  int* cnt = ws.dcounts.as<int>();  // [l][0]=nsrc [l][1]=ntgt [l][2]=ntyp [l][3..11] type bounds
+  int* cnt = ws.dcounts.as<int>();  // [l][0]=nsrc [l][1]=ntgt [l][2]=ntyp; [0] and [1] dense, sparse
   int* part = ws.leafpart.as<int>();
   la.prefix = part + leaf_need;
   la.bcount = la.prefix + leaf_need;
-  la.bchunk = la.bcount + list_blocks;
+  la.bchunk = la.bcount + list_counts;
   auto add = [&](int kind, int l, int* out, int* count, int slot) {
     ListJob& j = la.job[la.njobs++];
     j.kind = kind;
     j.shift = 3 * (L - l);
-    j.ncells = (int)cells_at(l);
+    j.ncells = (int)cells_at(kind == LIST_TYPED ? l - 1 : l);
     j.block0 = la.nblocks;
+    j.count0 = la.ncounts;
+    j.pieces = (int)list_pieces(j.ncells);
+    j.ncounts = (int)list_blocks(j.ncells) * (kind == LIST_TYPED ? 8 : 1);
     j.out = out;
     j.count = count;
     j.slot = slot;
-    j.bounds = kind == LIST_TYPED ? count + 1 : nullptr;
-    la.nblocks += (j.ncells + kListBlock - 1) / kListBlock;
+    la.nblocks += (int)list_blocks(j.ncells);
+    la.ncounts += j.ncounts;
   };
   int64_t off = 0;
   for (int l = 2; l <= L; ++l) {
@@ -408,7 +509,7 @@ int run_binning(pbbfmm_tree* t, const double* d_tgt, int64_t Nf, const double* d
     LL.typ_off[l] = off + ms + mt;
     for (int k = 0; k < 3; ++k)
       add(k, l, lists + (k == 0 ? LL.src_off[l] : k == 1 ? LL.tgt_off[l] : LL.typ_off[l]),
-          cnt + 12 * l + k, 12 * l + k);
+          cnt + 3 * l + k, 12 * l + k);
     off += ms + 2 * mt;
   }
   add(LIST_DENSE, L, part, cnt, -1);

@@ -4,9 +4,10 @@ sources and targets (binned once) against a copy of it (binned twice)."""
 import numpy as np
 import pytest
 
+import oracle
 import pbbfmm3d_b200 as fmm
-from helpers import make_tree
-from test_gpu_parity import _meta, phase_by_phase
+from helpers import host_ops, make_tree, oracle_ops, rel
+from test_gpu_parity import _meta, gpu_tree, phase_by_phase, run_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -48,4 +49,17 @@ def test_shared_buffer_is_binned_once_with_the_same_result(precision, cols):
     assert fmm.launch_count() - launches > once
     fmm.compute_device(t, p, p, w, cols, out[2], precision=precision)
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+    t.close()
+
+
+def test_deep_level_lists_match_oracle():
+    """Level 8: more counts than one step of the lists' scan covers."""
+    rng = np.random.default_rng(8)
+    p = rng.uniform(-0.5, 0.5, (3000, 3))
+    p[:1500] = 0.2 + 0.01 * rng.standard_normal((1500, 3))
+    w = rng.standard_normal(3000)
+    meta = _meta("Laplacian", 0.0, 1.0, 8, 2, 1e-2, 1, 1)
+    ops = host_ops("Laplacian", 0.0, 1.0, 8, 2, 1e-2, 1)
+    t = gpu_tree(meta, ops)
+    assert rel(run_gpu(t, p, p, w, 1), oracle.matvec(oracle_ops(ops, meta), p, p, w, 1)) < 1e-12
     t.close()
