@@ -236,6 +236,18 @@ struct FftCfg {
     return b > out_bytes ? b : out_bytes;
   }
   static constexpr int unroll = n <= 6 ? n : 1;  // the k3 loops: larger orders keep the code small
+  // inverse: threads of a row of outputs.  From order 8 (float32 9) on a thread's n^2
+  // outputs and the m inputs of a transform do not fit its registers (spills of
+  // up to 1 KB), and a thread per row leaves half of the warps idle: each then
+  // takes n / qparts of the outputs a2 and reads its inputs from shared memory as it
+  // uses them.  20,000 points on 4 levels, inverse of all levels, 1 column: float64,
+  // orders 8, 9, 10: 0.188, 0.466, 0.698 -> 0.101, 0.186, 0.310 ms (2, 3, 2 parts:
+  // 0.127, 0.186, 0.341); float32, orders 9, 10: 0.187, 0.264 -> 0.101, 0.184 ms.
+  static constexpr int qparts = sizeof(T) == 8 ? (n == 8 ? 4 : n == 9 ? 3 : n == 10 ? 5 : 1)
+                                               : (n == 9 ? 3 : n == 10 ? 2 : 1);
+  static_assert(n % qparts == 0, "equal parts");
+  static constexpr int threads_inv =
+      n * U * qparts <= threads ? threads : (n * U * qparts + 31) / 32 * 32;
 };
 
 // The z and y transforms of row l1 of one unit, for k3 = K0, K0 + STEP, ...
@@ -408,13 +420,51 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   }
 }
 
+// y and z of outputs a2 = Q0 .. Q0 + QN - 1 of one row a1 of one unit (see
+// k_fft_inv), the inputs read from shared memory as they are used.
+template <int n, typename T, int U, int Q0, int QN>
+__device__ __forceinline__ void inv_row_part(const cplx_t<T>* __restrict__ g, T (&acc)[QN][n]) {
+  using W = Tw<n, T>;
+  constexpr int m = 2 * n - 1;
+#pragma unroll 1
+  for (int k3 = 0; k3 < n; ++k3) {
+    T re[QN], im[QN];
+#pragma unroll
+    for (int q = 0; q < QN; ++q) re[q] = im[q] = 0;
+#pragma unroll
+    for (int k = 0; k < m; ++k) {
+      const bool mirror = k3 == 0 && k >= n;  // G(-k2, 0) = conj G(k2, 0)
+      cplx_t<T> v = g[unif_job_of(n, mirror ? m - k : k, k3) * U];
+      if (mirror) v.y = -v.y;
+#pragma unroll
+      for (int q = 0; q < QN; ++q) {
+        const int t = (Q0 + q + n) % m;
+        const T c = W::c((k * t) % m), s = W::s((k * t) % m);
+        re[q] = fma(v.x, c, fma(-v.y, s, re[q]));
+        im[q] = fma(v.y, c, fma(v.x, s, im[q]));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < QN; ++q)
+#pragma unroll
+      for (int a3 = 0; a3 < n; ++a3) {
+        const int t = (a3 + n) % m;
+        if (k3 == 0)
+          acc[q][a3] = re[q];
+        else
+          acc[q][a3] = fma(T(2), fma(re[q], W::c((k3 * t) % m), -im[q] * W::s((k3 * t) % m)),
+                           acc[q][a3]);
+      }
+  }
+}
+
 // F = scale * IDFT(Y)/P at grid positions (a + n) mod m;
 // (a + ib) e^{+2 pi i j / m} = (a c - b s) + i (b c + a s).
 // Units: U consecutive (cell, column) pairs of the nonempty target cells,
 // Y[(slot ncells + cell) C + column]; SPLIT: U consecutive (parent, column)
 // rows of one child, Y as the tensor-core MAC writes it (UnifPlanes).
 template <int n, typename T, bool SPLIT>
-__global__ void __launch_bounds__(FftCfg<n, T>::threads)
+__global__ void __launch_bounds__(FftCfg<n, T>::threads_inv)
     k_fft_inv(const FftInvArgs<T> a) {
   using C2 = cplx_t<T>;
   using W = Tw<n, T>;
@@ -426,7 +476,7 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   T* O = reinterpret_cast<T*>(smraw);    // [U][OP], after G
   __shared__ int64_t s_dst[U];           // unit: its locals, or -1
   const int tid = threadIdx.x, u = tid % U, job0 = tid / U;
-  constexpr int JS = Cfg::threads / U;
+  constexpr int JS = Cfg::threads_inv / U;
   int64_t src = 0;
   bool has;
   if constexpr (SPLIT) {
@@ -482,10 +532,24 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   __syncthreads();
   // y and z of row a1: H[a2][k3] = sum_k2 G[a1][k2][k3] e^{+2 pi i k2 t2 / m},
   // out = Re H[..][0] + 2 sum_{k3>=1} Re(H[..][k3] e^{+2 pi i k3 t3 / m})
-  T acc[n][n];
-  const bool row = job0 < n && has;
-  if (row) {
-    const C2* g = G + job0 * nj * U + u;
+  constexpr int QP = Cfg::qparts, QN = n / QP;
+  T acc[QN][n];
+  const bool row = job0 < n * QP && has;
+  const int a1 = job0 % n, part = job0 / n;
+  const C2* grow = G + a1 * nj * U + u;
+  if constexpr (QP > 1) {
+    if (row) {
+      if (part == 0) inv_row_part<n, T, U, 0, QN>(grow, acc);
+      if (part == 1) inv_row_part<n, T, U, QN, QN>(grow, acc);
+      if constexpr (QP > 2)
+        if (part == 2) inv_row_part<n, T, U, 2 * QN, QN>(grow, acc);
+      if constexpr (QP > 3)
+        if (part == 3) inv_row_part<n, T, U, 3 * QN, QN>(grow, acc);
+      if constexpr (QP > 4)
+        if (part == 4) inv_row_part<n, T, U, 4 * QN, QN>(grow, acc);
+    }
+  } else if (row) {
+    const C2* g = grow;
 #pragma unroll Cfg::unroll
     for (int k3 = 0; k3 < n; ++k3) {
       C2 v[m];
@@ -526,15 +590,15 @@ __global__ void __launch_bounds__(FftCfg<n, T>::threads)
   }
   __syncthreads();
   if (row) {
-    T* o = O + u * OP + job0 * n2;
+    T* o = O + u * OP + a1 * n2 + part * QN * n;
 #pragma unroll
-    for (int q = 0; q < n; ++q)
+    for (int q = 0; q < QN; ++q)
 #pragma unroll
       for (int a3 = 0; a3 < n; ++a3) o[q * n + a3] = a.scale * (acc[q][a3] * a.invP);
   }
   __syncthreads();
   // (a warp per unit, lanes over its row)
-  for (int v = tid >> 5; v < U; v += Cfg::threads / 32) {
+  for (int v = tid >> 5; v < U; v += Cfg::threads_inv / 32) {
     const int64_t o = s_dst[v];
     if (o < 0) continue;
 #pragma unroll
@@ -869,7 +933,7 @@ struct FftInvLaunch {
     auto kern = k_fft_inv<N, T, SPLIT>;
     PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)Cfg::smem_inv(SPLIT)));
-    kern<<<(unsigned)grid, Cfg::threads, Cfg::smem_inv(SPLIT), st>>>(a);
+    kern<<<(unsigned)grid, Cfg::threads_inv, Cfg::smem_inv(SPLIT), st>>>(a);
     PB_LAUNCH("fft_inv");
     return PBBFMM_OK;
   }

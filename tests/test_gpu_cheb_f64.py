@@ -1,6 +1,6 @@
 """The float64 Chebyshev far field at the edges of its kernels' tiles, against
 the oracle phase by phase with the same operators: ranks from one group of 8
-outputs to two blocks of 128, row counts that leave remainders of the 64-row
+outputs to three blocks of 128, row counts that leave remainders of the 64-row
 tiles, many columns, tiles cut along the offsets and not, sparse cells."""
 import numpy as np
 import pytest
@@ -18,6 +18,7 @@ CASES = [
     ("GaussSigma", 0.25, 4, 1e-6, 3, 2, 3000, False),
     ("GaussSigma", 0.1, 5, 1e-12, 3, 3, 2500, False),    # 125 outputs: 16 groups
     ("Laplacian", 0.0, 6, 1e-14, 3, 2, 2500, True),      # over 128 outputs: two blocks
+    ("Laplacian", 0.0, 7, 1e-13, 3, 1, 400, False),      # rank 328, 343 outputs: three blocks
 ]
 
 

@@ -6,9 +6,10 @@ in mixed precision within 2e-6 of float64 (the mixed path's bound)."""
 import numpy as np
 import pytest
 
+import oracle
 import pbbfmm3d_b200 as fmm
-from helpers import make_tree, rel
-from test_gpu_parity import _meta, phase_by_phase
+from helpers import host_ops, make_tree, oracle_ops, rel
+from test_gpu_parity import _meta, gpu_tree, phase_by_phase
 
 pytestmark = pytest.mark.gpu
 
@@ -22,7 +23,7 @@ def _points(n, clustered, seed):
 
 
 CASES = ([(3, 3, c, False) for c in (1, 2, 3, 4, 5, 6, 7, 8, 9, 12)] +
-         [(n, 3, 1, False) for n in (2, 4, 5, 6, 7, 8)] +
+         [(n, 3, 1, False) for n in (2, 4, 5, 6, 7, 8, 9)] +
          [(3, 2, 3, False), (4, 4, 2, True), (5, 4, 8, True)])
 
 
@@ -43,7 +44,7 @@ def _run(t, p, w, cols, precision):
 
 
 MIXED = ([(3, 4, c, False) for c in (1, 2, 3, 4, 5, 6, 7, 8, 11)] +
-         [(n, 3, 1, False) for n in (2, 4, 5, 6, 7, 8)] +
+         [(n, 3, 1, False) for n in (2, 4, 5, 6, 7, 8, 9)] +
          # tensor cores: 16 and 32 parents per side, orders with 32, 16 and 8 units per CTA
          [(2, 5, 8, False), (5, 5, 8, True), (6, 5, 16, False), (8, 5, 8, True), (4, 6, 8, True)])
 
@@ -59,4 +60,40 @@ def test_unif_mixed_matches_f64(case):
     t.buildFMMTree()
     ref = _run(t, p, w, cols, fmm.PREC_FP64)
     assert rel(_run(t, p, w, cols, fmm.PREC_MIXED), ref) < 2e-6
+    t.close()
+
+
+# The basis of 10 equidistant nodes amplifies rounding: its Lebesgue constant is
+# 17.8 (9 nodes: 10.9), cubed 5.7e3 in three dimensions.  Float64: 2^-53 times that,
+# for each of the 10 additions of a transform at the sources' and the targets' end
+# less what cancels: 16 times (1.3e-12 to 6.9e-12 seen, the same with the
+# transforms computed as direct sums).  Mixed: the bound of 2e-6, which
+# order 9 keeps, times (17.8 / 10.9)^2 for the basis at both ends.
+TOL10_F64 = 16 * 2.0 ** -53 * 17.85 ** 3
+TOL10_MIXED = 2e-6 * (17.85 / 10.95) ** 2
+
+
+@pytest.mark.parametrize("level", [2, 3])
+def test_unif_order_10(level):
+    p, rng = _points(600, False, level)
+    w = rng.standard_normal(600)
+    ops = host_ops("ExpCov", 0.3, 1.0, level, 10, 1e-5, 0)
+    meta = _meta("ExpCov", 0.3, 1.0, level, 10, 1e-5, 0, 1)
+    t = gpu_tree(meta, ops)
+    ref = oracle.matvec(oracle_ops(ops, meta), p, p, w, 1)
+    assert rel(_run(t, p, w, 1, fmm.PREC_FP64), ref) < TOL10_F64
+    assert rel(_run(t, p, w, 1, fmm.PREC_MIXED), ref) < TOL10_MIXED
+    t.close()
+
+
+@pytest.mark.parametrize("order", [9, 10])
+def test_unif_tensor_core_levels_of_the_largest_orders(order):
+    """Float64 takes these orders a column at a time."""
+    n = 3000
+    p, rng = _points(n, True, order)
+    w = rng.standard_normal((8, n))
+    t = make_tree("ExpCov", 0.3, 1.0, 5, order, 1e-5, 0)
+    t.buildFMMTree()
+    ref = np.concatenate([_run(t, p, w[c], 1, fmm.PREC_FP64) for c in range(8)])
+    assert rel(_run(t, p, w.ravel(), 8, fmm.PREC_MIXED), ref) < (2e-6 if order == 9 else TOL10_MIXED)
     t.close()
