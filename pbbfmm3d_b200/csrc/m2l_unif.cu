@@ -227,12 +227,16 @@ struct FftCfg {
   static constexpr size_t smem_s = sizeof(T) * (size_t)n3 * (U + 1);
   static constexpr size_t smem_fwd = alias ? (smem_y > smem_s ? smem_y : smem_s) : smem_y + smem_s + 16;
   static constexpr size_t out_bytes = sizeof(T) * (size_t)U * (n3 | 1);
-  // inverse: plain levels ask for n m n elements per unit and so keep three CTAs
-  // per SM at order 5, float32 (with four: 1M points, 1 column 0.334 -> 0.356 ms;
-  // 200,000 points, 3 columns 0.146 -> 0.166 ms); the split ones gain from four
-  // (2.20 -> 1.99 ms)
+  // inverse: plain levels of 32 units per CTA, four of which would fit an SM (order
+  // 4 in float64, 5 in float32), ask for so much that three do: 1M points, 1 column,
+  // order 5, float32 0.356 -> 0.334 ms; 800,000 points, 3 columns, order 4, float64
+  // 0.702 -> 0.653 ms.  The other plans lose by it (order 6, 120,000 points, 3
+  // columns: float64 0.369 -> 0.494, float32 0.227 -> 0.277 ms) or do not notice, and
+  // the split levels gain from four (2.20 -> 1.99 ms).
   static constexpr size_t smem_inv(bool split) {
-    const size_t b = split ? smem_y : 2 * sizeof(T) * (size_t)(n * m * n) * U;
+    constexpr size_t sm = 228 * 1024, cta = smem_y + 1024;  // (1 KB is the system's)
+    const bool three = !split && U == 32 && 4 * cta <= sm && 5 * cta > sm;
+    const size_t b = three ? (size_t)60 * 1024 : smem_y;
     return b > out_bytes ? b : out_bytes;
   }
   static constexpr int unroll = n <= 6 ? n : 1;  // the k3 loops: larger orders keep the code small
