@@ -510,13 +510,13 @@ static int upload_operators(pbbfmm_tree* t) {
 
 static void free_tree_device(pbbfmm_tree* t) {
   double** bufs[] = {&t->d_Tkz, &t->d_Kw, &t->d_Cw, &t->d_E,  &t->d_U,
-                     &t->d_VT,  &t->d_op, &t->d_twid, &t->d_kparam, &t->d_Ek};
+                     &t->d_VT,  &t->d_op, &t->d_kparam, &t->d_Ek};
   for (double** b : bufs) {
     if (*b) cudaFree(*b);
     *b = nullptr;
   }
   float** fbufs[] = {&t->f_Tkz, &t->f_Kw, &t->f_Cw, &t->f_E,    &t->f_U,
-                     &t->f_VT,  &t->f_op, &t->f_twid};
+                     &t->f_VT,  &t->f_op};
   for (float** b : fbufs) {
     if (*b) cudaFree(*b);
     *b = nullptr;
@@ -821,17 +821,6 @@ static int create_tree(const pbbfmm_tree_params* params, const pbbfmm_user_kerne
     return rc;
   }
   {
-    std::vector<double> tw(2 * t->m);
-    for (int j = 0; j < t->m; ++j) {
-      tw[j] = cos(2.0 * M_PI * j / t->m);
-      tw[t->m + j] = sin(2.0 * M_PI * j / t->m);
-    }
-    if ((rc = upload(&t->d_twid, tw.data(), tw.size())) ||
-        (rc = upload_f32(&t->f_twid, tw.data(), tw.size()))) {
-      free_tree_device(t);
-      delete t;
-      return rc;
-    }
     std::vector<int> offs = m2l_offsets(t->w.Ktable), terms;
     cheb_kara_tables(t->w.Ktable, &offs, &terms);
     offs.insert(offs.end(), terms.begin(), terms.end());

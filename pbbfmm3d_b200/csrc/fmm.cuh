@@ -145,7 +145,6 @@ struct pbbfmm_tree {
   // Cheb M2L: 8 types x 189 x 4 (ox, oy, oz, op index), then the same of the
   // combinations and their operators' terms (cheb_kara_tables)
   int* d_offs = nullptr;
-  double* d_twid = nullptr;  // Unif: cos/sin of 2 pi j / m, j < m
   double* d_kparam = nullptr;  // 4 kernel parameters
   // float32 copies of the weights and operators for the mixed path
   float* f_Tkz = nullptr;
@@ -160,7 +159,6 @@ struct pbbfmm_tree {
   // power-of-two exponents
   uint16_t* f_unif_tiles = nullptr;
   int* f_unif_bexp = nullptr;
-  float* f_twid = nullptr;
   // tensor-core Chebyshev M2L (mixed path); tc_fmt: PBBFMM_TC_F16 (scaled
   // F16 operands, default) or PBBFMM_TC_TF32
   bool use_tc = true;
