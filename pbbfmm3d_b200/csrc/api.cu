@@ -586,9 +586,11 @@ static int grow_pinned(void** p, size_t* cap, size_t bytes) {
 
 static int host_threads(size_t bytes) {
   const unsigned hw = std::thread::hardware_concurrency();
-  // 3 MB per thread at least: starting one costs 50 to 100 us here (14 MB in and
-  // out, whole call: 1 MB per thread 4.8, 3 MB 3.9, 8 MB 3.9 ms)
-  const size_t by_size = bytes / (3u << 20) + 1;
+  // 8 MB per thread at least: starting one costs 50 to 100 us here.  Whole calls of
+  // 100,000, 200,000, 400,000 and 1M points with 1, 3, 4 and 8 columns (4 to 150 MB
+  // in and out), 1 MB per thread: 1.31, 2.91, 4.79, 14.1 ms; 3 MB: 1.15, 2.68, 4.39,
+  // 13.9 ms; 8 MB: 1.06, 2.46, 3.91, 13.4 ms.
+  const size_t by_size = bytes / (8u << 20) + 1;
   size_t n = hw ? (hw < 16 ? hw : 16) : 4;
   return (int)(n < by_size ? n : by_size);
 }

@@ -1,6 +1,6 @@
 """The host-buffer entry stages its arrays by pieces of 1 MB over host threads:
 its result is the device entry's, bit for bit, whatever the arrays' sizes --
-within one piece, at its edges, and over several threads (more than 3 MB)."""
+within one piece, at its edges, and over several threads (more than 8 MB)."""
 import numpy as np
 import pytest
 import torch
@@ -18,7 +18,8 @@ PIECE = (1 << 20) // 8  # values of a piece
     (PIECE // 3 + 1, PIECE + 1, 1),
     (PIECE // 2, 0, 2),  # sources = targets; the weights one whole piece
     (150_001, 70_000, 5),  # several threads for the inputs, one for the result
-    (50_000, 200_003, 3),  # and for the result
+    (50_000, 200_003, 3),  # one thread
+    (50_000, 400_003, 3),  # several for inputs and result
 ])
 def test_same_as_device_entry(Ns, Nf, C):
     rng = np.random.default_rng(7)
