@@ -926,6 +926,51 @@ int run_m2l_cheb_tc(pbbfmm_tree* t, int C, cudaStream_t st) {
 // stay 12 steps long); otherwise the chunks accumulate in TMEM.
 constexpr int CG_TC_THREADS = 128;
 
+// A of rows that fit one chunk (K <= 64), the warp's 32 rows: lr lanes per row (two
+// values each), so that a load covers 32 / lr rows; a row's values stay in
+// registers between its maximum and the split.  With all lanes along K, as for
+// longer rows, most of them idle and the rows are read twice: 120,000 points, 16
+// columns, pre + post at orders 2, 3, 4: 0.62, 0.68, 0.83 ms, so 0.36, 0.46, 0.66 ms
+// (a row per thread: 0.35, 0.53, 0.75 ms).
+template <bool BSCALE>
+__device__ __forceinline__ void colgemm_rows_short(int K, const float* __restrict__ X,
+                                                   const float* __restrict__ bscale,
+                                                   const int64_t* s_row, int* s_exp,
+                                                   unsigned char* a_hi, unsigned char* a_lo) {
+  const int lane = threadIdx.x & 31, w0 = threadIdx.x & ~31;
+  const int lr = K <= 16 ? 8 : K <= 32 ? 16 : 32, rows = 32 / lr, l = lane & (lr - 1), k = 2 * l;
+  const bool k0 = k < K, k1 = k + 1 < K;
+  const float b0 = BSCALE && k0 ? bscale[k] : 1.f, b1 = BSCALE && k1 ? bscale[k + 1] : 1.f;
+  for (int r0 = w0 + lane / lr; r0 < w0 + 32; r0 += 8 * rows) {
+    float x[8][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int64_t r = s_row[r0 + i * rows];
+      x[i][0] = r >= 0 && k0 ? X[r * K + k] : 0.f;
+      x[i][1] = r >= 0 && k1 ? X[r * K + k + 1] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float v0 = BSCALE ? x[i][0] * b0 : x[i][0], v1 = BSCALE ? x[i][1] * b1 : x[i][1];
+      float mx = fmaxf(fabsf(v0), fabsf(v1));
+      for (int o = lr >> 1; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const int e = mx > 0.f ? 15 - exponent_of(mx) : 0, r = r0 + i * rows;
+      if (l == 0) s_exp[r] = e;
+      const float u0 = scale2(v0, e), u1 = scale2(v1, e);
+      const __half2 vh = __floats2half2_rn(u0, u1);
+      const float2 vf = __half22float2(vh);
+      const uint32_t off = sw128_off(r, l >> 2) + (l & 3) * 4;
+      *reinterpret_cast<__half2*>(a_hi + off) = vh;
+      *reinterpret_cast<__half2*>(a_lo + off) = __floats2half2_rn(u0 - vf.x, u1 - vf.y);
+    }
+  }
+  for (int ch = lr / 4; ch < 8; ++ch) {  // past the lanes' values: zeros
+    const uint32_t off = sw128_off(threadIdx.x, ch);
+    *reinterpret_cast<uint4*>(a_hi + off) = make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(a_lo + off) = make_uint4(0, 0, 0, 0);
+  }
+}
+
 template <bool BSCALE, bool OSCALE>
 __global__ void __launch_bounds__(CG_TC_THREADS, 1)
     k_colgemm_tc(int M, int mp, int K, int kp, const __grid_constant__ CUtensorMap tm_wh,
@@ -954,7 +999,8 @@ __global__ void __launch_bounds__(CG_TC_THREADS, 1)
   const int lane = tid & 31;
   s_row[tid] = valid ? row : -1;
   __syncwarp();
-  for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += 8) {
+  const bool one = K <= 64;  // one chunk holds the rows: read once, below
+  for (int r0 = 32 * warp; !one && r0 < 32 * warp + 32; r0 += 8) {
     float mx[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) mx[i] = 0.f;
@@ -973,8 +1019,6 @@ __global__ void __launch_bounds__(CG_TC_THREADS, 1)
       if (lane == 0) s_exp[r0 + i] = mx[i] > 0.f ? 15 - exponent_of(mx[i]) : 0;
     }
   }
-  __syncwarp();
-  const int e = s_exp[tid];
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                      smem_u32(&s_tmem)),
@@ -1003,7 +1047,8 @@ __global__ void __launch_bounds__(CG_TC_THREADS, 1)
   for (int c = 0; c < nchunks; ++c) {
     // A chunk: 64 values of each row (zero past K), scaled and split; lane k / 2
     // of a row's warp takes values k and k + 1
-    for (int r0 = 32 * warp; r0 < 32 * warp + 32; r0 += 8) {
+    if (one) colgemm_rows_short<BSCALE>(K, X, bscale, s_row, s_exp, a_hi, a_lo);
+    for (int r0 = 32 * warp; !one && r0 < 32 * warp + 32; r0 += 8) {
       const int k = c * 64 + 2 * lane;
       const bool k0 = k < K, k1 = k + 1 < K;
       float x[8][2];
@@ -1097,7 +1142,7 @@ __global__ void __launch_bounds__(CG_TC_THREADS, 1)
     // the unscaling 2^-(e + wexp) as two exact power-of-two factors applied
     // one after the other (never multiplied together, which could leave the
     // float range although the result lies inside it), then alpha
-    const int kt = -(e + wexp), k1 = min(max(kt, -126), 127), k2 = min(max(kt - k1, -149), 127);
+    const int kt = -(s_exp[tid] + wexp), k1 = min(max(kt, -126), 127), k2 = min(max(kt - k1, -149), 127);
     const float sc = exp2i(k1), sc2 = exp2i(k2);
     float* so = reinterpret_cast<float*>(base);  // [128 rows][129] (the tiles are done with)
     for (int m0 = 0; m0 < mp; m0 += 128) {  // uniform

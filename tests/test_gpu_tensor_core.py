@@ -206,3 +206,22 @@ def test_tensor_core_timeout_reports_and_recovers():
     assert np.all(out == 7.0)
     o = _run(t, p, w, 1, fmm.PREC_MIXED, fmt="f16")
     assert rel(o, o64) < 2e-6, rel(o, o64)
+
+
+@pytest.mark.parametrize("order,eps,cols", [(2, 1e-1, 1), (2, 1e-12, 3), (3, 1e-3, 5), (3, 1e-12, 1),
+                                            (4, 1e-3, 3), (4, 1e-12, 2)])
+def test_pre_post_transforms_of_short_rows(order, eps, cols):
+    """Rows of at most 64 values (one K chunk, 8, 16 or 32 lanes per row): orders 2
+    to 4, ranks from a few to n^3, counts that leave a part of the last 128 rows."""
+    rng = np.random.default_rng(order)
+    p = rng.uniform(-0.5, 0.5, (3000, 3))
+    w = rng.standard_normal(3000 * cols)
+    t = make_tree("GaussSigma", 0.25, 1.0, 3, order, eps, 1)
+    t.buildFMMTree()
+    out = []
+    for prec in (fmm.PREC_FP64, fmm.PREC_MIXED):
+        t.set_precision(prec)
+        out.append(np.zeros(3000 * cols))
+        fmm.H2_3D_Compute(t, p, p, w, cols, out[-1])
+    assert rel(out[1], out[0]) < 2e-6
+    t.close()
