@@ -54,7 +54,10 @@ void set_error(const std::string& msg) { g_err = msg; }
 
 int cuda_status(cudaError_t e, const char* what) {
   g_err = std::string(what) + ": " + cudaGetErrorString(e);
-  if (e == cudaErrorMemoryAllocation) return PBBFMM_ERR_ALLOC;
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // (a later launch check would report it again)
+    return PBBFMM_ERR_ALLOC;
+  }
   return PBBFMM_ERR_CUDA;
 }
 
@@ -1118,8 +1121,11 @@ int pbbfmm_compute_adjoint_device(pbbfmm_tree* t, const double* d_target, int64_
     // targets sources carrying g, the box stays the forward targets' one.
     PassGuard guard{t};
     if (t->p.use_chebyshev) {
-      if (!t->adj_ready)
-        if (int rc = build_adjoint_ops(t)) return rc;
+      if (!t->adj_ready) {
+        int rc = build_adjoint_ops(t);
+        if (rc == PBBFMM_ERR_ALLOC && release_combined(t)) rc = build_adjoint_ops(t);
+        if (rc) return rc;
+      }
       swap_adjoint_ops(t);
       guard.swapped = true;
     }

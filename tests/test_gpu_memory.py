@@ -174,3 +174,52 @@ def test_groups_of_combinations(share, cols, precision):
         got.append(o.cpu().numpy())
     assert rel(got[0], got[1]) < tol
     t.close()
+
+
+def test_adjoint_operators_take_the_place_of_combinations():
+    """The transposed operators (0.12 GB at order 6) are made at the first adjoint
+    call.  Where the combinations of earlier calls hold the memory that they need,
+    these give it back; without any, the call is refused and the next one is right."""
+    import torch
+
+    cols, n = 8, 20000
+    p, w = points(n, 1), weights(cols, n, 2)
+
+    def adjoint(t):
+        o = torch.zeros(cols, n, dtype=torch.float64, device="cuda")
+        fmm.compute_adjoint_device(t, p, p, w, w, cols, grad_weight=o)
+        return o.cpu().numpy()
+
+    def tree():
+        t = make_tree("Laplacian", 0.0, 1.0, 4, 6, 1e-7, 1)
+        t.buildFMMTree()
+        return t
+
+    t = tree()
+    ref = adjoint(t)
+    t.close()
+    t = tree()
+    run(t, p, w, fmm.PREC_FP64)
+    held = combined_bytes(t)
+    assert held > 200 * MB
+    spare = torch.empty(cols * n, dtype=torch.float64, device="cuda")  # the gradient's memory
+    full = fill_but(40 * MB)
+    del spare
+    assert rel(adjoint(t), ref) < 1e-13
+    assert combined_bytes(t) < held
+    del full
+    t.close()
+    torch.cuda.empty_cache()
+    t = tree()
+    combined_bytes(t, 0)
+    run(t, p, w, fmm.PREC_FP64)
+    spare = torch.empty(cols * n, dtype=torch.float64, device="cuda")
+    full = fill_but(40 * MB)
+    del spare
+    with pytest.raises(fmm.FMMError) as e:
+        adjoint(t)
+    assert e.value.code == _lib.ERR_ALLOC
+    del full
+    torch.cuda.empty_cache()
+    assert rel(adjoint(t), ref) < 1e-13
+    t.close()
