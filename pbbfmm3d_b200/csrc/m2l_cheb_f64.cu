@@ -22,7 +22,7 @@
 // operands lie in shared memory in the order of the instruction's fragments
 // (lane-contiguous 256-byte reads, no bank conflicts); the operators are
 // stored that way in global memory, so a K chunk is one contiguous copy.  A
-// tile of 64 rows leaves the running sum at 64 KB or less and two CTAs per SM:
+// tile of 64 rows leaves the running sum at 68 KB or less and two CTAs per SM:
 // one CTA's barriers, adds and copies hide behind the other's products.
 //
 // Measured, M2L of one matvec (B200), against one FMA kernel per level with
@@ -98,6 +98,13 @@ __host__ __device__ constexpr size_t fd_smem(int ntb, int kc, int nst) {
   return sizeof(double) *
          ((size_t)FD_R * fd_pitch(ntb) + (size_t)nst * kc * (FD_R + 8 * ntb));
 }
+
+// two CTAs of the widest plans fit an SM's 228 KB (the row lists and masks take less
+// than 5 KB, the system 1 KB per CTA)
+static_assert(2 * (fd_smem(16, 8, 3) + 6 * 1024) <= 228 * 1024 &&
+                  2 * (fd_smem(15, 16, 2) + 6 * 1024) <= 228 * 1024 &&
+                  2 * (fd_smem(8, 16, 3) + 6 * 1024) <= 228 * 1024,
+              "two CTAs per SM");
 
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() {

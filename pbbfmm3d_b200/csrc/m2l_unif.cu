@@ -198,15 +198,16 @@ int unif_slot_freq(int n, int slot) {
 //            transform of the n lines l2 and the y transform of the results;
 //            thread (j): the x transform of (k2, k3), straight to global memory;
 //   inverse: thread (j): the x transform, straight from global memory; thread
-//            (a1): for each k3 the y transform, added into the n^2 outputs of
-//            its row by the z transform; the outputs leave through shared
-//            memory in coalesced rows.
+//            (a1), of the largest orders several (qparts): for each k3 the y
+//            transform, added into the n^2 outputs of its row by the z
+//            transform; the outputs leave through shared memory in coalesced
+//            rows.
 // Spectra between the stages: the jobs (k2, k3) that are kept, n nj elements per
 // unit.  Bound: HBM and the latency of the stages (shared memory admits two to
 // four CTAs per SM).  Measured, 1M points at order 5, forward + inverse, against one
 // cell per CTA with a column per lane: 1 column, float32 2.57 + 1.56 -> 0.38 +
 // 0.34 ms (its stores covered 8 bytes of each frequency plane); 8 columns,
-// float64 3.77 + 5.38 -> 2.75 + 3.30 ms, float32 with the split 3.32 + 3.10 -> 2.57 +
+// float64 4.43 + 5.26 -> 2.75 + 3.31 ms, float32 with the split 3.32 + 3.10 -> 2.57 +
 // 2.19 ms, and with four CTAs per SM instead of three (the conjugate elements not
 // stored, the forward's moments under its spectra) 2.27 + 1.99 ms.
 template <int n, typename T>
