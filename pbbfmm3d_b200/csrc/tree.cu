@@ -208,6 +208,11 @@ __device__ __forceinline__ unsigned list_children(const ListArgs& a, const ListJ
   return m;
 }
 
+// LIST_TYPED: end of block b's parents
+__device__ __forceinline__ int64_t list_end(const ListJob& j, int b) {
+  return min((int64_t)j.ncells, (int64_t)(b + 1) * j.pieces * kListBlock);
+}
+
 // block-wide exclusive prefix of (x, y); *tx, *ty the totals
 __device__ __forceinline__ void block_scan2(int x, int y, int* ex, int* ey, int* tx, int* ty) {
   __shared__ int sx[kListThreads / 32], sy[kListThreads / 32];
@@ -239,9 +244,9 @@ __global__ void __launch_bounds__(kListThreads) k_list_count(const __grid_consta
     if (tid < 8) s_n[tid] = 0;
     __syncthreads();
     int n[8] = {};
-    for (int i = 0; i < kListItems * j.pieces; ++i) {
-      const unsigned m =
-          list_children(a, j, (int64_t)b * j.pieces * kListBlock + i * kListThreads + tid);
+    for (int64_t p0 = (int64_t)b * j.pieces * kListBlock, e = list_end(j, b); p0 < e;
+         p0 += kListThreads) {
+      const unsigned m = list_children(a, j, p0 + tid);
 #pragma unroll
       for (int t = 0; t < 8; ++t) n[t] += __popc(__ballot_sync(0xffffffffu, (m >> t) & 1u));
     }
@@ -266,39 +271,48 @@ __global__ void __launch_bounds__(kListThreads) k_list_count(const __grid_consta
   if (tid == 0) a.bcount[j.count0 + b] = tx, a.bchunk[j.count0 + b] = ty;
 }
 
-// one block per list: exclusive scan of its counts, in place, kScanItems of them per
-// thread and step
+// exclusive scan of a job's counts from k0 on, in place, N per thread; n, nc: the sums
+// of those before
+template <int N>
+__device__ __forceinline__ void scan_counts(const ListArgs& a, const ListJob& j, int k0, int* n,
+                                            int* nc) {
+  const bool dense = j.kind == LIST_DENSE;
+  const int first = k0 + threadIdx.x * N;
+  int x[N], y[N], sx = 0, sy = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const bool ok = first + i < j.ncounts;
+    x[i] = ok ? a.bcount[j.count0 + first + i] : 0;
+    y[i] = ok && dense ? a.bchunk[j.count0 + first + i] : 0;
+    sx += x[i], sy += y[i];
+  }
+  int ex, ey, tx, ty;
+  block_scan2(sx, sy, &ex, &ey, &tx, &ty);
+  ex += *n, ey += *nc;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    if (first + i < j.ncounts) {
+      a.bcount[j.count0 + first + i] = ex;
+      if (dense) a.bchunk[j.count0 + first + i] = ey;
+    }
+    ex += x[i], ey += y[i];
+  }
+  *n += tx;
+  *nc += ty;
+}
+
+// one block per list; several counts per thread and step where there are many
 __global__ void __launch_bounds__(kListThreads) k_list_scan(const __grid_constant__ ListArgs a) {
   const ListJob& j = a.job[blockIdx.x];
-  const bool dense = j.kind == LIST_DENSE;
   int n = 0, nc = 0;
-  for (int k0 = 0; k0 < j.ncounts; k0 += kListThreads * kScanItems) {
-    const int first = k0 + threadIdx.x * kScanItems;
-    int x[kScanItems], y[kScanItems], sx = 0, sy = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-      const bool ok = first + i < j.ncounts;
-      x[i] = ok ? a.bcount[j.count0 + first + i] : 0;
-      y[i] = ok && dense ? a.bchunk[j.count0 + first + i] : 0;
-      sx += x[i], sy += y[i];
-    }
-    int ex, ey, tx, ty;
-    block_scan2(sx, sy, &ex, &ey, &tx, &ty);
-    ex += n, ey += nc;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-      if (first + i < j.ncounts) {
-        a.bcount[j.count0 + first + i] = ex;
-        if (dense) a.bchunk[j.count0 + first + i] = ey;
-      }
-      ex += x[i], ey += y[i];
-    }
-    n += tx;
-    nc += ty;
-  }
+  if (j.ncounts <= kListThreads)
+    scan_counts<1>(a, j, 0, &n, &nc);
+  else
+    for (int k0 = 0; k0 < j.ncounts; k0 += kListThreads * kScanItems)
+      scan_counts<kScanItems>(a, j, k0, &n, &nc);
   if (threadIdx.x == 0) {
     *j.count = n;
-    if (dense) a.prefix[n] = nc;
+    if (j.kind == LIST_DENSE) a.prefix[n] = nc;
     if (j.slot >= 0) a.hcount[j.slot] = n;
     if (j.kind == LIST_TYPED) a.hcount[j.slot + 9] = n;
   }
@@ -316,8 +330,10 @@ __global__ void __launch_bounds__(kListThreads) k_list_write(const __grid_consta
 #pragma unroll
     for (int t = 0; t < 8; ++t) at[t] = a.bcount[j.count0 + t * nb + b];
     if (b == 0 && tid < 8) a.hcount[j.slot + 1 + tid] = a.bcount[j.count0 + tid * nb];
-    for (int i = 0; i < kListItems * j.pieces; ++i) {
-      const int64_t p = (int64_t)b * j.pieces * kListBlock + i * kListThreads + tid;
+    int i = 0;
+    for (int64_t p0 = (int64_t)b * j.pieces * kListBlock, e = list_end(j, b); p0 < e;
+         p0 += kListThreads, ++i) {
+      const int64_t p = p0 + tid;
       const unsigned m = list_children(a, j, p);
       unsigned v[8];
 #pragma unroll
