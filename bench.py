@@ -456,9 +456,9 @@ def per_step(kt, steps):
 
 # DRAM bytes per (cell, frequency, column) of the frequency-domain M2L, from
 # the ncu capture in profiles/k_m2l_unif_tc_expcov0.3_unif5_N262144_C8_L5.md
-# (the level-5 launch of k_m2l_unif_tc: 979.03 MB read + 725.68 MB written
+# (the level-5 launch of k_m2l_unif_tc: 978.98 MB read + 724.73 MB written
 # for 32,768 cells x 365 frequencies x 8 columns)
-MAC_DRAM_BYTES_PER_UNIT = (979.034e6 + 725.678e6) / (32768 * 365 * 8)
+MAC_DRAM_BYTES_PER_UNIT = (978.980e6 + 724.732e6) / (32768 * 365 * 8)
 # tensor-core MAC tiling (csrc/m2l_unif_tc.cu): items of 8 x 1 x 16 target
 # parents at one frequency, 10 source planes per item, 18 MMAs (M = 128,
 # K = 16) per plane with N = 32 x (target planes it serves)
